@@ -103,15 +103,129 @@ __global__ void __launch_bounds__(256) gram_partial_kernel(blk_cols X, int h, bl
     }
 }
 
-__global__ void gram_reduce_kernel(const double* __restrict__ partial, int splits, int h, int w,
-                                   double* __restrict__ G, int ldg)
+// G from the partials, in a fixed order: 32 entries per CTA; 64 splits at a time
+// are loaded by all its threads, then added in order by one thread an entry.
+// A split's value is the sum of its `chunks` partials in order (nparts in all;
+// chunks = 1: the split's own sum).  One thread an entry loading as it adds took
+// 44 us for 304 splits of 8 x 8, a chain of loads and FP64 additions; this takes 20.
+//   mode 0: entries e = j h + i of a full product
+//   mode 1: e = i (i + 1) / 2 + j, the packed lower triangle of X'X
+//   mode 2: the lower triangle of X'X at e = j h + i
+static __device__ __forceinline__ void tri_index(int e, int* i, int* j)
 {
-  int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= h * w) return;
+  int r = (int)((sqrtf(8.0f * (float)e + 1.0f) - 1.0f) * 0.5f);
+  while (r * (r + 1) / 2 > e) r--;
+  while ((r + 1) * (r + 2) / 2 <= e) r++;
+  *i = r;
+  *j = e - r * (r + 1) / 2;
+}
+
+__global__ void __launch_bounds__(256) gram_reduce_kernel(const double* __restrict__ partial, int splits, int chunks,
+                                                          long nparts, int E, int h, int mode,
+                                                          double* __restrict__ G, int ldg)
+{
+  __shared__ double sm[64][33];
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+  const int e0 = blockIdx.x * 32 + x;
+  const int e = min(e0, E - 1);
   double s = 0.0;
-  for (int p = 0; p < splits; p++) s += partial[(size_t)p * h * w + e];
-  int i = e % h, j = e / h;
+  for (int base = 0; base < splits; base += 64) {
+    const int cnt = min(64, splits - base);
+    if (chunks == 1) {
+#pragma unroll 8
+      for (int q = y; q < cnt; q += 8) sm[q][x] = partial[(size_t)(base + q) * E + e];
+    } else {
+      for (int q = y; q < cnt; q += 8) {
+        const long p0 = (long)(base + q) * chunks, p1 = min(p0 + chunks, nparts);
+        double v = 0.0;
+#pragma unroll 4
+        for (long c = p0; c < p1; c++) v += partial[(size_t)c * E + e];
+        sm[q][x] = v;
+      }
+    }
+    __syncthreads();
+    if (y == 0) {
+#pragma unroll 8
+      for (int q = 0; q < cnt; q++) s += sm[q][x];
+    }
+    __syncthreads();
+  }
+  if (y || e0 >= E) return;
+  int i, j;
+  if (mode == 1) {
+    tri_index(e, &i, &j);
+  } else {
+    i = e % h;
+    j = e / h;
+    if (mode == 2 && i < j) return;
+  }
   G[(size_t)j * ldg + i] = s;
+  if (mode) G[(size_t)i * ldg + j] = s;
+}
+
+// FP64 Gram of narrow blocks: E <= 512 entries -- h w, or for X'X the h (h + 1) / 2
+// of the lower triangle -- one to a thread, packed onto whole warps, since a
+// warp-wide FP64 instruction occupies the pipe 16 cycles whatever its lane
+// count: ceil(E / 32) of them per row, where a padded 32 x 32 tile spends 32.
+// The threads left over form groups that take different 32-row chunks, each
+// chunk's sum (32 FMAs in row order) being added to its entry's in chunk order
+// afterwards.  With few splits the CTAs of a split (`sub` of them) leave that
+// to the reduction, so that every SM has work.  Splits, chunks and the order of
+// all sums are those of gram_partial_kernel: the results are its bits.  (Above
+// 512 entries a thread's register tile wins: 32 x 32 65,536 rows 135 us against
+// 160 with two packed entries a thread.)
+//   8,000 x 10 x 10: 16 us with the reduction against 96 (padded tile, 28 CTAs);
+//   262,144 x 8 x 8: 60 us against 504.
+#define GRAMP_T 512
+template <bool SYM>
+__global__ void __launch_bounds__(GRAMP_T) gram_packed_kernel(blk_cols X, int h, blk_cols Y, int w, long n,
+                                                              long rows_per_split, int sub, int groups,
+                                                              double* __restrict__ partial)
+{
+  extern __shared__ double sm[];  // [32 groups][h (+ w), odd stride], then [groups][E32]
+  const int E = SYM ? h * (h + 1) / 2 : h * w, E32 = (E + 31) & ~31;
+  const int nc = SYM ? h : h + w, ld = nc | 1, RS = 32 * groups;
+  double* red = sm + RS * ld;
+  const int t = threadIdx.x, g = t / E32, e = t - g * E32;
+  const long chunks = rows_per_split / 32, per = (chunks + sub - 1) / sub;  // per split, per CTA
+  const long split = blockIdx.x / sub;
+  const long c0 = (long)(blockIdx.x % sub) * per, c1 = min(c0 + per, chunks);
+  const long r_end = min(n, (split + 1) * rows_per_split);
+  int xi, yj;
+  if (SYM) {
+    tri_index(min(e, E - 1), &xi, &yj);
+  } else {
+    xi = min(e, E - 1) % h;
+    yj = h + min(e, E - 1) / h;
+  }
+  const bool live = g < groups && e < E;
+  double acc = 0.0;
+  for (long c = c0; c < c1; c += groups) {
+    const long r0 = split * rows_per_split + 32 * c;
+    if (r0 >= r_end) break;
+    for (int q = t; q < RS * nc; q += GRAMP_T) {
+      const int rr = q % RS, cc = q / RS;
+      const double* col = (const double*)(cc < h ? X.col[cc] : Y.col[cc - h]);
+      const long r = r0 + rr;
+      sm[rr * ld + cc] = r < r_end ? col[r] : 0.0;
+    }
+    __syncthreads();
+    if (live) {
+      double a = 0.0;
+      const double* row = sm + 32 * g * ld;
+#pragma unroll 8
+      for (int rr = 0; rr < 32; rr++, row += ld) a = fma(row[xi], row[yj], a);
+      if (sub > 1) {
+        if (c + g < c1 && r0 + 32 * g < r_end) partial[(size_t)(split * chunks + c + g) * E + e] = a;
+      } else {
+        red[g * E32 + e] = a;
+      }
+    }
+    __syncthreads();
+    if (sub == 1 && live && g == 0)
+      for (int k = 0; k < groups && c + k < c1 && r0 + 32 * k < r_end; k++) acc += red[k * E32 + e];
+  }
+  if (sub == 1 && live && g == 0) partial[(size_t)split * E + e] = acc;
 }
 
 // Symmetric Gram X'X (h <= 64) on the lower triangle only.  Thread t owns
@@ -195,19 +309,6 @@ __global__ void __launch_bounds__(544) gram_sym_partial_kernel(blk_cols X, int h
     }
 }
 
-// G (h x h) from the lower-triangle partials, both triangles
-__global__ void gram_sym_reduce_kernel(const double* __restrict__ partial, int splits, int h,
-                                       double* __restrict__ G, int ldg)
-{
-  int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= h * h) return;
-  int i = e % h, j = e / h;
-  const int src = i >= j ? e : j + i * h;
-  double s = 0.0;
-  for (int p = 0; p < splits; p++) s += partial[(size_t)p * h * h + src];
-  G[(size_t)j * ldg + i] = s;
-}
-
 // the row splits of gram_launch for a single (gx = gy = 1) output tile
 static long gram_splits(gpu_Context* ctx, long n, long* rows)
 {
@@ -236,7 +337,7 @@ static int gram_sym_launch(gpu_Context* ctx, long n, const blk_cols* X, int h, d
   gb_prof_rec pr;
   gb_prof_begin(ctx, &pr, sizeof(T) == 8 ? GB_K_GRAM : GB_K_GRAM32);
   gram_sym_partial_kernel<T, BS><<<grid, threads, 0, S(ctx)>>>(*X, h, n, rows, partial);
-  gram_sym_reduce_kernel<<<(h * h + 255) / 256, 256, 0, S(ctx)>>>(partial, (int)splits, h, G, ldg);
+  gram_reduce_kernel<<<(h * h + 31) / 32, 256, 0, S(ctx)>>>(partial, (int)splits, 1, splits, h * h, h, 2, G, ldg);
   gb_prof_end(ctx, &pr, (double)sizeof(T) * n * h, (double)n * h * (h + 1));
   gb_count_launch(2);
   return CUDA_LAUNCH_CHECK(ctx, "gram_sym");
@@ -265,10 +366,42 @@ static int gram_launch(gpu_Context* ctx, long n, const blk_cols* X, int h, const
   gb_prof_begin(ctx, &pr, sizeof(T) == 8 ? GB_K_GRAM : GB_K_GRAM32);
   gram_partial_kernel<T, TM, TN><<<grid, 256, 0, S(ctx)>>>(*X, h, *Y, w, n, rows, partial);
   int tot = h * w;
-  gram_reduce_kernel<<<(tot + 255) / 256, 256, 0, S(ctx)>>>(partial, (int)splits, h, w, G, ldg);
+  gram_reduce_kernel<<<(tot + 31) / 32, 256, 0, S(ctx)>>>(partial, (int)splits, 1, splits, tot, h, 0, G, ldg);
   gb_prof_end(ctx, &pr, (double)sizeof(T) * n * (h + w), 2.0 * n * h * w);
   gb_count_launch(2);
   return CUDA_LAUNCH_CHECK(ctx, "gram");
+}
+
+template <bool SYM>
+static int gram_packed(gpu_Context* ctx, long n, const blk_cols* X, int h, const blk_cols* Y, int w, double* G, int ldg)
+{
+  long rows;
+  const long splits = gram_splits(ctx, n, &rows), chunks = rows / 32;
+  const int E = SYM ? h * (h + 1) / 2 : h * w, E32 = (E + 31) & ~31, nc = SYM ? h : h + w;
+  int groups = GRAMP_T / E32;
+  if (groups > chunks) groups = (int)chunks;
+  while (groups > 1 && 32 * groups * (nc | 1) * 8 > 64 * 1024) groups /= 2;
+  // few splits: several CTAs a split, each leaving its chunks' sums
+  int sub = 1;
+  if (splits <= ctx->num_sms) {
+    const long most = (chunks + groups - 1) / groups, want = 4L * ctx->num_sms / splits;
+    sub = (int)(want < most ? want : most);
+  }
+  const long nparts = sub > 1 ? (n + 31) / 32 : splits;
+  double* partial = (double*)gb_workspace(ctx, sizeof(double) * (size_t)nparts * E);
+  if (!partial) return -1;
+  const int smem = 8 * (32 * groups * (nc | 1) + groups * E32);
+  if (cudaFuncSetAttribute(gram_packed_kernel<SYM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+    return gb_fail(ctx, "gram: cannot reserve %d bytes of shared memory", smem);
+  gb_prof_rec pr;
+  gb_prof_begin(ctx, &pr, GB_K_GRAM);
+  gram_packed_kernel<SYM><<<(unsigned)(splits * sub), GRAMP_T, smem, S(ctx)>>>(*X, h, *Y, w, n, rows, sub, groups,
+                                                                               partial);
+  gram_reduce_kernel<<<(E + 31) / 32, 256, 0, S(ctx)>>>(partial, (int)splits, sub > 1 ? (int)chunks : 1, nparts, E, h,
+                                                        SYM ? 1 : 0, G, ldg);
+  gb_prof_end(ctx, &pr, 8.0 * n * nc, SYM ? (double)n * h * (h + 1) : 2.0 * n * h * w);
+  gb_count_launch(2);
+  return CUDA_LAUNCH_CHECK(ctx, "gram_packed");
 }
 
 extern "C" int gb_gram(gpu_Context* ctx, int dtype, long n, const blk_cols* X, int h,
@@ -276,17 +409,19 @@ extern "C" int gb_gram(gpu_Context* ctx, int dtype, long n, const blk_cols* X, i
 {
   if (h <= 0 || w <= 0) return 0;
   // X'X with h <= 64 (one output tile): the lower triangle only
-  if (h == w && h <= 64 && memcmp(X->col, Y->col, sizeof(void*) * (size_t)h) == 0) {
-    if (dtype == GPU_MV_FLOAT64)
+  const int sym = h == w && h <= 64 && memcmp(X->col, Y->col, sizeof(void*) * (size_t)h) == 0;
+  if (dtype == GPU_MV_FLOAT64) {
+    if (sym && h * (h + 1) / 2 <= GRAMP_T) return gram_packed<true>(ctx, n, X, h, Y, w, G, ldg);
+    if (!sym && h * w <= GRAMP_T && h <= 64 && w <= 64) return gram_packed<false>(ctx, n, X, h, Y, w, G, ldg);
+    if (sym)
       return h <= 32 ? gram_sym_launch<double, 1>(ctx, n, X, h, G, ldg)
                      : gram_sym_launch<double, 2>(ctx, n, X, h, G, ldg);
-    return h <= 32 ? gram_sym_launch<float, 1>(ctx, n, X, h, G, ldg)
-                   : gram_sym_launch<float, 2>(ctx, n, X, h, G, ldg);
-  }
-  if (dtype == GPU_MV_FLOAT64) {
     if (h <= 32 && w <= 32) return gram_launch<double, 2, 2>(ctx, n, X, h, Y, w, G, ldg);
     return gram_launch<double, 4, 4>(ctx, n, X, h, Y, w, G, ldg);
   }
+  if (sym)
+    return h <= 32 ? gram_sym_launch<float, 1>(ctx, n, X, h, G, ldg)
+                   : gram_sym_launch<float, 2>(ctx, n, X, h, G, ldg);
   if (h <= 32 && w <= 32) return gram_launch<float, 2, 2>(ctx, n, X, h, Y, w, G, ldg);
   return gram_launch<float, 4, 4>(ctx, n, X, h, Y, w, G, ldg);
 }
@@ -317,11 +452,12 @@ __global__ void __launch_bounds__(256) bymat_kernel(blk_cols X, int h, const dou
 
   const int kmax = tri ? min(h, j0 + BN) : h;
   for (int k0 = 0; k0 < kmax; k0 += KC) {
-    for (int e = t; e < KC * BM; e += 256) {
+    const int kc = min(KC, h - k0);  // (narrow blocks: no work on padding)
+    for (int e = t; e < kc * BM; e += 256) {
       int rr = e % BM, kk = e / BM;
       long r = r0 + rr;
       T v = T(0);
-      if (r < n && k0 + kk < h) v = ((const T*)X.col[k0 + kk])[r];
+      if (r < n) v = ((const T*)X.col[k0 + kk])[r];
       xs[kk][rr] = v;
     }
     for (int e = t; e < KC * BN; e += 256) {
@@ -331,12 +467,14 @@ __global__ void __launch_bounds__(256) bymat_kernel(blk_cols X, int h, const dou
       cs[kk][jj] = v;
     }
     __syncthreads();
-    const int kk_end = tri ? max(0, min(KC, j0 + cg * 8 + 8 - k0)) : KC;
+    const int nb = min(8, w - j0 - cg * 8);  // this warp's columns
+    const int kk_end = nb <= 0 ? 0 : (tri ? max(0, min(kc, j0 + cg * 8 + 8 - k0)) : kc);
 #pragma unroll 8
     for (int kk = 0; kk < kk_end; kk++) {
       T xv = xs[kk][rl];
 #pragma unroll
-      for (int b = 0; b < 8; b++) acc[b] = fma(xv, cs[kk][cg * 8 + b], acc[b]);
+      for (int b = 0; b < 8; b++)
+        if (b < nb) acc[b] = fma(xv, cs[kk][cg * 8 + b], acc[b]);
     }
     __syncthreads();
   }
@@ -886,7 +1024,7 @@ static int gram_noalloc_launch(long n, const blk_cols* X, int h, const blk_cols*
   // reduction reads it, so stale contents from an earlier call never leak
   gram_partial_kernel<T, TM, TN><<<grid, 256, 0, stream>>>(*X, h, *Y, w, n, rows, partial);
   if (cudaGetLastError() != cudaSuccess) return -3;
-  gram_reduce_kernel<<<(h * w + 255) / 256, 256, 0, stream>>>(partial, (int)splits, h, w, G, ldg);
+  gram_reduce_kernel<<<(h * w + 31) / 32, 256, 0, stream>>>(partial, (int)splits, 1, splits, h * w, h, 0, G, ldg);
   gb_count_launch(2);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
