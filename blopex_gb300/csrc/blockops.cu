@@ -521,6 +521,27 @@ extern "C" int gb_bymat(gpu_Context* ctx, int dtype, long n, const blk_cols* X, 
   return bymat_launch(ctx, dtype, n, X, h, C, ldc, Y, w, Z, 0);
 }
 
+// Callers' updates (the interpreter's entries, the adjoint): FP64 ones of at
+// least XC_TENSOR_MIN multiply-adds on the tensor cores (oz_xc64.cu), with a
+// smaller error: 2,097,152 x 32 x 32 0.43 ms against 3.5; 262,144 x 8 x 8 42 us
+// against 53; a launch costs it 20 us at least.  The solver keeps gb_bymat:
+// the signs of its Ritz vectors follow the last bits of these sums,
+// and a solve returns the same iterates, bit for bit, as it always did.
+#define XC_TENSOR_MIN 1.6e7
+
+extern "C" int gb_bymat_large(gpu_Context* ctx, int dtype, long n, const blk_cols* X, int h,
+                              const double* C, int ldc, const blk_cols* Y, int w, const blk_cols* Z)
+{
+  if (w <= 0 || n <= 0) return 0;
+  if (dtype != GPU_MV_FLOAT64 || h <= 0 || (double)n * h * w < XC_TENSOR_MIN)
+    return gb_bymat(ctx, dtype, n, X, h, C, ldc, Y, w, Z);
+  gb_prof_rec pr;
+  gb_prof_begin(ctx, &pr, GB_K_XC);
+  const int rc = gb_oz_bymat64(ctx, n, X, h, C, ldc, Y, w, Z);
+  gb_prof_end(ctx, &pr, 8.0 * n * (h + w + (Z ? w : 0)), 2.0 * n * h * w);
+  return rc;
+}
+
 extern "C" int gb_bymat_tri(gpu_Context* ctx, int dtype, long n, const blk_cols* X, int h,
                             const double* C, int ldc, const blk_cols* Y, int w)
 {

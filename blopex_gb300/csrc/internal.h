@@ -121,6 +121,9 @@ int gb_gram(gpu_Context* ctx, int dtype, long n, const blk_cols* X, int h, const
 /* Y(:,j) = sum_i X(:,i) C(i,j) [+ Z(:,j)], C FP64 device column-major (ldc) */
 int gb_bymat(gpu_Context* ctx, int dtype, long n, const blk_cols* X, int h, const double* C,
              int ldc, const blk_cols* Y, int w, const blk_cols* Z);
+/* the same for callers outside the solver: large FP64 products on the tensor cores */
+int gb_bymat_large(gpu_Context* ctx, int dtype, long n, const blk_cols* X, int h, const double* C,
+                   int ldc, const blk_cols* Y, int w, const blk_cols* Z);
 /* the same with C upper triangular (explicit zeros below the diagonal) */
 int gb_bymat_tri(gpu_Context* ctx, int dtype, long n, const blk_cols* X, int h, const double* C,
                  int ldc, const blk_cols* Y, int w);
@@ -192,6 +195,13 @@ int gb_tc_xc(gpu_Context* ctx, long n, const blk_cols* X, int h, const double* C
    or FP64 (z_dtype); Y32 optional FP32 copy of Y */
 int gb_oz_xc(gpu_Context* ctx, long n, const blk_cols* X, int h, const double* C, int ldc,
              const blk_cols* Y, int w, const blk_cols* Z, int z_dtype, const blk_cols* Y32);
+/* the same product with the accuracy of FP64 arithmetic (oz_xc64.cu) */
+int gb_oz_xc64(gpu_Context* ctx, long n, const blk_cols* X, int h, const double* C, int ldc,
+               const blk_cols* Y, int w, const blk_cols* Z, int z_dtype, const blk_cols* Y32);
+/* and for FP64 blocks of any widths and alignments; Z FP64, may be Y.  X must
+   not overlap Y when h or w > 64 */
+int gb_oz_bymat64(gpu_Context* ctx, long n, const blk_cols* X, int h, const double* C, int ldc,
+                  const blk_cols* Y, int w, const blk_cols* Z);
 /* FP64-accurate Gram G = L' [L Q_0 Q_1 ...] on the tensor cores (oz_gram.cu):
    L a block of h <= 64 columns, FP32 or FP64 (ldt); nq <= 4 blocks Q_b of up
    to 64 columns each, FP32 or FP64 (qdt[b]); every column 16-byte aligned and

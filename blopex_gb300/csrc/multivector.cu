@@ -360,7 +360,7 @@ static void vecmat(void* x_, BlopexInt gh, BlopexInt h, BlopexInt w, void* v, vo
   blk_cols a, b;
   gb_mv_fill_cols(x, &a, 0);
   gb_mv_fill_cols(y, &b, 0);
-  gb_bymat(ctx, x->dtype, x->size, &a, h, c, h, &b, w, add ? &b : NULL);
+  gb_bymat_large(ctx, x->dtype, x->size, &a, h, c, h, &b, w, add ? &b : NULL);
   gb_sync(ctx);
   gb_device_free(c);
 }

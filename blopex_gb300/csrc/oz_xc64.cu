@@ -1,0 +1,566 @@
+// oz_xc64.cu -- block update Y = X C (+ Z) with the accuracy of FP64 arithmetic on
+// the tensor cores, by error-free splitting (oz8_common.cuh): X an FP64 block of
+// n rows and h <= 64 columns, C the FP64 h x w coordinate block (w <= 64) on the
+// device, Z an optional FP32 or FP64 block, Y FP64 (and optionally its FP32
+// shadow Y32).  It is serial_Multi_VectorByMatrix (blopex_serial_double/
+// multivector/multi_vector.c:474-524), for callers' large FP64 blocks
+// (gb_bymat_large) and gpu_BlockUpdate's mode 2.
+//
+// Scales: each row of X (its h values) and each column of C share one power of
+// two; both are cut into 7 8-bit digits (55 fraction bits).  Level L = t + u of
+// the digit products is accumulated exactly in FP32 in TMEM (at most 7 products
+// of 2^14 over 64 columns: below 2^23); the epilogue recombines the eight levels
+// into one 64-bit integer, rounds it to FP64 with integer operations and adds Z.
+// |Y - (X C + Z)| is below that of a sum of h fused multiply-adds (6e-17
+// against 2.0e-16 relative on random blocks, h = 32).
+//
+// Rows or columns whose scale the digits cannot carry (infinities, NaN, values
+// below 2^-960) are summed directly with FP64 FMAs by the epilogue, entry by
+// entry.
+//
+// What bounds it: instruction issue, the half-rate integer pipe above all (~17
+// integer instructions per X value in the producers, ~30 per Y value in the
+// epilogue); FP64 FMAs instead would need h w / 2 cycles per row and SM (2 per
+// cycle), 2,048 at h = w = 64 against ~115 here.  Measured, 2,097,152 rows:
+// 32 x 32 0.43 ms (FMAs 3.5), 64 x 64 0.83 (11.7), 64 x 64 with an FP32 Z 1.11
+// (1.56 for oz_xc.cu, whose six 7-bit digits stop at 42 bits).  Hence no
+// shared-memory staging of X: its columns are read by coalesced 8-byte loads
+// straight into registers (any alignment and spacing of the columns), all 32 of
+// a thread in flight at once, while the MMAs of the previous tile run.
+//
+// Per CTA (one per SM, persistent over 128-row tiles; a tile's output columns
+// are taken 32 at a time, "units", into two alternating TMEM accumulator sets
+// so the MMAs of one unit overlap the epilogue of the previous one):
+//   warps 8-15  producers: warp p holds rows 32 (p mod 4) .. + 31 (lane = row)
+//               of 32 columns in registers, finds the rows' scales and writes
+//               the digit slices in the 128-byte-swizzled K-major layout;
+//   warp 16     allocates TMEM; one thread issues tcgen05.mma.kind::f16
+//               (M = 128, K = 16): for X slice t one MMA per K step against the
+//               C slices stacked along N, so that level t + u lands at TMEM
+//               column 32 (t + u);
+//   warps 0-7   read a unit's eight level accumulators (lane = row; warps w and
+//               w + 4 share TMEM lanes and take 16 of the unit's 32 columns
+//               each), recombine and store Y (and Y32).
+// Every wait is bounded; a timeout sets an error word and all roles finish.
+#include <cuda_runtime.h>
+#include <stdint.h>
+#include <string.h>
+
+#include "internal.h"
+#include "oz8_common.cuh"
+
+#define OZY_S OZ8_S
+#define OZY_THREADS 544
+#define OZY_NPROD 256
+#define OZY_ASLICE 16384          // 128 rows x 128 bytes
+#define OZY_BSLICE 4096           // 32 rows x 128 bytes (one unit's columns of one slice)
+#define OZY_UNIT 32               // output columns per unit
+#define OZY_SET (8 * OZY_UNIT)    // TMEM columns of one accumulator set
+#define OZY_C_BYTES (2 * OZY_S * OZY_BSLICE)  // [unit half][slice][32 rows][128 B]
+#define OZY_A_BYTES (OZY_S * OZY_ASLICE)
+#define OZY_SMEM (OZY_C_BYTES + OZY_A_BYTES + 1024)
+
+struct ozy_params {
+  const void *x[64], *z[64];
+  void *y[64], *y32[64];
+  const double* C;
+  int ldc, h, w, z_kind;  // z_kind: 0 none, 1 FP32, 2 FP64
+  int has_y32;
+  long n;
+  long polls;  // limit of one pipeline wait
+  int* err;
+};
+
+// global loads and stores through pointers kept in shared memory (the compiler
+// would take them for generic addresses, which cost several times as much)
+static __device__ __forceinline__ double ozy_ld(const void* p, long i)
+{
+  double v;
+  asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(__cvta_generic_to_global((const double*)p + i)));
+  return v;
+}
+static __device__ __forceinline__ uint32_t ozy_ld32(const void* p, long i)
+{
+  uint32_t v;
+  asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(__cvta_generic_to_global((const uint32_t*)p + i)));
+  return v;
+}
+static __device__ __forceinline__ void ozy_st(void* p, long i, double v)
+{
+  asm volatile("st.global.f64 [%0], %1;" ::"l"(__cvta_generic_to_global((double*)p + i)), "d"(v) : "memory");
+}
+static __device__ __forceinline__ void ozy_st32(void* p, long i, float v)
+{
+  asm volatile("st.global.f32 [%0], %1;" ::"l"(__cvta_generic_to_global((float*)p + i)), "f"(v) : "memory");
+}
+
+// the Z values of one row in columns j0 .. j0 + 3 (bit patterns; 0 outside)
+static __device__ __forceinline__ void ozy_load_z(int z_kind, const void* const* s_z, int j0, int w, long row,
+                                                  long n, unsigned long long (&zb)[4])
+{
+#pragma unroll
+  for (int jj = 0; jj < 4; jj++) {
+    const int j = j0 + jj;
+    zb[jj] = 0;
+    if (row < n && j < w) {
+      if (z_kind == 1)
+        zb[jj] = ozy_ld32(s_z[j], row);
+      else if (z_kind == 2)
+        zb[jj] = (unsigned long long)__double_as_longlong(ozy_ld(s_z[j], row));
+    }
+  }
+}
+
+// the eight levels of four output columns of this warp's rows (not waited for)
+static __device__ __forceinline__ void ozy_tmem_ld(uint32_t taddr, uint32_t (&v)[8][4])
+{
+#pragma unroll
+  for (int L = 0; L < 8; L++)
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(v[L][0]), "=r"(v[L][1]), "=r"(v[L][2]), "=r"(v[L][3])
+                 : "r"(taddr + (uint32_t)(L * OZY_UNIT)));
+}
+
+// one entry of X C by FP64 FMAs, in column order
+static __device__ __noinline__ double ozy_direct(const void* const* s_x, const double* C, int ldc, int h, int j,
+                                                 long row)
+{
+  double acc = 0.0;
+  for (int i = 0; i < h; i++) acc = fma(((const double*)s_x[i])[row], C[i + (size_t)j * ldc], acc);
+  return acc;
+}
+
+// a group's largest exponent, raised to 1 (unsafe) when it holds nothing but
+// subnormals
+static __device__ __forceinline__ int ozy_group_exp(uint32_t mag, bool nonzero)
+{
+  const int e = (int)(mag >> 20);
+  return e == 0 && nonzero ? 1 : e;
+}
+
+__global__ void __launch_bounds__(OZY_THREADS, 1) oz_xc64_kernel(const __grid_constant__ ozy_params prm)
+{
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char* smem = smem_align1024(smem_raw);
+  unsigned char* cdig = smem;                // [half][S][32 rows][128 B]
+  unsigned char* adig = smem + OZY_C_BYTES;  // [S][128 rows][128 B]
+  __shared__ uint64_t a_full[4], a_empty[4], acc_full[2], acc_empty[2], done_bar;
+  __shared__ uint32_t tmem_base;
+  __shared__ int abort_flag;
+  __shared__ int colexp[64];
+  __shared__ int any_odd;  // a column of C has a scale out of the ordinary
+  __shared__ uint32_t colpart[8][64];      // per (8-row group of C, column) largest magnitude word
+  __shared__ unsigned char colnz[8][64];   // and whether any value is not zero
+  __shared__ int rowexp[4][128];           // by tile modulo 4 (read by the epilogue)
+  __shared__ int rowpart[2][2][128];       // by tile modulo 2: per (column half, row) exponent
+  // column pointers: shared memory serves a runtime index in a few cycles,
+  // where the kernel-parameter table behind it does not
+  __shared__ const void* s_x[64];
+  __shared__ void* s_y[64];
+  __shared__ const void* s_z[64];
+  __shared__ void* s_y32[64];
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int h = prm.h, w = prm.w;
+  const int ksteps = (h + 15) >> 4;
+  const int nh = (w + OZY_UNIT - 1) / OZY_UNIT;  // units per tile
+  const long ntiles = (prm.n + 127) / 128;
+  const long my_tiles = (long)blockIdx.x < ntiles ? (ntiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
+
+  if (tid == 0) {
+    abort_flag = 0;
+    any_odd = 0;
+    for (int k = 0; k < 4; k++) {
+      mbar_init(&a_full[k], OZY_NPROD);
+      mbar_init(&a_empty[k], 1);
+    }
+    for (int b = 0; b < 2; b++) {
+      mbar_init(&acc_full[b], 1);
+      mbar_init(&acc_empty[b], 256);
+    }
+    mbar_init(&done_bar, 1);
+  }
+  if (tid < 64) {
+    s_x[tid] = tid < h ? prm.x[tid] : nullptr;
+    s_y[tid] = tid < w ? prm.y[tid] : nullptr;
+    s_z[tid] = (tid < w && prm.z_kind) ? prm.z[tid] : nullptr;
+    s_y32[tid] = (tid < w && prm.has_y32) ? prm.y32[tid] : nullptr;
+  }
+  // C: one scale per column, digits as the B operand (row j = output column,
+  // K = input column); rows j >= w and columns i >= h are zero
+  for (int e = tid; e < 64 * 8; e += OZY_THREADS) {
+    const int j = e & 63, cg = e >> 6;
+    uint32_t mag = 0;
+    bool nz = false;
+#pragma unroll
+    for (int c = 0; c < 8; c++) {
+      const int i = cg * 8 + c;
+      const double v = (j < w && i < h) ? prm.C[i + (size_t)j * prm.ldc] : 0.0;
+      mag = max(mag, (uint32_t)__double2hiint(v) & 0x7FFFFFFFu);
+      nz |= v != 0.0;
+    }
+    colpart[cg][j] = mag;
+    colnz[cg][j] = nz;
+  }
+  if (warp == 16) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     smem_u32(&tmem_base)),
+                 "r"(512u)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  __syncthreads();
+  for (int e = tid; e < 64 * 8; e += OZY_THREADS) {  // (column j, 8-row group cg)
+    const int j = e & 63, cg = e >> 6;
+    uint32_t mag = 0;
+    bool nz = false;
+#pragma unroll
+    for (int g = 0; g < 8; g++) {
+      mag = max(mag, colpart[g][j]);
+      nz |= colnz[g][j] != 0;
+    }
+    const int E = ozy_group_exp(mag, nz);
+    if (cg == 0) colexp[j] = E;
+    if (j < w && !oz8_plain(E)) any_odd = 1;
+    uint32_t lo[8], hi[8], pk[OZY_S][4];
+#pragma unroll
+    for (int c = 0; c < 8; c++) {
+      const int i = cg * 8 + c;
+      const double v = (j < w && i < h) ? prm.C[i + (size_t)j * prm.ldc] : 0.0;
+      lo[c] = (uint32_t)__double2loint(v);
+      hi[c] = (uint32_t)__double2hiint(v);
+    }
+    oz8_digits8(lo, hi, oz8_scale(E), pk);
+    // rows of one unit half hold its 32 output columns; within a half the
+    // slices are stacked, so one MMA takes several slices as a single operand
+    const int jr = j & 31, hf = j >> 5;
+    const uint32_t off = (uint32_t)jr * 128u + ((uint32_t)(cg ^ (jr & 7)) << 4);
+#pragma unroll
+    for (int t = 0; t < OZY_S; t++)
+      *(uint4*)(cdig + (hf * OZY_S + t) * OZY_BSLICE + off) = make_uint4(pk[t][0], pk[t][1], pk[t][2], pk[t][3]);
+  }
+  fence_proxy_async();
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = tmem_base;
+
+  if (warp >= 8 && warp < 16) {
+    // ------------------------------------------------------- digit slices
+    // (every producer runs every iteration: the named barrier of a pair of
+    // warps must be reached by both; an abort only skips the work)
+    // A thread holds the 8-column groups 2k + half of its row, so that K step
+    // k (columns 16 k .. + 15) is complete, and its MMAs start, while the next
+    // steps are still being cut.
+    const int pw = warp - 8, r = 32 * (pw & 3) + lane, half = pw >> 2;
+    for (long i = 0; i < my_tiles; i++) {
+      const long row = (blockIdx.x + i * gridDim.x) * 128 + r;
+      uint32_t lo[32], hi[32];
+#pragma unroll
+      for (int c = 0; c < 32; c++) {
+        const int col = 16 * (c >> 3) + 8 * half + (c & 7);
+        double v = 0.0;
+        if (row < prm.n && col < h) v = ozy_ld(s_x[col], row);
+        lo[c] = (uint32_t)__double2loint(v);
+        hi[c] = (uint32_t)__double2hiint(v);
+      }
+      if (i + 1 < my_tiles) {
+        // the next tile's X and Z (1 KB, 8 lines, of a column) on their way
+        // into L2
+        const long r1 = (blockIdx.x + (i + 1) * gridDim.x) * 128 + 16 * (lane & 7);
+        if (r1 < prm.n) {
+          for (int q = 4 * pw + (lane >> 3); q < h; q += 32)
+            asm volatile("prefetch.global.L2 [%0];" ::"l"((const char*)s_x[q] + 8 * r1));
+          if (prm.z_kind)
+            for (int q = 4 * pw + (lane >> 3); q < w; q += 32)
+              asm volatile("prefetch.global.L2 [%0];" ::"l"((const char*)s_z[q] + (prm.z_kind == 2 ? 8 : 4) * r1));
+        }
+      }
+      uint32_t mag = 0;
+#pragma unroll
+      for (int c = 0; c < 32; c++) mag = max(mag, hi[c] & 0x7FFFFFFFu);
+      int e = (int)(mag >> 20);
+      if (e == 0) {
+        uint32_t any = 0;
+#pragma unroll
+        for (int c = 0; c < 32; c++) any |= lo[c] | (hi[c] << 1);
+        e = any != 0;
+      }
+      rowpart[i & 1][half][r] = e;
+      // the rows' other half is warp pw ^ 4's; a slot is rewritten two tiles
+      // later, after another passage through this barrier
+      named_bar(1 + (pw & 3), 64);
+      const int E = max(rowpart[i & 1][0][r], rowpart[i & 1][1][r]);
+      const uint32_t es = oz8_scale(E);
+      if (half == 0) rowexp[i & 3][r] = E;
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        if (k >= ksteps) break;
+        // the step's part of the A slices is free once the previous tile's
+        // MMAs on it have completed
+        if (i >= 1 && !abort_flag && !mbar_wait_n(&a_empty[k], (uint32_t)((i - 1) & 1), &abort_flag, prm.polls)) {
+          abort_flag = 1;
+          atomicExch(prm.err, 13);
+        }
+        if (!abort_flag) {
+          tc_fence_after();
+          uint32_t pk[OZY_S][4];
+          oz8_digits8(lo + 8 * k, hi + 8 * k, es, pk);
+          // eight consecutive lanes (rows) write eight different 16-byte
+          // bank groups
+          const uint32_t off = (uint32_t)r * 128u + ((uint32_t)((2 * k + half) ^ (r & 7)) << 4);
+#pragma unroll
+          for (int t = 0; t < OZY_S; t++)
+            *(uint4*)(adig + t * OZY_ASLICE + off) = make_uint4(pk[t][0], pk[t][1], pk[t][2], pk[t][3]);
+          fence_proxy_async();
+          mbar_arrive(&a_full[k]);
+        }
+      }
+    }
+  } else if (warp == 16) {
+    if (lane == 0) {
+      // ------------------------------------------------------- MMA issuer
+      const uint32_t abase = smem_u32(adig), cbase = smem_u32(cdig);
+      long u = 0;  // units issued
+      for (long i = 0; i < my_tiles && !abort_flag; i++) {
+        for (int hf = 0; hf < nh; hf++, u++) {
+          const int set = (int)(u & 1);
+          if (u >= 2 && !mbar_wait_n(&acc_empty[set], (uint32_t)(((u >> 1) - 1) & 1), &abort_flag, prm.polls)) {
+            abort_flag = 1;
+            atomicExch(prm.err, 15);
+            break;
+          }
+          const uint32_t d = tmem + (uint32_t)(set * OZY_SET);
+          for (int ks = 0; ks < ksteps; ks++) {
+            if (hf == 0 && !mbar_wait_n(&a_full[ks], (uint32_t)(i & 1), &abort_flag, prm.polls)) {
+              abort_flag = 1;
+              atomicExch(prm.err, 14);
+              break;
+            }
+            tc_fence_after();
+            const uint32_t ab = abase + ks * 32, cb = cbase + hf * OZY_S * OZY_BSLICE + ks * 32;
+            // slice t against C slices u0 .. u0 + nu - 1 (levels t + u0 ..).
+            // t = 1 first: in the first K step its seven levels 1-7 start from
+            // zero, level 0 from t = 0, u = 0, and everything else accumulates
+            auto mma = [&](int t, int u0, int nu, bool fresh) {
+              mma_bf16(d + (uint32_t)((t + u0) * OZY_UNIT), sw128_desc(ab + t * OZY_ASLICE),
+                       sw128_desc(cb + u0 * OZY_BSLICE), f16_idesc(128, OZY_UNIT * nu),
+                       (!fresh || ks > 0) ? 1u : 0u);
+            };
+            mma(1, 0, 7, true);
+            if (ks == 0) {
+              mma(0, 0, 1, true);
+              mma(0, 1, 6, false);
+            } else {
+              mma(0, 0, 7, false);
+            }
+            for (int t = 2; t < OZY_S; t++) mma(t, 0, 8 - t, false);
+            if (hf + 1 == nh) mma_commit(&a_empty[ks]);
+          }
+          if (abort_flag) break;
+          mma_commit(&acc_full[set]);
+        }
+      }
+      mma_commit(&done_bar);
+    }
+  } else {
+    // ------------------------------------------------------- epilogue
+    const int quarter = warp & 3, chalf = warp >> 2;
+    const int r = 32 * quarter + lane;
+    long u = 0;
+    bool stop = false;
+    for (long i = 0; i < my_tiles && !stop; i++) {
+      const long row = (blockIdx.x + i * gridDim.x) * 128 + r;
+      for (int hf = 0; hf < nh; hf++, u++) {
+        const int set = (int)(u & 1);
+        const int jbase = hf * OZY_UNIT + 16 * chalf;  // this warp's 16 columns
+        unsigned long long zn[4];  // Z, four columns ahead
+        ozy_load_z(prm.z_kind, s_z, jbase, w, row, prm.n, zn);
+        const bool got = mbar_wait_n(&acc_full[set], (uint32_t)((u >> 1) & 1), &abort_flag, prm.polls);
+        if (!__all_sync(0xffffffffu, got)) {  // tcgen05.ld needs the whole warp
+          abort_flag = 1;
+          atomicExch(prm.err, 16);
+          stop = true;
+          break;
+        }
+        tc_fence_after();
+        const int er = rowexp[i & 3][r];
+        // scales out of the ordinary (zeros included): the general conversion,
+        // or the direct sum
+        const bool odd = !oz8_plain(er) || any_odd;
+        const uint32_t tl = tmem + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(set * OZY_SET + 16 * chalf);
+        double yp[4];
+        int jp = -1;
+        auto put = [&](const double(&y)[4], int j0) {
+#pragma unroll
+          for (int jj = 0; jj < 4; jj++)
+            if (row < prm.n && j0 + jj < w) ozy_st(s_y[j0 + jj], row, y[jj]);
+          if (prm.has_y32) {
+#pragma unroll
+            for (int jj = 0; jj < 4; jj++)
+              if (row < prm.n && j0 + jj < w) ozy_st32(s_y32[j0 + jj], row, oz_to_float(y[jj]));
+          }
+        };
+        // (not unrolled: the roles of a scheduler's warps share its instruction
+        // cache)
+#pragma unroll 1
+        for (int g = 0; g < 4; g++) {
+          const int j0 = jbase + 4 * g;
+          if (j0 >= w) break;
+          uint32_t x[8][4];  // the eight levels of four columns
+          ozy_tmem_ld(tl + (uint32_t)(4 * g), x);
+          // the previous four columns go out only now: their conversions and
+          // additions have had this group's start to finish in
+          if (g > 0) put(yp, jp);
+          unsigned long long zb[4];
+#pragma unroll
+          for (int jj = 0; jj < 4; jj++) zb[jj] = zn[jj];
+          if (g < 3) ozy_load_z(prm.z_kind, s_z, j0 + 4, w, row, prm.n, zn);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          // (no branch among the entries: their integer chains overlap)
+          double y[4];
+          long long T[4];
+          bool small = odd;
+#pragma unroll
+          for (int jj = 0; jj < 4; jj++) {
+            T[jj] = oz8_combine(x[0][jj], x[1][jj], x[2][jj], x[3][jj], x[4][jj], x[5][jj], x[6][jj], x[7][jj]);
+            small |= (uint32_t)((T[jj] >> 32) + 1) <= 1u;  // |T| < 2^32: cancellation, a zero
+          }
+          if (small) {
+#pragma unroll
+            for (int jj = 0; jj < 4; jj++) {
+              y[jj] = oz8_scaled(T[jj], er + colexp[j0 + jj] - OZ8_BASE);
+              if (row < prm.n && j0 + jj < w && (oz8_unsafe(er) || oz8_unsafe(colexp[j0 + jj])))
+                y[jj] = ozy_direct(s_x, prm.C, prm.ldc, h, j0 + jj, row);
+            }
+          } else {
+#pragma unroll
+            for (int jj = 0; jj < 4; jj++) y[jj] = oz8_scaled_fast(T[jj], er + colexp[j0 + jj] - OZ8_BASE);
+          }
+          if (prm.z_kind == 1) {
+            bool cvt = false;
+#pragma unroll
+            for (int jj = 0; jj < 4; jj++) cvt |= (((uint32_t)zb[jj] & 0x7FFFFFFFu) - 0x00800000u) >= 0x7F000000u;
+            if (cvt) {
+#pragma unroll
+              for (int jj = 0; jj < 4; jj++) y[jj] += (double)__uint_as_float((uint32_t)zb[jj]);
+            } else {
+              // a normal FP32 number widened on its bits: the conversion
+              // instruction would occupy the FP64 pipe as long as the addition
+#pragma unroll
+              for (int jj = 0; jj < 4; jj++) {
+                const uint32_t z = (uint32_t)zb[jj];
+                const uint32_t hi = (z & 0x80000000u) | (((z & 0x7FFFFFFFu) >> 3) + 0x38000000u);
+                y[jj] += __hiloint2double((int)hi, (int)(z << 29));
+              }
+            }
+          } else if (prm.z_kind == 2) {
+#pragma unroll
+            for (int jj = 0; jj < 4; jj++) y[jj] += __longlong_as_double((long long)zb[jj]);
+          }
+#pragma unroll
+          for (int jj = 0; jj < 4; jj++) yp[jj] = y[jj];
+          jp = j0;
+        }
+        tc_fence_before();
+        mbar_arrive(&acc_empty[set]);
+        if (jp >= 0) put(yp, jp);
+      }
+    }
+  }
+  // TMEM is freed only after the last MMA has completed (done_bar is always
+  // committed by the issuer) and every epilogue read has finished
+  if (warp == 16) {
+    mbar_drain(&done_bar, 0);
+    __syncwarp();
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 16) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+  }
+}
+
+__global__ void ozy_check_kernel(const int* err, int* status)
+{
+  if (*err) *status = *err;
+}
+
+// columns [0, h) x [0, w) of the tables, h, w <= 64; polls <= 0: the default limit
+static int ozy_launch(gpu_Context* ctx, long n, const void* const* X, int h, const double* C, int ldc,
+                      const void* const* Y, int w, const void* const* Z, int z_kind, const void* const* Y32,
+                      int polls, int* err)
+{
+  ozy_params prm;
+  memset(&prm, 0, sizeof(prm));
+  for (int c = 0; c < h; c++) prm.x[c] = X[c];
+  for (int j = 0; j < w; j++) {
+    prm.y[j] = (void*)Y[j];
+    if (z_kind) prm.z[j] = Z[j];
+    if (Y32) prm.y32[j] = (void*)Y32[j];
+  }
+  prm.C = C;
+  prm.ldc = ldc;
+  prm.h = h;
+  prm.w = w;
+  prm.z_kind = z_kind;
+  prm.has_y32 = Y32 != NULL;
+  prm.n = n;
+  prm.polls = polls > 0 ? (long)polls : TC_WAIT_LIMIT;
+  prm.err = err;
+  if (cudaFuncSetAttribute(oz_xc64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, OZY_SMEM) !=
+      cudaSuccess)
+    return gb_fail(ctx, "oz_xc64: cannot reserve %d bytes of shared memory", OZY_SMEM);
+  const long ntiles = (n + 127) / 128;
+  const unsigned nctas = (unsigned)(ntiles < ctx->num_sms ? ntiles : ctx->num_sms);
+  oz_xc64_kernel<<<nctas, OZY_THREADS, OZY_SMEM, (cudaStream_t)ctx->stream>>>(prm);
+  gb_count_launch(1);
+  return gb_cuda_check(ctx, (int)cudaGetLastError(), "oz_xc64");
+}
+
+extern "C" int gb_oz_xc64(gpu_Context* ctx, long n, const blk_cols* X, int h, const double* C, int ldc,
+                        const blk_cols* Y, int w, const blk_cols* Z, int z_dtype, const blk_cols* Y32)
+{
+  if (n <= 0 || w <= 0) return 0;
+  if (h < 1 || h > 64 || w > 64)
+    return gb_fail(ctx, "oz_xc64: block widths (%d -> %d) not supported", h, w);
+  for (int c = 0; c < h; c++)
+    if ((uintptr_t)X->col[c] & 15) return gb_fail(ctx, "oz_xc64: input column %d not 16-byte aligned", c);
+  int* err = (int*)gb_workspace(ctx, 256);
+  if (!err) return -1;
+  if (cudaMemsetAsync(err, 0, sizeof(int), (cudaStream_t)ctx->stream) != cudaSuccess)
+    return gb_fail(ctx, "oz_xc64: memset failed");
+  const int zk = Z ? (z_dtype == GPU_MV_FLOAT64 ? 2 : 1) : 0;
+  gb_prof_rec pr;
+  gb_prof_begin(ctx, &pr, GB_K_OZ_XC);
+  const int rc = ozy_launch(ctx, n, X->col, h, C, ldc, Y->col, w, Z ? Z->col : NULL, zk, Y32 ? Y32->col : NULL,
+                            ctx->opt.wait_polls, err);
+  const double zb = zk == 2 ? 8.0 * w : (zk == 1 ? 4.0 * w : 0.0);
+  gb_prof_end(ctx, &pr, (double)n * (8.0 * h + 8.0 * w + zb + (Y32 ? 4.0 * w : 0.0)),
+              2.0 * n * h * w);
+  if (rc) return rc;
+  ozy_check_kernel<<<1, 1, 0, (cudaStream_t)ctx->stream>>>(err, ctx->dcount + 5);
+  gb_count_launch(1);
+  return gb_cuda_check(ctx, (int)cudaGetLastError(), "oz_xc64_check");
+}
+
+// The FP64 block update of gb_bymat for any widths: 64 output columns at a
+// time, and within them 64 input columns at a time, the later ones added to
+// the sum so far.  A wait that gives up (with the default limit, whatever the
+// context's option) is reported in the device error word.
+extern "C" int gb_oz_bymat64(gpu_Context* ctx, long n, const blk_cols* X, int h, const double* C, int ldc,
+                             const blk_cols* Y, int w, const blk_cols* Z)
+{
+  for (int j0 = 0; j0 < w; j0 += 64) {
+    const int wj = w - j0 < 64 ? w - j0 : 64;
+    for (int i0 = 0; i0 < h; i0 += 64) {
+      const int hi = h - i0 < 64 ? h - i0 : 64;
+      const void* const* z = i0 ? Y->col + j0 : (Z ? Z->col + j0 : NULL);
+      if (ozy_launch(ctx, n, X->col + i0, hi, C + i0 + (size_t)j0 * ldc, ldc, Y->col + j0, wj, z, z ? 2 : 0,
+                     NULL, 0, ctx->dcount + 5))
+        return -1;
+    }
+  }
+  return 0;
+}

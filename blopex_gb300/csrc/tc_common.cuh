@@ -77,6 +77,18 @@ static __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
   return false;
 }
 
+// the same with the caller's limit
+static __device__ __forceinline__ bool mbar_wait_n(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
+                                                   long limit)
+{
+  const uint32_t addr = smem_u32(bar);
+  for (long i = 0; i < limit; i++) {
+    if (mbar_try_wait(addr, parity)) return true;
+    if (*abort_flag) return false;
+  }
+  return false;
+}
+
 // bounded drain: wait for work already in flight (copies landing in this
 // CTA's shared memory, the MMAs before TMEM is freed); never aborted early
 static __device__ __forceinline__ bool mbar_drain(uint64_t* bar, uint32_t parity)
