@@ -150,7 +150,7 @@ int project(adj_state* a, gpu_MultiVector* L, gpu_MultiVector* R, gpu_MultiVecto
   cols_of(R, &cr);
   cols_of(y, &cy);
   const int k = a->k;
-  if (gb_gram(a->ctx, GPU_MV_FLOAT64, a->n, &cr, k, &cy, k, a->M, k)) return -1;
+  if (gb_gram_large(a->ctx, GPU_MV_FLOAT64, a->n, &cr, k, &cy, k, a->M, k)) return -1;
   adj_neg_kernel<<<(k * k + 255) / 256, 256, 0, S(a->ctx)>>>(k * k, a->M);
   gb_count_launch(1);
   return gb_bymat_large(a->ctx, GPU_MV_FLOAT64, a->n, &cl, k, a->M, k, &cy, k, &cy);
@@ -285,7 +285,7 @@ extern "C" int gpu_EigenvectorAdjoint(gpu_MultiVector* X, const double* lambda, 
     for (int i = 0; i < k; i++) lmax = fmax(lmax, fabs(lambda[i]));
     const double tol_deg = 1e-12 * (lmax > 0.0 ? lmax : 1.0);
     // S = X'G; x_i'g_i for the mass term; W = X M (in-space part + glam)
-    rc = gb_gram(ctx, GPU_MV_FLOAT64, a.n, &cx, k, &cg, k, a.Sg, k);
+    rc = gb_gram_large(ctx, GPU_MV_FLOAT64, a.n, &cx, k, &cg, k, a.Sg, k);
     if (!rc) {
       adj_inspace_kernel<<<(unsigned)((kk + 255) / 256), 256, 0, S(ctx)>>>(k, a.Sg, a.lam, a.glam,
                                                                            tol_deg, a.M);

@@ -426,6 +426,34 @@ extern "C" int gb_gram(gpu_Context* ctx, int dtype, long n, const blk_cols* X, i
   return gram_launch<float, 4, 4>(ctx, n, X, h, Y, w, G, ldg);
 }
 
+// Callers' products (the interpreter's entry, the adjoint): FP64 ones of at
+// least GRAM_TENSOR_MIN multiply-adds on the tensor cores (oz_gram64.cu), with
+// an error no larger.  The FP64 pipe takes 0.17 ms for them at its 0.58 T
+// multiply-adds/s, the tensor-core kernel 0.05 to 0.07 (65,536 x 32 x 32: 45 us
+// against 125; 16,384 x 32 x 32: 51 against 30).  The solver keeps gb_gram: the
+// signs of its Ritz vectors follow the last bits of these sums, and a solve
+// returns the same iterates, bit for bit, as it always did.
+#define GRAM_TENSOR_MIN 1e8
+
+extern "C" int gb_gram_large(gpu_Context* ctx, int dtype, long n, const blk_cols* X, int h,
+                             const blk_cols* Y, int w, double* G, int ldg)
+{
+  if (h <= 0 || w <= 0) return 0;
+  if (dtype != GPU_MV_FLOAT64 || (double)n * h * w < GRAM_TENSOR_MIN)
+    return gb_gram(ctx, dtype, n, X, h, Y, w, G, ldg);
+  const int sym = h == w && memcmp(X->col, Y->col, sizeof(void*) * (size_t)h) == 0;
+  const double* partial;
+  long splits;
+  gb_prof_rec pr;
+  gb_prof_begin(ctx, &pr, GB_K_GRAM);
+  if (gb_oz_gram64(ctx, n, X, h, Y, w, sym, &partial, &splits)) return -1;
+  gram_reduce_kernel<<<(h * w + 31) / 32, 256, 0, S(ctx)>>>(partial, (int)splits, 1, splits, h * w, h, sym ? 2 : 0, G,
+                                                            ldg);
+  gb_prof_end(ctx, &pr, 8.0 * n * (sym ? h : h + w), sym ? (double)n * h * (h + 1) : 2.0 * n * h * w);
+  gb_count_launch(1);
+  return CUDA_LAUNCH_CHECK(ctx, "gram64");
+}
+
 // ------------------------------------------------------------------------
 // X*C update: Y(:, j0:j0+32) for 64 rows per CTA; thread t owns row t%64
 // and 8 columns (t/64)*8 ... ; K staged 32 at a time in shared memory.
@@ -524,9 +552,8 @@ extern "C" int gb_bymat(gpu_Context* ctx, int dtype, long n, const blk_cols* X, 
 // Callers' updates (the interpreter's entries, the adjoint): FP64 ones of at
 // least XC_TENSOR_MIN multiply-adds on the tensor cores (oz_xc64.cu), with a
 // smaller error: 2,097,152 x 32 x 32 0.43 ms against 3.5; 262,144 x 8 x 8 42 us
-// against 53; a launch costs it 20 us at least.  The solver keeps gb_bymat:
-// the signs of its Ritz vectors follow the last bits of these sums,
-// and a solve returns the same iterates, bit for bit, as it always did.
+// against 53; a launch costs it 20 us at least.  The solver keeps gb_bymat, for
+// the reason given at gb_gram_large.
 #define XC_TENSOR_MIN 1.6e7
 
 extern "C" int gb_bymat_large(gpu_Context* ctx, int dtype, long n, const blk_cols* X, int h,

@@ -305,7 +305,7 @@ static void gi_InnerProd(void* x_, void* y_, BlopexInt gh, BlopexInt h, BlopexIn
   blk_cols a, b;
   gb_mv_fill_cols(x, &a, 0);
   gb_mv_fill_cols(y, &b, 0);
-  if (gb_gram(ctx, x->dtype, x->size, &a, h, &b, w, g, h) == 0) {
+  if (gb_gram_large(ctx, x->dtype, x->size, &a, h, &b, w, g, h) == 0) {
     double* tmp = (double*)malloc(sizeof(double) * (size_t)h * w);
     if (gb_memcpy_d2h(ctx, tmp, g, sizeof(double) * (size_t)h * w) == 0)
       for (int j = 0; j < w; j++)

@@ -56,6 +56,17 @@ def _update(ctx, X, C, Y0=None, shift=0):
     return my.to_host()
 
 
+def _gram(ctx, mx, my):
+    h, w = mx.shape[1], my.shape[1]
+    interp = S._Interp(ctx.lib)
+    xx = ctx.lib.mv_MultiVectorWrap(interp.ptr, mx.handle, 0)
+    yy = ctx.lib.mv_MultiVectorWrap(interp.ptr, my.handle, 0)
+    G = np.empty((h, w), order="F")
+    ctx.lib.mv_MultiVectorByMultiVector(xx, yy, h, h, w, G.ctypes.data)
+    assert ctx.last_error() == ""
+    return G
+
+
 def _check_update(X, C, Y0, Y):
     L = np.longdouble
     ref = X.astype(L) @ C.astype(L)
@@ -119,3 +130,67 @@ def test_update_nonfinite(ctx):
     assert np.array_equal(np.isinf(Y), np.isinf(ref)) and np.array_equal(Y[np.isinf(Y)], ref[np.isinf(ref)])
     rows, cols = np.setdiff1d(np.arange(n), [100, 128, 29999]), np.setdiff1d(np.arange(w), [5, 8])
     _check_update(X[rows], C[:, cols], None, Y[np.ix_(rows, cols)])
+
+
+def _check_gram(X, Y, G):
+    L = np.longdouble
+    ref = np.zeros((X.shape[1], Y.shape[1]), dtype=L)
+    b = np.zeros(ref.shape)
+    # (the groups of the kernel are of 128 or 256 rows: bounds over 256)
+    for r in range(0, X.shape[0], 256):
+        x, y = X[r:r + 256], Y[r:r + 256]
+        ref += x.astype(L).T @ y.astype(L)
+        b += (len(x) * (2.0 ** -53 + 2.0 ** -58) + 2 * 2.0 ** -52) * np.outer(np.abs(x).max(0), np.abs(y).max(0))
+    # FP64 additions: over a CTA's groups (up to 8 sums by weight), then the CTAs
+    b += 2.0 ** -53 * (X.shape[0] / 128 / 152 + 8 + 64) * (np.abs(X).T @ np.abs(Y))
+    assert np.all(np.abs(G - ref) <= b), float((np.abs(G - ref) / b).max())
+
+
+# 2, 4 and 8 stacked slices (w > 32, > 16, <= 16), tiles of 64, units of 8
+# columns partly empty, a short last group
+@pytest.mark.parametrize("n,h,w,shift", [
+    (400003, 17, 15, 0), (25000, 64, 64, 0), (76001, 40, 33, 1), (98500, 33, 31, 0), (15001, 100, 70, 1),
+    (280001, 8, 45, 0), (1000003, 4, 26, 0), (30011, 65, 129, 0), (500000, 64, 4, 1)])
+def test_gram_on_tensor_cores(ctx, n, h, w, shift):
+    rng = np.random.default_rng(n + h + w)
+    X, Y = rng.standard_normal((n, h)) * np.exp(rng.standard_normal((1, h))), rng.standard_normal((n, w))
+    mx, my = _device(ctx, X, shift), _device(ctx, Y, shift)
+    _check_gram(X, Y, _gram(ctx, mx, my))
+
+
+@pytest.mark.parametrize("n,h", [(1000003, 11), (250000, 30), (40000, 64), (12001, 97)])
+def test_gram_of_one_block_is_symmetric(ctx, n, h):
+    rng = np.random.default_rng(n + h)
+    X = rng.standard_normal((n, h))
+    mx = _device(ctx, X)
+    G = _gram(ctx, mx, mx)
+    assert np.array_equal(G, G.T)
+    _check_gram(X, X, G)
+
+
+def test_gram_scales_and_nonfinite(ctx):
+    """Columns over 200 decades, zero and subnormal columns, a zero stretch;
+    then an infinity and a NaN, which reach their columns' entries only."""
+    rng = np.random.default_rng(8)
+    n, h, w = 120001, 30, 40
+    X = rng.standard_normal((n, h)) * 10.0 ** rng.uniform(-120, 80, size=(1, h))
+    Y = rng.standard_normal((n, w)) * 10.0 ** rng.uniform(-80, 60, size=(1, w))
+    X[:, 3] = 0.0
+    X[:, 4] = rng.standard_normal(n) * 1e-311
+    X[1000:9000] = 0.0
+    Y[:, 6] = 0.0
+    mx, my = _device(ctx, X), _device(ctx, Y)
+    G = _gram(ctx, mx, my)
+    assert np.all(G[3] == 0) and np.all(G[:, 6] == 0)
+    s = np.outer(np.linalg.norm(X, axis=0), np.linalg.norm(Y, axis=0))  # (of columns that keep off underflow)
+    keep = np.arange(h) != 4
+    ref = X.T.astype(np.longdouble) @ Y.astype(np.longdouble)
+    assert np.all(np.abs(G - ref)[keep] <= 1e-14 * s[keep])
+    assert np.all(np.abs(G[4] - ref[4]) <= 1e-14 * (np.abs(X[:, 4]).astype(np.longdouble) @ np.abs(Y))
+                  + n * 2.0 ** -1074)
+    X[7, 5], Y[n - 1, 2], Y[5000, 9] = np.inf, np.nan, np.inf
+    Y[7, :] = np.abs(Y[7, :])
+    G = _gram(ctx, _device(ctx, X), _device(ctx, Y))
+    with np.errstate(invalid="ignore"):
+        r = X.T @ Y
+    assert np.array_equal(np.isnan(G), np.isnan(r)) and np.array_equal(np.isinf(G), np.isinf(r))
