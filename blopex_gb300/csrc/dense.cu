@@ -398,7 +398,10 @@ __global__ void __launch_bounds__(DENSE_THREADS) sygv_kernel(double* A, double* 
     if (tid == 0) *info = 2 * m + 1;
     return;
   }
-  // 4. ascending order: rank of each eigenvalue (ties by index)
+  // 4. ascending order: rank of each eigenvalue (ties by index; NaN entries share
+  // a rank, and every entry must hold an index all the same)
+  for (int i = tid; i < m; i += nt) s_perm[i] = i;
+  __syncthreads();
   for (int i = tid; i < m; i += nt) {
     double di = C[i + (size_t)i * m];
     int r = 0;

@@ -401,6 +401,10 @@ __global__ void __launch_bounds__(RR_THREADS) rr_vsort_kernel(int m, rr_scratch 
   __shared__ int perm[512];
   const int tid = threadIdx.x, nt = blockDim.x;
   if (s.status[0]) return;
+  // NaN eigenvalues (a product poisoned by a timed-out wait) share a rank: every
+  // entry must hold an index all the same
+  for (int i = tid; i < m; i += nt) perm[i] = i;
+  __syncthreads();
   for (int i = tid; i < m; i += nt) {
     float di = s.lam32[i];
     int r = 0;
@@ -635,6 +639,8 @@ __global__ void __launch_bounds__(RR_THREADS) rr_refine_kernel(int m, rr_scratch
     }
     // ascending order inside the cluster
     __shared__ int cperm[512];
+    for (int a = tid; a < sz; a += nt) cperm[a] = a;  // (NaN entries share a rank)
+    __syncthreads();
     for (int a = tid; a < sz; a += nt) {
       double da = Mc[a + a * lm];
       int r = 0;
