@@ -64,12 +64,27 @@ static __device__ __forceinline__ bool mbar_try_wait(uint32_t addr, uint32_t par
   return done != 0;
 }
 
-// bounded pipeline wait for the phase with the given parity (tc_wait_polls
-// polls); false on timeout or when another role has aborted
-static __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag)
+// the phase's state now; try_wait may suspend the thread for a while first
+static __device__ __forceinline__ bool mbar_test_wait(uint32_t addr, uint32_t parity)
+{
+  uint32_t done;
+  asm volatile(
+      "{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+      " selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(done)
+      : "r"(addr), "r"(parity)
+      : "memory");
+  return done != 0;
+}
+
+// bounded pipeline wait for the phase with the given parity (limit polls; a limit
+// of one looks once, without suspension, and so gives up on any phase that has not
+// completed); false on timeout or when another role has aborted
+static __device__ __forceinline__ bool mbar_wait_n(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
+                                                   long limit)
 {
   const uint32_t addr = smem_u32(bar);
-  const long limit = tc_wait_polls;
+  if (limit == 1) return mbar_test_wait(addr, parity);
   for (long i = 0; i < limit; i++) {
     if (mbar_try_wait(addr, parity)) return true;
     if (*abort_flag) return false;
@@ -77,16 +92,10 @@ static __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
   return false;
 }
 
-// the same with the caller's limit
-static __device__ __forceinline__ bool mbar_wait_n(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
-                                                   long limit)
+// the same with the limit of the last launch (tc_wait_polls)
+static __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag)
 {
-  const uint32_t addr = smem_u32(bar);
-  for (long i = 0; i < limit; i++) {
-    if (mbar_try_wait(addr, parity)) return true;
-    if (*abort_flag) return false;
-  }
-  return false;
+  return mbar_wait_n(bar, parity, abort_flag, tc_wait_polls);
 }
 
 // bounded drain: wait for work already in flight (copies landing in this
