@@ -31,18 +31,82 @@ static __device__ __forceinline__ void acc_prod32x4(float& s, float& c, float4 a
   acc_prod32(s, c, a.w, b.w);
 }
 
+// (s, c) += (s2, c2), two compensated sums
+static __device__ __forceinline__ void acc_pair32(float& s, float& c, float s2, float c2)
+{
+  const float t = __fadd_rn(s, s2);
+  const float bp = __fsub_rn(t, s);
+  const float e = __fadd_rn(__fsub_rn(s, __fsub_rn(t, bp)), __fsub_rn(s2, bp));
+  s = t;
+  c = __fadd_rn(__fadd_rn(c, c2), e);
+}
+
+static __device__ __forceinline__ void warp_pair_sum32(float& s, float& c)
+{
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const float s2 = __shfl_xor_sync(0xffffffffu, s, o), c2 = __shfl_xor_sync(0xffffffffu, c, o);
+    acc_pair32(s, c, s2, c2);
+  }
+}
+
+// block-wide sum of the threads' compensated sums (blockDim.x = 256), the
+// result in thread 0, in a fixed order: the warps in FP32 pairs (an FP64 add
+// holds this GPU's FP64 pipe for 16 cycles), the eight warp sums in FP64
+static __device__ __forceinline__ double block_pair_sum256(float s, float c)
+{
+  __shared__ float2 red[8];
+  warp_pair_sum32(s, c);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = make_float2(s, c);
+  __syncthreads();
+  double v = 0.0;
+  if (threadIdx.x < 32) {
+    const float2 p = red[threadIdx.x & 7];
+    v = (double)p.x + (double)p.y;
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  }
+  return v;
+}
+
 // block-wide sum of one double per thread (blockDim.x = 256), the result in
-// thread 0, in a fixed order
+// thread 0, in a fixed order: halves of 128, 64, ..., 1.  All of it in warp 0
+// behind one branch: a tree over the block, its adds predicated off in the warps
+// that had no part in a level, held the FP64 pipe (16 cycles an instruction,
+// executed or not) for 1024 cycles a block instead of 192.
 static __device__ __forceinline__ double block_sum256(double v)
 {
   __shared__ double red[256];
-  red[threadIdx.x] = v;
+  const int t = threadIdx.x;
+  red[t] = v;
   __syncthreads();
-  for (int o = 128; o > 0; o >>= 1) {
-    if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
+  if (t < 32) {
+    const double a0 = red[t] + red[t + 128], a1 = red[t + 32] + red[t + 160];
+    const double a2 = red[t + 64] + red[t + 192], a3 = red[t + 96] + red[t + 224];
+    v = (a0 + a2) + (a1 + a3);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  }
+  return v;
+}
+
+// p[0] + p[1] + ... + p[n - 1] in that order, in thread 0 (blockDim.x = 256): the
+// loads by the whole block at once, the adds one by one (70 cycles each)
+static __device__ __forceinline__ double ordered_sum256(const double* p, int n)
+{
+  __shared__ double buf[256];
+  double s = 0.0;
+  for (int b0 = 0; b0 < n; b0 += 256) {
+    if (b0 + threadIdx.x < n) buf[threadIdx.x] = __ldcg(p + b0 + threadIdx.x);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      const int m = min(256, n - b0);
+#pragma unroll 8
+      for (int b = 0; b < m; b++) s += buf[b];
+    }
     __syncthreads();
   }
-  return red[0];
+  return s;
 }
 
 static inline bool cols_aligned16(const void* const* cols, int w)

@@ -665,24 +665,15 @@ __global__ void dot_partial_kernel(blk_cols X, blk_cols Y, long n, double* __res
   double s = 0.0;
   for (long r = blockIdx.x * (long)blockDim.x + threadIdx.x; r < n; r += (long)gridDim.x * blockDim.x)
     s += (double)x[r] * (double)y[r];
-  __shared__ double red[256];
-  red[threadIdx.x] = s;
-  __syncthreads();
-  for (int o = 128; o > 0; o >>= 1) {
-    if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) partial[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = red[0];
+  s = block_sum256(s);
+  if (threadIdx.x == 0) partial[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = s;
 }
 
 __global__ void dot_reduce_kernel(const double* __restrict__ partial, int nb, idx_table idx,
-                                  int w, double* __restrict__ out)
+                                  double* __restrict__ out)
 {
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= w) return;
-  double s = 0.0;
-  for (int b = 0; b < nb; b++) s += partial[(size_t)j * nb + b];
-  out[idx.v[j]] = s;
+  const double s = ordered_sum256(partial + (size_t)blockIdx.x * nb, nb);
+  if (threadIdx.x == 0) out[idx.v[blockIdx.x]] = s;
 }
 
 // FP32 blocks with 16-byte aligned columns: float4 loads, exact products in
@@ -695,14 +686,17 @@ __global__ void __launch_bounds__(256) dot32_partial_kernel(blk_cols X, blk_cols
   const long n4 = n >> 2, stride = (long)gridDim.x * blockDim.x;
   double acc = 0.0;
   float s = 0.f, c = 0.f;
-  int cnt = 0;
+  // the flush stands outside the inner loop: predicated off inside it, its four
+  // FP64 instructions still held the FP64 pipe (16 cycles each)
+  for (long v = blockIdx.x * (long)blockDim.x + threadIdx.x; v < n4;) {
+    if (v + 15 * stride < n4) {
 #pragma unroll 4
-  for (long v = blockIdx.x * (long)blockDim.x + threadIdx.x; v < n4; v += stride) {
-    acc_prod32x4(s, c, x[v], y[v]);
-    if (++cnt == 16) {
+      for (int i = 0; i < 16; i++, v += stride) acc_prod32x4(s, c, x[v], y[v]);
       acc += (double)s + (double)c;
       s = c = 0.f;
-      cnt = 0;
+    } else {
+#pragma unroll 4
+      for (; v < n4; v += stride) acc_prod32x4(s, c, x[v], y[v]);
     }
   }
   if (blockIdx.x == 0 && threadIdx.x < (n & 3)) {  // the last n % 4 rows
@@ -713,18 +707,6 @@ __global__ void __launch_bounds__(256) dot32_partial_kernel(blk_cols X, blk_cols
   const double t = block_sum256(acc);
   if (threadIdx.x == 0) partial[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = t;
 }
-
-extern "C" int gb_dot_reduce(gpu_Context* ctx, const double* partial, int nb, int w, double* out,
-                             const int* idx)
-{
-  idx_table t;
-  fill_idx(&t, idx, w);
-  dot_reduce_kernel<<<(w + 63) / 64, 64, 0, S(ctx)>>>(partial, nb, t, w, out);
-  gb_count_launch(1);
-  return CUDA_LAUNCH_CHECK(ctx, "dot_reduce");
-}
-
-extern "C" unsigned gb_row_blocks(gpu_Context* ctx, long n, int w) { return row_blocks(ctx, n, w); }
 
 extern "C" int gb_dot_cols(gpu_Context* ctx, int dtype, long n, const blk_cols* X,
                            const blk_cols* Y, int w, double* out, const int* idx)
@@ -744,7 +726,7 @@ extern "C" int gb_dot_cols(gpu_Context* ctx, int dtype, long n, const blk_cols* 
     dot32_partial_kernel<<<grid, 256, 0, S(ctx)>>>(*X, *Y, n, partial);
   else
     dot_partial_kernel<float><<<grid, 256, 0, S(ctx)>>>(*X, *Y, n, partial);
-  dot_reduce_kernel<<<(w + 63) / 64, 64, 0, S(ctx)>>>(partial, nb, t, w, out);
+  dot_reduce_kernel<<<w, 256, 0, S(ctx)>>>(partial, nb, t, out);
   gb_prof_end(ctx, &pr, (dtype == GPU_MV_FLOAT64 ? 8.0 : 4.0) * n * w * 2, 2.0 * n * w);
   gb_count_launch(2);
   return CUDA_LAUNCH_CHECK(ctx, "dot_cols");
@@ -778,14 +760,8 @@ __global__ void residual_partial_kernel(blk_cols BX, blk_cols AX, const double* 
     rr[r] = (TO)v;
     s += (double)v * (double)v;
   }
-  __shared__ double red[256];
-  red[threadIdx.x] = s;
-  __syncthreads();
-  for (int o = 128; o > 0; o >>= 1) {
-    if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) partial[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = red[0];
+  s = block_sum256(s);
+  if (threadIdx.x == 0) partial[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = s;
 }
 
 extern "C" int gb_residual(gpu_Context* ctx, int dtype, long n, const blk_cols* BX,
@@ -807,7 +783,7 @@ extern "C" int gb_residual(gpu_Context* ctx, int dtype, long n, const blk_cols* 
     residual_partial_kernel<float><<<grid, 256, 0, S(ctx)>>>(*BX, *AX, lambda, t, *R, n, partial);
   else  // FP64 inputs, FP32 residual
     residual_partial_kernel<double, 1><<<grid, 256, 0, S(ctx)>>>(*BX, *AX, lambda, t, *R, n, partial);
-  dot_reduce_kernel<<<(w + 63) / 64, 64, 0, S(ctx)>>>(partial, nb, t, w, norm2);
+  dot_reduce_kernel<<<w, 256, 0, S(ctx)>>>(partial, nb, t, norm2);
   gb_prof_end(ctx, &pr, (dtype == GPU_MV_FLOAT32 ? 12.0 : (dtype == GPU_MV_FLOAT64 ? 24.0 : 20.0)) * n * w,
               4.0 * n * w);
   gb_count_launch(2);

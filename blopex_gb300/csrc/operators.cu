@@ -58,7 +58,7 @@ struct gpu_Operator {
   int iters;
   gpu_MultiVector* work[4];  // r, z, p, q
   gpu_MultiVector* io32[2];  // FP32 copies of an FP64 input / output (mixed mode)
-  double* coef;              // 4 x BLK_MAXCOLS device doubles
+  double* coef;              // 4 x BLK_MAXCOLS device doubles, then BLK_MAXCOLS ints (zero between kernels)
 };
 
 static inline cudaStream_t S(gpu_Context* ctx) { return (cudaStream_t)ctx->stream; }
@@ -896,34 +896,38 @@ static int st7t_maps(const gpu_Operator* op, const gpu_MultiVector* X, CUtensorM
 
 static int pcg_apply(gpu_Operator* op, gpu_MultiVector* X, gpu_MultiVector* Y);
 
-// the per-column sums of the stencil kernel's warp partials, in a fixed order
+// the per-column sums of the stencil kernel's warp partials, in a fixed order,
+// and the CG coefficient num / sum
 __global__ void __launch_bounds__(256) st7t_dot_reduce_kernel(const double* __restrict__ parts,
-                                                              long nparts, double* __restrict__ out)
+                                                              long nparts, double* __restrict__ out,
+                                                              const double* __restrict__ num,
+                                                              double* __restrict__ ratio)
 {
   const double* p = parts + (size_t)blockIdx.x * nparts;
   double acc = 0.0;
+#pragma unroll 4
   for (long i = threadIdx.x; i < nparts; i += blockDim.x) acc += p[i];
   const double t = block_sum256(acc);
-  if (threadIdx.x == 0) out[blockIdx.x] = t;
+  if (threadIdx.x) return;
+  out[blockIdx.x] = t;
+  const double v = num[blockIdx.x];
+  ratio[blockIdx.x] = (t != 0.0 && v != 0.0) ? v / t : 0.0;
 }
 
-static int operator_apply(gpu_Operator* op, gpu_MultiVector* X, gpu_MultiVector* Y, double* dot_out);
+// Y = A X.  With dot_out: also dot_out[c] = X_c' Y_c and ratio[c] = num[c] /
+// dot_out[c] in the same pass where the operator's kernel can fold the inner
+// products in (the FP32 TMA 7-point stencil): 0; 1 when it cannot (nothing done:
+// apply and take the inner products apart); -1 on error
+static int operator_apply(gpu_Operator* op, gpu_MultiVector* X, gpu_MultiVector* Y, double* dot_out,
+                          const double* num, double* ratio);
 
 extern "C" int gb_operator_apply(gpu_Operator* op, gpu_MultiVector* X, gpu_MultiVector* Y)
 {
-  return operator_apply(op, X, Y, NULL);
+  return operator_apply(op, X, Y, NULL, NULL, NULL);
 }
 
-// Y = A X and out[c] = X_c' Y_c in one pass where the operator's kernel can
-// fold the inner products in (the FP32 TMA 7-point stencil): 0; 1 when it
-// cannot (nothing done: apply and take the inner products apart); -1 on error
-extern "C" int gb_operator_apply_dot(gpu_Operator* op, gpu_MultiVector* X, gpu_MultiVector* Y,
-                                     double* dot_out)
-{
-  return operator_apply(op, X, Y, dot_out);
-}
-
-static int operator_apply(gpu_Operator* op, gpu_MultiVector* X, gpu_MultiVector* Y, double* dot_out)
+static int operator_apply(gpu_Operator* op, gpu_MultiVector* X, gpu_MultiVector* Y, double* dot_out,
+                          const double* num, double* ratio)
 {
   if (op->kind == OPK_PCG) return dot_out ? 1 : pcg_apply(op, X, Y);
   gpu_Context* ctx = op->ctx;
@@ -1023,7 +1027,7 @@ static int operator_apply(gpu_Operator* op, gpu_MultiVector* X, gpu_MultiVector*
                                                       op->c32[2], (float)op->shift, tmc, tmz, pc, yc,
                                                       w, ctx->dcount + 5, dparts);
         if (dot_out) {
-          st7t_dot_reduce_kernel<<<w, 256, 0, S(ctx)>>>(dparts, 8L * st7t_ctas, dot_out);
+          st7t_dot_reduce_kernel<<<w, 256, 0, S(ctx)>>>(dparts, 8L * st7t_ctas, dot_out, num, ratio);
           gb_count_launch(1);
         }
       } else if (f32 && st7_ring_ok(op, &xc, w))
@@ -1395,128 +1399,227 @@ __global__ void pcg_ratio_kernel(int k, const double* num, const double* den, do
   if (i < k) out[i] = (den[i] != 0.0 && num[i] != 0.0) ? num[i] / den[i] : 0.0;
 }
 
-// FP32 blocks with 16-byte aligned columns and a diagonal (Jacobi) or no
-// inner preconditioner M: the column updates of a CG step fused with the
-// inner product that follows them, float4 access, and z = M r recomputed
-// where it is read instead of stored (M is one column, L2-resident).  Per
-// step 13 block passes instead of 17.  Inner products as gb_dot_cols' FP32
-// path (exact products, compensated FP32 sums flushed to FP64).
-//   init: r = x ; p = M x ; partial x' M x
-//   step: y = alpha p (first) or y += alpha p ; r -= alpha q ; partial r' M r
-//   dir:  p = M r + beta p
+// A diagonal (Jacobi) or no inner preconditioner M: the column updates of a CG
+// step fused with the inner product that follows them, z = M r recomputed where
+// it is read instead of stored (M is one column, L2-resident), and the CG
+// coefficients formed by the last CTA of a column to finish.  Per step:
+//   q = A p                                 the operator
+//   dot:  alpha = rho / p'q                 (folded into the FP32 TMA stencil)
+//   step: r -= alpha q ; rho' = r' M r ; beta = rho' / rho
+//   dir:  y += alpha p ; p = M r + beta p
+// 10 block passes (the update of y waits for the pass that reads p anyway; in
+// the first step r is read from x and y is not read), 3 in the last, which only
+// finishes y; 4 launches, where each product, reduction, quotient, preconditioner
+// application and update on its own took 10 (FP64) or 7 (FP32).
+//   512^2 5-point, 8 columns, FP64, 20 steps: 1700 us against 2390 (FP64 pipe: 14
+//   instructions an entry and step, 1010 us; the ordered sums 12 us a step);
+//   128^3 7-point, 17 columns, FP32, 20 steps: 5980 us against 7120 (HBM 4000).
+// FP32 (16-byte aligned columns): float4 access, inner products as gb_dot_cols'
+// FP32 path (exact products, compensated FP32 sums flushed to FP64).  FP64: the
+// rows of a thread and the order of every sum are those of gb_dot_cols.
+// at most this many vectors a thread (FP32), so that no flush of the compensated
+// sums stands in the loops: predicated off, its four FP64 instructions still held
+// the FP64 pipe for 64 cycles a vector and warp (75% of the step kernel's time)
+#define PCG_VECS 8
+enum { PCG_RHO = 0, PCG_ALPHA, PCG_BETA };
+// every CTA of an FP64 grid (8 an SM) resident; FP32: room for the float4 loads
+#define PCG_BOUNDS(T) __launch_bounds__(256, sizeof(T) == 8 ? 8 : 6)
+
+struct pcg_coef {
+  double *rho, *alpha, *beta;
+  int* cnt;
+};
+
+static __device__ __forceinline__ double pcg_ratio(double num, double den)
+{
+  return (den != 0.0 && num != 0.0) ? num / den : 0.0;
+}
+
+// this CTA's sum v (thread 0) of column j; the column's last CTA adds the
+// gridDim.x sums (FP64 blocks: in CTA order, 70 cycles an add; FP32: by threads,
+// in a fixed order) and forms the coefficient
+template <typename T>
+static __device__ __forceinline__ void pcg_finish(double v, int j, double* __restrict__ partial, const pcg_coef& k,
+                                                  int what)
+{
+  __shared__ int last;
+  double* p = partial + (size_t)j * gridDim.x;
+  const int nb = gridDim.x, t = threadIdx.x;
+  if (t == 0) {
+    p[blockIdx.x] = v;
+    __threadfence();
+    last = atomicAdd(&k.cnt[j], 1) == nb - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  double s = 0.0;
+  if (sizeof(T) == 8) {
+    s = ordered_sum256(p, nb);
+  } else {
+    for (int b = t; b < nb; b += 256) s += __ldcg(p + b);
+    s = block_sum256(s);
+  }
+  if (t) return;
+  k.cnt[j] = 0;
+  if (what == PCG_ALPHA) {
+    k.alpha[j] = pcg_ratio(k.rho[j], s);
+  } else {
+    if (what == PCG_BETA) k.beta[j] = pcg_ratio(s, k.rho[j]);
+    k.rho[j] = s;
+  }
+}
+
+// one element or four, with the arithmetic of each type
 template <bool HAVE_M>
-static __device__ __forceinline__ float4 pcg32_m(const float4* m, long v, float4 r)
+static __device__ __forceinline__ float4 pcg_m(const float4* m, long v, float4 r)
 {
   if (!HAVE_M) return r;
   const float4 d = m[v];
   return make_float4(d.x * r.x, d.y * r.y, d.z * r.z, d.w * r.w);
 }
-
 template <bool HAVE_M>
-__global__ void __launch_bounds__(256) pcg32_init_kernel(long n, blk_cols X, const float* __restrict__ m,
-                                                         blk_cols R, blk_cols P,
-                                                         double* __restrict__ partial)
+static __device__ __forceinline__ double pcg_m(const double* m, long v, double r)
 {
-  const float* x = (const float*)X.col[blockIdx.y];
-  float* r = (float*)R.col[blockIdx.y];
-  float* p = (float*)P.col[blockIdx.y];
-  const long n4 = n >> 2, stride = (long)gridDim.x * blockDim.x;
-  double acc = 0.0;
+  return HAVE_M ? m[v] * r : r;
+}
+static __device__ __forceinline__ float4 pcg_fma(float a, float4 x, float4 y)
+{
+  return make_float4(fmaf(a, x.x, y.x), fmaf(a, x.y, y.y), fmaf(a, x.z, y.z), fmaf(a, x.w, y.w));
+}
+static __device__ __forceinline__ double pcg_fma(double a, double x, double y) { return fma(a, x, y); }
+static __device__ __forceinline__ float4 pcg_mul(float a, float4 x)
+{
+  return make_float4(a * x.x, a * x.y, a * x.z, a * x.w);
+}
+static __device__ __forceinline__ double pcg_mul(double a, double x) { return fma(a, x, 0.0); }
+
+template <typename T>
+struct pcg_vec;
+template <>
+struct pcg_vec<float> {
+  typedef float4 type;
+  static constexpr int N = 4;
+};
+template <>
+struct pcg_vec<double> {
+  typedef double type;
+  static constexpr int N = 1;
+};
+
+// a thread's share of an inner product
+template <typename T>
+struct pcg_acc;
+template <>
+struct pcg_acc<double> {
+  double s = 0.0;
+  __device__ __forceinline__ void add(double a, double b) { s = fma(a, b, s); }
+  __device__ __forceinline__ void tail(double, double) {}
+  __device__ __forceinline__ double sum() { return block_sum256(s); }
+};
+template <>
+struct pcg_acc<float> {
   float s = 0.f, c = 0.f;
-  int cnt = 0;
-  for (long v = blockIdx.x * (long)blockDim.x + threadIdx.x; v < n4; v += stride) {
-    const float4 xv = ((const float4*)x)[v];
-    const float4 z = pcg32_m<HAVE_M>((const float4*)m, v, xv);
-    ((float4*)r)[v] = xv;
-    ((float4*)p)[v] = z;
-    acc_prod32x4(s, c, xv, z);
-    if (++cnt == 16) {
-      acc += (double)s + (double)c;
-      s = c = 0.f;
-      cnt = 0;
-    }
+  __device__ __forceinline__ void add(float4 a, float4 b) { acc_prod32x4(s, c, a, b); }
+  __device__ __forceinline__ void tail(float a, float b) { acc_prod32(s, c, a, b); }
+  __device__ __forceinline__ double sum() { return block_pair_sum256(s, c); }
+};
+
+// p = M x ; rho = x' M x
+template <typename T, bool HAVE_M>
+__global__ void PCG_BOUNDS(T)
+    pcg_init_kernel(long n, blk_cols X, const T* __restrict__ m, blk_cols P, double* __restrict__ partial, pcg_coef k)
+{
+  typedef typename pcg_vec<T>::type V;
+  constexpr int N = pcg_vec<T>::N;
+  const int j = blockIdx.y;
+  const T* x = (const T*)X.col[j];
+  T* p = (T*)P.col[j];
+  const long nv = n / N, stride = (long)gridDim.x * blockDim.x;
+  pcg_acc<T> acc;
+  for (long v = blockIdx.x * (long)blockDim.x + threadIdx.x; v < nv; v += stride) {
+    const V xv = ((const V*)x)[v], z = pcg_m<HAVE_M>((const V*)m, v, xv);
+    ((V*)p)[v] = z;
+    acc.add(xv, z);
   }
-  if (blockIdx.x == 0 && threadIdx.x < (n & 3)) {
-    const long e = 4 * n4 + threadIdx.x;
-    const float z = HAVE_M ? m[e] * x[e] : x[e];
-    r[e] = x[e];
+  if (N > 1 && blockIdx.x == 0 && threadIdx.x < n % N) {
+    const long e = N * nv + threadIdx.x;
+    const T z = HAVE_M ? m[e] * x[e] : x[e];
     p[e] = z;
-    acc_prod32(s, c, x[e], z);
+    acc.tail(x[e], z);
   }
-  acc += (double)s + (double)c;
-  const double t = block_sum256(acc);
-  if (threadIdx.x == 0) partial[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = t;
+  pcg_finish<T>(acc.sum(), j, partial, k, PCG_RHO);
 }
 
-template <bool HAVE_M, bool FIRST>
-__global__ void __launch_bounds__(256) pcg32_step_kernel(long n, blk_cols P, blk_cols Q, blk_cols Y,
-                                                         blk_cols R, const float* __restrict__ m,
-                                                         const double* __restrict__ alpha,
-                                                         double* __restrict__ partial)
+// alpha = rho / p'q
+template <typename T>
+__global__ void PCG_BOUNDS(T)
+    pcg_dot_kernel(long n, blk_cols P, blk_cols Q, double* __restrict__ partial, pcg_coef k)
 {
+  typedef typename pcg_vec<T>::type V;
+  constexpr int N = pcg_vec<T>::N;
   const int j = blockIdx.y;
-  const float a = (float)alpha[j];
-  const float* p = (const float*)P.col[j];
-  const float* q = (const float*)Q.col[j];
-  float* y = (float*)Y.col[j];
-  float* r = (float*)R.col[j];
-  const long n4 = n >> 2, stride = (long)gridDim.x * blockDim.x;
-  double acc = 0.0;
-  float s = 0.f, c = 0.f;
-  int cnt = 0;
-  for (long v = blockIdx.x * (long)blockDim.x + threadIdx.x; v < n4; v += stride) {
-    const float4 pv = ((const float4*)p)[v], qv = ((const float4*)q)[v];
-    float4 rv = ((float4*)r)[v];
-    float4 yv;
-    if (FIRST) {
-      yv = make_float4(a * pv.x, a * pv.y, a * pv.z, a * pv.w);
-    } else {
-      yv = ((float4*)y)[v];
-      yv = make_float4(fmaf(a, pv.x, yv.x), fmaf(a, pv.y, yv.y), fmaf(a, pv.z, yv.z), fmaf(a, pv.w, yv.w));
-    }
-    rv = make_float4(fmaf(-a, qv.x, rv.x), fmaf(-a, qv.y, rv.y), fmaf(-a, qv.z, rv.z), fmaf(-a, qv.w, rv.w));
-    ((float4*)y)[v] = yv;
-    ((float4*)r)[v] = rv;
-    if (partial) {
-      acc_prod32x4(s, c, rv, pcg32_m<HAVE_M>((const float4*)m, v, rv));
-      if (++cnt == 16) {
-        acc += (double)s + (double)c;
-        s = c = 0.f;
-        cnt = 0;
-      }
-    }
+  const T *p = (const T*)P.col[j], *q = (const T*)Q.col[j];
+  const long nv = n / N, stride = (long)gridDim.x * blockDim.x;
+  pcg_acc<T> acc;
+#pragma unroll 4
+  for (long v = blockIdx.x * (long)blockDim.x + threadIdx.x; v < nv; v += stride)
+    acc.add(((const V*)p)[v], ((const V*)q)[v]);
+  if (N > 1 && blockIdx.x == 0 && threadIdx.x < n % N) acc.tail(p[N * nv + threadIdx.x], q[N * nv + threadIdx.x]);
+  pcg_finish<T>(acc.sum(), j, partial, k, PCG_ALPHA);
+}
+
+// r = r0 - alpha q ; rho, beta from r' M r (r0 = x in the first step, then r)
+template <typename T, bool HAVE_M>
+__global__ void PCG_BOUNDS(T) pcg_step_kernel(long n, blk_cols Q, blk_cols R0, blk_cols R, const T* __restrict__ m,
+                                              double* __restrict__ partial, pcg_coef k)
+{
+  typedef typename pcg_vec<T>::type V;
+  constexpr int N = pcg_vec<T>::N;
+  const int j = blockIdx.y;
+  const T a = -(T)k.alpha[j];
+  const T *q = (const T*)Q.col[j], *r0 = (const T*)R0.col[j];
+  T* r = (T*)R.col[j];
+  const long nv = n / N, stride = (long)gridDim.x * blockDim.x;
+  pcg_acc<T> acc;
+#pragma unroll 2
+  for (long v = blockIdx.x * (long)blockDim.x + threadIdx.x; v < nv; v += stride) {
+    const V rv = pcg_fma(a, ((const V*)q)[v], ((const V*)r0)[v]);
+    ((V*)r)[v] = rv;
+    acc.add(rv, pcg_m<HAVE_M>((const V*)m, v, rv));
   }
-  if (blockIdx.x == 0 && threadIdx.x < (n & 3)) {
-    const long e = 4 * n4 + threadIdx.x;
-    y[e] = FIRST ? a * p[e] : fmaf(a, p[e], y[e]);
-    const float re = fmaf(-a, q[e], r[e]);
+  if (N > 1 && blockIdx.x == 0 && threadIdx.x < n % N) {
+    const long e = N * nv + threadIdx.x;
+    const T re = fma(a, q[e], r0[e]);
     r[e] = re;
-    if (partial) acc_prod32(s, c, re, HAVE_M ? m[e] * re : re);
+    acc.tail(re, HAVE_M ? m[e] * re : re);
   }
-  if (!partial) return;  // uniform over the grid
-  acc += (double)s + (double)c;
-  const double t = block_sum256(acc);
-  if (threadIdx.x == 0) partial[(size_t)j * gridDim.x + blockIdx.x] = t;
+  pcg_finish<T>(acc.sum(), j, partial, k, PCG_BETA);
 }
 
-template <bool HAVE_M>
-__global__ void __launch_bounds__(256) pcg32_dir_kernel(long n, blk_cols R, const float* __restrict__ m,
-                                                        blk_cols P, const double* __restrict__ beta)
+// y (+)= alpha p ; p = M r + beta p (not in the last step)
+template <typename T, bool HAVE_M, bool FIRST>
+__global__ void PCG_BOUNDS(T)
+    pcg_dir_kernel(long n, blk_cols R, const T* __restrict__ m, blk_cols P, blk_cols Y, int last, pcg_coef k)
 {
+  typedef typename pcg_vec<T>::type V;
+  constexpr int N = pcg_vec<T>::N;
   const int j = blockIdx.y;
-  const float b = (float)beta[j];
-  const float* r = (const float*)R.col[j];
-  float* p = (float*)P.col[j];
-  const long n4 = n >> 2, stride = (long)gridDim.x * blockDim.x;
-  for (long v = blockIdx.x * (long)blockDim.x + threadIdx.x; v < n4; v += stride) {
-    const float4 z = pcg32_m<HAVE_M>((const float4*)m, v, ((const float4*)r)[v]);
-    float4 pv = ((float4*)p)[v];
-    pv = make_float4(fmaf(b, pv.x, z.x), fmaf(b, pv.y, z.y), fmaf(b, pv.z, z.z), fmaf(b, pv.w, z.w));
-    ((float4*)p)[v] = pv;
+  const T a = (T)k.alpha[j], b = (T)k.beta[j];
+  const T* r = (const T*)R.col[j];
+  T *p = (T*)P.col[j], *y = (T*)Y.col[j];
+  const long nv = n / N, stride = (long)gridDim.x * blockDim.x;
+#pragma unroll 2
+  for (long v = blockIdx.x * (long)blockDim.x + threadIdx.x; v < nv; v += stride) {
+    const V pv = ((const V*)p)[v];
+    ((V*)y)[v] = FIRST ? pcg_mul(a, pv) : pcg_fma(a, pv, ((const V*)y)[v]);
+    if (!last) ((V*)p)[v] = pcg_fma(b, pv, pcg_m<HAVE_M>((const V*)m, v, ((const V*)r)[v]));
   }
-  if (blockIdx.x == 0 && threadIdx.x < (n & 3)) {
-    const long e = 4 * n4 + threadIdx.x;
-    p[e] = fmaf(b, p[e], HAVE_M ? m[e] * r[e] : r[e]);
+  if (N > 1 && blockIdx.x == 0 && threadIdx.x < n % N) {
+    const long e = N * nv + threadIdx.x;
+    const T pe = p[e];
+    y[e] = FIRST ? a * pe : fma(a, pe, y[e]);
+    if (!last) p[e] = fma(b, pe, HAVE_M ? m[e] * r[e] : r[e]);
   }
 }
 
@@ -1531,80 +1634,65 @@ extern "C" gpu_Operator* gpu_PCGPreconditionerCreate(gpu_Context* ctx, gpu_Opera
   op->inner = A;
   op->prec = M;
   op->iters = iterations;
-  op->coef = (double*)gb_device_alloc(ctx, sizeof(double) * 4 * BLK_MAXCOLS);
-  if (!op->coef) {
+  const size_t cbytes = (sizeof(double) * 4 + sizeof(int)) * BLK_MAXCOLS;
+  op->coef = (double*)gb_device_alloc(ctx, cbytes);
+  if (!op->coef || cudaMemsetAsync(op->coef, 0, cbytes, S(ctx)) != cudaSuccess) {
     gpu_OperatorDestroy(op);
     return NULL;
   }
   return op;
 }
 
-// the FP32 inner CG of pcg_apply on the fused kernels above (M diagonal or
-// absent, aligned columns); the same recurrences and coefficients
-static int pcg32_fused(gpu_Operator* op, gpu_MultiVector* X, const blk_cols* cx, const blk_cols* cy,
-                       const blk_cols* cr, const blk_cols* cp, const blk_cols* cq, int w, dim3 grid,
-                       const int* idx)
+// the inner CG of pcg_apply on the fused kernels above (M diagonal or absent;
+// FP32: aligned columns)
+template <typename T, bool HAVE_M>
+static int pcg_fused(gpu_Operator* op, const blk_cols* cx, const blk_cols* cy, const blk_cols* cr,
+                     const blk_cols* cp, const blk_cols* cq, int w, dim3 grid)
 {
   gpu_Context* ctx = op->ctx;
+  cudaStream_t st = S(ctx);
   const long n = op->n;
-  const float* m = op->prec ? op->prec->d32 : NULL;
-  double *rho = op->coef, *rho2 = rho + BLK_MAXCOLS, *pq = rho2 + BLK_MAXCOLS, *al = pq + BLK_MAXCOLS;
-  const double blk = 4.0 * (double)n * w, mb = m ? 4.0 * (double)n : 0.0;
-  gpu_MultiVector* p = op->work[2];
-  gpu_MultiVector* q = op->work[3];
+  const T* m = !HAVE_M ? NULL : (sizeof(T) == 8 ? (const T*)op->prec->d : (const T*)op->prec->d32);
+  pcg_coef k;
+  k.rho = op->coef;
+  k.alpha = k.rho + BLK_MAXCOLS;
+  k.beta = k.alpha + BLK_MAXCOLS;
+  k.cnt = (int*)(k.rho + 4 * BLK_MAXCOLS);
+  const double blk = (double)sizeof(T) * n * w, mb = HAVE_M ? (double)sizeof(T) * n : 0.0;
+  gpu_MultiVector *p = op->work[2], *q = op->work[3];
   gb_prof_rec pr;
-  // r = x ; p = M x ; rho = x' M x
   double* partial = (double*)gb_workspace(ctx, sizeof(double) * (size_t)grid.x * w);
   if (!partial) return -1;
   gb_prof_begin(ctx, &pr, GB_K_BLAS1);
-  if (m)
-    pcg32_init_kernel<true><<<grid, 256, 0, S(ctx)>>>(n, *cx, m, *cr, *cp, partial);
-  else
-    pcg32_init_kernel<false><<<grid, 256, 0, S(ctx)>>>(n, *cx, m, *cr, *cp, partial);
-  gb_prof_end(ctx, &pr, 3.0 * blk + mb, 2.0 * n * w);
+  pcg_init_kernel<T, HAVE_M><<<grid, 256, 0, st>>>(n, *cx, m, *cp, partial, k);
+  gb_prof_end(ctx, &pr, 2.0 * blk + mb, 2.0 * n * w);
   gb_count_launch(1);
-  if (gb_dot_reduce(ctx, partial, (int)grid.x, w, rho, idx)) return -1;
-  (void)X;
   for (int it = 0; it < op->iters; it++) {
-    // q = A p with p' q folded into the operator's kernel where it can be
-    const int fused = gb_operator_apply_dot(op->inner, p, q, pq);
-    if (fused < 0) return -1;
-    if (fused == 1 && (gb_operator_apply(op->inner, p, q) ||
-                       gb_dot_cols(ctx, GPU_MV_FLOAT32, n, cp, cq, w, pq, idx)))
-      return -1;
-    pcg_ratio_kernel<<<1, BLK_MAXCOLS, 0, S(ctx)>>>(w, rho, pq, al);
-    gb_count_launch(1);
-    const bool last = it + 1 == op->iters;
-    partial = last ? NULL : (double*)gb_workspace(ctx, sizeof(double) * (size_t)grid.x * w);
-    if (!last && !partial) return -1;
-    gb_prof_begin(ctx, &pr, GB_K_BLAS1);
-    if (it == 0) {
-      if (m)
-        pcg32_step_kernel<true, true><<<grid, 256, 0, S(ctx)>>>(n, *cp, *cq, *cy, *cr, m, al, partial);
-      else
-        pcg32_step_kernel<false, true><<<grid, 256, 0, S(ctx)>>>(n, *cp, *cq, *cy, *cr, m, al, partial);
-    } else {
-      if (m)
-        pcg32_step_kernel<true, false><<<grid, 256, 0, S(ctx)>>>(n, *cp, *cq, *cy, *cr, m, al, partial);
-      else
-        pcg32_step_kernel<false, false><<<grid, 256, 0, S(ctx)>>>(n, *cp, *cq, *cy, *cr, m, al, partial);
+    // q = A p, alpha with p' q folded into the operator's kernel where it can be
+    const int fused = operator_apply(op->inner, p, q, k.rho + 3 * BLK_MAXCOLS, k.rho, k.alpha);
+    if (fused < 0 || (fused == 1 && gb_operator_apply(op->inner, p, q))) return -1;
+    partial = (double*)gb_workspace(ctx, sizeof(double) * (size_t)grid.x * w);
+    if (!partial) return -1;
+    if (fused == 1) {
+      gb_prof_begin(ctx, &pr, GB_K_BLAS1);
+      pcg_dot_kernel<T><<<grid, 256, 0, st>>>(n, *cp, *cq, partial, k);
+      gb_prof_end(ctx, &pr, 2.0 * blk, 2.0 * n * w);
+      gb_count_launch(1);
     }
-    gb_prof_end(ctx, &pr, (it == 0 ? 5.0 : 6.0) * blk + (last ? 0.0 : mb), 4.0 * n * w);
-    gb_count_launch(1);
-    if (last) break;
-    if (gb_dot_reduce(ctx, partial, (int)grid.x, w, rho2, idx)) return -1;
-    pcg_ratio_kernel<<<1, BLK_MAXCOLS, 0, S(ctx)>>>(w, rho2, rho, al);  // beta
-    gb_count_launch(1);
+    const bool last = it + 1 == op->iters;
     gb_prof_begin(ctx, &pr, GB_K_BLAS1);
-    if (m)
-      pcg32_dir_kernel<true><<<grid, 256, 0, S(ctx)>>>(n, *cr, m, *cp, al);
+    if (!last) {
+      pcg_step_kernel<T, HAVE_M><<<grid, 256, 0, st>>>(n, *cq, it == 0 ? *cx : *cr, *cr, m, partial, k);
+      gb_count_launch(1);
+    }
+    if (it == 0)
+      pcg_dir_kernel<T, HAVE_M, true><<<grid, 256, 0, st>>>(n, *cr, m, *cp, *cy, last, k);
     else
-      pcg32_dir_kernel<false><<<grid, 256, 0, S(ctx)>>>(n, *cr, m, *cp, al);
-    gb_prof_end(ctx, &pr, 3.0 * blk + mb, 2.0 * n * w);
+      pcg_dir_kernel<T, HAVE_M, false><<<grid, 256, 0, st>>>(n, *cr, m, *cp, *cy, last, k);
+    // step: q, r -> r; dir: p, y (not the first time), r -> y, p; the last: p, y -> y
+    gb_prof_end(ctx, &pr, (last ? 3.0 : 8.0) * blk - (it == 0 ? blk : 0.0) + (last ? 0.0 : 2.0 * mb),
+                (last ? 2.0 : 8.0) * n * w);
     gb_count_launch(1);
-    double* t = rho;
-    rho = rho2;
-    rho2 = t;
   }
   return gb_cuda_check(ctx, (int)cudaGetLastError(), "pcg preconditioner");
 }
@@ -1675,6 +1763,9 @@ static int pcg_apply(gpu_Operator* op, gpu_MultiVector* X, gpu_MultiVector* Y)
   if (want > cap) want = cap;
   const dim3 grid((unsigned)want, w);
   const bool mdiag = !op->prec || op->prec->kind == OPK_DIAG;
+  if (!f32 && mdiag)
+    return op->prec ? pcg_fused<double, true>(op, &cx, &cy, &cr, &cp, &cq, w, grid)
+                    : pcg_fused<double, false>(op, &cx, &cy, &cr, &cp, &cq, w, grid);
   if (f32 && mdiag && cols_aligned16(cx.col, w) && cols_aligned16(cy.col, w) &&
       cols_aligned16(cr.col, w) && cols_aligned16(cp.col, w) && cols_aligned16(cq.col, w) &&
       (!op->prec || ensure_f32(op->prec) == 0)) {
@@ -1682,7 +1773,12 @@ static int pcg_apply(gpu_Operator* op, gpu_MultiVector* X, gpu_MultiVector* Y)
     // context asks for accurate FP32 operators
     const int acc_saved = ctx->op_accurate;
     if (ctx->opt.fp32_accurate_op) ctx->op_accurate = 1;
-    const int rc = pcg32_fused(op, X, &cx, &cy, &cr, &cp, &cq, w, grid, idx);
+    // PCG_VECS vectors a thread while that leaves 8 CTAs an SM, fewer on small blocks
+    long vecs = op->n * w / (4L * 256 * 8 * ctx->num_sms);
+    vecs = vecs < 1 ? 1 : vecs > PCG_VECS ? PCG_VECS : vecs;
+    const dim3 grid4((unsigned)((op->n + 4 * 256 * vecs - 1) / (4 * 256 * vecs)), w);
+    const int rc = op->prec ? pcg_fused<float, true>(op, &cx, &cy, &cr, &cp, &cq, w, grid4)
+                            : pcg_fused<float, false>(op, &cx, &cy, &cr, &cp, &cq, w, grid4);
     ctx->op_accurate = acc_saved;
     return rc;
   }
