@@ -13,10 +13,10 @@
 //                   blocks with FP64 arithmetic);
 //   csr32_kernel    FP32 CSR: the row's entries in registers, the gathers of
 //                   four columns issued ahead of their products;
-//   st7_tma_kernel  FP32 7-point: plane tiles staged by TMA into a
-//                   shared-memory column ring (st7_ring_kernel: the same
-//                   with cp.async copies; st7_kernel: scalar, FP64 and the
-//                   unaligned cases);
+//   st7_tma_kernel  FP32 7-point: tiles of one or two planes staged by TMA
+//                   into a shared-memory column ring (st7_ring_kernel: one
+//                   plane with cp.async copies; st7_kernel: scalar, FP64 and
+//                   the unaligned cases);
 //   st5_kernel, st27_kernel, diag_kernel;
 // plus the inner-CG preconditioner (pcg_apply) and the parameter gradients
 // of the adjoint module (grad_*_kernel).
@@ -378,20 +378,38 @@ __global__ void __launch_bounds__(256) st7_ring_kernel(int nx, int ny, int nz,
 // ------------------------------------------- 7-point, FP32, TMA column ring
 // The column ring of st7_ring_kernel with the copies done by the tensor
 // memory accelerator: per column one thread issues three 4D tensor loads
-// (x, y, z, block column) on one mbarrier -- the 40 x 34 centre box from
-// (i0 - 4, j0 - 1, k) and the 32 x 32 boxes of planes k - 1 and k + 1 --
-// and TMA writes the same shared-memory layout the cp.async plan builds
-// (centre rows of 40 floats, cells at offsets 4-35), filling everything off
-// the grid with zeros.  x coordinates are multiples of 4 floats (16 bytes);
+// (x, y, z, block column) on one mbarrier -- the 40 x 34 x NP centre box from
+// (i0 - 4, j0 - 1, k0) and the 32 x 32 boxes of planes k0 - 1 and k0 + NP --
+// and TMA fills everything off the grid with zeros (centre rows of 40 floats,
+// cells at offsets 4-35).  x coordinates are multiples of 4 floats (16 bytes);
 // every box starts on a 128-byte boundary of its slot.  Waits are bounded: a
 // timeout stops the issue of further copies, poisons the CTA's outputs with
 // NaN, sets the context's device error word and, before the CTA exits,
 // waits (bounded again) for the copies still in flight.
+//
+// Bound by HBM on large grids, by the latency of a CTA's column chain (0.5 us a
+// column) on small ones.
+//   NP planes a CTA: two share their halo planes and face weights, 2.3 floats
+//     staged a cell instead of 3.3; one leaves more CTAs (st7t_planes).
+//   A thread has four cells in x of one row (16-byte shared loads and stores,
+//     x neighbours by shuffles): a third fewer instructions than four rows of one.
+//   Strips of about ST7T_STRIP tiles, z before the next strip, so that the CTAs
+//     that share halo planes run within a few columns of each other; whole planes
+//     first let the z halo fall out of L2 (256^3, 64 columns: 1729 us, strips of
+//     8, 16, 32 tiles: 1474, 1459, 1513; 512 x 256 x 128: 1972, 1471, 1471, 1497).
+//   256^3, 64 columns: 1455 us, 5.9 TB/s of blocks and coefficients (6.1 with the
+//     halos read twice), before 1797; 128^3, 17 columns: 64 us against 71;
+//     32^3, 64 columns: 9 us against 39.
 #define ST7T_DEPTH 3
-#define ST7T_BELOW 1376  // floats: the 34 x 40 centre box, padded to 128 bytes
-#define ST7T_ABOVE (ST7T_BELOW + 1024)
-#define ST7T_SLOT (ST7T_ABOVE + 1024)            // 13696 bytes, a multiple of 128
-#define ST7T_BYTES ((34 * 40 + 2 * 32 * 32) * 4)  // bytes per column (13632)
+#define ST7T_STRIP 16
+template <int NP>  // planes a CTA
+struct st7t_cfg {
+  static constexpr int PLANE = 34 * 40;                                   // floats of a centre plane
+  static constexpr int BELOW = (NP * PLANE + 31) / 32 * 32;               // offsets in a slot: 128-byte steps
+  static constexpr int ABOVE = BELOW + 1024, SLOT = ABOVE + 1024;
+  static constexpr int BYTES = (NP * PLANE + 2 * 1024) * 4;               // one column's copies
+  static constexpr int SMEM = ST7T_DEPTH * SLOT * 4 + 128;
+};
 
 struct st7t_cols {
   int c[BLK_MAXCOLS];  // physical column of each active column
@@ -407,22 +425,58 @@ static __device__ __forceinline__ void st7t_load(uint32_t dst, const CUtensorMap
       : "memory");
 }
 
-__global__ void __launch_bounds__(256) st7_tma_kernel(
+template <int NP>
+static __device__ __forceinline__ void st7t_issue(uint32_t slot, const CUtensorMap* tm_c, const CUtensorMap* tm_z,
+                                                  int i0, int j0, int k0, int col, uint64_t* bar)
+{
+  using C = st7t_cfg<NP>;
+  const uint32_t b = smem_u32(bar);
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"((uint32_t)C::BYTES)
+               : "memory");
+  st7t_load(slot, tm_c, i0 - 4, j0 - 1, k0, col, b);
+  st7t_load(slot + 4u * C::BELOW, tm_z, i0, j0, k0 - 1, col, b);
+  st7t_load(slot + 4u * C::ABOVE, tm_z, i0, j0, k0 + NP, col, b);
+}
+
+// a column's sum over the CTA of the threads' compensated sums, by one warp (all
+// eight warps' values in a fixed order), into the CTA's partial
+static __device__ __forceinline__ void st7t_dot_store(const float2* red, double* out, int lane)
+{
+  float s = 0.f, c = 0.f;
+#pragma unroll
+  for (int q = 0; q < 8; q++) {
+    const float2 v = red[32 * q + lane];
+    acc_pair32(s, c, v.x, v.y);
+  }
+  warp_pair_sum32(s, c);
+  if (lane == 0) *out = (double)s + (double)c;
+}
+
+template <int NP, bool DOT>
+__global__ void __launch_bounds__(256, NP == 1 ? 4 : 3) st7_tma_kernel(
     int nx, int ny, int nz, const float* __restrict__ cx, const float* __restrict__ cy,
     const float* __restrict__ cz, float shift, const __grid_constant__ CUtensorMap tm_c,
     const __grid_constant__ CUtensorMap tm_z, const __grid_constant__ st7t_cols XC,
-    const __grid_constant__ blk_cols Y, int w, int* err, double* __restrict__ dotp)
+    const __grid_constant__ blk_cols Y, int wall, int cpg, int strip, int yvec, int* err, double* __restrict__ dotp)
 {
-  __shared__ __align__(128) float ring[ST7T_DEPTH * ST7T_SLOT];
+  using C = st7t_cfg<NP>;
+  extern __shared__ float ring_raw[];
+  float* ring = ring_raw + ((128u - (smem_u32(ring_raw) & 127u)) & 127u) / 4;
   __shared__ __align__(8) uint64_t bar[ST7T_DEPTH];
   __shared__ int abort_flag;
-  const int t = threadIdx.x, tx = t & 31, ty = t >> 5;
+  __shared__ float2 red[DOT ? 2 : 1][DOT ? 256 : 1];
+  const int t = threadIdx.x, tx = t & 7, ty = t >> 3, warp = t >> 5, lane = t & 31;
   const int tiles_x = (nx + 31) / 32, tiles_y = (ny + 31) / 32;
-  const long b = blockIdx.x;
-  const int tile = (int)(b % ((long)tiles_x * tiles_y));
-  const int k = (int)(b / ((long)tiles_x * tiles_y));
-  const int i0 = (tile % tiles_x) * 32, j0 = (tile / tiles_x) * 32;
+  const unsigned b = blockIdx.x;
+  // tiles in strips of `strip` tile rows, z before the next strip
+  const unsigned per = (unsigned)(tiles_x * strip) * ((nz + NP - 1) / NP);
+  const int s0 = (int)(b / per) * strip;
+  const unsigned rest = b % per, in_strip = (unsigned)(tiles_x * min(strip, tiles_y - s0));
+  const int k0 = NP * (int)(rest / in_strip), tile = (int)(rest % in_strip);
+  const int i0 = (tile % tiles_x) * 32, j0 = (s0 + tile / tiles_x) * 32;
   const long plane = (long)nx * ny;
+  // columns c0 .. c0 + w - 1
+  const int c0 = blockIdx.y * cpg, w = min(cpg, wall - c0);
   if (t == 0) {
     abort_flag = 0;
     for (int q = 0; q < ST7T_DEPTH; q++) mbar_init(&bar[q], 1);
@@ -431,47 +485,54 @@ __global__ void __launch_bounds__(256) st7_tma_kernel(
   __syncthreads();
   const uint32_t ring_s = smem_u32(ring);
   int issued = 0, waited = 0;  // thread 0: columns issued / columns whose copies it saw land
-  if (t == 0) {
-    for (int c = 0; c < ST7T_DEPTH - 1 && c < w; c++) {
-      const uint32_t bq = smem_u32(&bar[c]), d = ring_s + 4u * ST7T_SLOT * c;
-      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bq),
-                   "r"((uint32_t)ST7T_BYTES)
-                   : "memory");
-      st7t_load(d, &tm_c, i0 - 4, j0 - 1, k, XC.c[c], bq);
-      st7t_load(d + 4u * ST7T_BELOW, &tm_z, i0, j0, k - 1, XC.c[c], bq);
-      st7t_load(d + 4u * ST7T_ABOVE, &tm_z, i0, j0, k + 1, XC.c[c], bq);
-      issued++;
-    }
-  }
+  if (t == 0)
+    for (; issued < ST7T_DEPTH - 1 && issued < w; issued++)
+      st7t_issue<NP>(ring_s + 4u * C::SLOT * issued, &tm_c, &tm_z, i0, j0, k0, XC.c[c0 + issued], &bar[issued]);
 
-  // coefficients of the thread's four cells (rows j0 + 4 ty .. + 3)
-  const int i = i0 + tx, jb = j0 + 4 * ty;
-  float dg[4], ww[4], we[4], ws[4], wn[4], wb[4], wt[4];
-  bool valid[4];
+  // coefficients of the thread's cells: four in x (all or none on the grid, nx a
+  // multiple of 4) of row j in NP planes; neighbours share a face's weight, which
+  // is zero on the boundary
+  const int i = i0 + 4 * tx, j = j0 + ty;
+  const bool on = i < nx && j < ny;
+  float dg[NP][4], wx[NP][5], ws[NP][4], wn[NP][4], wz[NP + 1][4];
+  {
+    float4 f[NP + 1];
 #pragma unroll
-  for (int s = 0; s < 4; s++) {
-    const int j = jb + s;
-    valid[s] = i < nx && j < ny;
-    dg[s] = ww[s] = we[s] = ws[s] = wn[s] = wb[s] = wt[s] = 0.f;
-    if (valid[s]) {
-      const long cell = (long)i + (long)nx * j + plane * k;
-      const long jk = (long)j + (long)ny * k;
-      const float cw = cx[i + (long)(nx + 1) * jk];
-      const float ce = cx[i + 1 + (long)(nx + 1) * jk];
-      const float cs = cy[i + (long)nx * (j + (long)(ny + 1) * k)];
-      const float cn = cy[i + (long)nx * (j + 1 + (long)(ny + 1) * k)];
-      const float cb = cz[cell];
-      const float ct = cz[cell + plane];
-      dg[s] = cw + ce + cs + cn + cb + ct + shift;
-      ww[s] = i > 0 ? cw : 0.f;
-      we[s] = i < nx - 1 ? ce : 0.f;
-      ws[s] = j > 0 ? cs : 0.f;
-      wn[s] = j < ny - 1 ? cn : 0.f;
-      wb[s] = k > 0 ? cb : 0.f;
-      wt[s] = k < nz - 1 ? ct : 0.f;
+    for (int p = 0; p <= NP; p++) {
+      const int k = k0 + p;
+      f[p] = on && k <= nz ? *(const float4*)(cz + i + (long)nx * j + plane * k) : make_float4(0.f, 0.f, 0.f, 0.f);
+      const bool in = k > 0 && k < nz;
+      wz[p][0] = in ? f[p].x : 0.f, wz[p][1] = in ? f[p].y : 0.f;
+      wz[p][2] = in ? f[p].z : 0.f, wz[p][3] = in ? f[p].w : 0.f;
+    }
+#pragma unroll
+    for (int p = 0; p < NP; p++) {
+      const int k = k0 + p;
+      float4 s4 = make_float4(0.f, 0.f, 0.f, 0.f), n4 = s4;
+#pragma unroll
+      for (int x = 0; x < 5; x++) wx[p][x] = 0.f;
+      if (on && k < nz) {
+        const float* fx = cx + i + (long)(nx + 1) * (j + (long)ny * k);
+#pragma unroll
+        for (int x = 0; x < 5; x++) wx[p][x] = fx[x];
+        const float* fy = cy + i + (long)nx * (j + (long)(ny + 1) * k);
+        s4 = *(const float4*)fy;
+        n4 = *(const float4*)(fy + nx);
+      }
+      const float s_[4] = {s4.x, s4.y, s4.z, s4.w}, n_[4] = {n4.x, n4.y, n4.z, n4.w};
+      const float b_[4] = {f[p].x, f[p].y, f[p].z, f[p].w};
+      const float t_[4] = {f[p + 1].x, f[p + 1].y, f[p + 1].z, f[p + 1].w};
+#pragma unroll
+      for (int x = 0; x < 4; x++) {
+        dg[p][x] = wx[p][x] + wx[p][x + 1] + s_[x] + n_[x] + b_[x] + t_[x] + shift;
+        ws[p][x] = j > 0 ? s_[x] : 0.f;
+        wn[p][x] = j < ny - 1 ? n_[x] : 0.f;
+      }
+      if (i == 0) wx[p][0] = 0.f;
+      if (i + 4 >= nx) wx[p][4] = 0.f;
     }
   }
-  const long cell0 = (long)i + (long)nx * jb + plane * k;
+  const long cell0 = (long)i + (long)nx * j + plane * k0;
 
   int slot = 0, ahead_slot = ST7T_DEPTH - 1;
 #pragma unroll 1
@@ -484,61 +545,66 @@ __global__ void __launch_bounds__(256) st7_tma_kernel(
     const bool go = !abort_flag;
     const int ahead = col + ST7T_DEPTH - 1;
     if (go && t == 0 && ahead < w) {
-      const uint32_t bq = smem_u32(&bar[ahead_slot]), d = ring_s + 4u * ST7T_SLOT * ahead_slot;
       fence_proxy_async();
-      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bq),
-                   "r"((uint32_t)ST7T_BYTES)
-                   : "memory");
-      st7t_load(d, &tm_c, i0 - 4, j0 - 1, k, XC.c[ahead], bq);
-      st7t_load(d + 4u * ST7T_BELOW, &tm_z, i0, j0, k - 1, XC.c[ahead], bq);
-      st7t_load(d + 4u * ST7T_ABOVE, &tm_z, i0, j0, k + 1, XC.c[ahead], bq);
+      st7t_issue<NP>(ring_s + 4u * C::SLOT * ahead_slot, &tm_c, &tm_z, i0, j0, k0, XC.c[c0 + ahead],
+                     &bar[ahead_slot]);
       issued++;
     }
-    float* y = (float*)Y.col[col] + cell0;
+    // the column before: its threads' sums were written ahead of the barrier
+    if (DOT && col > 0 && warp == ((col - 1) & 7))
+      st7t_dot_store(red[(col - 1) & 1], dotp + (long)(c0 + col - 1) * gridDim.x + b, lane);
+    float* y = (float*)Y.col[c0 + col] + cell0;
     float xs = 0.f, xc = 0.f;  // this thread's share of x' (A x): compensated sum
     if (go) {
-      const float* sl = ring + ST7T_SLOT * slot;
-      float cv[6];
+      const float* sl = ring + C::SLOT * slot;
+      float4 v[NP + 2];
+      v[0] = *(const float4*)(sl + C::BELOW + 32 * ty + 4 * tx);
 #pragma unroll
-      for (int r = 0; r < 6; r++) cv[r] = sl[(4 * ty + r) * 40 + 4 + tx];
+      for (int p = 0; p < NP; p++) v[p + 1] = *(const float4*)(sl + p * C::PLANE + 40 * (ty + 1) + 4 + 4 * tx);
+      v[NP + 1] = *(const float4*)(sl + C::ABOVE + 32 * ty + 4 * tx);
 #pragma unroll
-      for (int s = 0; s < 4; s++) {
-        const int m = (4 * ty + 1 + s) * 40 + 4 + tx;
-        const float v1 = sl[m - 1], v2 = sl[m + 1];
-        const float v5 = sl[ST7T_BELOW + (4 * ty + s) * 32 + tx];
-        const float v6 = sl[ST7T_ABOVE + (4 * ty + s) * 32 + tx];
-        if (valid[s]) {
-          const float yv = dg[s] * cv[s + 1] - ww[s] * v1 - we[s] * v2 - ws[s] * cv[s] -
-                           wn[s] * cv[s + 2] - wb[s] * v5 - wt[s] * v6;
-          __stcs(y + (long)nx * s, yv);
-          if (dotp) acc_prod32(xs, xc, cv[s + 1], yv);
+      for (int p = 0; p < NP; p++) {
+        const float* r = sl + p * C::PLANE + 40 * (ty + 1) + 4 + 4 * tx;
+        const float4 vs = *(const float4*)(r - 40), vn = *(const float4*)(r + 40);
+        const float4 c = v[p + 1], lo = v[p], up = v[p + 2];
+        // x neighbours of the quad: the next lanes' cells, from the tile at its rims
+        float e = 0.f;
+        if (tx == 0 || tx == 7) e = r[tx == 0 ? -1 : 4];
+        float vw = __shfl_up_sync(0xffffffffu, c.w, 1), ve = __shfl_down_sync(0xffffffffu, c.x, 1);
+        if (tx == 0) vw = e;
+        if (tx == 7) ve = e;
+        float4 o;
+        o.x = dg[p][0] * c.x - wx[p][0] * vw - wx[p][1] * c.y - ws[p][0] * vs.x - wn[p][0] * vn.x - wz[p][0] * lo.x -
+              wz[p + 1][0] * up.x;
+        o.y = dg[p][1] * c.y - wx[p][1] * c.x - wx[p][2] * c.z - ws[p][1] * vs.y - wn[p][1] * vn.y - wz[p][1] * lo.y -
+              wz[p + 1][1] * up.y;
+        o.z = dg[p][2] * c.z - wx[p][2] * c.y - wx[p][3] * c.w - ws[p][2] * vs.z - wn[p][2] * vn.z - wz[p][2] * lo.z -
+              wz[p + 1][2] * up.z;
+        o.w = dg[p][3] * c.w - wx[p][3] * c.z - wx[p][4] * ve - ws[p][3] * vs.w - wn[p][3] * vn.w - wz[p][3] * lo.w -
+              wz[p + 1][3] * up.w;
+        if (on && k0 + p < nz) {
+          float* yp = y + plane * p;
+          if (yvec) {
+            __stcs((float4*)yp, o);
+          } else {
+            __stcs(yp, o.x), __stcs(yp + 1, o.y), __stcs(yp + 2, o.z), __stcs(yp + 3, o.w);
+          }
+          if (DOT) acc_prod32x4(xs, xc, c, o);
         }
       }
-    }
-    if (dotp) {
-      // per warp: exact products in compensated FP32 sums, combined across
-      // the lanes by two-sums, into FP64 partials that a second kernel sums
-      // in a fixed order (the inner CG's p' A p, as accurate as its
-      // separate inner-product kernel)
+    } else {
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const float s2 = __shfl_xor_sync(0xffffffffu, xs, o);
-        const float c2 = __shfl_xor_sync(0xffffffffu, xc, o);
-        const float t2 = __fadd_rn(xs, s2);
-        const float bp = __fsub_rn(t2, xs);
-        const float e = __fadd_rn(__fsub_rn(xs, __fsub_rn(t2, bp)), __fsub_rn(s2, bp));
-        xs = t2;
-        xc = __fadd_rn(__fadd_rn(xc, c2), e);
-      }
-      if (tx == 0) dotp[(long)col * gridDim.x * 8 + blockIdx.x * 8 + ty] = go ? (double)xs + (double)xc : 0.0;
+      for (int p = 0; p < NP; p++)
+        if (on && k0 + p < nz)
+          for (int x = 0; x < 4; x++) y[plane * p + x] = __int_as_float(0x7fc00000);  // NaN: output incomplete
     }
-    if (!go) {
-#pragma unroll
-      for (int s = 0; s < 4; s++)
-        if (valid[s]) y[(long)nx * s] = __int_as_float(0x7fc00000);  // NaN: output incomplete
-    }
+    if (DOT) red[col & 1][t] = make_float2(xs, xc);
     slot = slot == ST7T_DEPTH - 1 ? 0 : slot + 1;
     ahead_slot = ahead_slot == ST7T_DEPTH - 1 ? 0 : ahead_slot + 1;
+  }
+  if (DOT) {
+    __syncthreads();
+    if (warp == ((w - 1) & 7)) st7t_dot_store(red[(w - 1) & 1], dotp + (long)(c0 + w - 1) * gridDim.x + b, lane);
   }
   if (t == 0 && abort_flag) {
     atomicExch(err, 1);
@@ -870,10 +936,10 @@ static PFN_cuTensorMapEncodeTiled_v12000 st7t_encoder(void)
 }
 
 // tensor maps of the FP32 block X as (x, y, z, column) for st7_tma_kernel:
-// boxes 40 x 34 (centre plane with halo) and 32 x 32 (planes above and
+// boxes 40 x 34 x np (centre planes with halo) and 32 x 32 (planes above and
 // below).  TMA needs 16-byte-aligned bases and strides: nx a multiple of 4
 // and ld * 4 a multiple of 16.  Returns 0 when both maps were encoded.
-static int st7t_maps(const gpu_Operator* op, const gpu_MultiVector* X, CUtensorMap* mc,
+static int st7t_maps(const gpu_Operator* op, const gpu_MultiVector* X, int np, CUtensorMap* mc,
                      CUtensorMap* mz)
 {
   PFN_cuTensorMapEncodeTiled_v12000 enc = st7t_encoder();
@@ -882,7 +948,7 @@ static int st7t_maps(const gpu_Operator* op, const gpu_MultiVector* X, CUtensorM
                               (cuuint64_t)X->num_vectors};
   const cuuint64_t strides[3] = {(cuuint64_t)op->nx * 4, (cuuint64_t)op->nx * op->ny * 4,
                                  (cuuint64_t)X->ld * 4};
-  const cuuint32_t boxc[4] = {40, 34, 1, 1}, boxz[4] = {32, 32, 1, 1}, es[4] = {1, 1, 1, 1};
+  const cuuint32_t boxc[4] = {40, 34, (cuuint32_t)np, 1}, boxz[4] = {32, 32, 1, 1}, es[4] = {1, 1, 1, 1};
   if (enc(mc, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, X->data, dims, strides, boxc, es,
           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
@@ -896,7 +962,44 @@ static int st7t_maps(const gpu_Operator* op, const gpu_MultiVector* X, CUtensorM
 
 static int pcg_apply(gpu_Operator* op, gpu_MultiVector* X, gpu_MultiVector* Y);
 
-// the per-column sums of the stencil kernel's warp partials, in a fixed order,
+static long st7t_ctas(const gpu_Operator* op, int np)
+{
+  return (long)((op->nx + 31) / 32) * ((op->ny + 31) / 32) * ((op->nz + np - 1) / np);
+}
+
+// two planes a CTA once that fills the GPU's 3 resident CTAs an SM twice over
+// (128^3, 64 columns, 1024 CTAs: 201 us, one plane 213; 96 x 100 x 101, 612 CTAs:
+// 120 us, one plane 111)
+static int st7t_planes(const gpu_Operator* op) { return st7t_ctas(op, 2) >= 6L * op->ctx->num_sms ? 2 : 1; }
+
+static_assert(st7t_cfg<1>::SMEM + 4096 + 64 <= 48 * 1024, "one plane must fit the default shared memory");
+
+template <int NP, bool DOT>
+static int st7t_launch(gpu_Operator* op, const CUtensorMap& tmc, const CUtensorMap& tmz, const st7t_cols& pc,
+                       const blk_cols& yc, int w, int yvec, double* dparts)
+{
+  gpu_Context* ctx = op->ctx;
+  const int smem = st7t_cfg<NP>::SMEM;
+  if (NP > 1 &&  // (one plane fits the 48 KB every kernel has)
+      cudaFuncSetAttribute(st7_tma_kernel<NP, DOT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
+          cudaSuccess)
+    return gb_fail(ctx, "stencil7: cannot reserve %d bytes of shared memory", smem);
+  // small grids: the columns dealt to several CTAs a tile, as many as fit the GPU at
+  // once, four columns each at least (32^3, 64 columns: 9 us, all in one CTA 31)
+  const long ctas = st7t_ctas(op, NP);
+  long groups = (NP == 1 ? 4L : 3L) * ctx->num_sms / ctas;
+  if (groups > (w + 3) / 4) groups = (w + 3) / 4;
+  if (groups < 1) groups = 1;
+  const int cpg = (int)((w + groups - 1) / groups);
+  const int tiles_x = (op->nx + 31) / 32, strip = tiles_x < ST7T_STRIP ? ST7T_STRIP / tiles_x : 1;
+  const dim3 grid((unsigned)ctas, (unsigned)((w + cpg - 1) / cpg));
+  st7_tma_kernel<NP, DOT><<<grid, 256, smem, S(ctx)>>>(op->nx, op->ny, op->nz, op->c32[0], op->c32[1], op->c32[2],
+                                                       (float)op->shift, tmc, tmz, pc, yc, w, cpg, strip, yvec,
+                                                       ctx->dcount + 5, dparts);
+  return 0;
+}
+
+// the per-column sums of the stencil kernel's CTA partials, in a fixed order,
 // and the CG coefficient num / sum
 __global__ void __launch_bounds__(256) st7t_dot_reduce_kernel(const double* __restrict__ parts,
                                                               long nparts, double* __restrict__ out,
@@ -953,11 +1056,12 @@ static int operator_apply(gpu_Operator* op, gpu_MultiVector* X, gpu_MultiVector*
   const int acc64 = f32 && ctx->op_accurate && (op->kind == OPK_CSR || op->kind == OPK_ST7);
   // the FP32 7-point stencil staged by TMA (nx a multiple of 4, aligned block)
   CUtensorMap tmc, tmz;
-  const int tma = op->kind == OPK_ST7 && f32 && !acc64 && st7t_maps(op, X, &tmc, &tmz) == 0;
+  const int np = op->kind == OPK_ST7 ? st7t_planes(op) : 1;
+  const int tma = op->kind == OPK_ST7 && f32 && !acc64 && st7t_maps(op, X, np, &tmc, &tmz) == 0;
   if (dot_out && !tma) return 1;
-  const unsigned st7t_ctas = (unsigned)(((op->nx + 31) / 32) * ((op->ny + 31) / 32) * (long)op->nz);
+  const long nparts = dot_out ? st7t_ctas(op, np) : 0;
   double* dparts = NULL;
-  if (dot_out && !(dparts = (double*)gb_workspace(ctx, sizeof(double) * 8 * (size_t)st7t_ctas * w)))
+  if (dot_out && !(dparts = (double*)gb_workspace(ctx, sizeof(double) * (size_t)nparts * w)))
     return -1;
   const long n = op->n;
   const unsigned blocks = (unsigned)((n + 255) / 256);
@@ -1023,11 +1127,14 @@ static int operator_apply(gpu_Operator* op, gpu_MultiVector* X, gpu_MultiVector*
         for (int c = 0; c < w; c++) pc.c[c] = X->active[c];
         if (tc_apply_wait_polls(ctx->opt.wait_polls, S(ctx)) != cudaSuccess)
           return gb_fail(ctx, "stencil7: cannot set the wait limit");
-        st7_tma_kernel<<<st7t_ctas, 256, 0, S(ctx)>>>(op->nx, op->ny, op->nz, op->c32[0], op->c32[1],
-                                                      op->c32[2], (float)op->shift, tmc, tmz, pc, yc,
-                                                      w, ctx->dcount + 5, dparts);
+        const int yvec = cols_aligned16(yc.col, w);
+        const int rc = np == 1 ? (dot_out ? st7t_launch<1, true>(op, tmc, tmz, pc, yc, w, yvec, dparts)
+                                          : st7t_launch<1, false>(op, tmc, tmz, pc, yc, w, yvec, NULL))
+                               : (dot_out ? st7t_launch<2, true>(op, tmc, tmz, pc, yc, w, yvec, dparts)
+                                          : st7t_launch<2, false>(op, tmc, tmz, pc, yc, w, yvec, NULL));
+        if (rc) return rc;
         if (dot_out) {
-          st7t_dot_reduce_kernel<<<w, 256, 0, S(ctx)>>>(dparts, 8L * st7t_ctas, dot_out, num, ratio);
+          st7t_dot_reduce_kernel<<<w, 256, 0, S(ctx)>>>(dparts, nparts, dot_out, num, ratio);
           gb_count_launch(1);
         }
       } else if (f32 && st7_ring_ok(op, &xc, w))
