@@ -17,7 +17,9 @@
 //                   into a shared-memory column ring (st7_ring_kernel: one
 //                   plane with cp.async copies; st7_kernel: scalar, FP64 and
 //                   the unaligned cases);
-//   st5_kernel, st27_kernel, diag_kernel;
+//   st27_tma_kernel  the same for 27 points (st27_kernel: FP64, unaligned and
+//                   small cases);
+//   st5_kernel, diag_kernel;
 // plus the inner-CG preconditioner (pcg_apply) and the parameter gradients
 // of the adjoint module (grad_*_kernel).
 #include <cuda.h>
@@ -688,6 +690,168 @@ __global__ void __launch_bounds__(256) st27_kernel(int nx, int ny, int nz, const
   }
 }
 
+// ------------------------------------------ 27-point, FP32, TMA column ring
+// The column ring of st7_tma_kernel for the 27-point stencil: one 4D tensor load a
+// column of the 40 x 6 x 4 box from (i0 - 4, j0 - 1, k0 - 1), zeros off the grid,
+// four columns a step; a thread has two cells of a z line and keeps their 52
+// weights in registers over the columns.  Same terms in the same order as
+// st27_kernel, which gathers 27 values a cell through L1 by 64-bit addresses.
+//
+// Bound by shared-memory reads (18 a cell: 74% of the pipe).  The four layers are
+// read once for both cells; three cells (15 a cell) spill, and four columns a step
+// share a wait and a barrier and interleave their dependent sums (100^3, 128
+// columns: 640 us with one column a step and 3 x 256 threads at 80 registers, 456
+// with three columns and 4 x 128 threads at 124, 412 with four).
+//   100^3, 128 columns: 412 us, st27_kernel 1759 (HBM 159, the tiles' overhang 28%);
+//   64^3, 128 columns: 97 against 489; 88 x 75 x 90, 32 columns: 71 against 266.
+static __device__ __forceinline__ int st27_di(int e) { return e == 0 ? 1 : e < 4 ? e - 2 : (e - 4) % 3 - 1; }
+static __device__ __forceinline__ int st27_dj(int e) { return e == 0 ? 0 : e < 4 ? 1 : (e - 4) / 3 - 1; }
+static __device__ __forceinline__ int st27_dk(int e) { return e < 4 ? 0 : 1; }
+#define ST27T_ROWS 4
+#define ST27T_NZ 2
+#define ST27T_MINB 4
+#define ST27T_DEPTH 2
+#define ST27T_CB 4  // columns a step
+template <int NZ>
+struct st27t_cfg {
+  static constexpr int LAYER = 40 * (ST27T_ROWS + 2);
+  static constexpr int COL = ((NZ + 2) * LAYER + 31) / 32 * 32;  // floats of a column, 128-byte steps
+  static constexpr int SLOT = ST27T_CB * COL;
+  static constexpr int BYTES = (NZ + 2) * LAYER * 4;
+  static constexpr int SMEM = ST27T_DEPTH * SLOT * 4 + 128;
+};
+
+// the copies of columns col .. min(col + ST27T_CB, w) - 1 (of those from c0 on)
+template <int NZ>
+static __device__ __forceinline__ void st27t_issue(uint32_t slot, const CUtensorMap* tm, int i0, int j0, int k0,
+                                                   const st7t_cols& XC, int c0, int col, int w, uint64_t* bar)
+{
+  using C = st27t_cfg<NZ>;
+  const uint32_t b = smem_u32(bar);
+  const int m = min(ST27T_CB, w - col);
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"((uint32_t)(m * C::BYTES))
+               : "memory");
+  for (int q = 0; q < m; q++)
+    st7t_load(slot + 4u * C::COL * q, tm, i0 - 4, j0 - 1, k0 - 1, XC.c[c0 + col + q], b);
+}
+
+template <int NZ>
+__global__ void __launch_bounds__(32 * ST27T_ROWS, ST27T_MINB)
+    st27_tma_kernel(int nx, int ny, int nz, const float* __restrict__ wt, float shift,
+                    const __grid_constant__ CUtensorMap tm, const __grid_constant__ st7t_cols XC,
+                    const __grid_constant__ blk_cols Y, int wall, int cpg, int strip, int* err)
+{
+  using C = st27t_cfg<NZ>;
+  extern __shared__ float ring_raw[];
+  float* ring = ring_raw + ((128u - (smem_u32(ring_raw) & 127u)) & 127u) / 4;
+  __shared__ __align__(8) uint64_t bar[ST27T_DEPTH];
+  __shared__ int abort_flag;
+  const int t = threadIdx.x, tx = t & 31, ty = t >> 5;
+  const int tiles_x = (nx + 31) / 32, tiles_y = (ny + ST27T_ROWS - 1) / ST27T_ROWS;
+  const unsigned b = blockIdx.x;
+  const unsigned per = (unsigned)(tiles_x * strip) * ((nz + NZ - 1) / NZ);
+  const int s0 = (int)(b / per) * strip;
+  const unsigned rest = b % per, in_strip = (unsigned)(tiles_x * min(strip, tiles_y - s0));
+  const int k0 = NZ * (int)(rest / in_strip), tile = (int)(rest % in_strip);
+  const int i0 = (tile % tiles_x) * 32, j0 = (s0 + tile / tiles_x) * ST27T_ROWS;
+  const int c0 = blockIdx.y * cpg, w = min(cpg, wall - c0);
+  if (t == 0) {
+    abort_flag = 0;
+    for (int q = 0; q < ST27T_DEPTH; q++) mbar_init(&bar[q], 1);
+  }
+  fence_proxy_async();
+  __syncthreads();
+  const uint32_t ring_s = smem_u32(ring);
+  int issued = 0, waited = 0;  // thread 0: steps issued / steps whose copies it saw land
+  const int steps = (w + ST27T_CB - 1) / ST27T_CB;
+  if (t == 0)
+    for (; issued < ST27T_DEPTH - 1 && issued < steps; issued++)
+      st27t_issue<NZ>(ring_s + 4u * C::SLOT * issued, &tm, i0, j0, k0, XC, c0, ST27T_CB * issued, w, &bar[issued]);
+
+  const int i = i0 + tx, j = j0 + ty;
+  const long n = (long)nx * ny * nz, plane = (long)nx * ny;
+  const long cell0 = (long)i + (long)nx * j + plane * k0;
+  const bool on = i < nx && j < ny;
+  float we[NZ][26], dg[NZ];
+#pragma unroll
+  for (int p = 0; p < NZ; p++) {
+    const int k = k0 + p;
+    const long c = cell0 + plane * p;
+    dg[p] = shift;
+#pragma unroll
+    for (int e = 0; e < 13; e++) {
+      // forward edge (c, c + off_e) and backward edge (c - off_e, c)
+      const int di = st27_di(e), dj = st27_dj(e), dk = st27_dk(e);
+      const long off = di + (long)nx * dj + plane * dk;
+      const bool in = on && k < nz;
+      const bool fw = in && (unsigned)(i + di) < (unsigned)nx && (unsigned)(j + dj) < (unsigned)ny && k + dk < nz;
+      const bool bw = in && (unsigned)(i - di) < (unsigned)nx && (unsigned)(j - dj) < (unsigned)ny && k - dk >= 0;
+      we[p][e] = fw ? wt[e * n + c] : 0.f;
+      we[p][13 + e] = bw ? wt[e * n + c - off] : 0.f;
+      dg[p] += we[p][e] + we[p][13 + e];
+    }
+  }
+
+  int slot = 0, ahead_slot = ST27T_DEPTH - 1;
+#pragma unroll 1
+  for (int st = 0; st < steps; st++) {
+    const uint32_t parity = (uint32_t)((st / ST27T_DEPTH) & 1);
+    const bool ok = !abort_flag && mbar_wait(&bar[slot], parity, &abort_flag);
+    if (!ok) abort_flag = 1;
+    else if (t == 0) waited = st + 1;
+    __syncthreads();  // step st landed; every thread is done with the slot of st - 1
+    const bool go = !abort_flag;
+    const int ahead = st + ST27T_DEPTH - 1;
+    if (go && t == 0 && ahead < steps) {
+      fence_proxy_async();
+      st27t_issue<NZ>(ring_s + 4u * C::SLOT * ahead_slot, &tm, i0, j0, k0, XC, c0, ST27T_CB * ahead, w,
+                      &bar[ahead_slot]);
+      issued++;
+    }
+    auto column = [&](int cb) {
+      const int col = ST27T_CB * st + cb;
+      const float* r = ring + C::SLOT * slot + C::COL * cb + C::LAYER + 40 * (ty + 1) + 4 + tx;  // cell p: + p LAYER
+      float v[NZ], x[NZ + 2][3][3];  // layers k0 - 1 .. k0 + NZ, each read once
+#pragma unroll
+      for (int l = 0; l < NZ + 2; l++)
+#pragma unroll
+        for (int a = 0; a < 3; a++)
+#pragma unroll
+          for (int q = 0; q < 3; q++) x[l][a][q] = r[(l - 1) * C::LAYER + 40 * (a - 1) + q - 1];
+#pragma unroll
+      for (int p = 0; p < NZ; p++) {
+        v[p] = dg[p] * x[p + 1][1][1];
+#pragma unroll
+        for (int e = 0; e < 26; e++) {
+          const int sg = e < 13 ? 1 : -1;
+          v[p] -= we[p][e] * x[p + 1 + sg * st27_dk(e % 13)][1 + sg * st27_dj(e % 13)][1 + sg * st27_di(e % 13)];
+        }
+      }
+      if (on) {
+        float* y = (float*)Y.col[c0 + col] + cell0;
+#pragma unroll
+        for (int p = 0; p < NZ; p++)
+          if (k0 + p < nz) __stcs(y + plane * p, go ? v[p] : __int_as_float(0x7fc00000));  // NaN: not computed
+      }
+    };
+    if (ST27T_CB * (st + 1) <= w) {
+#pragma unroll
+      for (int cb = 0; cb < ST27T_CB; cb++) column(cb);
+    } else {
+#pragma unroll 1
+      for (int cb = 0; ST27T_CB * st + cb < w; cb++) column(cb);
+    }
+    slot = slot == ST27T_DEPTH - 1 ? 0 : slot + 1;
+    ahead_slot = ahead_slot == ST27T_DEPTH - 1 ? 0 : ahead_slot + 1;
+  }
+  if (t == 0 && abort_flag) {
+    atomicExch(err, 1);
+    // copies issued but not seen landing: wait for them before the CTA exits
+    for (int c = waited; c < issued; c++)
+      mbar_drain(&bar[c % ST27T_DEPTH], (uint32_t)((c / ST27T_DEPTH) & 1));
+  }
+}
+
 // ----------------------------------------------------------- diagonal
 template <typename T, typename V>
 __global__ void diag_kernel(long n, const V* __restrict__ d, blk_cols X, blk_cols Y)
@@ -960,6 +1124,50 @@ static int st7t_maps(const gpu_Operator* op, const gpu_MultiVector* X, int np, C
   return 0;
 }
 
+// the map of st27_tma_kernel: boxes 40 x 10 x np (the conditions of st7t_maps)
+static int st27t_map(const gpu_Operator* op, const gpu_MultiVector* X, int np, CUtensorMap* m)
+{
+  PFN_cuTensorMapEncodeTiled_v12000 enc = st7t_encoder();
+  if (!enc || op->nx % 4 || ((uintptr_t)X->data & 15) || (X->ld * 4) % 16) return -1;
+  const cuuint64_t dims[4] = {(cuuint64_t)op->nx, (cuuint64_t)op->ny, (cuuint64_t)op->nz,
+                              (cuuint64_t)X->num_vectors};
+  const cuuint64_t strides[3] = {(cuuint64_t)op->nx * 4, (cuuint64_t)op->nx * op->ny * 4,
+                                 (cuuint64_t)X->ld * 4};
+  const cuuint32_t box[4] = {40, ST27T_ROWS + 2, (cuuint32_t)np, 1}, es[4] = {1, 1, 1, 1};
+  return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, X->data, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+             CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS
+             ? 0
+             : -1;
+}
+
+static long st27t_ctas(const gpu_Operator* op)
+{
+  return (long)((op->nx + 31) / 32) * ((op->ny + ST27T_ROWS - 1) / ST27T_ROWS) * ((op->nz + ST27T_NZ - 1) / ST27T_NZ);
+}
+
+// a few columns on a few CTAs: the host's tensor map and the CTAs' start take longer
+// than st27_kernel (20 x 18 x 23, 2 columns: 10.9 us against 7.5; 8 columns 8.7
+// against 11.1; 48^3, 576 CTAs, 1 column 8.7 against 9.4)
+static int st27t_pays(const gpu_Operator* op, int w)
+{
+  return w >= 6 || st27t_ctas(op) >= 2L * op->ctx->num_sms;
+}
+
+static void st27t_launch(gpu_Operator* op, const CUtensorMap& tm, const st7t_cols& pc, const blk_cols& yc, int w)
+{
+  gpu_Context* ctx = op->ctx;
+  const int tiles_x = (op->nx + 31) / 32, strip = tiles_x < ST7T_STRIP ? ST7T_STRIP / tiles_x : 1;
+  const long ctas = st27t_ctas(op);
+  long groups = (long)ST27T_MINB * ctx->num_sms / ctas;  // as st7t_launch
+  if (groups > (w + 3) / 4) groups = (w + 3) / 4;
+  if (groups < 1) groups = 1;
+  const int cpg = (int)((w + groups - 1) / groups);
+  const dim3 grid((unsigned)ctas, (unsigned)((w + cpg - 1) / cpg));
+  st27_tma_kernel<ST27T_NZ><<<grid, 32 * ST27T_ROWS, st27t_cfg<ST27T_NZ>::SMEM, S(ctx)>>>(
+      op->nx, op->ny, op->nz, op->w32, (float)op->shift, tm, pc, yc, w, cpg, strip, ctx->dcount + 5);
+}
+
 static int pcg_apply(gpu_Operator* op, gpu_MultiVector* X, gpu_MultiVector* Y);
 
 static long st7t_ctas(const gpu_Operator* op, int np)
@@ -1159,7 +1367,13 @@ static int operator_apply(gpu_Operator* op, gpu_MultiVector* X, gpu_MultiVector*
                                                        op->shift, xc, yc, w);
       break;
     case OPK_ST27:
-      if (f32)
+      if (f32 && st27t_pays(op, w) && st27t_map(op, X, ST27T_NZ + 2, &tmc) == 0) {
+        st7t_cols pc;
+        for (int c = 0; c < w; c++) pc.c[c] = X->active[c];
+        if (tc_apply_wait_polls(ctx->opt.wait_polls, S(ctx)) != cudaSuccess)
+          return gb_fail(ctx, "stencil27: cannot set the wait limit");
+        st27t_launch(op, tmc, pc, yc, w);
+      } else if (f32)
         st27_kernel<float><<<blocks, 256, 0, S(ctx)>>>(op->nx, op->ny, op->nz, op->w32,
                                                        (float)op->shift, xc, yc, w);
       else
