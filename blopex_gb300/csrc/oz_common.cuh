@@ -69,13 +69,6 @@ static __device__ __forceinline__ int oz_bexp64(double v)
 {
   return (int)((__double_as_longlong(v) >> 52) & 0x7FF);
 }
-// the same scale for an FP32 value, on the FP64 exponent scale
-static __device__ __forceinline__ int oz_bexp32(float v)
-{
-  const int e = (int)((__float_as_uint(v) >> 23) & 0xFF);
-  return e ? e + 896 : 0;
-}
-
 // |v| in fixed point with F fractional bits relative to 2^(E - 1022), E the
 // group's largest biased exponent: U = round(|v| 2^(F - (E - 1022))),
 // 0 <= U <= 2^F.  F <= 52.
@@ -276,16 +269,7 @@ static __device__ __forceinline__ void oz_digits4x8_hl(float h, float l, float (
   d[3] = (fmaf(d[2], -256.0f, l) + OZ_RINT_MAGIC) - OZ_RINT_MAGIC;
 }
 
-// FP32 value; scale = 2^(32 - (E - 1022)) as a float
-static __device__ __forceinline__ void oz_digits4x8_f32(float v, float scale, float (&d)[4])
-{
-  const float u = v * scale;
-  const float h = fmaf(u, 0.0000152587890625f, OZ_RINT_MAGIC) - OZ_RINT_MAGIC;  // 2^-16
-  const float l = fmaf(h, -65536.0f, u);
-  oz_digits4x8_hl(h, l, d);
-}
-
-// the scale of oz_digits4x8_f32 for a group exponent E, 0 when E is outside
+// the scale 2^(32 - (E - 1022)) of an FP32 group as a float, 0 when E is outside
 // the range the float can hold (the caller then takes the integer path)
 static __device__ __forceinline__ float oz_scale4x8(int E)
 {
@@ -302,14 +286,89 @@ static __device__ __forceinline__ void oz_digits4x8_u(uint64_t U, uint32_t sg, f
   oz_digits4x8_hl(h, l, d);
 }
 
-// FP64 value: the 32-bit fixed point integer from its bits, then as above
-static __device__ __forceinline__ void oz_digits4x8_f64(double v, int E, float (&d)[4])
-{
-  oz_digits4x8_u(oz_fixed64<32>(v, E), (uint32_t)((uint64_t)__double_as_longlong(v) >> 63) << 31, d);
-}
-
 // two digits (floats holding integers) as one word of two bf16 patterns
 static __device__ __forceinline__ uint32_t oz_pack_bf16(float lo, float hi)
 {
   return __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632);
+}
+
+// ------------------------------------------------ two FP32 values a register pair
+// Blackwell's packed FP32 arithmetic: the same roundings as one value at a time in
+// half the issue slots.
+typedef unsigned long long f32x2;
+static __device__ __forceinline__ f32x2 f2_pack(float lo, float hi)
+{
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+static __device__ __forceinline__ void f2_unpack(f32x2 v, float& lo, float& hi)
+{
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+static __device__ __forceinline__ f32x2 f2_add(f32x2 a, f32x2 b)
+{
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+static __device__ __forceinline__ f32x2 f2_mul(f32x2 a, f32x2 b)
+{
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+static __device__ __forceinline__ f32x2 f2_fma(f32x2 a, f32x2 b, f32x2 c)
+{
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+// the digits of two rows, from the halves, an FP32 value and an FP64 value
+static __device__ __forceinline__ void oz_digits4x8_hlx2(f32x2 h, f32x2 l, f32x2 (&d)[4])
+{
+  const f32x2 s = f2_pack(0.00390625f, 0.00390625f), m256 = f2_pack(-256.f, -256.f);
+  const f32x2 M = f2_pack(OZ_RINT_MAGIC, OZ_RINT_MAGIC), mM = f2_pack(-OZ_RINT_MAGIC, -OZ_RINT_MAGIC);
+  d[0] = f2_add(f2_fma(h, s, M), mM);
+  d[1] = f2_fma(d[0], m256, h);
+  d[2] = f2_add(f2_fma(l, s, M), mM);
+  d[3] = f2_add(f2_add(f2_fma(d[2], m256, l), M), mM);
+}
+static __device__ __forceinline__ void oz_digits4x8_f32x2(f32x2 v, f32x2 scale, f32x2 (&d)[4])
+{
+  const f32x2 s = f2_pack(0.0000152587890625f, 0.0000152587890625f), m = f2_pack(-65536.f, -65536.f);
+  const f32x2 M = f2_pack(OZ_RINT_MAGIC, OZ_RINT_MAGIC), mM = f2_pack(-OZ_RINT_MAGIC, -OZ_RINT_MAGIC);
+  const f32x2 u = f2_mul(v, scale);
+  const f32x2 h = f2_add(f2_fma(u, s, M), mM);
+  oz_digits4x8_hlx2(h, f2_fma(h, m, u), d);
+}
+
+// the 16-bit halves of oz_fixed64<32>(v, E) as floats 2^23 above, for E >= 64: with
+// T.R the 53-bit mantissa at the top of 64 bits and d = E - (v's exponent), U is
+// T >> d plus the bit below (0 for d > 32, zeros and subnormals among them)
+static __device__ __forceinline__ void oz_halves32(uint32_t lo, uint32_t hi, int E, float& h, float& l)
+{
+  const int d = E - (int)((hi >> 20) & 0x7FF);
+  const bool in = d <= 32;
+  const uint32_t T = in ? __funnelshift_l(lo, hi, 11) | 0x80000000u : 0u;
+  const uint32_t R = in ? lo << 11 : 0u;
+  const uint32_t U = __funnelshift_rc(T, 0u, (uint32_t)d), below = __funnelshift_rc(R, T, (uint32_t)d);
+  const uint32_t l17 = (U & 0xFFFFu) + (below >> 31);
+  h = __uint_as_float(0x4B000000u + (U >> 16) + (l17 >> 16));
+  l = __uint_as_float(0x4B000000u | (l17 & 0xFFFFu));
+}
+// two FP64 rows (their four words)
+static __device__ __forceinline__ void oz_digits4x8_f64x2(uint4 v, int E, f32x2 (&d)[4])
+{
+  const f32x2 b = f2_pack(-8388608.f, -8388608.f);
+  float h0, l0, h1, l1;
+  oz_halves32(v.x, v.y, E, h0, l0);
+  oz_halves32(v.z, v.w, E, h1, l1);
+  const f32x2 sg = ((f32x2)(v.w & 0x80000000u) << 32) | (v.y & 0x80000000u);
+  oz_digits4x8_hlx2(f2_add(f2_pack(h0, h1), b) ^ sg, f2_add(f2_pack(l0, l1), b) ^ sg, d);
+}
+static __device__ __forceinline__ uint32_t oz_pack_bf16x2(f32x2 d)
+{
+  return __byte_perm((uint32_t)d, (uint32_t)(d >> 32), 0x7632);
 }

@@ -18,22 +18,33 @@
 // bias; each CTA writes its sums in FP64 and a second kernel adds the CTAs
 // in a fixed order.
 //
-// Tile b of the grid pairs L with Q_b: the A operand has 128 rows, L's
-// columns in rows 0-63 and Q_b's in rows 64-127; the B operand is rows 0-63
-// of the same slices (L).  Per CTA (one per SM):
-//   warp 1          copies a chunk's columns into one of two raw buffers:
+// Tile b of the grid pairs L with Q_b: the A operand has 128 rows, L's and
+// Q_b's columns in alternating groups of eight; the B operand is every other
+// group (L) of one or more slices.  Per CTA (one per SM):
+//   warp 1          copies a chunk's columns into one of two to four raw buffers:
 //                   a run of equally spaced columns (a block's columns at
 //                   its leading dimension) as one 2-D TMA tile, other
 //                   columns one cp.async.bulk each (the per-request cost of
 //                   128 column copies per chunk otherwise bounds the kernel);
-//   warps 2-3, 12-15 find each column's chunk scale and write the digit
-//                   slices (128-byte-swizzled K-major, K = the chunk's rows);
+//   warps 2, 3, 12  find each column's chunk scale;
+//   warps 13-19     write the digit slices (128-byte-swizzled K-major, K = the
+//                   chunk's rows), half the rows at a time;
 //   warp 0          allocates TMEM; one thread issues tcgen05.mma.kind::f16
-//                   (M = 128, N = 64, K = 16) for the pairs t + u < S into one
-//                   of two accumulator sets;
+//                   (M = 128, K = 16): digit t of every column with digits
+//                   0 .. S - 1 - t of L stacked (N = 64 (S - t)) onto levels
+//                   t .. S - 1 of one of two accumulator sets;
 //   warps 4-11      fold a finished chunk into the double-float sums (lane =
 //                   column of [L Q_b]; warps w and w + 4 share TMEM lanes and
 //                   take 32 of the 64 L columns each).
+// Bound by the instructions that cut the digits (integer and FP32 pipes; 20 warps
+// of 96 registers cover each other's latencies to half the issue rate).  Measured,
+// 2 M rows, 64 FP64 + 33 + 33 FP32 columns (HBM 240 us): 2240 us with 64-bit
+// shifts and one value at a time, six warps for scales and digits, a barrier
+// between them, and one MMA a digit pair (40 of N = 64, bound by the shared-memory
+// reads of A: 87 cycles each); 1850 with packed FP32 arithmetic and 32-bit funnel
+// shifts; 1580 with ten warps and 96 registers; 1520 with stacked MMAs (16 a chunk);
+// 1480 with the scales on warps of their own and three raw buffers.  Folding on the
+// digit warps (2160) thrashes the instruction cache.
 // Every wait is bounded; a timeout sets an error word, the outputs become NaN.
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -47,17 +58,21 @@
 
 #define OZG_S 4
 #define OZG_F (8 * OZG_S)                // 8-bit digits (oz_digits4x8_*)
-#define OZG_THREADS 512
-#define OZG_NPROD 192
+#define OZG_THREADS 640
+#define OZG_NSCALE 96   // threads that find the scales
+#define OZG_NPROD 224   // threads that write the digits
+#define OZG_CSLOTS 8    // chunks whose scales are kept
 #define OZG_ROWS 64                      // rows per chunk
 // a staged column: 64 rows and 16 bytes more, so that consecutive columns
 // start 16 bytes apart modulo 128 (different shared-memory bank groups); a
 // TMA tile of 66 FP64 / 68 FP32 rows lands its columns at exactly this stride
 #define OZG_STRIDE64 528
 #define OZG_STRIDE32 272
-#define OZG_RAW 69632                    // one raw buffer: 128 columns + run alignment
+#define OZG_RAW 69632                    // most of one raw buffer: 128 columns + run alignment
+#define OZG_RAWS 153600                  // of all of them: 3 of 64 FP64 and 64 FP32 columns
+#define OZG_MAXSLOTS 4
 #define OZG_SLICE 16384                  // 128 operand rows x 128 bytes
-#define OZG_SMEM (2 * OZG_RAW + OZG_S * OZG_SLICE + 1024)
+#define OZG_SMEM (OZG_RAWS + OZG_S * OZG_SLICE + 1024)
 #define OZG_MAXQ 4  // 64 + 64 * OZG_MAXQ column slots fit blk_cols
 #define OZG_MAXMAPS 12
 
@@ -73,6 +88,7 @@ struct ozg_params {
   unsigned short roff[OZG_MAXQ][128];   // raw-buffer offset of each slot, 16-byte units
   unsigned char by_map[OZG_MAXQ][128];  // 1: the slot arrives with a map's tile
   long n;
+  int raw, nslots;  // bytes and number of the raw buffers
   double* partial;  // [tile][cta][128][64]
   int* err;
 };
@@ -81,8 +97,8 @@ struct ozg_params {
 // digit slices behind them 1024-byte aligned (the MMA descriptors' swizzle
 // atom); dynamic plus static shared memory within the 227 KB of a CTA
 static_assert(sizeof(ozg_params) <= 32764, "oz_gram parameters exceed the kernel parameter space");
-static_assert(OZG_RAW % 1024 == 0, "raw buffers must keep the digit slices 1024-byte aligned");
-static_assert(OZG_SMEM + 8192 <= 232448, "oz_gram shared memory exceeds a CTA's 227 KB");
+static_assert(OZG_RAW % 1024 == 0 && 2 * OZG_RAW <= OZG_RAWS && OZG_MAXSLOTS + 3 < OZG_CSLOTS + 1, "raw buffers must keep the digit slices 1024-byte aligned");
+static_assert(OZG_SMEM + 12288 <= 232448, "oz_gram shared memory exceeds a CTA's 227 KB");
 
 // rows x columns tile of a column run: x = first row, the run's columns all
 static __device__ __forceinline__ void ozg_tile_load(uint32_t dst, const CUtensorMap* map, int x, uint64_t* bar)
@@ -110,15 +126,6 @@ static __device__ __forceinline__ int ozg_col_kind(const ozg_params& prm, int b,
 
 // eight consecutive values of a staged column (16-byte aligned) with 16-byte
 // shared-memory loads
-static __device__ __forceinline__ void ozg_load8(const unsigned char* src, double (&v)[8])
-{
-#pragma unroll
-  for (int x = 0; x < 4; x++) {
-    const double2 d = ((const double2*)src)[x];
-    v[2 * x] = d.x;
-    v[2 * x + 1] = d.y;
-  }
-}
 static __device__ __forceinline__ void ozg_load8(const unsigned char* src, float (&v)[8])
 {
   const float4 a = ((const float4*)src)[0], b = ((const float4*)src)[1];
@@ -129,9 +136,10 @@ __global__ void __launch_bounds__(OZG_THREADS, 1) oz_gram_kernel(const __grid_co
 {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = smem_align1024(smem_raw);
-  unsigned char* raws = smem;                  // [2][OZG_RAW]: columns at s_off
-  unsigned char* adig = smem + 2 * OZG_RAW;    // [S][128 rows][128 B]
-  __shared__ uint64_t raw_full[2], raw_empty[2], a_full, a_empty, acc_full[2], acc_empty[2], done_bar;
+  unsigned char* raws = smem;                  // [nslots][raw]: columns at s_off
+  unsigned char* adig = smem + prm.nslots * prm.raw;    // [S][128 rows][128 B]
+  // a_full, a_empty: the digits of rows 0-31 and 32-63
+  __shared__ uint64_t raw_full[OZG_MAXSLOTS], raw_empty[OZG_MAXSLOTS], scale_full[OZG_MAXSLOTS], a_full[2], a_empty[2], acc_full[2], acc_empty[2], done_bar;
   __shared__ uint32_t tmem_base;
   __shared__ int abort_flag;
   // this tile's column pointers and kinds (0 absent, 1 FP32, 2 FP64) in shared
@@ -140,7 +148,10 @@ __global__ void __launch_bounds__(OZG_THREADS, 1) oz_gram_kernel(const __grid_co
   __shared__ int s_kind[128];
   __shared__ int s_off[128];   // raw-buffer offset of each column
   __shared__ int s_copy[128];  // the column's own bulk copy: 0 none, 1 FP32, 2 FP64
-  __shared__ int cexp[4][128];     // chunk scales, by chunk modulo 4
+  __shared__ int cexp[OZG_CSLOTS][128];  // chunk scales, by chunk
+  // 2^(E - 1022 - 8), the scale of a column's digit sums (they carry 2^-8), 0 where
+  // FP32 cannot hold the products
+  __shared__ __align__(16) float cscale[OZG_CSLOTS][128];
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int b = blockIdx.y;
@@ -155,16 +166,25 @@ __global__ void __launch_bounds__(OZG_THREADS, 1) oz_gram_kernel(const __grid_co
     s_off[tid] = 16 * (int)prm.roff[b][tid];
     s_copy[tid] = prm.by_map[b][tid] ? 0 : kind;
   }
+  // absent columns: digits and scales of zero throughout
+  for (int e = tid; e < OZG_S * OZG_SLICE / 16; e += OZG_THREADS) ((uint4*)adig)[e] = make_uint4(0, 0, 0, 0);
+  for (int e = tid; e < OZG_CSLOTS * 128; e += OZG_THREADS) {
+    (&cexp[0][0])[e] = 0;
+    (&cscale[0][0])[e] = 0.f;
+  }
   if (tid == 0) {
     abort_flag = 0;
-    for (int s = 0; s < 2; s++) {
+    for (int s = 0; s < OZG_MAXSLOTS; s++) {
       mbar_init(&raw_full[s], 1);
       mbar_init(&raw_empty[s], OZG_NPROD);
+      mbar_init(&scale_full[s], OZG_NSCALE);
+    }
+    for (int s = 0; s < 2; s++) {
+      mbar_init(&a_full[s], OZG_NPROD);
+      mbar_init(&a_empty[s], 1);
       mbar_init(&acc_full[s], 1);
       mbar_init(&acc_empty[s], 256);
     }
-    mbar_init(&a_full, OZG_NPROD);
-    mbar_init(&a_empty, 1);
     mbar_init(&done_bar, 1);
   }
   if (warp == 0) {
@@ -180,9 +200,13 @@ __global__ void __launch_bounds__(OZG_THREADS, 1) oz_gram_kernel(const __grid_co
   tc_fence_after();
   const uint32_t tmem = tmem_base;
 
+  // groups of eight columns, L's first (s_col[64 ..]: Q_b's)
+  const int nl = (prm.h + 7) / 8, groups = nl + ((b < prm.nq ? prm.qw[b] : 0) + 7) / 8;
+  auto group_of = [&](int v) { return v < nl ? v : 8 + v - nl; };
+
   if (warp == 1) {
     // ------------------------------------------------------- bulk copies
-    long issued[2] = {0, 0};  // chunks issued per slot
+    long issued = 0;           // chunks
     int ncol8 = 0, ncol4 = 0;  // FP64 and FP32 columns copied one by one
     for (int j = 0; j < 128; j++) {
       ncol8 += s_copy[j] == 2;
@@ -191,11 +215,12 @@ __global__ void __launch_bounds__(OZG_THREADS, 1) oz_gram_kernel(const __grid_co
     uint32_t mapbytes = 0;  // the tiles of this CTA's runs
     for (int m = 0; m < prm.nmaps; m++)
       if (prm.map_tile[m] < 0 || prm.map_tile[m] == b) mapbytes += (uint32_t)prm.map_bytes[m];
+    int slot = 0;
+    uint32_t par = 0;
     for (long c = 0; c < my_chunks; c++) {
-      const int slot = (int)(c & 1);
       int stop = 0;
       if (lane == 0) {
-        if (c >= 2 && !mbar_wait(&raw_empty[slot], (uint32_t)(((c >> 1) - 1) & 1), &abort_flag)) {
+        if (c >= prm.nslots && !mbar_wait(&raw_empty[slot], par ^ 1u, &abort_flag)) {
           abort_flag = 1;
           atomicExch(prm.err, 21);
         }
@@ -210,7 +235,7 @@ __global__ void __launch_bounds__(OZG_THREADS, 1) oz_gram_kernel(const __grid_co
       const uint32_t total = mapbytes + (uint32_t)ncol8 * b8 + (uint32_t)ncol4 * b4;
       if (lane == 0) mbar_expect_tx(&raw_full[slot], total);
       __syncwarp();
-      unsigned char* raw = raws + slot * OZG_RAW;
+      unsigned char* raw = raws + slot * prm.raw;
       for (int m = lane; m < prm.nmaps; m += 32)
         if (prm.map_tile[m] < 0 || prm.map_tile[m] == b)
           ozg_tile_load(smem_u32(raw + s_off[prm.map_slot[m]]), &prm.maps[m], (int)r0, &raw_full[slot]);
@@ -222,165 +247,227 @@ __global__ void __launch_bounds__(OZG_THREADS, 1) oz_gram_kernel(const __grid_co
         else if (kind == 1)
           bulk_g2s(raw + s_off[j], (const float*)ptr + r0, b4, &raw_full[slot]);
       }
-      issued[slot] = c + 1;
+      issued = c + 1;
+      if (++slot == prm.nslots) {
+        slot = 0;
+        par ^= 1u;
+      }
     }
     // no copy may still be landing when the CTA exits
-    for (int s = 0; s < 2; s++)
-      if (issued[s] > 0) mbar_drain(&raw_full[s], (uint32_t)(((issued[s] - 1) >> 1) & 1));
-  } else if (warp == 2 || warp == 3 || warp >= 12) {
-    // ------------------------------------------------------- digit slices
-    // (every producer runs every iteration: the named barrier below must be
-    // reached by all of them; an abort only skips the work)
-    const int p = (warp < 4 ? warp - 2 : warp - 10) * 32 + lane;
+    for (long c = max(0L, issued - prm.nslots); c < issued; c++)
+      mbar_drain(&raw_full[c % prm.nslots], (uint32_t)((c / prm.nslots) & 1));
+  } else if (warp == 2 || warp == 3 || warp == 12) {
+    // ------------------------------------------------------- chunk scales
+    const int pw = warp < 4 ? warp - 2 : 2;
+    int slot = 0;
+    uint32_t par = 0;
     for (long c = 0; c < my_chunks; c++) {
-      const int slot = (int)(c & 1);
-      if (!abort_flag && !mbar_wait(&raw_full[slot], (uint32_t)((c >> 1) & 1), &abort_flag)) {
+      const bool got = mbar_wait(&raw_full[slot], par, &abort_flag);
+      if (!__all_sync(0xffffffffu, got)) {  // the shuffles below need the whole warp
         abort_flag = 1;
         atomicExch(prm.err, 22);
+        break;
       }
       const long r0 = (blockIdx.x + c * gridDim.x) * OZG_ROWS;
       const int rows = (int)min((long)OZG_ROWS, prm.n - r0);
-      const unsigned char* raw = raws + slot * OZG_RAW;
-      // pass 1: each column's largest exponent over the chunk.  The eight
+      const unsigned char* raw = raws + slot * prm.raw;
+      // each column's largest exponent over the chunk.  The eight
       // 8-row groups of column j sit in eight consecutive lanes (every lane
       // of a warp runs the same number of iterations), which combine theirs
       // by shuffles.  Only the maximum matters here, so the lanes read their
       // 16-byte pieces in rotated orders: the eight lanes of a column then
       // touch eight different bank groups.
-      for (int u = p; u < 1024; u += OZG_NPROD) {
-        const int j = u >> 3, q = u & 7;
-        const int kind = abort_flag ? 0 : s_kind[j];
+#pragma unroll 2
+      for (int v = pw; v < 2 * groups; v += OZG_NSCALE / 32) {
+        const int j = 8 * group_of(v >> 1) + 4 * (v & 1) + (lane >> 3), q = lane & 7;
+        const int kind = s_kind[j];
         const int nr = min(8, rows - 8 * q);
         int e = 0;
         if (kind == 2) {
           const unsigned char* src = raw + s_off[j] + 64 * q;
+          uint32_t a[8];  // the high words without their signs
 #pragma unroll
           for (int x = 0; x < 4; x++) {
             const int xx = (x + (q >> 1)) & 3;  // rows 2 xx, 2 xx + 1
-            const double2 d = *(const double2*)(src + 16 * xx);
-            if (2 * xx < nr) e = max(e, oz_bexp64(d.x));
-            if (2 * xx + 1 < nr) e = max(e, oz_bexp64(d.y));
+            const uint4 d = *(const uint4*)(src + 16 * xx);
+            a[2 * x] = 2 * xx < nr ? d.y & 0x7FFFFFFFu : 0u;
+            a[2 * x + 1] = 2 * xx + 1 < nr ? d.w & 0x7FFFFFFFu : 0u;
           }
+          const uint32_t m = max(max(max(a[0], a[1]), max(a[2], a[3])), max(max(a[4], a[5]), max(a[6], a[7])));
+          e = (int)(m >> 20);
         } else if (kind == 1) {
           const unsigned char* src = raw + s_off[j] + 32 * q;
+          uint32_t m = 0;
 #pragma unroll
           for (int x = 0; x < 2; x++) {
             const int hx = x ^ ((q >> 2) & 1);  // rows 4 hx .. 4 hx + 3
-            const float4 f = *(const float4*)(src + 16 * hx);
-            if (4 * hx < nr) e = max(e, oz_bexp32(f.x));
-            if (4 * hx + 1 < nr) e = max(e, oz_bexp32(f.y));
-            if (4 * hx + 2 < nr) e = max(e, oz_bexp32(f.z));
-            if (4 * hx + 3 < nr) e = max(e, oz_bexp32(f.w));
+            const uint4 f = *(const uint4*)(src + 16 * hx);
+            m = max(m, 4 * hx < nr ? f.x & 0x7FFFFFFFu : 0u);
+            m = max(m, 4 * hx + 1 < nr ? f.y & 0x7FFFFFFFu : 0u);
+            m = max(m, 4 * hx + 2 < nr ? f.z & 0x7FFFFFFFu : 0u);
+            m = max(m, 4 * hx + 3 < nr ? f.w & 0x7FFFFFFFu : 0u);
           }
+          e = (int)(m >> 23);
+          e = e ? e + 896 : 0;
         }
         e = max(e, __shfl_xor_sync(0xffffffffu, e, 1));
         e = max(e, __shfl_xor_sync(0xffffffffu, e, 2));
         e = max(e, __shfl_xor_sync(0xffffffffu, e, 4));
-        // the chunk scale (absent columns: 0).  Slot c mod 4 was last read by
-        // the epilogue of chunk c - 4, which finished before the MMAs of
-        // chunk c - 2 started (their accumulator buffer), and those completed
-        // before the previous chunk's pass 2 (its a_empty wait)
-        if (q == 0) cexp[c & 3][j] = e;
+        // the chunk scale (absent columns: 0).  Its slot was last read when chunk
+        // c - 8 was folded; chunk c was copied after the digits of chunk c - nslots
+        // had been written, hence the MMAs of the chunk before it been done and the
+        // chunk two before that been folded: c - nslots - 3 >= c - 8
+        if (q == 0) {
+          cexp[c % OZG_CSLOTS][j] = e;
+          cscale[c % OZG_CSLOTS][j] = (e >= 904 && e <= 1157) ? __uint_as_float((uint32_t)(e - 1030 + 127) << 23) : 0.f;
+        }
       }
-      named_bar(1, OZG_NPROD);
-      // the digit slices are free once the previous chunk's MMAs completed
-      if (c >= 1 && !abort_flag && !mbar_wait(&a_empty, (uint32_t)((c - 1) & 1), &abort_flag)) {
+      mbar_arrive(&scale_full[slot]);
+      if (++slot == prm.nslots) {
+        slot = 0;
+        par ^= 1u;
+      }
+    }
+  } else if (warp > 12) {
+    // ------------------------------------------------------- digit slices
+    // the warps take the units of all chunks in turn
+    int v = warp - 13;
+    int slot = 0;
+    uint32_t par = 0;
+    for (long c = 0; c < my_chunks && !abort_flag; c++, v -= 2 * groups) {
+      if (!mbar_wait(&raw_full[slot], par, &abort_flag) || !mbar_wait(&scale_full[slot], par, &abort_flag)) {
         abort_flag = 1;
-        atomicExch(prm.err, 23);
+        atomicExch(prm.err, 27);
       }
-      if (!abort_flag) {
+      const long r0 = (blockIdx.x + c * gridDim.x) * OZG_ROWS;
+      const int rows = (int)min((long)OZG_ROWS, prm.n - r0);
+      const unsigned char* raw = raws + slot * prm.raw;
+      // (column j, rows 8q .. 8q + 7), half the rows at a time: one half's MMAs run
+      // while the other is written.  Eight consecutive lanes take eight consecutive
+      // columns at the same q: the raw column stride (528 or 272, 16 mod 128) and
+      // the slices' swizzle then put their 16-byte loads and stores in eight
+      // different bank groups.
+#pragma unroll 1
+      for (int hf = 0; hf < 2; hf++) {
+        // this half of the slices is free once the previous chunk's MMAs on it completed
+        if (c >= 1 && !abort_flag && !mbar_wait(&a_empty[hf], (uint32_t)((c - 1) & 1), &abort_flag)) {
+          abort_flag = 1;
+          atomicExch(prm.err, 23);
+        }
+        if (abort_flag) break;
         tc_fence_after();
-        // pass 2: the digits of (column j, rows 8q .. 8q + 7).  Eight
-        // consecutive lanes take eight consecutive columns at the same q:
-        // the raw column stride (528 or 272, 16 mod 128) and the slices' swizzle
-        // then put their 16-byte loads and stores in eight different bank
-        // groups.
-        for (int u = p; u < 1024; u += OZG_NPROD) {
-          const int j = (u & 7) | ((u >> 6) << 3), q = (u >> 3) & 7;
-          const int E = cexp[c & 3][j];
+#pragma unroll 1
+        for (; v < (hf + 1) * groups; v += OZG_NPROD / 32) {
+          const int j = 8 * group_of(v - hf * groups) + (lane & 7), q = 4 * hf + (lane >> 3);
+          const int E = cexp[c % OZG_CSLOTS][j];
           const int kind = s_kind[j];
-          // the eight rows' digits with FP32 arithmetic (integer fixed point
-          // first for FP64 values, or for FP32 groups whose scale leaves the
-          // float range)
-          float dg[8][OZG_S];
+          if (kind == 0) continue;
+          // the eight rows' digits with FP32 arithmetic, two rows at a time
+          // (integer fixed point first for FP64 values, or for FP32 groups
+          // whose scale leaves the float range)
+          uint32_t pk[OZG_S][4];
           const float sc = oz_scale4x8(E);
           const int nr = min(8, rows - 8 * q);
           if (kind == 1) {
             float v[8];
             ozg_load8(raw + s_off[j] + 32 * q, v);
+            if (nr < 8) {
 #pragma unroll
-            for (int x = 0; x < 8; x++) v[x] = x < nr ? v[x] : 0.0f;
+              for (int x = 0; x < 8; x++) v[x] = x < nr ? v[x] : 0.0f;
+            }
             if (sc != 0.0f) {
 #pragma unroll
-              for (int x = 0; x < 8; x++) oz_digits4x8_f32(v[x], sc, dg[x]);
+              for (int k = 0; k < 4; k++) {
+                f32x2 dg[OZG_S];
+                oz_digits4x8_f32x2(f2_pack(v[2 * k], v[2 * k + 1]), f2_pack(sc, sc), dg);
+#pragma unroll
+                for (int t = 0; t < OZG_S; t++) pk[t][k] = oz_pack_bf16x2(dg[t]);
+              }
             } else {
 #pragma unroll
-              for (int x = 0; x < 8; x++)
-                oz_digits4x8_u(oz_fixed32<OZG_F>(v[x], E), __float_as_uint(v[x]) & 0x80000000u, dg[x]);
+              for (int k = 0; k < 4; k++) {
+                float d0[OZG_S], d1[OZG_S];
+                oz_digits4x8_u(oz_fixed32<OZG_F>(v[2 * k], E), __float_as_uint(v[2 * k]) & 0x80000000u, d0);
+                oz_digits4x8_u(oz_fixed32<OZG_F>(v[2 * k + 1], E), __float_as_uint(v[2 * k + 1]) & 0x80000000u, d1);
+#pragma unroll
+                for (int t = 0; t < OZG_S; t++) pk[t][k] = oz_pack_bf16(d0[t], d1[t]);
+              }
             }
-          } else if (kind == 2) {
-            double v[8];
-            ozg_load8(raw + s_off[j] + 64 * q, v);
-#pragma unroll
-            for (int x = 0; x < 8; x++) oz_digits4x8_f64(x < nr ? v[x] : 0.0, E, dg[x]);
           } else {
+            const uint4* src = (const uint4*)(raw + s_off[j] + 64 * q);
+            // (scales below 904 enter the sums with a factor of 0)
+            const int Ed = max(E, 64);
 #pragma unroll
-            for (int x = 0; x < 8; x++)
+            for (int k = 0; k < 4; k++) {
+              uint4 d = src[k];
+              if (2 * k >= nr) d.x = d.y = 0u;
+              if (2 * k + 1 >= nr) d.z = d.w = 0u;
+              f32x2 dg[OZG_S];
+              oz_digits4x8_f64x2(d, Ed, dg);
 #pragma unroll
-              for (int t = 0; t < OZG_S; t++) dg[x][t] = 0.0f;
+              for (int t = 0; t < OZG_S; t++) pk[t][k] = oz_pack_bf16x2(dg[t]);
+            }
           }
-          uint32_t pk[OZG_S][4];
-#pragma unroll
-          for (int t = 0; t < OZG_S; t++)
-#pragma unroll
-            for (int k = 0; k < 4; k++) pk[t][k] = oz_pack_bf16(dg[2 * k][t], dg[2 * k + 1][t]);
-          const uint32_t off = (uint32_t)j * 128u + ((uint32_t)(q ^ (j & 7)) << 4);
+          // groups of eight rows: L's even, Q's odd
+          const uint32_t off = (uint32_t)(2 * ((j & 63) >> 3) + (j >> 6)) * 1024u + (uint32_t)(j & 7) * 128u +
+                               ((uint32_t)(q ^ (j & 7)) << 4);
 #pragma unroll
           for (int t = 0; t < OZG_S; t++)
             *(uint4*)(adig + t * OZG_SLICE + off) = make_uint4(pk[t][0], pk[t][1], pk[t][2], pk[t][3]);
         }
         fence_proxy_async();
-        mbar_arrive(&a_full);
-        mbar_arrive(&raw_empty[slot]);
+        mbar_arrive(&a_full[hf]);
+        if (hf == 1) mbar_arrive(&raw_empty[slot]);
       }
-      // no barrier here: the next chunk's pass 1 writes another scale slot
-      // and reads the other raw buffer
+      if (++slot == prm.nslots) {
+        slot = 0;
+        par ^= 1u;
+      }
     }
   } else if (warp == 0 && lane == 0) {
     // ------------------------------------------------------- MMA issuer
-    const uint32_t idesc = bf16_idesc(128, 64);
-    const uint32_t abase = smem_u32(adig);
+    // A: 16 groups of eight rows 1024 bytes apart; B: every other of them (L's), on
+    // through the slices (the address fields do not carry)
+    const uint64_t adesc = sw128_desc(smem_u32(adig)), bdesc = adesc + ((uint64_t)(1024 >> 4) << 32);
     for (long c = 0; c < my_chunks && !abort_flag; c++) {
       const int buf = (int)(c & 1);
-      if (!mbar_wait(&a_full, (uint32_t)(c & 1), &abort_flag)) {
-        abort_flag = 1;
-        atomicExch(prm.err, 24);
-        break;
-      }
       if (c >= 2 && !mbar_wait(&acc_empty[buf], (uint32_t)(((c >> 1) - 1) & 1), &abort_flag)) {
         abort_flag = 1;
         atomicExch(prm.err, 25);
         break;
       }
-      tc_fence_after();
-      for (int t = 0; t < OZG_S; t++)
-        for (int u = 0; u + t < OZG_S; u++) {
-          const uint32_t d = tmem + (uint32_t)(buf * 256 + (t + u) * 64);
-          for (int ks = 0; ks < 4; ks++)
-            mma_bf16(d, sw128_desc(abase + t * OZG_SLICE + ks * 32), sw128_desc(abase + u * OZG_SLICE + ks * 32),
-                     idesc, (t > 0 || ks > 0) ? 1u : 0u);
+      const uint32_t d = tmem + (uint32_t)(buf * 256);
+#pragma unroll
+      for (int hf = 0; hf < 2; hf++) {
+        if (abort_flag || !mbar_wait(&a_full[hf], (uint32_t)(c & 1), &abort_flag)) {
+          abort_flag = 1;
+          atomicExch(prm.err, 24);
+          break;
         }
-      mma_commit(&a_empty);
+        tc_fence_after();
+        // digit t of every column with digits 0 .. S - 1 - t of L at once: the levels
+        // t .. S - 1 of the sums
+#pragma unroll
+        for (int t = 0; t < OZG_S; t++)
+#pragma unroll
+          for (int ks = 2 * hf; ks < 2 * hf + 2; ks++)
+            mma_bf16(d + t * 64, adesc + ((t * OZG_SLICE + ks * 32) >> 4), bdesc + ((ks * 32) >> 4),
+                     bf16_idesc(128, 64 * (OZG_S - t)), (t > 0 || ks > 0) ? 1u : 0u);
+        mma_commit(&a_empty[hf]);
+      }
+      if (abort_flag) break;
       mma_commit(&acc_full[buf]);
     }
     mma_commit(&done_bar);
   } else if (warp >= 4 && warp < 12) {
     // ------------------------------------------------------- epilogue
     const int quarter = warp & 3, ihalf = (warp - 4) >> 2;
-    const int j = 32 * quarter + lane;
-    float hi[32], lo[32];
+    // the column in TMEM lane 32 quarter + lane (groups of eight: L, Q_b, L, ...)
+    const int j = 64 * ((lane >> 3) & 1) + 16 * quarter + 8 * (lane >> 4) + (lane & 7);
+    f32x2 hi[16], lo[16];  // the sums of L columns 32 ihalf + 2 i, 2 i + 1
 #pragma unroll
-    for (int i = 0; i < 32; i++) hi[i] = lo[i] = 0.f;
+    for (int i = 0; i < 16; i++) hi[i] = lo[i] = f2_pack(0.f, 0.f);
+    const f32x2 neg1 = f2_pack(-1.f, -1.f), s8 = f2_pack(0.00390625f, 0.00390625f);
     bool ok = true;
     for (long c = 0; c < my_chunks; c++) {
       const int buf = (int)(c & 1);
@@ -392,46 +479,42 @@ __global__ void __launch_bounds__(OZG_THREADS, 1) oz_gram_kernel(const __grid_co
         break;
       }
       tc_fence_after();
-      const int* ce = cexp[c & 3];
-      const int ej = ce[j];
-      // 2^(E - 1022 - 8) per factor: the digit sums carry 2^-8 per factor
-      const float fj = (ej >= 904 && ej <= 1157) ? __uint_as_float((uint32_t)(ej - 1030 + 127) << 23) : 0.f;
+      const float* ce = cscale[c % OZG_CSLOTS];
+      const f32x2 fj = f2_pack(ce[j], ce[j]);
       const uint32_t tl = tmem + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(buf * 256 + 32 * ihalf);
 #pragma unroll
-      for (int g = 0; g < 4; g++) {
-        // the four level accumulators of these 8 columns, one wait for all
-        uint32_t r[OZG_S][8];
+      for (int g = 0; g < 8; g++) {
+        // the four level accumulators of these 4 columns, one wait for all
+        uint32_t r[OZG_S][4];
 #pragma unroll
         for (int L = 0; L < OZG_S; L++)
-          asm volatile(
-              "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-              : "=r"(r[L][0]), "=r"(r[L][1]), "=r"(r[L][2]), "=r"(r[L][3]), "=r"(r[L][4]),
-                "=r"(r[L][5]), "=r"(r[L][6]), "=r"(r[L][7])
-              : "r"(tl + (uint32_t)(L * 64 + 8 * g)));
+          asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                       : "=r"(r[L][0]), "=r"(r[L][1]), "=r"(r[L][2]), "=r"(r[L][3])
+                       : "r"(tl + (uint32_t)(L * 64 + 4 * g)));
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        // levels 1.. by Horner, highest first: rest = sum_{L>=1} S_L 2^(8 - 8 L)
-        float rest[8];
+        const float4 fa = *(const float4*)(ce + 32 * ihalf + 4 * g);
+        const f32x2 fi[2] = {f2_pack(fa.x, fa.y), f2_pack(fa.z, fa.w)};
 #pragma unroll
-        for (int x = 0; x < 8; x++) {
-          rest[x] = __uint_as_float(r[OZG_S - 1][x]);
+        for (int x = 0; x < 2; x++) {
+          const int ii = 2 * g + x;
+          f32x2 S[OZG_S];
 #pragma unroll
-          for (int L = OZG_S - 2; L >= 1; L--) rest[x] = fmaf(rest[x], 0.00390625f, __uint_as_float(r[L][x]));
-        }
+          for (int L = 0; L < OZG_S; L++)
+            S[L] = f2_pack(__uint_as_float(r[L][2 * x]), __uint_as_float(r[L][2 * x + 1]));
+          // levels 1.. by Horner, highest first: rest = sum_{L>=1} S_L 2^(8 - 8 L)
+          f32x2 rest = S[OZG_S - 1];
 #pragma unroll
-        for (int x = 0; x < 8; x++) {
-          const int ii = 8 * g + x;
-          const int ei = ce[32 * ihalf + ii];
-          const float fi = (ei >= 904 && ei <= 1157) ? __uint_as_float((uint32_t)(ei - 1030 + 127) << 23) : 0.f;
-          const float fij = __fmul_rn(fj, fi);
+          for (int L = OZG_S - 2; L >= 1; L--) rest = f2_fma(rest, s8, S[L]);
+          const f32x2 fij = f2_mul(fj, fi[x]);
           // level 0 (an integer below 2^22) scaled exactly, added by a
-          // two-sum (hi + a = sum + err exactly; intrinsics: no contraction);
-          // the levels below it, 2^-8 smaller, into the low word
-          const float a = __fmul_rn(__uint_as_float(r[0][x]), fij);
-          const float sum = __fadd_rn(hi[ii], a);
-          const float bv = __fsub_rn(sum, hi[ii]);
-          const float err = __fadd_rn(__fsub_rn(hi[ii], __fsub_rn(sum, bv)), __fsub_rn(a, bv));
+          // two-sum (hi + a = sum + err exactly; a - b as b (-1) + a, rounded
+          // once); the levels below it, 2^-8 smaller, into the low word
+          const f32x2 a = f2_mul(S[0], fij);
+          const f32x2 sum = f2_add(hi[ii], a);
+          const f32x2 bv = f2_fma(hi[ii], neg1, sum);
+          const f32x2 err = f2_add(f2_fma(f2_fma(bv, neg1, sum), neg1, hi[ii]), f2_fma(bv, neg1, a));
           hi[ii] = sum;
-          lo[ii] = fmaf(rest[x], __fmul_rn(fij, 0.00390625f), __fadd_rn(lo[ii], err));
+          lo[ii] = f2_fma(rest, f2_mul(fij, s8), f2_add(lo[ii], err));
         }
       }
       tc_fence_before();
@@ -440,17 +523,23 @@ __global__ void __launch_bounds__(OZG_THREADS, 1) oz_gram_kernel(const __grid_co
       // small and its own FP32 roundings negligible
       if ((c & 7) == 7) {
 #pragma unroll
-        for (int i = 0; i < 32; i++) {
-          const float sum = __fadd_rn(hi[i], lo[i]);
-          const float bv = __fsub_rn(sum, hi[i]);
-          lo[i] = __fadd_rn(__fsub_rn(hi[i], __fsub_rn(sum, bv)), __fsub_rn(lo[i], bv));
+        for (int i = 0; i < 16; i++) {
+          const f32x2 sum = f2_add(hi[i], lo[i]);
+          const f32x2 bv = f2_fma(hi[i], neg1, sum);
+          lo[i] = f2_add(f2_fma(f2_fma(bv, neg1, sum), neg1, hi[i]), f2_fma(bv, neg1, lo[i]));
           hi[i] = sum;
         }
       }
     }
     double* out = prm.partial + ((size_t)b * gridDim.x + blockIdx.x) * 128 * 64 + (size_t)j * 64 + 32 * ihalf;
 #pragma unroll
-    for (int i = 0; i < 32; i++) out[i] = ok ? (double)hi[i] + (double)lo[i] : 0.0;
+    for (int i = 0; i < 16; i++) {
+      float h0, h1, l0, l1;
+      f2_unpack(hi[i], h0, h1);
+      f2_unpack(lo[i], l0, l1);
+      out[2 * i] = ok ? (double)h0 + (double)l0 : 0.0;
+      out[2 * i + 1] = ok ? (double)h1 + (double)l1 : 0.0;
+    }
   }
   // TMEM is freed only after the last MMA has completed and every epilogue
   // read has finished
@@ -573,7 +662,11 @@ static int ozg_layout(gpu_Context* ctx, ozg_params* prm, int ntiles)
       j++;
     }
     if (off > OZG_RAW) return gb_fail(ctx, "oz_gram: tile %d needs %ld bytes of staging", t, off);
+    if (off > prm->raw) prm->raw = (int)((off + 1023) & ~1023L);
   }
+  // as many raw buffers as fit: a chunk's copies, scales and digits each take about as
+  // long, and with two buffers each role waits for another
+  prm->nslots = OZG_RAWS / prm->raw < OZG_MAXSLOTS ? OZG_RAWS / prm->raw : OZG_MAXSLOTS;
   return 0;
 }
 
