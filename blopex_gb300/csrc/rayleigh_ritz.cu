@@ -75,11 +75,10 @@ __global__ void __launch_bounds__(RR_THREADS) rr_chol64_kernel(const double* __r
                                                                double report_below)
 {
   extern __shared__ double Ls[];
+  __shared__ double piv[RR_MAX_M];  // L_jj^2
   __shared__ int bad;
   double* L = SMEM ? Ls : s.L64;
   const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
-  double qmin = HUGE_VAL;
-  int jmin = 0;
   if (tid == 0) {
     bad = 0;
     s.status[0] = 0;
@@ -90,38 +89,62 @@ __global__ void __launch_bounds__(RR_THREADS) rr_chol64_kernel(const double* __r
     L[e] = (i >= j) ? B[i + (size_t)j * ld] : 0.0;
   }
   __syncthreads();
-  for (int j = 0; j < m; j++) {
-    if (tid == 0) {
-      double d = L[j + (size_t)j * m];
-      if (!(d > 0.0) || !isfinite(d)) {
-        bad = j + 1;
-      } else {
-        L[j + (size_t)j * m] = sqrt(d);
-        const double q = d / B[j + (size_t)j * ld];
-        if (q < qmin) {
-          qmin = q;
-          jmin = j;
-        }
-      }
+  auto pivot = [&](int j, double d) {  // thread 0
+    if (!(d > 0.0) || !isfinite(d)) {
+      bad = j + 1;
+    } else {
+      L[j + (size_t)j * m] = sqrt(d);
+      piv[j] = d;
     }
-    __syncthreads();
-    if (bad) break;
+  };
+  if (tid == 0) pivot(0, L[0]);
+  __syncthreads();
+  for (int j = 0; j < m && !bad; j++) {
     const double djj = L[j + (size_t)j * m];
     for (int i = j + 1 + tid; i < m; i += nt) L[i + (size_t)j * m] /= djj;
     __syncthreads();
-    // trailing update, a warp per column: L(i, l) -= L(i, j) L(l, j), i >= l > j
-    for (int l = j + 1 + warp; l < m; l += nw) {
+    // trailing update, a warp per column: L(i, l) -= L(i, j) L(l, j), i >= l > j; the
+    // next pivot and its root (a chain of 500 cycles) by warp 0 meanwhile (order 72:
+    // 77 us against 100, the ratios to B's diagonal now taken after the loop)
+    if (tid == 0 && j + 1 < m) {
+      const double a = L[j + 1 + (size_t)j * m];
+      double d = L[j + 1 + (size_t)(j + 1) * m];
+      d -= a * a;
+      pivot(j + 1, d);
+    }
+    for (int l = j + warp; l < m && warp > 0; l += nw - 1) {
       const double llj = L[l + (size_t)j * m];
-      for (int i = l + lane; i < m; i += 32) L[i + (size_t)l * m] -= L[i + (size_t)j * m] * llj;
+      for (int i = l + lane; i < m; i += 32)
+        if (i > j + 1) L[i + (size_t)l * m] -= L[i + (size_t)j * m] * llj;
     }
     __syncthreads();
   }
-  if (tid == 0 && !bad) {
-    if (qmin < report_below) {
-      bad = jmin + 1;
-    } else if (qmin < RR_GRADED_BELOW) {
-      s.status[0] = 7;
-      atomicAdd(&s.count[4], 1);
+  // the smallest pivot ratio, the first of equal ones
+  if (warp == 0 && !bad) {
+    double qmin = HUGE_VAL;
+    int jmin = 0;
+    for (int j = lane; j < m; j += 32) {
+      const double q = piv[j] / B[j + (size_t)j * ld];
+      if (q < qmin) {
+        qmin = q;
+        jmin = j;
+      }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      const double q = __shfl_xor_sync(0xffffffffu, qmin, o);
+      const int jq = __shfl_xor_sync(0xffffffffu, jmin, o);
+      if (q < qmin || (q == qmin && jq < jmin)) {
+        qmin = q;
+        jmin = jq;
+      }
+    }
+    if (lane == 0) {
+      if (qmin < report_below) {
+        bad = jmin + 1;
+      } else if (qmin < RR_GRADED_BELOW) {
+        s.status[0] = 7;
+        atomicAdd(&s.count[4], 1);
+      }
     }
   }
   __syncthreads();
@@ -175,37 +198,54 @@ __global__ void __launch_bounds__(32) rr_trsm64_kernel(int mode, const double* _
     }
     y[q] = a;
   }
+  // column i of L (row i of L' backwards) is loaded while step i - 1 (i + 1) runs: a
+  // load in the chain cost as much as its division (order 72: 41 us against 71)
+  const double* T = mode < 2 ? s.L64 : s.LT64;
+  double nx[SL], nd;
+  auto load = [&](int i) {
+    const double* t = T + (size_t)i * m;
+    nd = t[i];
+#pragma unroll
+    for (int q = 0; q < SL; q++) nx[q] = q * 32 + lane < m ? t[q * 32 + lane] : 0.0;
+  };
+  load(mode < 2 ? 0 : m - 1);
   if (mode < 2) {
-    const double* L = s.L64;
 #pragma unroll
     for (int q = 0; q < SL; q++) {
       for (int il = 0; il < 32; il++) {
         const int i = q * 32 + il;
         if (i >= m) break;
-        const double* li = L + (size_t)i * m;
-        const double xi = __shfl_sync(0xffffffffu, y[q], il) / li[i];
+        double li[SL];
+        const double lii = nd;
+#pragma unroll
+        for (int q2 = 0; q2 < SL; q2++) li[q2] = nx[q2];
+        if (i + 1 < m) load(i + 1);
+        const double xi = __shfl_sync(0xffffffffu, y[q], il) / lii;
         if (lane == il) y[q] = xi;
 #pragma unroll
         for (int q2 = q; q2 < SL; q2++) {
           const int p = q2 * 32 + lane;
-          if (p > i && p < m) y[q2] -= li[p] * xi;
+          if (p > i && p < m) y[q2] -= li[q2] * xi;
         }
       }
     }
   } else {
-    const double* LT = s.LT64;
 #pragma unroll
     for (int q = SL - 1; q >= 0; q--) {
       for (int il = 31; il >= 0; il--) {
         const int i = q * 32 + il;
         if (i >= m) continue;
-        const double* lti = LT + (size_t)i * m;  // lti[p] = L(i, p)
-        const double xi = __shfl_sync(0xffffffffu, y[q], il) / lti[i];
+        double li[SL];  // li[q2]: L(i, 32 q2 + lane)
+        const double lii = nd;
+#pragma unroll
+        for (int q2 = 0; q2 < SL; q2++) li[q2] = nx[q2];
+        if (i > 0) load(i - 1);
+        const double xi = __shfl_sync(0xffffffffu, y[q], il) / lii;
         if (lane == il) y[q] = xi;
 #pragma unroll
         for (int q2 = 0; q2 <= q; q2++) {
           const int p = q2 * 32 + lane;
-          if (p < i) y[q2] -= lti[p] * xi;
+          if (p < i) y[q2] -= li[q2] * xi;
         }
       }
     }
@@ -434,19 +474,31 @@ struct rr_gemm_t {
   int M, N, K;
 };
 
-__global__ void __launch_bounds__(256) rr_gemm_kernel(rr_gemm_t g0, rr_gemm_t g1, const int* status)
+// Tiles of 8 x 16, one entry a thread: the orders are small, and a 32 x 32 tile held one
+// SM's FP64 pipe for 128 instructions of 16 cycles a column of A where the chain of an
+// entry's own multiply-adds takes 70 (57 x 20 x 57: 5.2 us, in 32 x 32 tiles 12.6).
+#define RR_GEMM_TM 8
+#define RR_GEMM_TN 16
+static dim3 rr_gemm_grid(int M, int N, int batch)
+{
+  return dim3((M + RR_GEMM_TM - 1) / RR_GEMM_TM, (N + RR_GEMM_TN - 1) / RR_GEMM_TN, batch);
+}
+
+__global__ void __launch_bounds__(RR_GEMM_TM * RR_GEMM_TN) rr_gemm_kernel(rr_gemm_t g0, rr_gemm_t g1,
+                                                                          const int* status)
 {
   if (status[0]) return;
   const rr_gemm_t g = blockIdx.z == 0 ? g0 : g1;
-  __shared__ double As[32][33], Bs[32][33];
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int i0 = blockIdx.x * 32, j0 = blockIdx.y * 32;
+  __shared__ double As[RR_GEMM_TM][33], Bs[RR_GEMM_TN][33];
+  const int tx = threadIdx.x % RR_GEMM_TN, ty = threadIdx.x / RR_GEMM_TN;
+  const int i0 = blockIdx.x * RR_GEMM_TM, j0 = blockIdx.y * RR_GEMM_TN;
   if (i0 >= g.M || j0 >= g.N) return;
-  double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+  double acc = 0.0;
   for (int k0 = 0; k0 < g.K; k0 += 32) {
-    for (int e = threadIdx.x; e < 32 * 32; e += 256) {
-      int ii = e % 32, kk = e / 32;
-      int i = i0 + ii, k = k0 + kk;
+    for (int e = threadIdx.x; e < RR_GEMM_TM * 32; e += RR_GEMM_TM * RR_GEMM_TN) {
+      // along the index that is contiguous in memory
+      const int ii = g.amode == 1 ? e / 32 : e % RR_GEMM_TM, kk = g.amode == 1 ? e % 32 : e / RR_GEMM_TM;
+      const int i = i0 + ii, k = k0 + kk;
       double v = 0.0;
       if (i < g.M && k < g.K) {
         if (g.amode == 0)
@@ -457,27 +509,18 @@ __global__ void __launch_bounds__(256) rr_gemm_kernel(rr_gemm_t g0, rr_gemm_t g1
           v = (i >= k) ? g.A[i + (size_t)k * g.lda] : g.A[k + (size_t)i * g.lda];
       }
       As[ii][kk] = v;
-      int jj = e / 32, kb = e % 32;
-      int j = j0 + jj, k2 = k0 + kb;
-      Bs[kb][jj] = (j < g.N && k2 < g.K) ? g.B[k2 + (size_t)j * g.ldb] : 0.0;
+    }
+    for (int e = threadIdx.x; e < RR_GEMM_TN * 32; e += RR_GEMM_TM * RR_GEMM_TN) {
+      const int jj = e / 32, kk = e % 32, j = j0 + jj, k = k0 + kk;
+      Bs[jj][kk] = (j < g.N && k < g.K) ? g.B[k + (size_t)j * g.ldb] : 0.0;
     }
     __syncthreads();
+    const int kn = min(32, g.K - k0);
 #pragma unroll 8
-    for (int kk = 0; kk < 32; kk++) {
-      double a0 = As[ty][kk], a1 = As[ty + 16][kk];
-      double b0 = Bs[kk][tx], b1 = Bs[kk][tx + 16];
-      acc[0][0] = fma(a0, b0, acc[0][0]);
-      acc[0][1] = fma(a0, b1, acc[0][1]);
-      acc[1][0] = fma(a1, b0, acc[1][0]);
-      acc[1][1] = fma(a1, b1, acc[1][1]);
-    }
+    for (int kk = 0; kk < kn; kk++) acc = fma(As[ty][kk], Bs[tx][kk], acc);
     __syncthreads();
   }
-  for (int a = 0; a < 2; a++)
-    for (int b = 0; b < 2; b++) {
-      int i = i0 + ty + 16 * a, j = j0 + tx + 16 * b;
-      if (i < g.M && j < g.N) g.C[i + (size_t)j * g.ldc] = acc[a][b];
-    }
+  if (i0 + ty < g.M && j0 + tx < g.N) g.C[i0 + ty + (size_t)(j0 + tx) * g.ldc] = acc;
 }
 
 // FP64 cyclic Jacobi on the c x c matrix M (leading dimension lm); V (same
@@ -782,29 +825,42 @@ __global__ void __launch_bounds__(RR_TRD_THREADS) rr_tridiag_kernel(int m, rr_sc
 #define RR_TRD_SMEM_M 224
 __device__ __forceinline__ int rr_pk(int r, int c, int m) { return c * m - ((c * (c - 1)) >> 1) + (r - c); }
 
-// sum over threads of v, computed by warp 0 from per-thread values staged in
-// buf (blockDim.x entries); all threads return the sum
-__device__ double rr_sum_w0(double v, double* buf, double* out)
+// the reflector of column j (warp 0): x = the column below row j + 1
+__device__ __forceinline__ void rr_trd_reflector(const double* Lp, int j, int m, const rr_scratch& s,
+                                                 double* sh_tau, double* sh_scale)
 {
-  const int tid = threadIdx.x;
-  buf[tid] = v;
-  __syncthreads();
-  if (tid < 32) {
-    double t = 0.0;
-    for (int i = tid; i < (int)blockDim.x; i += 32) t += buf[i];
-    t = rr_warp_sum(t);
-    if (tid == 0) *out = t;
+  const int lane = threadIdx.x & 31, n1 = m - j - 1, cj = rr_pk(j + 1, j, m);
+  double acc = 0.0;
+  for (int i = 1 + lane; i < n1; i += 32) acc += Lp[cj + i] * Lp[cj + i];
+  acc = rr_warp_sum(acc);
+  if (lane == 0) {
+    const double alpha = Lp[cj];
+    double tau = 0.0, beta = alpha, scale = 0.0;
+    if (acc > 0.0) {
+      beta = -copysign(hypot(alpha, sqrt(acc)), alpha);
+      tau = (beta - alpha) / beta;
+      scale = 1.0 / (alpha - beta);
+    }
+    s.d[j] = Lp[rr_pk(j, j, m)];
+    s.e[j] = beta;
+    s.tau[j] = tau;
+    *sh_tau = tau;
+    *sh_scale = scale;
   }
-  __syncthreads();
-  return *out;
 }
 
+// Bound by chains of dependent FP64 instructions (70 cycles each): a step is the dot
+// products of p (one multiply-add a row), their sum, and a square root, hypot and two
+// divisions for the reflector.  The rows of a warp run one loop over both parts (the
+// lanes of a warp change part at different columns: two loops took 31 more steps), the
+// sum adds the n1 values that are there, and warp 0 updates the next column first and
+// forms its reflector while the others update the rest.
+//   order 57: 110 us against 152; order 72: 306 against 430.
 __global__ void __launch_bounds__(RR_TRD_THREADS) rr_tridiag_smem_kernel(int m, rr_scratch s)
 {
   extern __shared__ double Lp[];  // packed lower triangle, m(m+1)/2
-  __shared__ double v[RR_TRD_SMEM_M], p[RR_TRD_SMEM_M];
-  __shared__ double buf[RR_TRD_THREADS];
-  __shared__ double sh_sum, sh_tau, sh_scale;
+  __shared__ double v[RR_TRD_SMEM_M], p[RR_TRD_SMEM_M], buf[RR_TRD_SMEM_M];
+  __shared__ double sh_sum, sh_tau[2], sh_scale[2];  // by step parity
   if (s.status[0]) return;
   double* A = s.C64;
   const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5;
@@ -812,60 +868,60 @@ __global__ void __launch_bounds__(RR_TRD_THREADS) rr_tridiag_smem_kernel(int m, 
   for (int c = warp; c < m; c += nw)
     for (int r = c + lane; r < m; r += 32) Lp[rr_pk(r, c, m)] = A[r + (size_t)c * m];
   __syncthreads();
+  if (warp == 0 && m > 2) rr_trd_reflector(Lp, 0, m, s, &sh_tau[0], &sh_scale[0]);
+  __syncthreads();
   for (int j = 0; j + 2 < m; j++) {
     const int n1 = m - j - 1, o = j + 1;  // trailing block rows/cols o .. m-1
     const int cj = rr_pk(o, j, m);        // x = Lp[cj .. cj + n1)
-    if (warp == 0) {
-      double acc = 0.0;
-      for (int i = 1 + lane; i < n1; i += 32) acc += Lp[cj + i] * Lp[cj + i];
-      acc = rr_warp_sum(acc);
-      if (lane == 0) {
-        const double alpha = Lp[cj];
-        double tau = 0.0, beta = alpha, scale = 0.0;
-        if (acc > 0.0) {
-          beta = -copysign(hypot(alpha, sqrt(acc)), alpha);
-          tau = (beta - alpha) / beta;
-          scale = 1.0 / (alpha - beta);
-        }
-        s.d[j] = Lp[rr_pk(j, j, m)];
-        s.e[j] = beta;
-        s.tau[j] = tau;
-        sh_tau = tau;
-        sh_scale = scale;
-      }
+    const double tau = sh_tau[j & 1], scale = sh_scale[j & 1];
+    double* next_tau = &sh_tau[(j + 1) & 1];
+    double* next_scale = &sh_scale[(j + 1) & 1];
+    if (tau == 0.0) {  // uniform
+      if (warp == 0 && o + 2 < m) rr_trd_reflector(Lp, o, m, s, next_tau, next_scale);
+      __syncthreads();
+      continue;
     }
-    __syncthreads();
-    const double tau = sh_tau, scale = sh_scale;
-    if (tau == 0.0) continue;  // uniform
     for (int i = tid; i < n1; i += nt) {
       const double vi = (i == 0) ? 1.0 : Lp[cj + i] * scale;
       v[i] = vi;
       if (i > 0) A[(o + i) + (size_t)j * m] = vi;  // reflector for the back-transformation
     }
     __syncthreads();
-    // p_i = tau * (sum_{c <= i} A22(i, c) v_c + sum_{r > i} A22(r, i) v_r)
-    double pv = 0.0;
-    for (int i = tid; i < n1; i += nt) {
+    // p_i = tau * sum_c A22(i, c) v_c, entries above the diagonal from their mirror
+    // images: along row i up to the diagonal, then down column i
+    static_assert(RR_TRD_SMEM_M <= RR_TRD_THREADS, "a thread a row");
+    if (tid < n1) {
       double t = 0.0;
-      int a = rr_pk(o + i, o, m);  // (i, c = 0)
-      for (int c = 0; c <= i; c++) {
+      int a = rr_pk(o + tid, o, m);
+#pragma unroll 8
+      for (int c = 0; c < n1; c++) {
         t += Lp[a] * v[c];
-        a += m - (o + c) - 1;  // next column, same row
+        a += c < tid ? m - (o + c) - 1 : 1;
       }
-      const int b = rr_pk(o + i, o + i, m);
-      for (int r = i + 1; r < n1; r++) t += Lp[b + (r - i)] * v[r];
       t *= tau;
-      p[i] = t;
-      pv += t * v[i];
+      p[tid] = t;
+      buf[tid] = t * v[tid];
     }
-    const double K = 0.5 * tau * rr_sum_w0(pv, buf, &sh_sum);  // (its barriers order p)
-    for (int i = tid; i < n1; i += nt) p[i] -= K * v[i];     // p <- w
     __syncthreads();
-    // A22 -= v w' + w v' (lower): warp per column
-    for (int c = warp; c < n1; c += nw) {
+    if (warp == 0) {
+      double t = 0.0;
+      for (int i = lane; i < n1; i += 32) t += buf[i];
+      t = rr_warp_sum(t);
+      if (lane == 0) sh_sum = t;
+    }
+    __syncthreads();
+    const double K = 0.5 * tau * sh_sum;
+    if (tid < n1) p[tid] -= K * v[tid];  // p <- w
+    __syncthreads();
+    // A22 -= v w' + w v' (lower): column 0 and its reflector by warp 0, a warp a column
+    for (int c = warp; c < n1; c += warp == 0 ? n1 : nw - 1) {
       const int base = rr_pk(o + c, o + c, m) - c;
       const double vc = v[c], wc = p[c];
       for (int r = c + lane; r < n1; r += 32) Lp[base + r] -= v[r] * wc + p[r] * vc;
+    }
+    if (warp == 0 && o + 2 < m) {
+      __syncwarp();
+      rr_trd_reflector(Lp, o, m, s, next_tau, next_scale);
     }
     __syncthreads();
   }
@@ -879,36 +935,83 @@ __global__ void __launch_bounds__(RR_TRD_THREADS) rr_tridiag_smem_kernel(int m, 
   }
 }
 
-// number of eigenvalues of T below x (Sturm count of the LDL' pivots)
+// number of eigenvalues of T below x (Sturm count of the LDL' pivots); the high words
+// of the pivots go to piv[32 i].  The comparisons read the bits: as FP64 instructions
+// each added 70 cycles to the chain of a pivot.
 __device__ __forceinline__ int rr_sturm(const double* d, const double* e2, int m, double x,
-                                        double pivmin)
+                                        double pivmin, int* piv)
 {
+  const long long pm = __double_as_longlong(pivmin);
   double q = d[0] - x;
-  if (fabs(q) < pivmin) q = -pivmin;
-  int cnt = q < 0.0;
+  if ((__double_as_longlong(q) & 0x7FFFFFFFFFFFFFFFll) < pm) q = -pivmin;
+  int cnt = __double2hiint(q) < 0;
+  piv[0] = __double2hiint(q);
   for (int i = 1; i < m; i++) {
     q = (d[i] - x) - e2[i - 1] / q;
-    if (fabs(q) < pivmin) q = -pivmin;
-    cnt += q < 0.0;
+    if ((__double_as_longlong(q) & 0x7FFFFFFFFFFFFFFFll) < pm) q = -pivmin;
+    cnt += __double2hiint(q) < 0;
+    piv[32 * i] = __double2hiint(q);
   }
   return cnt;
 }
 
-// 4. eigenvalue j of T (ascending) by multisection: the 32 lanes count at
-// 31 interior points of [lo, hi]; the bracket shrinks 32-fold per step
-__global__ void __launch_bounds__(32) rr_bisect_kernel(int m, rr_scratch s)
+// the same in FP32, for a first guess (a zero pivot gives an infinity, which counts
+// on as it should)
+__device__ __forceinline__ int rr_sturm32(const float* d, const float* e2, int m, float x)
 {
+  float q = d[0] - x;
+  int cnt = q < 0.f;
+  for (int i = 1; i < m; i++) {
+    q = (d[i] - x) - __fdividef(e2[i - 1], q);
+    cnt += q < 0.f;
+  }
+  return cnt;
+}
+
+__device__ __forceinline__ double rr_bis_point(double lo, double hi, int lane)
+{
+  return (lane == 31) ? hi : lo + (hi - lo) * (double)(lane + 1) * (1.0 / 32.0);
+}
+
+__device__ __forceinline__ bool rr_bis_done(double lo, double hi, double tnorm)
+{
+  return hi - lo <= fmax(2.0 * DBL_EPSILON * fmax(fabs(lo), fabs(hi)), 0.25 * DBL_EPSILON * tnorm);
+}
+
+// 4. eigenvalue j of T (ascending) by multisection: the 32 lanes count at
+// 31 interior points of [lo, hi]; the bracket shrinks 32-fold per step, about 11
+// steps, each a chain of m divisions (600 cycles a pivot).
+//
+// The FP64 pipe takes the chains of two or three warps at once, so RR_BIS_WARPS steps
+// go together: warp w counts at the points of the bracket that w more steps would
+// reach if the eigenvalue were at `est`, and its counts are used if they do.  The
+// brackets, points and counts are those of one step at a time.  est: from FP32 counts
+// first, then the secant of det(T - x), the product of the pivots (their high words),
+// between the bracket's ends.
+// 4 rounds of 1100 cycles a pivot instead of 11 steps of 720.
+//   order 57, 19 eigenvalues: 90 us against 153; order 72, 24: 164 against 309.
+#define RR_BIS_WARPS 3
+static size_t rr_bisect_smem(int m) { return ((size_t)RR_BIS_WARPS * 32 + 2) * m * sizeof(int); }
+
+__global__ void __launch_bounds__(32 * RR_BIS_WARPS) rr_bisect_kernel(int m, rr_scratch s)
+{
+  extern __shared__ int piv[];  // [RR_BIS_WARPS][m][32] pivots, then those at lo and at hi
   __shared__ double d[RR_MAX_M], e2[RR_MAX_M];
+  __shared__ float d32[RR_MAX_M], e32[RR_MAX_M];
+  __shared__ double plo[RR_BIS_WARPS], phi[RR_BIS_WARPS];
+  __shared__ unsigned pge[RR_BIS_WARPS];
   if (s.status[0]) return;
-  const int lane = threadIdx.x, j = blockIdx.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, j = blockIdx.x;
+  int *pivlo = piv + RR_BIS_WARPS * 32 * m, *pivhi = pivlo + m;
   double emax2 = 0.0, glo = HUGE_VAL, ghi = -HUGE_VAL;
   for (int i = lane; i < m; i += 32) {
     const double di = s.d[i];
     const double el = i > 0 ? fabs(s.e[i - 1]) : 0.0, er = i + 1 < m ? fabs(s.e[i]) : 0.0;
-    d[i] = di;
+    if (warp == 0) d[i] = di;
     if (i + 1 < m) {
-      e2[i] = s.e[i] * s.e[i];
-      emax2 = fmax(emax2, e2[i]);
+      const double ee = s.e[i] * s.e[i];
+      if (warp == 0) e2[i] = ee;
+      emax2 = fmax(emax2, ee);
     }
     glo = fmin(glo, di - el - er);
     ghi = fmax(ghi, di + el + er);
@@ -918,24 +1021,76 @@ __global__ void __launch_bounds__(32) rr_bisect_kernel(int m, rr_scratch s)
     glo = fmin(glo, __shfl_xor_sync(0xffffffffu, glo, o));
     ghi = fmax(ghi, __shfl_xor_sync(0xffffffffu, ghi, o));
   }
-  __syncwarp();
   const double pivmin = DBL_MIN * fmax(1.0, emax2);
   const double tnorm = fmax(fabs(glo), fabs(ghi));
   const double pad = 2.0 * DBL_EPSILON * tnorm * m + 2.0 * pivmin;
   double lo = glo - pad, hi = ghi + pad;
-  for (int step = 0; step < 16; step++) {
-    if (hi - lo <= fmax(2.0 * DBL_EPSILON * fmax(fabs(lo), fabs(hi)), 0.25 * DBL_EPSILON * tnorm))
-      break;
-    const double x = (lane == 31) ? hi : lo + (hi - lo) * (double)(lane + 1) * (1.0 / 32.0);
-    const int cnt = (lane == 31) ? m : rr_sturm(d, e2, m, x, pivmin);
-    const unsigned ge = __ballot_sync(0xffffffffu, cnt >= j + 1);
-    const int f = __ffs(ge) - 1;  // first point with at least j+1 eigenvalues below it
-    const double xf = __shfl_sync(0xffffffffu, x, f);
-    const double xl = __shfl_sync(0xffffffffu, x, f > 0 ? f - 1 : 0);
-    hi = xf;
-    if (f > 0) lo = xl;
+  const double inv = tnorm > DBL_MIN ? 1.0 / tnorm : 1.0;
+  __syncthreads();
+  for (int i = threadIdx.x; i < m; i += 32 * RR_BIS_WARPS) {
+    d32[i] = (float)(d[i] * inv);
+    if (i + 1 < m) e32[i] = (float)(e2[i] * inv * inv);
+    pivlo[i] = pivhi[i] = 0;
   }
-  if (lane == 0) s.lam[j] = 0.5 * (lo + hi);
+  __syncthreads();
+  double est;
+  {
+    float a = (float)(lo * inv), b = (float)(hi * inv);
+    for (int step = 0; step < 5; step++) {
+      const float x = lane == 31 ? b : a + (b - a) * (float)(lane + 1) * (1.f / 32.f);
+      const int cnt = lane == 31 ? m : rr_sturm32(d32, e32, m, x);
+      const int f = __ffs(__ballot_sync(0xffffffffu, cnt >= j + 1)) - 1;
+      const float xf = __shfl_sync(0xffffffffu, x, f), xl = __shfl_sync(0xffffffffu, x, f > 0 ? f - 1 : 0);
+      b = xf;
+      if (f > 0) a = xl;
+    }
+    est = (0.5 * ((double)a + (double)b)) / inv;
+  }
+  for (int step = 0; step < 16 && !rr_bis_done(lo, hi, tnorm);) {
+    // this warp's bracket, were the eigenvalue at est
+    double a = lo, b = hi;
+    for (int l = 0; l < warp; l++) {
+      const double x = rr_bis_point(a, b, lane);
+      const int f = __ffs(__ballot_sync(0xffffffffu, lane == 31 || x >= est)) - 1;
+      const double xl = __shfl_sync(0xffffffffu, x, f > 0 ? f - 1 : 0);
+      b = __shfl_sync(0xffffffffu, x, f);
+      if (f > 0) a = xl;
+    }
+    const int cnt =
+        (lane == 31) ? m : rr_sturm(d, e2, m, rr_bis_point(a, b, lane), pivmin, piv + warp * 32 * m + lane);
+    const unsigned ge = __ballot_sync(0xffffffffu, cnt >= j + 1);
+    if (lane == 0) {
+      pge[warp] = ge;
+      plo[warp] = a;
+      phi[warp] = b;
+    }
+    __syncthreads();
+    int src_lo = -1, src_hi = -1;  // the points that lo and hi moved to
+    for (int l = 0; l < RR_BIS_WARPS && step < 16; l++, step++) {
+      if (l > 0 && (plo[l] != lo || phi[l] != hi || rr_bis_done(lo, hi, tnorm))) break;
+      const int f = __ffs(pge[l]) - 1;  // first point with at least j+1 eigenvalues below it
+      const double xf = rr_bis_point(lo, hi, f), xl = rr_bis_point(lo, hi, f > 0 ? f - 1 : 0);
+      hi = xf;
+      if (f < 31) src_hi = l * 32 * m + f;
+      if (f > 0) {
+        lo = xl;
+        src_lo = l * 32 * m + f - 1;
+      }
+    }
+    for (int i = threadIdx.x; i < m; i += 32 * RR_BIS_WARPS) {
+      if (src_lo >= 0) pivlo[i] = piv[src_lo + 32 * i];
+      if (src_hi >= 0) pivhi[i] = piv[src_hi + 32 * i];
+    }
+    __syncthreads();
+    // det(T - hi) / det(T - lo), negative around one eigenvalue (NaN while an end has
+    // not been counted at)
+    double ratio = 1.0;
+    for (int i = lane; i < m; i += 32)
+      ratio *= __hiloint2double(pivhi[i], 0) / __hiloint2double(pivlo[i], 0);
+    for (int o = 16; o > 0; o >>= 1) ratio *= __shfl_xor_sync(0xffffffffu, ratio, o);
+    est = ratio < 0.0 ? lo + (hi - lo) / (1.0 - ratio) : 0.5 * (lo + hi);
+  }
+  if (threadIdx.x == 0) s.lam[j] = 0.5 * (lo + hi);
 }
 
 __device__ __forceinline__ double rr_start_value(int j, int i)
@@ -1036,27 +1191,46 @@ __global__ void __launch_bounds__(32) rr_invit_kernel(int m, rr_scratch s)
 
 // Cholesky of the nev x nev Gram matrix s.S (upper, U'U = S) and U^-1 into
 // s.P; status 6 when the vectors are not numerically independent
-__global__ void __launch_bounds__(256) rr_cholinv_kernel(int nev, rr_scratch s)
+#define RR_CHOLINV_SMEM_M 112
+__global__ void __launch_bounds__(256) rr_cholinv_kernel(int nev, rr_scratch s, int smem)
 {
+  extern __shared__ double sh[];  // up to order RR_CHOLINV_SMEM_M: U, then its inverse
   __shared__ int bad;
+  __shared__ double rinv;  // 1 / U_jj: by one thread, 8 warps' divisions at once take the FP64 pipe 1800 cycles
   if (s.status[0]) return;
-  double* U = s.S;
+  double *U = smem ? sh : s.S, *V = smem ? sh + (size_t)nev * nev : s.P;
   const int tid = threadIdx.x, nt = blockDim.x;
-  if (tid == 0) bad = 0;
-  __syncthreads();
-  for (int j = 0; j < nev; j++) {
-    if (tid == 0) {
-      const double djj = U[j + (size_t)j * nev];
-      if (!(djj > 1e-6)) bad = 1;  // the vectors are unit vectors
-      else U[j + (size_t)j * nev] = sqrt(djj);
-    }
+  if (smem) {
+    for (int e = tid; e < nev * nev; e += nt) U[e] = s.S[e];
     __syncthreads();
-    if (bad) break;
-    const double r = 1.0 / U[j + (size_t)j * nev];
+  }
+  auto pivot = [&](int j, double djj) {  // thread 0
+    if (!(djj > 1e-6)) {  // the vectors are unit vectors
+      bad = 1;
+    } else {
+      const double u = sqrt(djj);
+      U[j + (size_t)j * nev] = u;
+      rinv = 1.0 / u;
+    }
+  };
+  if (tid == 0) {
+    bad = 0;
+    pivot(0, U[0]);
+  }
+  __syncthreads();
+  for (int j = 0; j < nev && !bad; j++) {
+    const double r = rinv;
     for (int c = j + 1 + tid; c < nev; c += nt) U[j + (size_t)c * nev] *= r;
     __syncthreads();
     const int w = nev - j - 1;
-    for (int e = tid; e < w * w; e += nt) {
+    if (tid == 0 && w > 0) {  // the next pivot while the others update the rest
+      const double a = U[j + (size_t)(j + 1) * nev];
+      double d = U[j + 1 + (size_t)(j + 1) * nev];
+      d -= a * a;
+      pivot(j + 1, d);
+    }
+    for (int e = tid < 32 ? w * w : tid - 32; e < w * w; e += nt - 32) {  // (not warp 0)
+      if (e == 0) continue;  // element (j + 1, j + 1)
       const int a = j + 1 + e % w, c = j + 1 + e / w;
       if (a <= c) U[a + (size_t)c * nev] -= U[j + (size_t)a * nev] * U[j + (size_t)c * nev];
     }
@@ -1068,7 +1242,7 @@ __global__ void __launch_bounds__(256) rr_cholinv_kernel(int nev, rr_scratch s)
   }
   // inverse of the upper factor, one thread per column
   for (int c = tid; c < nev; c += nt) {
-    double* x = s.P + (size_t)c * nev;
+    double* x = V + (size_t)c * nev;
     for (int i = nev - 1; i > c; i--) x[i] = 0.0;
     x[c] = 1.0 / U[c + (size_t)c * nev];
     for (int i = c - 1; i >= 0; i--) {
@@ -1076,6 +1250,10 @@ __global__ void __launch_bounds__(256) rr_cholinv_kernel(int nev, rr_scratch s)
       for (int l = i + 1; l <= c; l++) t += U[i + (size_t)l * nev] * x[l];
       x[i] = -t / U[i + (size_t)i * nev];
     }
+  }
+  if (smem) {
+    __syncthreads();
+    for (int e = tid; e < nev * nev; e += nt) s.P[e] = V[e];
   }
 }
 
@@ -1095,10 +1273,22 @@ __global__ void __launch_bounds__(32) rr_backtr_kernel(int m, int nev, rr_scratc
     const int i = q * 32 + lane;
     z[q] = i < m ? zc[i] : 0.0;
   }
-  for (int h = m - 3; h >= 0; h--) {
-    const double tau = s.tau[h];
-    if (tau == 0.0) continue;
+  // reflector h - 1 is loaded while reflector h is applied
+  double nv[SL], ntau = 0.0;
+  auto load = [&](int h) {
+    ntau = s.tau[h];
     const double* vh = s.C64 + (size_t)h * m;  // v(h+1) = 1, v(i) = C[i, h] for i >= h+2
+#pragma unroll
+    for (int q = 0; q < SL; q++) nv[q] = q * 32 + lane < m ? vh[q * 32 + lane] : 0.0;
+  };
+  if (m >= 3) load(m - 3);
+  for (int h = m - 3; h >= 0; h--) {
+    const double tau = ntau;
+    double vh[SL];
+#pragma unroll
+    for (int q = 0; q < SL; q++) vh[q] = nv[q];
+    if (h > 0) load(h - 1);
+    if (tau == 0.0) continue;
     double t = 0.0;
 #pragma unroll
     for (int q = 0; q < SL; q++) {
@@ -1106,7 +1296,7 @@ __global__ void __launch_bounds__(32) rr_backtr_kernel(int m, int nev, rr_scratc
       if (i == h + 1)
         t += z[q];
       else if (i > h + 1 && i < m)
-        t += vh[i] * z[q];
+        t += vh[q] * z[q];
     }
     t = tau * rr_warp_sum(t);
 #pragma unroll
@@ -1115,7 +1305,7 @@ __global__ void __launch_bounds__(32) rr_backtr_kernel(int m, int nev, rr_scratc
       if (i == h + 1)
         z[q] -= t;
       else if (i > h + 1 && i < m)
-        z[q] -= t * vh[i];
+        z[q] -= t * vh[q];
     }
   }
 #pragma unroll
@@ -1227,16 +1417,22 @@ static void rr_tridiag_path(gpu_Context* ctx, double* A, int ld, int m, int nev,
   } else {
     RR_STAGE(GB_K_RR_TRID, 4.0 * m3 / 3.0, (rr_tridiag_kernel<<<1, RR_TRD_THREADS, 0, st>>>(m, s)));
   }
-  RR_STAGE(GB_K_RR_EIG, 0.0, (rr_bisect_kernel<<<nev, 32, 0, st>>>(m, s)));
+  const int sb = (int)rr_bisect_smem(m);
+  if (sb > 32 * 1024)
+    cudaFuncSetAttribute(rr_bisect_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sb);
+  RR_STAGE(GB_K_RR_EIG, 0.0, (rr_bisect_kernel<<<nev, 32 * RR_BIS_WARPS, sb, st>>>(m, s)));
   RR_STAGE(GB_K_RR_EIG, 0.0, (rr_invit_kernel<<<nev, 32, 0, st>>>(m, s)));
   // Cholesky-QR twice: Z <- Z inv(U), U'U = Z'Z
-  const dim3 gs((nev + 31) / 32, (nev + 31) / 32, 1), gz((m + 31) / 32, (nev + 31) / 32, 1);
+  const dim3 gs = rr_gemm_grid(nev, nev, 1), gz = rr_gemm_grid(m, nev, 1);
+  const int sc = nev <= RR_CHOLINV_SMEM_M ? (int)(2 * sizeof(double) * (size_t)nev * nev) : 0;
+  if (sc > 40 * 1024)
+    cudaFuncSetAttribute(rr_cholinv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sc);
   for (int round = 0; round < 2; round++) {
     rr_gemm_t zz = {s.X, m, 1, s.X, m, s.S, nev, nev, nev, m};
-    RR_STAGE(GB_K_RR_GEMM, 2.0 * m * nev * nev, (rr_gemm_kernel<<<gs, 256, 0, st>>>(zz, zz, s.status)));
-    RR_STAGE(GB_K_RR_EIG, 0.0, (rr_cholinv_kernel<<<1, 256, 0, st>>>(nev, s)));
+    RR_STAGE(GB_K_RR_GEMM, 2.0 * m * nev * nev, (rr_gemm_kernel<<<gs, RR_GEMM_TM * RR_GEMM_TN, 0, st>>>(zz, zz, s.status)));
+    RR_STAGE(GB_K_RR_EIG, 0.0, (rr_cholinv_kernel<<<1, 256, sc, st>>>(nev, s, sc > 0)));
     rr_gemm_t zu = {s.X, m, 0, s.P, nev, s.Xn, m, m, nev, nev};
-    RR_STAGE(GB_K_RR_GEMM, 2.0 * m * nev * nev, (rr_gemm_kernel<<<gz, 256, 0, st>>>(zu, zu, s.status)));
+    RR_STAGE(GB_K_RR_GEMM, 2.0 * m * nev * nev, (rr_gemm_kernel<<<gz, RR_GEMM_TM * RR_GEMM_TN, 0, st>>>(zu, zu, s.status)));
     double* t = s.X;
     s.X = s.Xn;
     s.Xn = t;
@@ -1264,18 +1460,18 @@ static void rr_jacobi32_path(gpu_Context* ctx, double* A, int ld, int m, int nev
   int launches = 2;
   const size_t sm_ref = 2 * sizeof(double) * RR_CLUSTER_SMEM * rr_pad(RR_CLUSTER_SMEM);
   cudaFuncSetAttribute(rr_refine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_ref);
-  const dim3 g1((m + 31) / 32, (m + 31) / 32, 1), g2((m + 31) / 32, (m + 31) / 32, 2);
+  const dim3 g1 = rr_gemm_grid(m, m, 1), g2 = rr_gemm_grid(m, m, 2);
   for (int round = 0; round < 2; round++) {
     rr_gemm_t ta = {s.C64, m, 0, s.X, m, s.TA, m, m, m, m};  // C X
-    RR_STAGE(GB_K_RR_GEMM, 2 * m3, (rr_gemm_kernel<<<g1, 256, 0, st>>>(ta, ta, s.status)));
+    RR_STAGE(GB_K_RR_GEMM, 2 * m3, (rr_gemm_kernel<<<g1, RR_GEMM_TM * RR_GEMM_TN, 0, st>>>(ta, ta, s.status)));
     rr_gemm_t sa = {s.X, m, 1, s.TA, m, s.S, m, m, m, m};  // X' C X
     rr_gemm_t sb = {s.X, m, 1, s.X, m, s.P, m, m, m, m};   // X' X
-    RR_STAGE(GB_K_RR_GEMM, 4 * m3, (rr_gemm_kernel<<<g2, 256, 0, st>>>(sa, sb, s.status)));
+    RR_STAGE(GB_K_RR_GEMM, 4 * m3, (rr_gemm_kernel<<<g2, RR_GEMM_TM * RR_GEMM_TN, 0, st>>>(sa, sb, s.status)));
     RR_STAGE(GB_K_RR_REFINE, 0.0, (rr_refine_kernel<<<1, RR_THREADS, sm_ref, st>>>(m, s, round == 1)));
     rr_gemm_t fq = {s.EI, m, 0, s.Q, m, s.F, m, m, m, m};
-    RR_STAGE(GB_K_RR_GEMM, 2 * m3, (rr_gemm_kernel<<<g1, 256, 0, st>>>(fq, fq, s.status)));
+    RR_STAGE(GB_K_RR_GEMM, 2 * m3, (rr_gemm_kernel<<<g1, RR_GEMM_TM * RR_GEMM_TN, 0, st>>>(fq, fq, s.status)));
     rr_gemm_t xf = {s.X, m, 0, s.F, m, s.Xn, m, m, m, m};
-    RR_STAGE(GB_K_RR_GEMM, 2 * m3, (rr_gemm_kernel<<<g1, 256, 0, st>>>(xf, xf, s.status)));
+    RR_STAGE(GB_K_RR_GEMM, 2 * m3, (rr_gemm_kernel<<<g1, RR_GEMM_TM * RR_GEMM_TN, 0, st>>>(xf, xf, s.status)));
     double* t = s.X;
     s.X = s.Xn;
     s.Xn = t;
