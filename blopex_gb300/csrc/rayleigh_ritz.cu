@@ -825,6 +825,11 @@ __global__ void __launch_bounds__(RR_TRD_THREADS) rr_tridiag_kernel(int m, rr_sc
 #define RR_TRD_SMEM_M 224
 __device__ __forceinline__ int rr_pk(int r, int c, int m) { return c * m - ((c * (c - 1)) >> 1) + (r - c); }
 
+// the warps that work beside a chain of warp 0: those of the three schedulers it does
+// not sit on, so that its FP64 instructions queue behind one of each at most; their
+// index, -1 for the others
+__device__ __forceinline__ int rr_side_warp(int warp, int nw) { return (warp & 3) ? (warp >> 2) * 3 + (warp & 3) - 1 : -1; }
+
 // the reflector of column j (warp 0): x = the column below row j + 1
 __device__ __forceinline__ void rr_trd_reflector(const double* Lp, int j, int m, const rr_scratch& s,
                                                  double* sh_tau, double* sh_scale)
@@ -914,7 +919,8 @@ __global__ void __launch_bounds__(RR_TRD_THREADS) rr_tridiag_smem_kernel(int m, 
     if (tid < n1) p[tid] -= K * v[tid];  // p <- w
     __syncthreads();
     // A22 -= v w' + w v' (lower): column 0 and its reflector by warp 0, a warp a column
-    for (int c = warp; c < n1; c += warp == 0 ? n1 : nw - 1) {
+    const int uw = rr_side_warp(warp, nw);
+    for (int c = warp == 0 ? 0 : uw < 0 ? n1 : 1 + uw; c < n1; c += warp == 0 ? n1 : 3 * nw / 4) {
       const int base = rr_pk(o + c, o + c, m) - c;
       const double vc = v[c], wc = p[c];
       for (int r = c + lane; r < n1; r += 32) Lp[base + r] -= v[r] * wc + p[r] * vc;
