@@ -15,6 +15,7 @@
 #include <string.h>
 
 #include "internal.h"
+#include "pdl.cuh"
 #include "blas32.cuh"
 
 #define CUDA_LAUNCH_CHECK(ctx, what) gb_cuda_check((ctx), (int)cudaGetLastError(), (what))
@@ -32,6 +33,7 @@ __global__ void __launch_bounds__(256) gram_partial_kernel(blk_cols X, int h, bl
                                                            long n, long rows_per_split,
                                                            double* __restrict__ partial)
 {
+  gb_pdl_entry();
   constexpr int BM = 16 * TM, BN = 16 * TN, RK = 32;
   __shared__ T xs[RK][BM + 1];
   __shared__ T ys[RK][BN + 1];
@@ -124,6 +126,7 @@ __global__ void __launch_bounds__(256) gram_reduce_kernel(const double* __restri
                                                           long nparts, int E, int h, int mode,
                                                           double* __restrict__ G, int ldg)
 {
+  gb_pdl_entry();
   __shared__ double sm[64][33];
   const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
   const int e0 = blockIdx.x * 32 + x;
@@ -182,6 +185,7 @@ __global__ void __launch_bounds__(GRAMP_T) gram_packed_kernel(blk_cols X, int h,
                                                               long rows_per_split, int sub, int groups,
                                                               double* __restrict__ partial)
 {
+  gb_pdl_entry();
   extern __shared__ double sm[];  // [32 groups][h (+ w), odd stride], then [groups][E32]
   const int E = SYM ? h * (h + 1) / 2 : h * w, E32 = (E + 31) & ~31;
   const int nc = SYM ? h : h + w, ld = nc | 1, RS = 32 * groups;
@@ -241,6 +245,7 @@ __global__ void __launch_bounds__(544) gram_sym_partial_kernel(blk_cols X, int h
                                                                long rows_per_split,
                                                                double* __restrict__ partial)
 {
+  gb_pdl_entry();
   constexpr int BM = 32 * BS, RK = 32;
   __shared__ T xs[RK][BM + 1];
   const int t = threadIdx.x;
@@ -336,8 +341,8 @@ static int gram_sym_launch(gpu_Context* ctx, long n, const blk_cols* X, int h, d
   dim3 grid(1, 1, (unsigned)splits);
   gb_prof_rec pr;
   gb_prof_begin(ctx, &pr, sizeof(T) == 8 ? GB_K_GRAM : GB_K_GRAM32);
-  gram_sym_partial_kernel<T, BS><<<grid, threads, 0, S(ctx)>>>(*X, h, n, rows, partial);
-  gram_reduce_kernel<<<(h * h + 31) / 32, 256, 0, S(ctx)>>>(partial, (int)splits, 1, splits, h * h, h, 2, G, ldg);
+  gb_pdl(gram_sym_partial_kernel<T, BS>, grid, threads, 0, S(ctx), *X, h, n, rows, partial);
+  gb_pdl(gram_reduce_kernel, (h * h + 31) / 32, 256, 0, S(ctx), partial, (int)splits, 1, splits, h * h, h, 2, G, ldg);
   gb_prof_end(ctx, &pr, (double)sizeof(T) * n * h, (double)n * h * (h + 1));
   gb_count_launch(2);
   return CUDA_LAUNCH_CHECK(ctx, "gram_sym");
@@ -364,9 +369,9 @@ static int gram_launch(gpu_Context* ctx, long n, const blk_cols* X, int h, const
   dim3 grid(gx, gy, (unsigned)splits);
   gb_prof_rec pr;
   gb_prof_begin(ctx, &pr, sizeof(T) == 8 ? GB_K_GRAM : GB_K_GRAM32);
-  gram_partial_kernel<T, TM, TN><<<grid, 256, 0, S(ctx)>>>(*X, h, *Y, w, n, rows, partial);
+  gb_pdl(gram_partial_kernel<T, TM, TN>, grid, 256, 0, S(ctx), *X, h, *Y, w, n, rows, partial);
   int tot = h * w;
-  gram_reduce_kernel<<<(tot + 31) / 32, 256, 0, S(ctx)>>>(partial, (int)splits, 1, splits, tot, h, 0, G, ldg);
+  gb_pdl(gram_reduce_kernel, (tot + 31) / 32, 256, 0, S(ctx), partial, (int)splits, 1, splits, tot, h, 0, G, ldg);
   gb_prof_end(ctx, &pr, (double)sizeof(T) * n * (h + w), 2.0 * n * h * w);
   gb_count_launch(2);
   return CUDA_LAUNCH_CHECK(ctx, "gram");
@@ -395,9 +400,9 @@ static int gram_packed(gpu_Context* ctx, long n, const blk_cols* X, int h, const
     return gb_fail(ctx, "gram: cannot reserve %d bytes of shared memory", smem);
   gb_prof_rec pr;
   gb_prof_begin(ctx, &pr, GB_K_GRAM);
-  gram_packed_kernel<SYM><<<(unsigned)(splits * sub), GRAMP_T, smem, S(ctx)>>>(*X, h, *Y, w, n, rows, sub, groups,
+  gb_pdl(gram_packed_kernel<SYM>, (unsigned)(splits * sub), GRAMP_T, smem, S(ctx), *X, h, *Y, w, n, rows, sub, groups,
                                                                                partial);
-  gram_reduce_kernel<<<(E + 31) / 32, 256, 0, S(ctx)>>>(partial, (int)splits, sub > 1 ? (int)chunks : 1, nparts, E, h,
+  gb_pdl(gram_reduce_kernel, (E + 31) / 32, 256, 0, S(ctx), partial, (int)splits, sub > 1 ? (int)chunks : 1, nparts, E, h,
                                                         SYM ? 1 : 0, G, ldg);
   gb_prof_end(ctx, &pr, 8.0 * n * nc, SYM ? (double)n * h * (h + 1) : 2.0 * n * h * w);
   gb_count_launch(2);
@@ -447,7 +452,7 @@ extern "C" int gb_gram_large(gpu_Context* ctx, int dtype, long n, const blk_cols
   gb_prof_rec pr;
   gb_prof_begin(ctx, &pr, GB_K_GRAM);
   if (gb_oz_gram64(ctx, n, X, h, Y, w, sym, &partial, &splits)) return -1;
-  gram_reduce_kernel<<<(h * w + 31) / 32, 256, 0, S(ctx)>>>(partial, (int)splits, 1, splits, h * w, h, sym ? 2 : 0, G,
+  gb_pdl(gram_reduce_kernel, (h * w + 31) / 32, 256, 0, S(ctx), partial, (int)splits, 1, splits, h * w, h, sym ? 2 : 0, G,
                                                             ldg);
   gb_prof_end(ctx, &pr, 8.0 * n * (sym ? h : h + w), sym ? (double)n * h * (h + 1) : 2.0 * n * h * w);
   gb_count_launch(1);
@@ -467,6 +472,7 @@ __global__ void __launch_bounds__(256) bymat_kernel(blk_cols X, int h, const dou
                                                     int ldc, blk_cols Y, int w, blk_cols Z,
                                                     int has_z, long n, int tri)
 {
+  gb_pdl_entry();
   constexpr int BM = 64, BN = 32, KC = 32;
   __shared__ T xs[KC][BM];
   __shared__ T cs[KC][BN];
@@ -532,9 +538,9 @@ static int bymat_launch(gpu_Context* ctx, int dtype, long n, const blk_cols* X, 
   gb_prof_rec pr;
   gb_prof_begin(ctx, &pr, dtype == GPU_MV_FLOAT64 ? GB_K_XC : GB_K_XC32);
   if (dtype == GPU_MV_FLOAT64)
-    bymat_kernel<double><<<grid, 256, 0, S(ctx)>>>(*X, h, C, ldc, *Y, w, *z, Z != NULL, n, tri);
+    gb_pdl(bymat_kernel<double>, grid, 256, 0, S(ctx), *X, h, C, ldc, *Y, w, *z, Z != NULL, n, tri);
   else
-    bymat_kernel<float><<<grid, 256, 0, S(ctx)>>>(*X, h, C, ldc, *Y, w, *z, Z != NULL, n, tri);
+    gb_pdl(bymat_kernel<float>, grid, 256, 0, S(ctx), *X, h, C, ldc, *Y, w, *z, Z != NULL, n, tri);
   // a triangular C: sum over j of min(j + 1, h) products per row
   const double kw = tri ? (double)w * (w + 1) / 2 - (w > h ? (double)(w - h) * (w - h + 1) / 2 : 0.0)
                         : (double)h * w;
@@ -581,6 +587,7 @@ extern "C" int gb_bymat_tri(gpu_Context* ctx, int dtype, long n, const blk_cols*
 template <typename T>
 __global__ void axpby_kernel(blk_cols X, double alpha, blk_cols Y, double beta, long n)
 {
+  gb_pdl_entry();
   const T* x = (const T*)X.col[blockIdx.y];
   T* y = (T*)Y.col[blockIdx.y];
   const T a = (T)alpha, b = (T)beta;
@@ -610,9 +617,9 @@ extern "C" int gb_axpby(gpu_Context* ctx, int dtype, long n, double alpha, const
   gb_prof_rec pr;
   gb_prof_begin(ctx, &pr, GB_K_BLAS1);
   if (dtype == GPU_MV_FLOAT64)
-    axpby_kernel<double><<<grid, 256, 0, S(ctx)>>>(*X, alpha, *Y, beta, n);
+    gb_pdl(axpby_kernel<double>, grid, 256, 0, S(ctx), *X, alpha, *Y, beta, n);
   else
-    axpby_kernel<float><<<grid, 256, 0, S(ctx)>>>(*X, alpha, *Y, beta, n);
+    gb_pdl(axpby_kernel<float>, grid, 256, 0, S(ctx), *X, alpha, *Y, beta, n);
   gb_prof_end(ctx, &pr, (dtype == GPU_MV_FLOAT64 ? 8.0 : 4.0) * n * w * (beta == 0.0 ? 2 : 3), 0.0);
   gb_count_launch(1);
   return CUDA_LAUNCH_CHECK(ctx, "axpby");
@@ -626,6 +633,7 @@ template <typename T>
 __global__ void scale_cols_kernel(blk_cols X, const double* __restrict__ d, idx_table idx,
                                   blk_cols Y, long n)
 {
+  gb_pdl_entry();
   const T* x = (const T*)X.col[blockIdx.y];
   T* y = (T*)Y.col[blockIdx.y];
   const T a = (T)d[idx.v[blockIdx.y]];
@@ -648,9 +656,9 @@ extern "C" int gb_scale_cols(gpu_Context* ctx, int dtype, long n, const blk_cols
   gb_prof_rec pr;
   gb_prof_begin(ctx, &pr, GB_K_BLAS1);
   if (dtype == GPU_MV_FLOAT64)
-    scale_cols_kernel<double><<<grid, 256, 0, S(ctx)>>>(*X, d, t, *Y, n);
+    gb_pdl(scale_cols_kernel<double>, grid, 256, 0, S(ctx), *X, d, t, *Y, n);
   else
-    scale_cols_kernel<float><<<grid, 256, 0, S(ctx)>>>(*X, d, t, *Y, n);
+    gb_pdl(scale_cols_kernel<float>, grid, 256, 0, S(ctx), *X, d, t, *Y, n);
   gb_prof_end(ctx, &pr, (dtype == GPU_MV_FLOAT64 ? 8.0 : 4.0) * n * w * 2, 0.0);
   gb_count_launch(1);
   return CUDA_LAUNCH_CHECK(ctx, "scale_cols");
@@ -660,6 +668,7 @@ extern "C" int gb_scale_cols(gpu_Context* ctx, int dtype, long n, const blk_cols
 template <typename T>
 __global__ void dot_partial_kernel(blk_cols X, blk_cols Y, long n, double* __restrict__ partial)
 {
+  gb_pdl_entry();
   const T* x = (const T*)X.col[blockIdx.y];
   const T* y = (const T*)Y.col[blockIdx.y];
   double s = 0.0;
@@ -672,6 +681,7 @@ __global__ void dot_partial_kernel(blk_cols X, blk_cols Y, long n, double* __res
 __global__ void dot_reduce_kernel(const double* __restrict__ partial, int nb, idx_table idx,
                                   double* __restrict__ out)
 {
+  gb_pdl_entry();
   const double s = ordered_sum256(partial + (size_t)blockIdx.x * nb, nb);
   if (threadIdx.x == 0) out[idx.v[blockIdx.x]] = s;
 }
@@ -681,6 +691,7 @@ __global__ void dot_reduce_kernel(const double* __restrict__ partial, int nb, id
 __global__ void __launch_bounds__(256) dot32_partial_kernel(blk_cols X, blk_cols Y, long n,
                                                             double* __restrict__ partial)
 {
+  gb_pdl_entry();
   const float4* x = (const float4*)X.col[blockIdx.y];
   const float4* y = (const float4*)Y.col[blockIdx.y];
   const long n4 = n >> 2, stride = (long)gridDim.x * blockDim.x;
@@ -721,12 +732,12 @@ extern "C" int gb_dot_cols(gpu_Context* ctx, int dtype, long n, const blk_cols* 
   gb_prof_rec pr;
   gb_prof_begin(ctx, &pr, GB_K_BLAS1);
   if (dtype == GPU_MV_FLOAT64)
-    dot_partial_kernel<double><<<grid, 256, 0, S(ctx)>>>(*X, *Y, n, partial);
+    gb_pdl(dot_partial_kernel<double>, grid, 256, 0, S(ctx), *X, *Y, n, partial);
   else if (cols_aligned16(X->col, w) && cols_aligned16(Y->col, w))
-    dot32_partial_kernel<<<grid, 256, 0, S(ctx)>>>(*X, *Y, n, partial);
+    gb_pdl(dot32_partial_kernel, grid, 256, 0, S(ctx), *X, *Y, n, partial);
   else
-    dot_partial_kernel<float><<<grid, 256, 0, S(ctx)>>>(*X, *Y, n, partial);
-  dot_reduce_kernel<<<w, 256, 0, S(ctx)>>>(partial, nb, t, out);
+    gb_pdl(dot_partial_kernel<float>, grid, 256, 0, S(ctx), *X, *Y, n, partial);
+  gb_pdl(dot_reduce_kernel, w, 256, 0, S(ctx), partial, nb, t, out);
   gb_prof_end(ctx, &pr, (dtype == GPU_MV_FLOAT64 ? 8.0 : 4.0) * n * w * 2, 2.0 * n * w);
   gb_count_launch(2);
   return CUDA_LAUNCH_CHECK(ctx, "dot_cols");
@@ -747,6 +758,7 @@ __global__ void residual_partial_kernel(blk_cols BX, blk_cols AX, const double* 
                                         idx_table idx, blk_cols R, long n,
                                         double* __restrict__ partial)
 {
+  gb_pdl_entry();
   // T: arithmetic and input type; the residual is stored as TO (FP32 for the
   // FP64-accumulated explicit phase: its norm is taken before the rounding)
   using TO = typename rr_out<T, OUT32>::type;
@@ -778,12 +790,12 @@ extern "C" int gb_residual(gpu_Context* ctx, int dtype, long n, const blk_cols* 
   gb_prof_rec pr;
   gb_prof_begin(ctx, &pr, GB_K_RESID);
   if (dtype == GPU_MV_FLOAT64)
-    residual_partial_kernel<double><<<grid, 256, 0, S(ctx)>>>(*BX, *AX, lambda, t, *R, n, partial);
+    gb_pdl(residual_partial_kernel<double>, grid, 256, 0, S(ctx), *BX, *AX, lambda, t, *R, n, partial);
   else if (dtype == GPU_MV_FLOAT32)
-    residual_partial_kernel<float><<<grid, 256, 0, S(ctx)>>>(*BX, *AX, lambda, t, *R, n, partial);
+    gb_pdl(residual_partial_kernel<float>, grid, 256, 0, S(ctx), *BX, *AX, lambda, t, *R, n, partial);
   else  // FP64 inputs, FP32 residual
-    residual_partial_kernel<double, 1><<<grid, 256, 0, S(ctx)>>>(*BX, *AX, lambda, t, *R, n, partial);
-  dot_reduce_kernel<<<w, 256, 0, S(ctx)>>>(partial, nb, t, norm2);
+    gb_pdl(residual_partial_kernel<double, 1>, grid, 256, 0, S(ctx), *BX, *AX, lambda, t, *R, n, partial);
+  gb_pdl(dot_reduce_kernel, w, 256, 0, S(ctx), partial, nb, t, norm2);
   gb_prof_end(ctx, &pr, (dtype == GPU_MV_FLOAT32 ? 12.0 : (dtype == GPU_MV_FLOAT64 ? 24.0 : 20.0)) * n * w,
               4.0 * n * w);
   gb_count_launch(2);
@@ -795,6 +807,7 @@ extern "C" int gb_residual(gpu_Context* ctx, int dtype, long n, const blk_cols* 
 // relative to its own size) and its FP32 shadow
 __global__ void acc64_kernel(blk_cols X, blk_cols D, blk_cols Y, long n)
 {
+  gb_pdl_entry();
   const double* x = (const double*)X.col[blockIdx.y];
   float* d = (float*)D.col[blockIdx.y];
   double* y = (double*)Y.col[blockIdx.y];
@@ -812,7 +825,7 @@ extern "C" int gb_accumulate64(gpu_Context* ctx, long n, const blk_cols* X64, co
   dim3 grid(row_blocks(ctx, n, w), w);
   gb_prof_rec pr;
   gb_prof_begin(ctx, &pr, GB_K_BLAS1);
-  acc64_kernel<<<grid, 256, 0, S(ctx)>>>(*X64, *D32, *Y64, n);
+  gb_pdl(acc64_kernel, grid, 256, 0, S(ctx), *X64, *D32, *Y64, n);
   gb_prof_end(ctx, &pr, 24.0 * n * w, (double)n * w);
   gb_count_launch(1);
   return CUDA_LAUNCH_CHECK(ctx, "accumulate64");
@@ -836,6 +849,7 @@ __global__ void split_pencil_kernel(const double* __restrict__ Hx, const double*
                                     double* G, double* H, int ld, const double* __restrict__ lam,
                                     int k, int nR, int nP)
 {
+  gb_pdl_entry();
   const int m = k + nR + nP;
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= m * m) return;
@@ -878,13 +892,14 @@ extern "C" int gb_split_pencil(gpu_Context* ctx, const double* Hx, const double*
                                int nR, int nP)
 {
   const int m = k + nR + nP;
-  split_pencil_kernel<<<(m * m + 255) / 256, 256, 0, S(ctx)>>>(Hx, Hr, Hp, Gt, G, H, ld, lam, k, nR, nP);
+  gb_pdl(split_pencil_kernel, (m * m + 255) / 256, 256, 0, S(ctx), Hx, Hr, Hp, Gt, G, H, ld, lam, k, nR, nP);
   gb_count_launch(1);
   return CUDA_LAUNCH_CHECK(ctx, "split pencil");
 }
 
 __global__ void rayleigh_kernel(int w, const double* num, const double* den, double* lam)
 {
+  gb_pdl_entry();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < w) lam[i] = den[i] > 0.0 ? num[i] / den[i] : 0.0;
 }
@@ -896,7 +911,7 @@ extern "C" int gb_rayleigh_quotients(gpu_Context* ctx, int dtype, long n, const 
   for (int c = 0; c < w; c++) idx[c] = c;
   if (gb_dot_cols(ctx, dtype, n, X, AX, w, scratch, idx)) return -1;
   if (gb_dot_cols(ctx, dtype, n, X, X, w, scratch + w, idx)) return -1;
-  rayleigh_kernel<<<(w + 127) / 128, 128, 0, S(ctx)>>>(w, scratch, scratch + w, lam);
+  gb_pdl(rayleigh_kernel, (w + 127) / 128, 128, 0, S(ctx), w, scratch, scratch + w, lam);
   gb_count_launch(1);
   return CUDA_LAUNCH_CHECK(ctx, "rayleigh quotients");
 }
@@ -904,6 +919,7 @@ extern "C" int gb_rayleigh_quotients(gpu_Context* ctx, int dtype, long n, const 
 template <typename TI, typename TO>
 __global__ void convert_kernel(blk_cols X, blk_cols Y, long n)
 {
+  gb_pdl_entry();
   const TI* x = (const TI*)X.col[blockIdx.y];
   TO* y = (TO*)Y.col[blockIdx.y];
   for (long r = blockIdx.x * (long)blockDim.x + threadIdx.x; r < n; r += (long)gridDim.x * blockDim.x)
@@ -918,13 +934,13 @@ extern "C" int gb_convert(gpu_Context* ctx, long n, int dtype_x, const blk_cols*
   gb_prof_rec pr;
   gb_prof_begin(ctx, &pr, GB_K_BLAS1);
   if (dtype_x == GPU_MV_FLOAT64 && dtype_y == GPU_MV_FLOAT32)
-    convert_kernel<double, float><<<grid, 256, 0, S(ctx)>>>(*X, *Y, n);
+    gb_pdl(convert_kernel<double, float>, grid, 256, 0, S(ctx), *X, *Y, n);
   else if (dtype_x == GPU_MV_FLOAT32 && dtype_y == GPU_MV_FLOAT64)
-    convert_kernel<float, double><<<grid, 256, 0, S(ctx)>>>(*X, *Y, n);
+    gb_pdl(convert_kernel<float, double>, grid, 256, 0, S(ctx), *X, *Y, n);
   else if (dtype_x == GPU_MV_FLOAT64)
-    convert_kernel<double, double><<<grid, 256, 0, S(ctx)>>>(*X, *Y, n);
+    gb_pdl(convert_kernel<double, double>, grid, 256, 0, S(ctx), *X, *Y, n);
   else
-    convert_kernel<float, float><<<grid, 256, 0, S(ctx)>>>(*X, *Y, n);
+    gb_pdl(convert_kernel<float, float>, grid, 256, 0, S(ctx), *X, *Y, n);
   gb_prof_end(ctx, &pr, ((dtype_x == GPU_MV_FLOAT64 ? 8.0 : 4.0) + (dtype_y == GPU_MV_FLOAT64 ? 8.0 : 4.0)) * n * w, 0.0);
   gb_count_launch(1);
   return CUDA_LAUNCH_CHECK(ctx, "convert");
@@ -954,6 +970,7 @@ template <typename T>
 __global__ void drand48_kernel(T* data, long n, long ld, idx_table idx, int w,
                                unsigned long long state0, lcg_table tab)
 {
+  gb_pdl_entry();
   const unsigned long long M = (1ULL << 48) - 1;
   const unsigned long long A = 0x5DEECE66DULL, Cc = 0xBULL;
   long total = n * (long)w;
@@ -992,9 +1009,9 @@ extern "C" int gb_drand48_fill(gpu_Context* ctx, int dtype, void* data, long n, 
   long threads = (total + 63) / 64;
   unsigned blocks = (unsigned)((threads + 255) / 256);
   if (dtype == GPU_MV_FLOAT64)
-    drand48_kernel<double><<<blocks, 256, 0, S(ctx)>>>((double*)data, n, ld, t, w, state0, tab);
+    gb_pdl(drand48_kernel<double>, blocks, 256, 0, S(ctx), (double*)data, n, ld, t, w, state0, tab);
   else
-    drand48_kernel<float><<<blocks, 256, 0, S(ctx)>>>((float*)data, n, ld, t, w, state0, tab);
+    gb_pdl(drand48_kernel<float>, blocks, 256, 0, S(ctx), (float*)data, n, ld, t, w, state0, tab);
   gb_count_launch(1);
   return CUDA_LAUNCH_CHECK(ctx, "drand48_fill");
 }

@@ -19,6 +19,7 @@
 #include <math.h>
 
 #include "internal.h"
+#include "pdl.cuh"
 
 static inline cudaStream_t S(gpu_Context* ctx) { return (cudaStream_t)ctx->stream; }
 
@@ -104,6 +105,7 @@ __global__ void __launch_bounds__(DENSE_THREADS) cholqr_factor_kernel(double* A,
                                                                       int* info, double* W,
                                                                       int force_fail, int smem)
 {
+  gb_pdl_entry();
   extern __shared__ double sh[];
   double* U = A;
   int ldu = ld;
@@ -144,6 +146,7 @@ __global__ void __launch_bounds__(DENSE_THREADS) chol_deflate_kernel(double* A, 
                                                                      double tol, int* dropped,
                                                                      int* ndrop, double* W)
 {
+  gb_pdl_entry();
   __shared__ int s_drop;
   __shared__ int s_cnt;
   const int tid = threadIdx.x, nt = blockDim.x;
@@ -198,7 +201,7 @@ extern "C" int gb_chol_deflate(gpu_Context* ctx, double* A, int ld, int m, doubl
 {
   double* W = (double*)gb_workspace(ctx, sizeof(double) * (size_t)m * m + 64);
   if (!W) return -1;
-  chol_deflate_kernel<<<1, DENSE_THREADS, 0, S(ctx)>>>(A, ld, m, tol, dropped, ndrop, W);
+  gb_pdl(chol_deflate_kernel, 1, DENSE_THREADS, 0, S(ctx), A, ld, m, tol, dropped, ndrop, W);
   gb_count_launch(1);
   return gb_cuda_check(ctx, (int)cudaGetLastError(), "chol_deflate");
 }
@@ -211,6 +214,7 @@ extern "C" int gb_chol_deflate(gpu_Context* ctx, double* A, int ld, int m, doubl
 __global__ void deflate_pencil_kernel(double* G, double* H, int ld, int mtot, int off, int m,
                                       const int* dropped, int kx)
 {
+  gb_pdl_entry();
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= m * mtot) return;
   const int j = e % m, o = e / m;
@@ -230,7 +234,7 @@ extern "C" int gb_deflate_pencil(gpu_Context* ctx, double* G, double* H, int ld,
                                  int m, const int* dropped, int kx)
 {
   if (m <= 0) return 0;
-  deflate_pencil_kernel<<<(m * mtot + 255) / 256, 256, 0, S(ctx)>>>(G, H, ld, mtot, off, m, dropped, kx);
+  gb_pdl(deflate_pencil_kernel, (m * mtot + 255) / 256, 256, 0, S(ctx), G, H, ld, mtot, off, m, dropped, kx);
   gb_count_launch(1);
   return gb_cuda_check(ctx, (int)cudaGetLastError(), "deflate_pencil");
 }
@@ -248,7 +252,7 @@ extern "C" int gb_cholqr_factor(gpu_Context* ctx, double* A, int ld, int m, int*
   if (smem > 48 * 1024 &&
       cudaFuncSetAttribute(cholqr_factor_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
     return gb_fail(ctx, "cholqr_factor: cannot reserve %d bytes of shared memory", smem);
-  cholqr_factor_kernel<<<1, DENSE_THREADS, smem, S(ctx)>>>(A, ld, m, info, W, force, smem > 0);
+  gb_pdl(cholqr_factor_kernel, 1, DENSE_THREADS, smem, S(ctx), A, ld, m, info, W, force, smem > 0);
   gb_prof_end(ctx, &pr, 16.0 * m * m, (double)m * m * m / 1.5);
   gb_count_launch(1);
   return gb_cuda_check(ctx, (int)cudaGetLastError(), "cholqr_factor");
@@ -265,6 +269,7 @@ __global__ void __launch_bounds__(DENSE_THREADS) sygv_kernel(double* A, double* 
                                                              double* V, int force_fail,
                                                              const int* gate, int* count)
 {
+  gb_pdl_entry();
   // gate: status word of the fast path; this solver runs only when the fast
   // path failed for a reason it can fix (5 = B not positive definite, which
   // the fast path has already reported through *info)
@@ -461,7 +466,7 @@ extern "C" int gb_sygv_fp64(gpu_Context* ctx, double* A, double* B, int ld, int 
   if (!scratch) return -1;
   gb_prof_rec pr;
   gb_prof_begin(ctx, &pr, gate ? GB_K_SYGV_FALLBACK : GB_K_SYGV);
-  sygv_kernel<<<1, DENSE_THREADS, 0, S(ctx)>>>(A, B, ld, m, w, info, scratch,
+  gb_pdl(sygv_kernel, 1, DENSE_THREADS, 0, S(ctx), A, B, ld, m, w, info, scratch,
                                                scratch + (size_t)m * m, force, gate,
                                                ctx->dcount);
   gb_prof_end(ctx, &pr, 32.0 * m * m, 0.0);
@@ -472,6 +477,7 @@ extern "C" int gb_sygv_fp64(gpu_Context* ctx, double* A, double* B, int ld, int 
 // --------------------------------------------------------------- helpers
 __global__ void small_symmetrize_kernel(double* A, int ld, int m)
 {
+  gb_pdl_entry();
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < m * m; e += gridDim.x * blockDim.x) {
     int i = e % m, j = e / m;
     if (i > j) {
@@ -484,6 +490,7 @@ __global__ void small_symmetrize_kernel(double* A, int ld, int m)
 
 __global__ void small_identity_kernel(double* A, int ld, int h, int w)
 {
+  gb_pdl_entry();
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < h * w; e += gridDim.x * blockDim.x) {
     int i = e % h, j = e / h;
     A[i + (size_t)j * ld] = (i == j) ? 1.0 : 0.0;
@@ -492,6 +499,7 @@ __global__ void small_identity_kernel(double* A, int ld, int h, int w)
 
 __global__ void small_diag_kernel(double* A, int ld, int m, const double* d)
 {
+  gb_pdl_entry();
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < m * m; e += gridDim.x * blockDim.x) {
     int i = e % m, j = e / m;
     A[i + (size_t)j * ld] = (i == j) ? d[i] : 0.0;
@@ -506,6 +514,7 @@ __global__ void __launch_bounds__(SGEMM_TM * SGEMM_TN) small_gemm_kernel(const d
                                                                          const double* B, int ldb, int tb, double* C,
                                                                          int ldc, int h, int w, int l)
 {
+  gb_pdl_entry();
   __shared__ double As[SGEMM_TM][33], Bs[SGEMM_TN][33];
   const int tx = threadIdx.x % SGEMM_TN, ty = threadIdx.x / SGEMM_TN;
   const int i0 = blockIdx.x * SGEMM_TM, j0 = blockIdx.y * SGEMM_TN;
@@ -539,7 +548,7 @@ static unsigned small_blocks(int count)
 extern "C" int gb_small_symmetrize(gpu_Context* ctx, double* A, int ld, int m)
 {
   if (m <= 1) return 0;
-  small_symmetrize_kernel<<<small_blocks(m * m), 256, 0, S(ctx)>>>(A, ld, m);
+  gb_pdl(small_symmetrize_kernel, small_blocks(m * m), 256, 0, S(ctx), A, ld, m);
   gb_count_launch(1);
   return gb_cuda_check(ctx, (int)cudaGetLastError(), "symmetrize");
 }
@@ -547,13 +556,14 @@ extern "C" int gb_small_symmetrize(gpu_Context* ctx, double* A, int ld, int m)
 extern "C" int gb_small_identity(gpu_Context* ctx, double* A, int ld, int h, int w)
 {
   if (h <= 0 || w <= 0) return 0;
-  small_identity_kernel<<<small_blocks(h * w), 256, 0, S(ctx)>>>(A, ld, h, w);
+  gb_pdl(small_identity_kernel, small_blocks(h * w), 256, 0, S(ctx), A, ld, h, w);
   gb_count_launch(1);
   return gb_cuda_check(ctx, (int)cudaGetLastError(), "identity");
 }
 
 __global__ void small_add_diag_kernel(double* A, int ld, int m, double alpha)
 {
+  gb_pdl_entry();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < m) A[i + (size_t)i * ld] += alpha;
 }
@@ -561,7 +571,7 @@ __global__ void small_add_diag_kernel(double* A, int ld, int m, double alpha)
 extern "C" int gb_small_add_diag(gpu_Context* ctx, double* A, int ld, int m, double alpha)
 {
   if (m <= 0) return 0;
-  small_add_diag_kernel<<<(m + 255) / 256, 256, 0, S(ctx)>>>(A, ld, m, alpha);
+  gb_pdl(small_add_diag_kernel, (m + 255) / 256, 256, 0, S(ctx), A, ld, m, alpha);
   gb_count_launch(1);
   return gb_cuda_check(ctx, (int)cudaGetLastError(), "add_diag");
 }
@@ -569,7 +579,7 @@ extern "C" int gb_small_add_diag(gpu_Context* ctx, double* A, int ld, int m, dou
 extern "C" int gb_small_diag(gpu_Context* ctx, double* A, int ld, int m, const double* d)
 {
   if (m <= 0) return 0;
-  small_diag_kernel<<<small_blocks(m * m), 256, 0, S(ctx)>>>(A, ld, m, d);
+  gb_pdl(small_diag_kernel, small_blocks(m * m), 256, 0, S(ctx), A, ld, m, d);
   gb_count_launch(1);
   return gb_cuda_check(ctx, (int)cudaGetLastError(), "diag");
 }
@@ -579,7 +589,7 @@ extern "C" int gb_small_gemm(gpu_Context* ctx, const double* A, int lda, int ta,
 {
   if (h <= 0 || w <= 0) return 0;
   const dim3 grid((h + SGEMM_TM - 1) / SGEMM_TM, (w + SGEMM_TN - 1) / SGEMM_TN);
-  small_gemm_kernel<<<grid, SGEMM_TM * SGEMM_TN, 0, S(ctx)>>>(A, lda, ta, B, ldb, tb, C, ldc, h, w, l);
+  gb_pdl(small_gemm_kernel, grid, SGEMM_TM * SGEMM_TN, 0, S(ctx), A, lda, ta, B, ldb, tb, C, ldc, h, w, l);
   gb_count_launch(1);
   return gb_cuda_check(ctx, (int)cudaGetLastError(), "small_gemm");
 }
@@ -591,6 +601,7 @@ extern "C" int gb_small_gemm(gpu_Context* ctx, const double* A, int lda, int ta,
 __global__ void scale_pencil_kernel(const double* G, const double* H, double* Gs, double* Hs,
                                     double* d, int ld, int m)
 {
+  gb_pdl_entry();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
     double h = H[i + (size_t)i * ld];
     d[i] = h > 0.0 ? 1.0 / sqrt(h) : 1.0;
@@ -609,7 +620,7 @@ __global__ void scale_pencil_kernel(const double* G, const double* H, double* Gs
 extern "C" int gb_scale_pencil(gpu_Context* ctx, const double* G, const double* H, double* Gs,
                                double* Hs, double* d, int ld, int m)
 {
-  scale_pencil_kernel<<<1, 1024, 0, S(ctx)>>>(G, H, Gs, Hs, d, ld, m);
+  gb_pdl(scale_pencil_kernel, 1, 1024, 0, S(ctx), G, H, Gs, Hs, d, ld, m);
   gb_count_launch(1);
   return gb_cuda_check(ctx, (int)cudaGetLastError(), "scale_pencil");
 }
@@ -617,6 +628,7 @@ extern "C" int gb_scale_pencil(gpu_Context* ctx, const double* G, const double* 
 // C(0:m, 0:k) = D C (undo the scaling of the eigenvector coordinates)
 __global__ void scale_rows_kernel(double* C, const double* d, int ld, int m, int k)
 {
+  gb_pdl_entry();
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < m * k; e += gridDim.x * blockDim.x) {
     int i = e % m, j = e / m;
     C[i + (size_t)j * ld] *= d[i];
@@ -625,13 +637,14 @@ __global__ void scale_rows_kernel(double* C, const double* d, int ld, int m, int
 
 extern "C" int gb_scale_rows(gpu_Context* ctx, double* C, const double* d, int ld, int m, int k)
 {
-  scale_rows_kernel<<<small_blocks(m * k), 256, 0, S(ctx)>>>(C, d, ld, m, k);
+  gb_pdl(scale_rows_kernel, small_blocks(m * k), 256, 0, S(ctx), C, d, ld, m, k);
   gb_count_launch(1);
   return gb_cuda_check(ctx, (int)cudaGetLastError(), "scale_rows");
 }
 
 __global__ void small_copy_kernel(const double* A, int lda, double* B, int ldb, int h, int w)
 {
+  gb_pdl_entry();
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < h * w; e += gridDim.x * blockDim.x) {
     int i = e % h, j = e / h;
     B[i + (size_t)j * ldb] = A[i + (size_t)j * lda];
@@ -642,7 +655,7 @@ extern "C" int gb_small_copy(gpu_Context* ctx, const double* A, int lda, double*
                              int w)
 {
   if (h <= 0 || w <= 0) return 0;
-  small_copy_kernel<<<small_blocks(h * w), 256, 0, S(ctx)>>>(A, lda, B, ldb, h, w);
+  gb_pdl(small_copy_kernel, small_blocks(h * w), 256, 0, S(ctx), A, lda, B, ldb, h, w);
   gb_count_launch(1);
   return gb_cuda_check(ctx, (int)cudaGetLastError(), "small_copy");
 }

@@ -32,6 +32,7 @@
 #include "internal.h"
 #include "tc_common.cuh"
 #include "blas32.cuh"
+#include "pdl.cuh"
 
 enum { OPK_CSR = 1, OPK_ST7 = 2, OPK_ST5 = 3, OPK_ST27 = 4, OPK_DIAG = 5, OPK_PCG = 6 };
 
@@ -84,6 +85,7 @@ __global__ void __launch_bounds__(256) csr_kernel(long n, const int* __restrict_
                                                   const V* __restrict__ vals, blk_cols X,
                                                   blk_cols Y, int w)
 {
+  gb_pdl_entry();
   long r = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (r >= n) return;
   const int p0 = rowptr[r], p1 = rowptr[r + 1];
@@ -118,6 +120,7 @@ __global__ void __launch_bounds__(256) csr32_kernel(long n, const int* __restric
                                                     const __grid_constant__ blk_cols X,
                                                     const __grid_constant__ blk_cols Y, int w)
 {
+  gb_pdl_entry();
   const long r = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (r >= n) return;
   const int p0 = rowptr[r], len = rowptr[r + 1] - p0;
@@ -175,6 +178,7 @@ __global__ void __launch_bounds__(ST_TX* ST_TY) st7_kernel(int nx, int ny, int n
                                                            const A* __restrict__ cz, A shift,
                                                            blk_cols X, blk_cols Y, int w)
 {
+  gb_pdl_entry();
   const int tiles_x = (nx + ST_TX - 1) / ST_TX, tiles_y = (ny + ST_TY - 1) / ST_TY;
   const long b = blockIdx.x;
   const int tile = (int)(b % ((long)tiles_x * tiles_y));
@@ -261,6 +265,7 @@ __global__ void __launch_bounds__(256) st7_ring_kernel(int nx, int ny, int nz,
                                                        const __grid_constant__ blk_cols X,
                                                        const __grid_constant__ blk_cols Y, int w)
 {
+  gb_pdl_entry();
   __shared__ __align__(16) float ring[ST7R_DEPTH * ST7R_SLOT];
   const int t = threadIdx.x, tx = t & 31, ty = t >> 5;
   const int tiles_x = (nx + 31) / 32, tiles_y = (ny + 31) / 32;
@@ -461,6 +466,7 @@ __global__ void __launch_bounds__(256, NP == 1 ? 4 : 3) st7_tma_kernel(
     const __grid_constant__ CUtensorMap tm_z, const __grid_constant__ st7t_cols XC,
     const __grid_constant__ blk_cols Y, int wall, int cpg, int strip, int yvec, int* err, double* __restrict__ dotp)
 {
+  gb_pdl_entry();
   using C = st7t_cfg<NP>;
   extern __shared__ float ring_raw[];
   float* ring = ring_raw + ((128u - (smem_u32(ring_raw) & 127u)) & 127u) / 4;
@@ -622,6 +628,7 @@ __global__ void __launch_bounds__(256) st5_kernel(int nx, int ny, const T* __res
                                                   const T* __restrict__ cy, T shift, blk_cols X,
                                                   blk_cols Y, int w)
 {
+  gb_pdl_entry();
   long c = blockIdx.x * (long)blockDim.x + threadIdx.x;
   long n = (long)nx * ny;
   if (c >= n) return;
@@ -649,6 +656,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) st27_kernel(int nx, int ny, int nz, const T* __restrict__ wt,
                                                    T shift, blk_cols X, blk_cols Y, int w)
 {
+  gb_pdl_entry();
   long c = blockIdx.x * (long)blockDim.x + threadIdx.x;
   const long n = (long)nx * ny * nz;
   if (c >= n) return;
@@ -741,6 +749,7 @@ __global__ void __launch_bounds__(32 * ST27T_ROWS, ST27T_MINB)
                     const __grid_constant__ CUtensorMap tm, const __grid_constant__ st7t_cols XC,
                     const __grid_constant__ blk_cols Y, int wall, int cpg, int strip, int* err)
 {
+  gb_pdl_entry();
   using C = st27t_cfg<NZ>;
   extern __shared__ float ring_raw[];
   float* ring = ring_raw + ((128u - (smem_u32(ring_raw) & 127u)) & 127u) / 4;
@@ -856,6 +865,7 @@ __global__ void __launch_bounds__(32 * ST27T_ROWS, ST27T_MINB)
 template <typename T, typename V>
 __global__ void diag_kernel(long n, const V* __restrict__ d, blk_cols X, blk_cols Y)
 {
+  gb_pdl_entry();
   const T* x = (const T*)X.col[blockIdx.y];
   T* y = (T*)Y.col[blockIdx.y];
   for (long r = blockIdx.x * (long)blockDim.x + threadIdx.x; r < n; r += (long)gridDim.x * blockDim.x)
@@ -866,6 +876,7 @@ __global__ void diag_kernel(long n, const V* __restrict__ d, blk_cols X, blk_col
 template <typename TI, typename TO>
 __global__ void cast_kernel(const TI* __restrict__ a, TO* __restrict__ b, long n)
 {
+  gb_pdl_entry();
   for (long r = blockIdx.x * (long)blockDim.x + threadIdx.x; r < n; r += (long)gridDim.x * blockDim.x)
     b[r] = (TO)a[r];
 }
@@ -1164,7 +1175,7 @@ static void st27t_launch(gpu_Operator* op, const CUtensorMap& tm, const st7t_col
   if (groups < 1) groups = 1;
   const int cpg = (int)((w + groups - 1) / groups);
   const dim3 grid((unsigned)ctas, (unsigned)((w + cpg - 1) / cpg));
-  st27_tma_kernel<ST27T_NZ><<<grid, 32 * ST27T_ROWS, st27t_cfg<ST27T_NZ>::SMEM, S(ctx)>>>(
+  gb_pdl(st27_tma_kernel<ST27T_NZ>, grid, 32 * ST27T_ROWS, st27t_cfg<ST27T_NZ>::SMEM, S(ctx), 
       op->nx, op->ny, op->nz, op->w32, (float)op->shift, tm, pc, yc, w, cpg, strip, ctx->dcount + 5);
 }
 
@@ -1201,7 +1212,7 @@ static int st7t_launch(gpu_Operator* op, const CUtensorMap& tmc, const CUtensorM
   const int cpg = (int)((w + groups - 1) / groups);
   const int tiles_x = (op->nx + 31) / 32, strip = tiles_x < ST7T_STRIP ? ST7T_STRIP / tiles_x : 1;
   const dim3 grid((unsigned)ctas, (unsigned)((w + cpg - 1) / cpg));
-  st7_tma_kernel<NP, DOT><<<grid, 256, smem, S(ctx)>>>(op->nx, op->ny, op->nz, op->c32[0], op->c32[1], op->c32[2],
+  gb_pdl(st7_tma_kernel<NP, DOT>, grid, 256, smem, S(ctx), op->nx, op->ny, op->nz, op->c32[0], op->c32[1], op->c32[2],
                                                        (float)op->shift, tmc, tmz, pc, yc, w, cpg, strip, yvec,
                                                        ctx->dcount + 5, dparts);
   return 0;
@@ -1214,6 +1225,7 @@ __global__ void __launch_bounds__(256) st7t_dot_reduce_kernel(const double* __re
                                                               const double* __restrict__ num,
                                                               double* __restrict__ ratio)
 {
+  gb_pdl_entry();
   const double* p = parts + (size_t)blockIdx.x * nparts;
   double acc = 0.0;
 #pragma unroll 4
@@ -1315,19 +1327,19 @@ static int operator_apply(gpu_Operator* op, gpu_MultiVector* X, gpu_MultiVector*
   switch (op->kind) {
     case OPK_CSR:
       if (acc64)
-        csr_kernel<float, double, double><<<blocks, 256, 0, S(ctx)>>>(n, op->rowptr, op->colidx,
+        gb_pdl(csr_kernel<float, double, double>, blocks, 256, 0, S(ctx), n, op->rowptr, op->colidx,
                                                                       op->vals, xc, yc, w);
       else if (f32)
-        csr32_kernel<<<blocks, 256, 0, S(ctx)>>>(n, op->rowptr, op->colidx, op->vals32, xc, yc, w);
+        gb_pdl(csr32_kernel, blocks, 256, 0, S(ctx), n, op->rowptr, op->colidx, op->vals32, xc, yc, w);
       else
-        csr_kernel<double, double><<<blocks, 256, 0, S(ctx)>>>(n, op->rowptr, op->colidx,
+        gb_pdl(csr_kernel<double, double>, blocks, 256, 0, S(ctx), n, op->rowptr, op->colidx,
                                                                op->vals, xc, yc, w);
       break;
     case OPK_ST7: {
       const unsigned tb = (unsigned)(((op->nx + ST_TX - 1) / ST_TX) * ((op->ny + ST_TY - 1) / ST_TY) *
                                      (long)op->nz);
       if (acc64)
-        st7_kernel<float, double><<<tb, ST_TX * ST_TY, 0, S(ctx)>>>(op->nx, op->ny, op->nz, op->c[0],
+        gb_pdl(st7_kernel<float, double>, tb, ST_TX * ST_TY, 0, S(ctx), op->nx, op->ny, op->nz, op->c[0],
                                                                     op->c[1], op->c[2], op->shift,
                                                                     xc, yc, w);
       else if (tma) {
@@ -1342,28 +1354,27 @@ static int operator_apply(gpu_Operator* op, gpu_MultiVector* X, gpu_MultiVector*
                                           : st7t_launch<2, false>(op, tmc, tmz, pc, yc, w, yvec, NULL));
         if (rc) return rc;
         if (dot_out) {
-          st7t_dot_reduce_kernel<<<w, 256, 0, S(ctx)>>>(dparts, nparts, dot_out, num, ratio);
+          gb_pdl(st7t_dot_reduce_kernel, w, 256, 0, S(ctx), dparts, nparts, dot_out, num, ratio);
           gb_count_launch(1);
         }
       } else if (f32 && st7_ring_ok(op, &xc, w))
-        st7_ring_kernel<<<(unsigned)(((op->nx + 31) / 32) * ((op->ny + 31) / 32) * (long)op->nz), 256,
-                          0, S(ctx)>>>(op->nx, op->ny, op->nz, op->c32[0], op->c32[1],
+        gb_pdl(st7_ring_kernel, (unsigned)(((op->nx + 31) / 32) * ((op->ny + 31) / 32) * (long)op->nz), 256, 0, S(ctx), op->nx, op->ny, op->nz, op->c32[0], op->c32[1],
                                                 op->c32[2], (float)op->shift, xc, yc, w);
       else if (f32)
-        st7_kernel<float><<<tb, ST_TX * ST_TY, 0, S(ctx)>>>(op->nx, op->ny, op->nz, op->c32[0],
+        gb_pdl(st7_kernel<float>, tb, ST_TX * ST_TY, 0, S(ctx), op->nx, op->ny, op->nz, op->c32[0],
                                                             op->c32[1], op->c32[2], (float)op->shift,
                                                             xc, yc, w);
       else
-        st7_kernel<double><<<tb, ST_TX * ST_TY, 0, S(ctx)>>>(op->nx, op->ny, op->nz, op->c[0],
+        gb_pdl(st7_kernel<double>, tb, ST_TX * ST_TY, 0, S(ctx), op->nx, op->ny, op->nz, op->c[0],
                                                              op->c[1], op->c[2], op->shift, xc, yc, w);
     }
       break;
     case OPK_ST5:
       if (f32)
-        st5_kernel<float><<<blocks, 256, 0, S(ctx)>>>(op->nx, op->ny, op->c32[0], op->c32[1],
+        gb_pdl(st5_kernel<float>, blocks, 256, 0, S(ctx), op->nx, op->ny, op->c32[0], op->c32[1],
                                                       (float)op->shift, xc, yc, w);
       else
-        st5_kernel<double><<<blocks, 256, 0, S(ctx)>>>(op->nx, op->ny, op->c[0], op->c[1],
+        gb_pdl(st5_kernel<double>, blocks, 256, 0, S(ctx), op->nx, op->ny, op->c[0], op->c[1],
                                                        op->shift, xc, yc, w);
       break;
     case OPK_ST27:
@@ -1374,10 +1385,10 @@ static int operator_apply(gpu_Operator* op, gpu_MultiVector* X, gpu_MultiVector*
           return gb_fail(ctx, "stencil27: cannot set the wait limit");
         st27t_launch(op, tmc, pc, yc, w);
       } else if (f32)
-        st27_kernel<float><<<blocks, 256, 0, S(ctx)>>>(op->nx, op->ny, op->nz, op->w32,
+        gb_pdl(st27_kernel<float>, blocks, 256, 0, S(ctx), op->nx, op->ny, op->nz, op->w32,
                                                        (float)op->shift, xc, yc, w);
       else
-        st27_kernel<double><<<blocks, 256, 0, S(ctx)>>>(op->nx, op->ny, op->nz, op->w, op->shift,
+        gb_pdl(st27_kernel<double>, blocks, 256, 0, S(ctx), op->nx, op->ny, op->nz, op->w, op->shift,
                                                         xc, yc, w);
       break;
     case OPK_DIAG: {
@@ -1387,9 +1398,9 @@ static int operator_apply(gpu_Operator* op, gpu_MultiVector* X, gpu_MultiVector*
       if (want > cap) want = cap;
       dim3 grid((unsigned)want, w);
       if (f32)
-        diag_kernel<float, float><<<grid, 256, 0, S(ctx)>>>(n, op->d32, xc, yc);
+        gb_pdl(diag_kernel<float, float>, grid, 256, 0, S(ctx), n, op->d32, xc, yc);
       else
-        diag_kernel<double, double><<<grid, 256, 0, S(ctx)>>>(n, op->d, xc, yc);
+        gb_pdl(diag_kernel<double, double>, grid, 256, 0, S(ctx), n, op->d, xc, yc);
       break;
     }
     default:
@@ -1413,6 +1424,7 @@ extern "C" void gpu_OperatorApply(void* op, void* X, void* Y)
 __global__ void csr_diag_kernel(long n, const int* rowptr, const int* colidx, const double* vals,
                                 double* out)
 {
+  gb_pdl_entry();
   long r = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (r >= n) return;
   double d = 0.0;
@@ -1515,6 +1527,7 @@ __device__ __forceinline__ double grad_pair(const blk_cols& X, const blk_cols& W
 __global__ void grad_csr_kernel(long n, const int* __restrict__ rowptr, const int* __restrict__ colidx,
                                 blk_cols X, blk_cols W, int k, double* __restrict__ g)
 {
+  gb_pdl_entry();
   const long p = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (p >= n) return;
   for (int e = rowptr[p]; e < rowptr[p + 1]; e++) {
@@ -1530,6 +1543,7 @@ __global__ void grad_csr_kernel(long n, const int* __restrict__ rowptr, const in
 __global__ void grad_faces_kernel(int nx, int ny, int nz, int dir, blk_cols X, blk_cols W, int k,
                                   double* __restrict__ g)
 {
+  gb_pdl_entry();
   const int ex = nx + (dir == 0), ey = ny + (dir == 1), ez = nz + (dir == 2);
   const long nf = (long)ex * ey * ez;
   const long f = blockIdx.x * (long)blockDim.x + threadIdx.x;
@@ -1554,6 +1568,7 @@ __global__ void grad_faces_kernel(int nx, int ny, int nz, int dir, blk_cols X, b
 __global__ void grad_st27_kernel(int nx, int ny, int nz, blk_cols X, blk_cols W, int k,
                                  double* __restrict__ g)
 {
+  gb_pdl_entry();
   const long n = (long)nx * ny * nz;
   const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (t >= n * 13) return;
@@ -1571,6 +1586,7 @@ __global__ void grad_st27_kernel(int nx, int ny, int nz, blk_cols X, blk_cols W,
 __global__ void grad_diag_kernel(long n, blk_cols X, blk_cols W, int k, const double* lam,
                                  const double* xg, double* __restrict__ g)
 {
+  gb_pdl_entry();
   const long p = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (p >= n) return;
   double s = 0.0;
@@ -1695,6 +1711,7 @@ template <typename T>
 __global__ void pcg_cols_kernel(long n, int mode, blk_cols A, blk_cols B, blk_cols C, blk_cols D,
                                 const double* __restrict__ a)
 {
+  gb_pdl_entry();
   // mode 0: C_i = a_i A_i (first step: Y = alpha P), D_i -= a_i B_i
   // mode 1: C_i += a_i A_i,  D_i -= a_i B_i
   // mode 2: C_i = A_i + a_i C_i  (P = Z + beta P)
@@ -1716,6 +1733,7 @@ __global__ void pcg_cols_kernel(long n, int mode, blk_cols A, blk_cols B, blk_co
 
 __global__ void pcg_ratio_kernel(int k, const double* num, const double* den, double* out)
 {
+  gb_pdl_entry();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < k) out[i] = (den[i] != 0.0 && num[i] != 0.0) ? num[i] / den[i] : 0.0;
 }
@@ -1851,6 +1869,7 @@ template <typename T, bool HAVE_M>
 __global__ void PCG_BOUNDS(T)
     pcg_init_kernel(long n, blk_cols X, const T* __restrict__ m, blk_cols P, double* __restrict__ partial, pcg_coef k)
 {
+  gb_pdl_entry();
   typedef typename pcg_vec<T>::type V;
   constexpr int N = pcg_vec<T>::N;
   const int j = blockIdx.y;
@@ -1877,6 +1896,7 @@ template <typename T>
 __global__ void PCG_BOUNDS(T)
     pcg_dot_kernel(long n, blk_cols P, blk_cols Q, double* __restrict__ partial, pcg_coef k)
 {
+  gb_pdl_entry();
   typedef typename pcg_vec<T>::type V;
   constexpr int N = pcg_vec<T>::N;
   const int j = blockIdx.y;
@@ -1895,6 +1915,7 @@ template <typename T, bool HAVE_M>
 __global__ void PCG_BOUNDS(T) pcg_step_kernel(long n, blk_cols Q, blk_cols R0, blk_cols R, const T* __restrict__ m,
                                               double* __restrict__ partial, pcg_coef k)
 {
+  gb_pdl_entry();
   typedef typename pcg_vec<T>::type V;
   constexpr int N = pcg_vec<T>::N;
   const int j = blockIdx.y;
@@ -1923,6 +1944,7 @@ template <typename T, bool HAVE_M, bool FIRST>
 __global__ void PCG_BOUNDS(T)
     pcg_dir_kernel(long n, blk_cols R, const T* __restrict__ m, blk_cols P, blk_cols Y, int last, pcg_coef k)
 {
+  gb_pdl_entry();
   typedef typename pcg_vec<T>::type V;
   constexpr int N = pcg_vec<T>::N;
   const int j = blockIdx.y;
@@ -1985,7 +2007,7 @@ static int pcg_fused(gpu_Operator* op, const blk_cols* cx, const blk_cols* cy, c
   double* partial = (double*)gb_workspace(ctx, sizeof(double) * (size_t)grid.x * w);
   if (!partial) return -1;
   gb_prof_begin(ctx, &pr, GB_K_BLAS1);
-  pcg_init_kernel<T, HAVE_M><<<grid, 256, 0, st>>>(n, *cx, m, *cp, partial, k);
+  gb_pdl(pcg_init_kernel<T, HAVE_M>, grid, 256, 0, st, n, *cx, m, *cp, partial, k);
   gb_prof_end(ctx, &pr, 2.0 * blk + mb, 2.0 * n * w);
   gb_count_launch(1);
   for (int it = 0; it < op->iters; it++) {
@@ -1996,20 +2018,20 @@ static int pcg_fused(gpu_Operator* op, const blk_cols* cx, const blk_cols* cy, c
     if (!partial) return -1;
     if (fused == 1) {
       gb_prof_begin(ctx, &pr, GB_K_BLAS1);
-      pcg_dot_kernel<T><<<grid, 256, 0, st>>>(n, *cp, *cq, partial, k);
+      gb_pdl(pcg_dot_kernel<T>, grid, 256, 0, st, n, *cp, *cq, partial, k);
       gb_prof_end(ctx, &pr, 2.0 * blk, 2.0 * n * w);
       gb_count_launch(1);
     }
     const bool last = it + 1 == op->iters;
     gb_prof_begin(ctx, &pr, GB_K_BLAS1);
     if (!last) {
-      pcg_step_kernel<T, HAVE_M><<<grid, 256, 0, st>>>(n, *cq, it == 0 ? *cx : *cr, *cr, m, partial, k);
+      gb_pdl(pcg_step_kernel<T, HAVE_M>, grid, 256, 0, st, n, *cq, it == 0 ? *cx : *cr, *cr, m, partial, k);
       gb_count_launch(1);
     }
     if (it == 0)
-      pcg_dir_kernel<T, HAVE_M, true><<<grid, 256, 0, st>>>(n, *cr, m, *cp, *cy, last, k);
+      gb_pdl(pcg_dir_kernel<T, HAVE_M, true>, grid, 256, 0, st, n, *cr, m, *cp, *cy, last, k);
     else
-      pcg_dir_kernel<T, HAVE_M, false><<<grid, 256, 0, st>>>(n, *cr, m, *cp, *cy, last, k);
+      gb_pdl(pcg_dir_kernel<T, HAVE_M, false>, grid, 256, 0, st, n, *cr, m, *cp, *cy, last, k);
     // step: q, r -> r; dir: p, y (not the first time), r -> y, p; the last: p, y -> y
     gb_prof_end(ctx, &pr, (last ? 3.0 : 8.0) * blk - (it == 0 ? blk : 0.0) + (last ? 0.0 : 2.0 * mb),
                 (last ? 2.0 : 8.0) * n * w);

@@ -36,6 +36,7 @@
 #include <math.h>
 
 #include "internal.h"
+#include "pdl.cuh"
 
 static inline cudaStream_t S_(gpu_Context* ctx) { return (cudaStream_t)ctx->stream; }
 
@@ -74,6 +75,7 @@ __global__ void __launch_bounds__(RR_THREADS) rr_chol64_kernel(const double* __r
                                                                int m, rr_scratch s, int* info,
                                                                double report_below)
 {
+  gb_pdl_entry();
   extern __shared__ double Ls[];
   __shared__ double piv[RR_MAX_M];  // L_jj^2
   __shared__ int bad;
@@ -179,6 +181,7 @@ __global__ void __launch_bounds__(32) rr_trsm64_kernel(int mode, const double* _
                                                        int ldy, double* __restrict__ X, int ldx,
                                                        int m, int ncols, rr_scratch s)
 {
+  gb_pdl_entry();
   if (s.status[0]) return;
   const int lane = threadIdx.x;
   const int j = blockIdx.x;
@@ -261,6 +264,7 @@ __global__ void __launch_bounds__(32) rr_trsm64_kernel(int mode, const double* _
 // symmetrise the FP64 reduced matrix and make the FP32 copy for Jacobi
 __global__ void rr_sym_kernel(int m, rr_scratch s)
 {
+  gb_pdl_entry();
   if (s.status[0]) return;
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < m * m; e += gridDim.x * blockDim.x) {
     int i = e % m, j = e / m;
@@ -271,6 +275,7 @@ __global__ void rr_sym_kernel(int m, rr_scratch s)
 
 __global__ void rr_sym_store_kernel(int m, rr_scratch s)
 {
+  gb_pdl_entry();
   if (s.status[0]) return;
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < m * m; e += gridDim.x * blockDim.x) {
     int i = e % m, j = e / m;
@@ -390,6 +395,7 @@ __host__ __device__ __forceinline__ int rr_pad(int m) { return m | 1; }
 
 __global__ void __launch_bounds__(RR_THREADS) rr_jacobi32_kernel(int m, int rows, rr_scratch s)
 {
+  gb_pdl_entry();
   extern __shared__ float sm[];
   const int lc = rr_pad(m);
   float* Cs = sm;             // m x m, column-major, leading dimension lc
@@ -438,6 +444,7 @@ __global__ void __launch_bounds__(RR_THREADS) rr_jacobi32_kernel(int m, int rows
 // eigenvectors of C sorted by the FP32 eigenvalues, widened to FP64
 __global__ void __launch_bounds__(RR_THREADS) rr_vsort_kernel(int m, rr_scratch s)
 {
+  gb_pdl_entry();
   __shared__ int perm[512];
   const int tid = threadIdx.x, nt = blockDim.x;
   if (s.status[0]) return;
@@ -487,6 +494,7 @@ static dim3 rr_gemm_grid(int M, int N, int batch)
 __global__ void __launch_bounds__(RR_GEMM_TM * RR_GEMM_TN) rr_gemm_kernel(rr_gemm_t g0, rr_gemm_t g1,
                                                                           const int* status)
 {
+  gb_pdl_entry();
   if (status[0]) return;
   const rr_gemm_t g = blockIdx.z == 0 ? g0 : g1;
   __shared__ double As[RR_GEMM_TM][33], Bs[RR_GEMM_TN][33];
@@ -570,6 +578,7 @@ __device__ int rr_jacobi64(double* M, double* V, int c, int lm)
 
 __global__ void __launch_bounds__(RR_THREADS) rr_refine_kernel(int m, rr_scratch s, int last)
 {
+  gb_pdl_entry();
   extern __shared__ double csm[];  // 2 x RR_CLUSTER_SMEM x rr_pad(RR_CLUSTER_SMEM)
   __shared__ double lt[512];
   __shared__ int cstart[513];
@@ -705,6 +714,7 @@ __global__ void __launch_bounds__(RR_THREADS) rr_refine_kernel(int m, rr_scratch
 
 __global__ void rr_finish_kernel(int nev, rr_scratch s, double* w, int* info)
 {
+  gb_pdl_entry();
   if (s.status[0]) return;  // the FP64 fallback writes the outputs
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nev; i += gridDim.x * blockDim.x)
     w[i] = s.lam[i];
@@ -740,6 +750,7 @@ __device__ double rr_block_sum(double v, double* red)
 #define RR_TRD_THREADS 512
 __global__ void __launch_bounds__(RR_TRD_THREADS) rr_tridiag_kernel(int m, rr_scratch s)
 {
+  gb_pdl_entry();
   __shared__ double v[RR_MAX_M], p[RR_MAX_M];
   __shared__ double red[RR_TRD_THREADS / 32];
   __shared__ double sh_tau, sh_scale;
@@ -863,6 +874,7 @@ __device__ __forceinline__ void rr_trd_reflector(const double* Lp, int j, int m,
 //   order 57: 110 us against 152; order 72: 306 against 430.
 __global__ void __launch_bounds__(RR_TRD_THREADS) rr_tridiag_smem_kernel(int m, rr_scratch s)
 {
+  gb_pdl_entry();
   extern __shared__ double Lp[];  // packed lower triangle, m(m+1)/2
   __shared__ double v[RR_TRD_SMEM_M], p[RR_TRD_SMEM_M], buf[RR_TRD_SMEM_M];
   __shared__ double sh_sum, sh_tau[2], sh_scale[2];  // by step parity
@@ -1001,6 +1013,7 @@ static size_t rr_bisect_smem(int m) { return ((size_t)RR_BIS_WARPS * 32 + 2) * m
 
 __global__ void __launch_bounds__(32 * RR_BIS_WARPS) rr_bisect_kernel(int m, rr_scratch s)
 {
+  gb_pdl_entry();
   extern __shared__ int piv[];  // [RR_BIS_WARPS][m][32] pivots, then those at lo and at hi
   __shared__ double d[RR_MAX_M], e2[RR_MAX_M];
   __shared__ float d32[RR_MAX_M], e32[RR_MAX_M];
@@ -1113,6 +1126,7 @@ __device__ __forceinline__ double rr_start_value(int j, int i)
 // solves from a pseudo-random start; vector j into s.X (ld m)
 __global__ void __launch_bounds__(32) rr_invit_kernel(int m, rr_scratch s)
 {
+  gb_pdl_entry();
   __shared__ double u0i[RR_MAX_M], u1[RR_MAX_M], u2[RR_MAX_M], mu[RR_MAX_M], y[RR_MAX_M];
   __shared__ unsigned char sw[RR_MAX_M];
   __shared__ int bad;
@@ -1200,6 +1214,7 @@ __global__ void __launch_bounds__(32) rr_invit_kernel(int m, rr_scratch s)
 #define RR_CHOLINV_SMEM_M 112
 __global__ void __launch_bounds__(256) rr_cholinv_kernel(int nev, rr_scratch s, int smem)
 {
+  gb_pdl_entry();
   extern __shared__ double sh[];  // up to order RR_CHOLINV_SMEM_M: U, then its inverse
   __shared__ int bad;
   __shared__ double rinv;  // 1 / U_jj: by one thread, 8 warps' divisions at once take the FP64 pipe 1800 cycles
@@ -1268,6 +1283,7 @@ __global__ void __launch_bounds__(256) rr_cholinv_kernel(int nev, rr_scratch s, 
 template <int SL>
 __global__ void __launch_bounds__(32) rr_backtr_kernel(int m, int nev, rr_scratch s)
 {
+  gb_pdl_entry();
   if (s.status[0]) return;
   const int lane = threadIdx.x;
   const int j = blockIdx.x;
@@ -1329,7 +1345,7 @@ static void rr_trsm(cudaStream_t st, int mode, const double* Y, int ldy, double*
 {
   switch ((m + 31) / 32) {
 #define RR_TRSM_CASE(n) \
-  case n: rr_trsm64_kernel<n><<<ncols, 32, 0, st>>>(mode, Y, ldy, X, ldx, m, ncols, s); break;
+  case n: gb_pdl(rr_trsm64_kernel<n>, ncols, 32, 0, st, mode, Y, ldy, X, ldx, m, ncols, s); break;
     RR_SL_CASES(RR_TRSM_CASE)
 #undef RR_TRSM_CASE
   }
@@ -1339,7 +1355,7 @@ static void rr_backtr(cudaStream_t st, int m, int nev, const rr_scratch& s)
 {
   switch ((m + 31) / 32) {
 #define RR_BACKTR_CASE(n) \
-  case n: rr_backtr_kernel<n><<<nev, 32, 0, st>>>(m, nev, s); break;
+  case n: gb_pdl(rr_backtr_kernel<n>, nev, 32, 0, st, m, nev, s); break;
     RR_SL_CASES(RR_BACKTR_CASE)
 #undef RR_BACKTR_CASE
   }
@@ -1397,15 +1413,15 @@ static void rr_reduce(gpu_Context* ctx, double* A, double* B, int ld, int m, int
     const int sm = (int)(sizeof(double) * (size_t)m * m);
     cudaFuncSetAttribute(rr_chol64_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
     RR_STAGE(GB_K_RR_CHOL, m3 / 3,
-             (rr_chol64_kernel<true><<<1, RR_THREADS, sm, st>>>(B, ld, m, s, info, report_below)));
+             (gb_pdl(rr_chol64_kernel<true>, 1, RR_THREADS, sm, st, B, ld, m, s, info, report_below)));
   } else {
     RR_STAGE(GB_K_RR_CHOL, m3 / 3,
-             (rr_chol64_kernel<false><<<1, RR_THREADS, 0, st>>>(B, ld, m, s, info, report_below)));
+             (gb_pdl(rr_chol64_kernel<false>, 1, RR_THREADS, 0, st, B, ld, m, s, info, report_below)));
   }
   RR_STAGE(GB_K_RR_TRSM, m3, (rr_trsm(st, 0, A, ld, s.W64, m, m, m, s)));
   RR_STAGE(GB_K_RR_TRSM, m3, (rr_trsm(st, 1, s.W64, m, s.C64, m, m, m, s)));
-  if (jacobi32) rr_sym_kernel<<<(unsigned)((mm + 255) / 256), 256, 0, st>>>(m, s);
-  rr_sym_store_kernel<<<(unsigned)((mm + 255) / 256), 256, 0, st>>>(m, s);
+  if (jacobi32) gb_pdl(rr_sym_kernel, (unsigned)((mm + 255) / 256), 256, 0, st, m, s);
+  gb_pdl(rr_sym_store_kernel, (unsigned)((mm + 255) / 256), 256, 0, st, m, s);
   gb_count_launch(4 + jacobi32);
 }
 
@@ -1419,15 +1435,15 @@ static void rr_tridiag_path(gpu_Context* ctx, double* A, int ld, int m, int nev,
     const int sm = (int)(sizeof(double) * (size_t)m * (m + 1) / 2);
     cudaFuncSetAttribute(rr_tridiag_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
     RR_STAGE(GB_K_RR_TRID, 4.0 * m3 / 3.0,
-             (rr_tridiag_smem_kernel<<<1, RR_TRD_THREADS, sm, st>>>(m, s)));
+             (gb_pdl(rr_tridiag_smem_kernel, 1, RR_TRD_THREADS, sm, st, m, s)));
   } else {
-    RR_STAGE(GB_K_RR_TRID, 4.0 * m3 / 3.0, (rr_tridiag_kernel<<<1, RR_TRD_THREADS, 0, st>>>(m, s)));
+    RR_STAGE(GB_K_RR_TRID, 4.0 * m3 / 3.0, (gb_pdl(rr_tridiag_kernel, 1, RR_TRD_THREADS, 0, st, m, s)));
   }
   const int sb = (int)rr_bisect_smem(m);
   if (sb > 32 * 1024)
     cudaFuncSetAttribute(rr_bisect_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sb);
-  RR_STAGE(GB_K_RR_EIG, 0.0, (rr_bisect_kernel<<<nev, 32 * RR_BIS_WARPS, sb, st>>>(m, s)));
-  RR_STAGE(GB_K_RR_EIG, 0.0, (rr_invit_kernel<<<nev, 32, 0, st>>>(m, s)));
+  RR_STAGE(GB_K_RR_EIG, 0.0, (gb_pdl(rr_bisect_kernel, nev, 32 * RR_BIS_WARPS, sb, st, m, s)));
+  RR_STAGE(GB_K_RR_EIG, 0.0, (gb_pdl(rr_invit_kernel, nev, 32, 0, st, m, s)));
   // Cholesky-QR twice: Z <- Z inv(U), U'U = Z'Z
   const dim3 gs = rr_gemm_grid(nev, nev, 1), gz = rr_gemm_grid(m, nev, 1);
   const int sc = nev <= RR_CHOLINV_SMEM_M ? (int)(2 * sizeof(double) * (size_t)nev * nev) : 0;
@@ -1435,10 +1451,10 @@ static void rr_tridiag_path(gpu_Context* ctx, double* A, int ld, int m, int nev,
     cudaFuncSetAttribute(rr_cholinv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sc);
   for (int round = 0; round < 2; round++) {
     rr_gemm_t zz = {s.X, m, 1, s.X, m, s.S, nev, nev, nev, m};
-    RR_STAGE(GB_K_RR_GEMM, 2.0 * m * nev * nev, (rr_gemm_kernel<<<gs, RR_GEMM_TM * RR_GEMM_TN, 0, st>>>(zz, zz, s.status)));
-    RR_STAGE(GB_K_RR_EIG, 0.0, (rr_cholinv_kernel<<<1, 256, sc, st>>>(nev, s, sc > 0)));
+    RR_STAGE(GB_K_RR_GEMM, 2.0 * m * nev * nev, (gb_pdl(rr_gemm_kernel, gs, RR_GEMM_TM * RR_GEMM_TN, 0, st, zz, zz, s.status)));
+    RR_STAGE(GB_K_RR_EIG, 0.0, (gb_pdl(rr_cholinv_kernel, 1, 256, sc, st, nev, s, sc > 0)));
     rr_gemm_t zu = {s.X, m, 0, s.P, nev, s.Xn, m, m, nev, nev};
-    RR_STAGE(GB_K_RR_GEMM, 2.0 * m * nev * nev, (rr_gemm_kernel<<<gz, RR_GEMM_TM * RR_GEMM_TN, 0, st>>>(zu, zu, s.status)));
+    RR_STAGE(GB_K_RR_GEMM, 2.0 * m * nev * nev, (gb_pdl(rr_gemm_kernel, gz, RR_GEMM_TM * RR_GEMM_TN, 0, st, zu, zu, s.status)));
     double* t = s.X;
     s.X = s.Xn;
     s.Xn = t;
@@ -1446,7 +1462,7 @@ static void rr_tridiag_path(gpu_Context* ctx, double* A, int ld, int m, int nev,
   RR_STAGE(GB_K_RR_TRSM, 2.0 * m * m * nev, (rr_backtr(st, m, nev, s)));
   RR_STAGE(GB_K_RR_TRSM, (double)m * m * nev,
            (rr_trsm(st, 2, s.X, m, A, ld, m, nev, s)));
-  rr_finish_kernel<<<(unsigned)((nev + 255) / 256), 256, 0, st>>>(nev, s, w, info);
+  gb_pdl(rr_finish_kernel, (unsigned)((nev + 255) / 256), 256, 0, st, nev, s, w, info);
   gb_count_launch(12);
 }
 
@@ -1461,23 +1477,23 @@ static void rr_jacobi32_path(gpu_Context* ctx, double* A, int ld, int m, int nev
   const int rows = (m + nsplit - 1) / nsplit;
   const size_t sm_jac = ((size_t)m * rr_pad(m) + (size_t)rows * rr_pad(m)) * sizeof(float);
   cudaFuncSetAttribute(rr_jacobi32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_jac);
-  RR_STAGE(GB_K_RR_JAC32, 0.0, (rr_jacobi32_kernel<<<nsplit, RR_THREADS, sm_jac, st>>>(m, rows, s)));
-  rr_vsort_kernel<<<1, RR_THREADS, 0, st>>>(m, s);
+  RR_STAGE(GB_K_RR_JAC32, 0.0, (gb_pdl(rr_jacobi32_kernel, nsplit, RR_THREADS, sm_jac, st, m, rows, s)));
+  gb_pdl(rr_vsort_kernel, 1, RR_THREADS, 0, st, m, s);
   int launches = 2;
   const size_t sm_ref = 2 * sizeof(double) * RR_CLUSTER_SMEM * rr_pad(RR_CLUSTER_SMEM);
   cudaFuncSetAttribute(rr_refine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_ref);
   const dim3 g1 = rr_gemm_grid(m, m, 1), g2 = rr_gemm_grid(m, m, 2);
   for (int round = 0; round < 2; round++) {
     rr_gemm_t ta = {s.C64, m, 0, s.X, m, s.TA, m, m, m, m};  // C X
-    RR_STAGE(GB_K_RR_GEMM, 2 * m3, (rr_gemm_kernel<<<g1, RR_GEMM_TM * RR_GEMM_TN, 0, st>>>(ta, ta, s.status)));
+    RR_STAGE(GB_K_RR_GEMM, 2 * m3, (gb_pdl(rr_gemm_kernel, g1, RR_GEMM_TM * RR_GEMM_TN, 0, st, ta, ta, s.status)));
     rr_gemm_t sa = {s.X, m, 1, s.TA, m, s.S, m, m, m, m};  // X' C X
     rr_gemm_t sb = {s.X, m, 1, s.X, m, s.P, m, m, m, m};   // X' X
-    RR_STAGE(GB_K_RR_GEMM, 4 * m3, (rr_gemm_kernel<<<g2, RR_GEMM_TM * RR_GEMM_TN, 0, st>>>(sa, sb, s.status)));
-    RR_STAGE(GB_K_RR_REFINE, 0.0, (rr_refine_kernel<<<1, RR_THREADS, sm_ref, st>>>(m, s, round == 1)));
+    RR_STAGE(GB_K_RR_GEMM, 4 * m3, (gb_pdl(rr_gemm_kernel, g2, RR_GEMM_TM * RR_GEMM_TN, 0, st, sa, sb, s.status)));
+    RR_STAGE(GB_K_RR_REFINE, 0.0, (gb_pdl(rr_refine_kernel, 1, RR_THREADS, sm_ref, st, m, s, round == 1)));
     rr_gemm_t fq = {s.EI, m, 0, s.Q, m, s.F, m, m, m, m};
-    RR_STAGE(GB_K_RR_GEMM, 2 * m3, (rr_gemm_kernel<<<g1, RR_GEMM_TM * RR_GEMM_TN, 0, st>>>(fq, fq, s.status)));
+    RR_STAGE(GB_K_RR_GEMM, 2 * m3, (gb_pdl(rr_gemm_kernel, g1, RR_GEMM_TM * RR_GEMM_TN, 0, st, fq, fq, s.status)));
     rr_gemm_t xf = {s.X, m, 0, s.F, m, s.Xn, m, m, m, m};
-    RR_STAGE(GB_K_RR_GEMM, 2 * m3, (rr_gemm_kernel<<<g1, RR_GEMM_TM * RR_GEMM_TN, 0, st>>>(xf, xf, s.status)));
+    RR_STAGE(GB_K_RR_GEMM, 2 * m3, (gb_pdl(rr_gemm_kernel, g1, RR_GEMM_TM * RR_GEMM_TN, 0, st, xf, xf, s.status)));
     double* t = s.X;
     s.X = s.Xn;
     s.Xn = t;
@@ -1485,7 +1501,7 @@ static void rr_jacobi32_path(gpu_Context* ctx, double* A, int ld, int m, int nev
   }
   // eigenvectors of the pencil: inv(L)' X into A; values into w
   RR_STAGE(GB_K_RR_TRSM, m3, (rr_trsm(st, 2, s.X, m, A, ld, m, m, s)));
-  rr_finish_kernel<<<(unsigned)((m + 255) / 256), 256, 0, st>>>(nev, s, w, info);
+  gb_pdl(rr_finish_kernel, (unsigned)((m + 255) / 256), 256, 0, st, nev, s, w, info);
   gb_count_launch(launches + 2);
 }
 #undef RR_STAGE
