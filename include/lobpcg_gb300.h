@@ -228,9 +228,9 @@ int gpu_ExplicitGram(gpu_MultiVector* X, gpu_MultiVector* R, gpu_MultiVector* P,
    (blopex_serial_double/multivector/multi_vector.c:474-524) with the fused
    accumulate of the solver's X update.  mode 0: CUDA-core kernel (FP64 or FP32
    blocks); mode 1: tensor cores, compensated 3xTF32 (FP32 blocks, h <= 128,
-   w <= 64, 16-byte aligned columns); mode 2: tensor cores, FP64-accurate
-   products by error-free splitting into bf16 digits (FP64 X and Y, h <= 64,
-   w <= 64; Z FP32 or FP64).  Z may be NULL. */
+   w <= 64, 16-byte aligned columns); mode 2: tensor cores, products with the
+   accuracy of FP64 arithmetic by error-free splitting into seven 8-bit digits
+   (FP64 X and Y, h <= 64, w <= 64; Z FP32 or FP64).  Z may be NULL. */
 int gpu_BlockUpdate(gpu_MultiVector* X, const double* C_host, int ldc, gpu_MultiVector* Y,
                     gpu_MultiVector* Z, int mode);
 
