@@ -1750,9 +1750,11 @@ __global__ void pcg_ratio_kernel(int k, const double* num, const double* den, do
 // the first step r is read from x and y is not read), 3 in the last, which only
 // finishes y; 4 launches, where each product, reduction, quotient, preconditioner
 // application and update on its own took 10 (FP64) or 7 (FP32).
-//   512^2 5-point, 8 columns, FP64, 20 steps: 1700 us against 2390 (FP64 pipe: 14
-//   instructions an entry and step, 1010 us; the ordered sums 12 us a step);
-//   128^3 7-point, 17 columns, FP32, 20 steps: 5980 us against 7120 (HBM 4000).
+//   512^2 5-point, 8 columns, FP64, 20 steps: 1700 us against 2390, 1530 with the
+//   launches overlapped (FP64 pipe: 14 instructions an entry and step, 1010 us; the
+//   ordered sums 11 us a step);
+//   128^3 7-point, 17 columns, FP32, 20 steps: 5980 us against 7120, 5400 with the
+//   two-plane stencil and the launches overlapped (HBM 4000).
 // FP32 (16-byte aligned columns): float4 access, inner products as gb_dot_cols'
 // FP32 path (exact products, compensated FP32 sums flushed to FP64).  FP64: the
 // rows of a thread and the order of every sum are those of gb_dot_cols.

@@ -871,7 +871,7 @@ __device__ __forceinline__ void rr_trd_reflector(const double* Lp, int j, int m,
 // lanes of a warp change part at different columns: two loops took 31 more steps), the
 // sum adds the n1 values that are there, and warp 0 updates the next column first and
 // forms its reflector while the others update the rest.
-//   order 57: 110 us against 152; order 72: 306 against 430.
+//   order 57: 106 us against 152; order 72: 288 against 430.
 __global__ void __launch_bounds__(RR_TRD_THREADS) rr_tridiag_smem_kernel(int m, rr_scratch s)
 {
   gb_pdl_entry();
