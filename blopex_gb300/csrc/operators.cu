@@ -415,6 +415,10 @@ struct st7t_cfg {
   static constexpr int BELOW = (NP * PLANE + 31) / 32 * 32;               // offsets in a slot: 128-byte steps
   static constexpr int ABOVE = BELOW + 1024, SLOT = ABOVE + 1024;
   static constexpr int BYTES = (NP * PLANE + 2 * 1024) * 4;               // one column's copies
+  // columns whose inner products are reduced together, a warp each: a column at a time
+  // every barrier waited for the reducing warp (inner CG 128^3, 17 columns: 5400 us
+  // against 5140; packed FP32 sums instead: 5455)
+  static constexpr int RB = NP == 1 ? 4 : 8;
   static constexpr int SMEM = ST7T_DEPTH * SLOT * 4 + 128;
 };
 
@@ -472,7 +476,7 @@ __global__ void __launch_bounds__(256, NP == 1 ? 4 : 3) st7_tma_kernel(
   float* ring = ring_raw + ((128u - (smem_u32(ring_raw) & 127u)) & 127u) / 4;
   __shared__ __align__(8) uint64_t bar[ST7T_DEPTH];
   __shared__ int abort_flag;
-  __shared__ float2 red[DOT ? 2 : 1][DOT ? 256 : 1];
+  __shared__ float2 red[DOT ? C::RB + 1 : 1][DOT ? 256 : 1];  // (one slot is written while RB are read)
   const int t = threadIdx.x, tx = t & 7, ty = t >> 3, warp = t >> 5, lane = t & 31;
   const int tiles_x = (nx + 31) / 32, tiles_y = (ny + 31) / 32;
   const unsigned b = blockIdx.x;
@@ -558,9 +562,11 @@ __global__ void __launch_bounds__(256, NP == 1 ? 4 : 3) st7_tma_kernel(
                      &bar[ahead_slot]);
       issued++;
     }
-    // the column before: its threads' sums were written ahead of the barrier
-    if (DOT && col > 0 && warp == ((col - 1) & 7))
-      st7t_dot_store(red[(col - 1) & 1], dotp + (long)(c0 + col - 1) * gridDim.x + b, lane);
+    // the RB columns before: their threads' sums were written ahead of the barrier
+    if (DOT && col > 0 && col % C::RB == 0 && warp < C::RB) {
+      const int cr = col - C::RB + warp;
+      st7t_dot_store(red[cr % (C::RB + 1)], dotp + (long)(c0 + cr) * gridDim.x + b, lane);
+    }
     float* y = (float*)Y.col[c0 + col] + cell0;
     float xs = 0.f, xc = 0.f;  // this thread's share of x' (A x): compensated sum
     if (go) {
@@ -606,13 +612,15 @@ __global__ void __launch_bounds__(256, NP == 1 ? 4 : 3) st7_tma_kernel(
         if (on && k0 + p < nz)
           for (int x = 0; x < 4; x++) y[plane * p + x] = __int_as_float(0x7fc00000);  // NaN: output incomplete
     }
-    if (DOT) red[col & 1][t] = make_float2(xs, xc);
+    if (DOT) red[col % (C::RB + 1)][t] = make_float2(xs, xc);
     slot = slot == ST7T_DEPTH - 1 ? 0 : slot + 1;
     ahead_slot = ahead_slot == ST7T_DEPTH - 1 ? 0 : ahead_slot + 1;
   }
   if (DOT) {
     __syncthreads();
-    if (warp == ((w - 1) & 7)) st7t_dot_store(red[(w - 1) & 1], dotp + (long)(c0 + w - 1) * gridDim.x + b, lane);
+    const int cr = (w - 1) / C::RB * C::RB + warp;
+    if (warp < C::RB && cr < w)
+      st7t_dot_store(red[cr % (C::RB + 1)], dotp + (long)(c0 + cr) * gridDim.x + b, lane);
   }
   if (t == 0 && abort_flag) {
     atomicExch(err, 1);
@@ -1191,7 +1199,7 @@ static long st7t_ctas(const gpu_Operator* op, int np)
 // 120 us, one plane 111)
 static int st7t_planes(const gpu_Operator* op) { return st7t_ctas(op, 2) >= 6L * op->ctx->num_sms ? 2 : 1; }
 
-static_assert(st7t_cfg<1>::SMEM + 4096 + 64 <= 48 * 1024, "one plane must fit the default shared memory");
+static_assert(st7t_cfg<1>::SMEM + 64 <= 48 * 1024, "one plane must fit the default shared memory");
 
 template <int NP, bool DOT>
 static int st7t_launch(gpu_Operator* op, const CUtensorMap& tmc, const CUtensorMap& tmz, const st7t_cols& pc,
@@ -1199,7 +1207,7 @@ static int st7t_launch(gpu_Operator* op, const CUtensorMap& tmc, const CUtensorM
 {
   gpu_Context* ctx = op->ctx;
   const int smem = st7t_cfg<NP>::SMEM;
-  if (NP > 1 &&  // (one plane fits the 48 KB every kernel has)
+  if ((NP > 1 || DOT) &&  // (one plane fits the 48 KB every kernel has)
       cudaFuncSetAttribute(st7_tma_kernel<NP, DOT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
           cudaSuccess)
     return gb_fail(ctx, "stencil7: cannot reserve %d bytes of shared memory", smem);
@@ -1753,7 +1761,7 @@ __global__ void pcg_ratio_kernel(int k, const double* num, const double* den, do
 //   512^2 5-point, 8 columns, FP64, 20 steps: 1700 us against 2390, 1530 with the
 //   launches overlapped (FP64 pipe: 14 instructions an entry and step, 1010 us; the
 //   ordered sums 11 us a step);
-//   128^3 7-point, 17 columns, FP32, 20 steps: 5980 us against 7120, 5400 with the
+//   128^3 7-point, 17 columns, FP32, 20 steps: 5980 us against 7120, 5140 with the
 //   two-plane stencil and the launches overlapped (HBM 4000).
 // FP32 (16-byte aligned columns): float4 access, inner products as gb_dot_cols'
 // FP32 path (exact products, compensated FP32 sums flushed to FP64).  FP64: the
