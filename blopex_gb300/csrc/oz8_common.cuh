@@ -90,14 +90,22 @@ static __device__ __forceinline__ void oz8_digits8(const uint32_t* lo, const uin
 }
 
 // The exact integer T = sum_L S_L 256^(7 - L) of the eight level sums, in
-// units of 2^15 (rounded once, at 2^-53 of the scales' product): |S_0| <= 2^20,
-// |S_1..3| <= 2^22, the others below 2^23; |T| < 2^62.  FP32 to integer by
-// adding 1.5 2^23 (exact to 2^22); the larger levels 4-6 by adding 1.5 2^24,
-// which gives the nearest even integer, the odd unit left over moving down a
-// level as 256; of level 7 only the leading bits count.  (Conversion
-// instructions run at a sixteenth of the additions' rate.)
-// The product of the two values is T 2^(Ex + Ey - 2099).
+// units of 2^15 (rounded once, at 2^-55 of the scales' product): |S_0..3| <=
+// 2^22, the others up to 2^23.  FP32 to integer by adding 1.5 2^23 (exact to
+// 2^22); the larger levels 4-6 by adding 1.5 2^24, which gives the nearest even
+// integer, the odd unit left over moving down a level as 256; of level 7 only
+// the leading bits count.  (Conversion instructions run at a sixteenth of the
+// additions' rate.)  The product of the two values is T 2^(Ex + Ey - 2099).
+//
+// Factors are below 1 but for a top digit rounded up to 128 (and, where the
+// slices of a row block are 0 and 4, the digit 4 beside it), so that R rows or
+// columns give |T| < R 2^55 (1 + 2^-32): 2^62 and a little for the 64 columns of
+// an update and the 128 rows of a Gram group, but just above 2^63 for 256 rows of
+// values next to a power of two.  HALF drops a bit of T for those (the product is
+// T 2^(Ex + Ey - 2098)); the one-instruction normalisation of oz8_scaled_fast
+// needs |T| < 2^63 too.
 #define OZ8_BASE 2099
+template <bool HALF>
 static __device__ __forceinline__ long long oz8_combine(uint32_t s0, uint32_t s1, uint32_t s2, uint32_t s3,
                                                         uint32_t s4, uint32_t s5, uint32_t s6, uint32_t s7)
 {
@@ -119,10 +127,10 @@ static __device__ __forceinline__ long long oz8_combine(uint32_t s0, uint32_t s1
   const int a4 = (int)(__float_as_uint(y4) - b24), a5 = (int)(__float_as_uint(y5) - b24);
   const int a6 = (int)(i6 * 256u + i7 - b24 * 257u + 8192u) >> 14;
   const long long t = (long long)a1 * 131072 + ((long long)a4 * 1024 + (long long)(a5 * 4 + a6));
-  return t + ((long long)a0 << 33);
+  return HALF ? ((t + 1) >> 1) + ((long long)a0 << 32) : t + ((long long)a0 << 33);
 }
 
-// FP64 nearest to T 2^base, |T| < 2^62, from integer operations only (ties
+// FP64 nearest to T 2^base, |T| < 2^63, from integer operations only (ties
 // away from zero): the FP64 pipe's conversion of a 64-bit integer takes longer
 // than all of these.  Fast form: needs |T| >= 2^32 and a result in the normal
 // range.

@@ -100,7 +100,9 @@ template <int F>  // slices of A stacked in an MMA: 2, 4, 8 (wpad = 64, 32, 16)
 __global__ void __launch_bounds__(OZH_THREADS, 1) oz_gram64_kernel(const __grid_constant__ ozh_params prm)
 {
   constexpr int WPAD = 128 / F;
-  constexpr int SPG = F == 2 ? 4 : 8;   // stages per group: the level sums stay below 2^23
+  constexpr int SPG = F == 2 ? 4 : 8;   // stages per group: the level sums stay within 2^23
+  constexpr bool HALF = SPG == 8;       // 256 rows: T would take 64 bits
+  constexpr int BASE = OZ8_BASE - HALF;
   constexpr long R = SPG * OZH_STAGE;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = smem_align1024(smem_raw);
@@ -386,7 +388,7 @@ __global__ void __launch_bounds__(OZH_THREADS, 1) oz_gram64_kernel(const __grid_
 #pragma unroll
         for (int e = 0; e < 4; e++) {
           ei[e] = i + e < h ? cexp[g & 3][i + e] : 1023;
-          T[e] = oz8_combine(x[0][e], x[1][e], x[2][e], x[3][e], x[4][e], x[5][e], x[6][e], x[7][e]);
+          T[e] = oz8_combine<HALF>(x[0][e], x[1][e], x[2][e], x[3][e], x[4][e], x[5][e], x[6][e], x[7][e]);
           // (|T| < 2^32: cancellation, a zero; absent entries do not count)
           odd |= !oz8_plain(ei[e]) || ((uint32_t)((T[e] >> 32) + 1) <= 1u && live && i + e < h);
         }
@@ -394,7 +396,7 @@ __global__ void __launch_bounds__(OZH_THREADS, 1) oz_gram64_kernel(const __grid_
         if (odd) {
 #pragma unroll
           for (int e = 0; e < 4; e++) {
-            v[e] = oz8_scaled(T[e], ei[e] + ej - OZ8_BASE - 8 * q);
+            v[e] = oz8_scaled(T[e], ei[e] + ej - BASE - 8 * q);
             if (oz8_unsafe(ei[e]) || oz8_unsafe(ej)) {
               const long r0 = (blockIdx.x + g * gridDim.x) * R;
               v[e] = live && q == 0 && i + e < h
@@ -404,7 +406,7 @@ __global__ void __launch_bounds__(OZH_THREADS, 1) oz_gram64_kernel(const __grid_
           }
         } else {
 #pragma unroll
-          for (int e = 0; e < 4; e++) v[e] = oz8_scaled_fast(T[e], ei[e] + ej - OZ8_BASE - 8 * q);
+          for (int e = 0; e < 4; e++) v[e] = oz8_scaled_fast(T[e], ei[e] + ej - BASE - 8 * q);
         }
 #pragma unroll
         for (int e = 0; e < 4; e++) acc[(size_t)(i + e) * 128 + r] += v[e];

@@ -423,7 +423,7 @@ __global__ void __launch_bounds__(OZY_THREADS, 1) oz_xc64_kernel(const __grid_co
           bool small = odd;
 #pragma unroll
           for (int jj = 0; jj < 4; jj++) {
-            T[jj] = oz8_combine(x[0][jj], x[1][jj], x[2][jj], x[3][jj], x[4][jj], x[5][jj], x[6][jj], x[7][jj]);
+            T[jj] = oz8_combine<false>(x[0][jj], x[1][jj], x[2][jj], x[3][jj], x[4][jj], x[5][jj], x[6][jj], x[7][jj]);
             small |= (uint32_t)((T[jj] >> 32) + 1) <= 1u;  // |T| < 2^32: cancellation, a zero
           }
           if (small) {

@@ -1,0 +1,71 @@
+"""FP64 block updates and Gram products of large blocks against the bounds that
+FP64 multiply-adds keep, entry by entry: (h + 2) 2^-53 sum |x_i c_ij| for an
+update, (32 + n / 32 / 304 + 310) 2^-53 sum |x_ri y_rj| for a Gram product (32
+roundings in a chunk, the chunks of a split, at most 304 splits).  The blocks
+are graded, localised and extreme ones, which a scale shared by a group of
+values does not absorb."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+from blopex_gb300 import solver as S  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+
+L = np.longdouble
+EPS = L(2) ** -53
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    c = S.Context(0)
+    yield c
+    assert c.device_error() == 0
+    c.close()
+
+
+def _wrap(ctx, mv):
+    interp = S._Interp(ctx.lib)
+    return interp, ctx.lib.mv_MultiVectorWrap(interp.ptr, mv.handle, 0)
+
+
+def _gram(ctx, X, Y):
+    h, w = X.shape[1], Y.shape[1]
+    mx = S.MultiVector.from_host(ctx, X)
+    my = mx if Y is X else S.MultiVector.from_host(ctx, Y)
+    (i, xx), (j, yy) = _wrap(ctx, mx), _wrap(ctx, my)
+    G = np.full((h, w), 7.0, order="F")
+    ctx.lib.mv_MultiVectorByMultiVector(xx, yy, h, h, w, G.ctypes.data)
+    assert ctx.last_error() == ""
+    return G
+
+
+def _products(X, Y):
+    """X' Y to 16 roundings of sum |x_ri y_rj| (16 rows at a time in FP64, these in
+    extended precision)."""
+    n = X.shape[0] // 16 * 16
+    p = np.matmul(X[:n].reshape(-1, 16, X.shape[1]).transpose(0, 2, 1), Y[:n].reshape(-1, 16, Y.shape[1]))
+    return p.astype(L).sum(0) + X[n:].T.astype(L) @ Y[n:]
+
+
+def _check_gram(X, Y, G):
+    n = X.shape[0]
+    mag = _products(np.abs(X), np.abs(Y))
+    err = np.abs(G - _products(X, Y))
+    b = (32 + L(n) / 32 / 304 + 310 + 16) * EPS * mag
+    assert np.all(err <= b), (float((err[mag > 0] / b[mag > 0]).max()), np.argwhere(err > b)[:3])
+
+
+# columns of constants next to a power of two: the largest sums that a group of
+# rows can hold (w in 17 .. 32 stacks two slices on a row block of 256 rows)
+@pytest.mark.parametrize("n,h,w", [(300001, 16, 24), (200003, 20, 32), (400000, 33, 16), (60001, 40, 50)])
+def test_gram_of_constant_columns(ctx, n, h, w):
+    consts = [1 - 2.0 ** -53, 0.997, 1 - 1e-12, 0.99609375, 1.998, 0.999]
+    X = np.empty((n, h))
+    Y = np.empty((n, w))
+    for c in range(h):
+        X[:, c] = consts[c % 6] * (-1 if c // 6 % 2 else 1)
+    for c in range(w):
+        Y[:, c] = consts[(c + c // 6) % 6] * (-1 if c // 3 % 2 else 1)
+    _check_gram(X, Y, _gram(ctx, X, Y))
