@@ -26,10 +26,22 @@ static __device__ __forceinline__ uint32_t oz8_scale(int E)
   return E ? ((uint32_t)E << 20) | 0xFFFFFu : 0xFFFFFFFFu;
 }
 
-// a group whose largest biased exponent E makes the digits unusable: holds
-// infinities or NaN (2047), or only values so small (below 2^-960) that
-// subnormals would matter; E = 0: zeros
-static __device__ __forceinline__ bool oz8_unsafe(int E) { return E == 2047 || (E != 0 && E < 64); }
+// The exponent word the kernels keep of a group: its largest biased exponent E,
+// or OZ8_UNSAFE when the digits cannot carry it: infinities or NaN (2047), or
+// only values so small (below 2^-960) that subnormals would matter; 0: zeros
+#define OZ8_UNSAFE 0x10000
+static __device__ __forceinline__ int oz8_code(int E) { return E == 2047 || (E != 0 && E < 64) ? OZ8_UNSAFE : E; }
+// the sum of two groups' words: products that the fast conversion can scale from
+// |T| >= 2^32 on (also at the weight 2^-56 of a Gram's last row block) without
+// leaving FP64's normal range
+static __device__ __forceinline__ bool oz8_ordinary(int e2) { return (unsigned)(e2 - 1120) <= 1900u; }
+// products to be summed with FP64 FMAs: unusable digits, or so small that the
+// roundings of subnormal sums would show (above the ordinary range the general
+// conversion is right)
+static __device__ __forceinline__ bool oz8_direct(int ex, int ey)
+{
+  return ((ex | ey) & OZ8_UNSAFE) || (ex && ey && ex + ey < 1120);
+}
 
 // |v| (v's bits hi:lo) in fixed point against its group's scale, as the bytes
 // digit 0, digits 1-6 + 128 (from the top down, below a byte 0x64)
@@ -132,8 +144,7 @@ static __device__ __forceinline__ long long oz8_combine(uint32_t s0, uint32_t s1
 
 // FP64 nearest to T 2^base, |T| < 2^63, from integer operations only (ties
 // away from zero): the FP64 pipe's conversion of a 64-bit integer takes longer
-// than all of these.  Fast form: needs |T| >= 2^32 and a result in the normal
-// range.
+// than all of these.  Fast form: |T| >= 2^32 and an ordinary sum of exponents.
 static __device__ __forceinline__ double oz8_scaled_fast(long long T, int base)
 {
   const uint64_t sg = (uint64_t)(T >> 63);
@@ -158,9 +169,6 @@ static __device__ __noinline__ double oz8_scaled(long long T, int base)
   if ((unsigned)e >= 2046u) bits = e > 0 ? 0x7FF0000000000000ull : 0ull;
   return __longlong_as_double((long long)(bits | ((uint64_t)T & 0x8000000000000000ull)));
 }
-// exponents whose products the fast form can always scale
-static __device__ __forceinline__ bool oz8_plain(int E) { return E >= 256 && E <= 1790; }
-
 // instruction descriptor of tcgen05.mma.kind::f16: D = F32, A = B = FP16,
 // both K-major, M x N (type code 0)
 static __host__ __device__ constexpr uint32_t f16_idesc(int M, int N)

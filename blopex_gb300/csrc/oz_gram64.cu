@@ -32,7 +32,8 @@
 // 1.25 (7.9).  Relative error 2.1e-16 on random blocks (FMAs 6 to 9e-16).
 //
 // Columns whose scale the digits cannot carry in some group (infinities, NaN,
-// values below 2^-960) are summed directly there with FP64 FMAs.
+// values below 2^-960) and pairs of columns whose product's scale is below 2^-924
+// are summed directly there with FP64 FMAs.
 //
 // Per CTA:
 //   warps 8-15  producers: a warp cuts 8 columns (a unit) of a 32-row stage at a
@@ -214,8 +215,8 @@ __global__ void __launch_bounds__(OZH_THREADS, 1) oz_gram64_kernel(const __grid_
       // slot g mod 4 was last read by the epilogue of group g - 4, which ended
       // before the MMAs of group g - 1, now well under way, began
       if (q == 0) {
-        cexp[g & 3][slot[m]] = E;
-        if (same) cexp[g & 3][64 + slot[m]] = E;
+        cexp[g & 3][slot[m]] = oz8_code(E);
+        if (same) cexp[g & 3][64 + slot[m]] = oz8_code(E);
       }
       emax[m] = anyb[m] = 0;
     };
@@ -384,20 +385,20 @@ __global__ void __launch_bounds__(OZH_THREADS, 1) oz_gram64_kernel(const __grid_
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         int ei[4];
         long long T[4];
-        bool odd = !oz8_plain(ej);
+        bool odd = false;
 #pragma unroll
         for (int e = 0; e < 4; e++) {
           ei[e] = i + e < h ? cexp[g & 3][i + e] : 1023;
           T[e] = oz8_combine<HALF>(x[0][e], x[1][e], x[2][e], x[3][e], x[4][e], x[5][e], x[6][e], x[7][e]);
           // (|T| < 2^32: cancellation, a zero; absent entries do not count)
-          odd |= !oz8_plain(ei[e]) || ((uint32_t)((T[e] >> 32) + 1) <= 1u && live && i + e < h);
+          odd |= !oz8_ordinary(ei[e] + ej) || ((uint32_t)((T[e] >> 32) + 1) <= 1u && live && i + e < h);
         }
         double v[4];
         if (odd) {
 #pragma unroll
           for (int e = 0; e < 4; e++) {
             v[e] = oz8_scaled(T[e], ei[e] + ej - BASE - 8 * q);
-            if (oz8_unsafe(ei[e]) || oz8_unsafe(ej)) {
+            if (oz8_direct(ei[e], ej)) {
               const long r0 = (blockIdx.x + g * gridDim.x) * R;
               v[e] = live && q == 0 && i + e < h
                          ? ozh_direct(s_col[i + e], s_col[64 + j], r0, min(r0 + R, prm.n))

@@ -15,8 +15,8 @@
 // against 2.0e-16 relative on random blocks, h = 32).
 //
 // Rows or columns whose scale the digits cannot carry (infinities, NaN, values
-// below 2^-960) are summed directly with FP64 FMAs by the epilogue, entry by
-// entry.
+// below 2^-960), and products whose scale is below 2^-924, are summed directly
+// with FP64 FMAs by the epilogue, entry by entry.
 //
 // What bounds it: instruction issue, the half-rate integer pipe above all (~17
 // integer instructions per X value in the producers, ~30 per Y value in the
@@ -148,7 +148,6 @@ __global__ void __launch_bounds__(OZY_THREADS, 1) oz_xc64_kernel(const __grid_co
   __shared__ uint32_t tmem_base;
   __shared__ int abort_flag;
   __shared__ int colexp[64];
-  __shared__ int any_odd;  // a column of C has a scale out of the ordinary
   __shared__ uint32_t colpart[8][64];      // per (8-row group of C, column) largest magnitude word
   __shared__ unsigned char colnz[8][64];   // and whether any value is not zero
   __shared__ int rowexp[4][128];           // by tile modulo 4 (read by the epilogue)
@@ -169,7 +168,6 @@ __global__ void __launch_bounds__(OZY_THREADS, 1) oz_xc64_kernel(const __grid_co
 
   if (tid == 0) {
     abort_flag = 0;
-    any_odd = 0;
     for (int k = 0; k < 4; k++) {
       mbar_init(&a_full[k], OZY_NPROD);
       mbar_init(&a_empty[k], 1);
@@ -220,8 +218,7 @@ __global__ void __launch_bounds__(OZY_THREADS, 1) oz_xc64_kernel(const __grid_co
       nz |= colnz[g][j] != 0;
     }
     const int E = ozy_group_exp(mag, nz);
-    if (cg == 0) colexp[j] = E;
-    if (j < w && !oz8_plain(E)) any_odd = 1;
+    if (cg == 0) colexp[j] = oz8_code(E);
     uint32_t lo[8], hi[8], pk[OZY_S][4];
 #pragma unroll
     for (int c = 0; c < 8; c++) {
@@ -292,7 +289,7 @@ __global__ void __launch_bounds__(OZY_THREADS, 1) oz_xc64_kernel(const __grid_co
       named_bar(1 + (pw & 3), 64);
       const int E = max(rowpart[i & 1][0][r], rowpart[i & 1][1][r]);
       const uint32_t es = oz8_scale(E);
-      if (half == 0) rowexp[i & 3][r] = E;
+      if (half == 0) rowexp[i & 3][r] = oz8_code(E);
 #pragma unroll
       for (int k = 0; k < 4; k++) {
         if (k >= ksteps) break;
@@ -385,9 +382,6 @@ __global__ void __launch_bounds__(OZY_THREADS, 1) oz_xc64_kernel(const __grid_co
         }
         tc_fence_after();
         const int er = rowexp[i & 3][r];
-        // scales out of the ordinary (zeros included): the general conversion,
-        // or the direct sum
-        const bool odd = !oz8_plain(er) || any_odd;
         const uint32_t tl = tmem + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(set * OZY_SET + 16 * chalf);
         double yp[4];
         int jp = -1;
@@ -420,22 +414,26 @@ __global__ void __launch_bounds__(OZY_THREADS, 1) oz_xc64_kernel(const __grid_co
           // (no branch among the entries: their integer chains overlap)
           double y[4];
           long long T[4];
-          bool small = odd;
+          // out of the ordinary: the general conversion, or the direct sum
+          int e2[4];
+          bool odd = false;
 #pragma unroll
           for (int jj = 0; jj < 4; jj++) {
             T[jj] = oz8_combine<false>(x[0][jj], x[1][jj], x[2][jj], x[3][jj], x[4][jj], x[5][jj], x[6][jj], x[7][jj]);
-            small |= (uint32_t)((T[jj] >> 32) + 1) <= 1u;  // |T| < 2^32: cancellation, a zero
+            e2[jj] = er + colexp[j0 + jj];
+            // (|T| < 2^32: cancellation, a zero)
+            odd |= !oz8_ordinary(e2[jj]) || (uint32_t)((T[jj] >> 32) + 1) <= 1u;
           }
-          if (small) {
+          if (odd) {
 #pragma unroll
             for (int jj = 0; jj < 4; jj++) {
-              y[jj] = oz8_scaled(T[jj], er + colexp[j0 + jj] - OZ8_BASE);
-              if (row < prm.n && j0 + jj < w && (oz8_unsafe(er) || oz8_unsafe(colexp[j0 + jj])))
+              y[jj] = oz8_scaled(T[jj], e2[jj] - OZ8_BASE);
+              if (row < prm.n && j0 + jj < w && oz8_direct(er, colexp[j0 + jj]))
                 y[jj] = ozy_direct(s_x, prm.C, prm.ldc, h, j0 + jj, row);
             }
           } else {
 #pragma unroll
-            for (int jj = 0; jj < 4; jj++) y[jj] = oz8_scaled_fast(T[jj], er + colexp[j0 + jj] - OZ8_BASE);
+            for (int jj = 0; jj < 4; jj++) y[jj] = oz8_scaled_fast(T[jj], e2[jj] - OZ8_BASE);
           }
           if (prm.z_kind == 1) {
             bool cvt = false;

@@ -69,3 +69,55 @@ def test_gram_of_constant_columns(ctx, n, h, w):
     for c in range(w):
         Y[:, c] = consts[(c + c // 6) % 6] * (-1 if c // 3 % 2 else 1)
     _check_gram(X, Y, _gram(ctx, X, Y))
+
+
+def _update(ctx, X, C, Y0=None):
+    """X C, or Y0 + X C in place."""
+    h, w = C.shape
+    mx = S.MultiVector.from_host(ctx, X)
+    my = S.MultiVector.from_host(ctx, Y0 if Y0 is not None else np.full((X.shape[0], w), 7.0))
+    Cf = np.asfortranarray(C)
+    (i, xx), (j, yy) = _wrap(ctx, mx), _wrap(ctx, my)
+    f = ctx.lib.mv_MultiVectorXapy if Y0 is not None else ctx.lib.mv_MultiVectorByMatrix
+    f(xx, h, h, w, Cf.ctypes.data, yy)
+    assert ctx.last_error() == ""
+    return my.to_host()
+
+
+TINY = L(2) ** -1074
+
+
+# products whose scale is below or near FP64's smallest normal numbers, and above
+# its largest, of factors that are themselves well inside the range
+def test_update_products_out_of_range(ctx):
+    rng = np.random.default_rng(21)
+    n, h, w = 40000, 32, 20
+    X, C = rng.standard_normal((n, h)), rng.standard_normal((h, w))
+    X *= 10.0 ** rng.uniform(-200, 150, size=(n, 1))
+    C *= 10.0 ** rng.choice([-200, -150, -130, -110, -104, 0, 100, 150, 160, 200], size=(1, w))
+    Y = _update(ctx, X, C)
+    ref, mag = X.astype(L) @ C.astype(L), np.abs(X).astype(L) @ np.abs(C)
+    big = mag > 1.7e308
+    assert np.all(np.isinf(Y[np.abs(ref) > 1.8e308]))
+    err = np.abs(Y - ref)[~big]
+    b = ((h + 2) * EPS * mag + (h + 1) * TINY)[~big]
+    assert np.all(err <= b), float((err / b).max())
+
+
+def test_gram_products_out_of_range(ctx):
+    rng = np.random.default_rng(22)
+    n, h, w = 120001, 24, 36
+    X = rng.standard_normal((n, h)) * 10.0 ** rng.choice([-200, -160, -120, 0, 120, 150], size=(1, h))
+    Y = rng.standard_normal((n, w)) * 10.0 ** rng.choice([-200, -148, -105, 0, 100, 151], size=(1, w))
+    G = _gram(ctx, X, Y)
+    xs, ys = np.abs(X).max(0), np.abs(Y).max(0)
+    with np.errstate(under="ignore", over="ignore"):
+        norm = np.outer(xs.astype(L), ys.astype(L))
+        mag = _products(np.abs(X) / xs, np.abs(Y) / ys) * norm
+        ref = _products(X / xs, Y / ys) * norm
+    fits = mag < 1.7e308
+    err = np.abs(G - ref)[fits]
+    # (the divisions by the largest values: two roundings of each product)
+    b = ((32 + L(n) / 32 / 304 + 310 + 20) * EPS * mag + n * TINY)[fits]
+    assert np.all(err <= b), float((err / b).max())
+    assert np.all(np.isinf(G[np.abs(ref) > 1.8e308]))

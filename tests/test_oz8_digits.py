@@ -185,3 +185,23 @@ def test_update_rows_fit_63_bits():
             assert reg == T and abs(T) < 1 << 62
             want = 64 * value(x, E) * value(-y, E)
             assert abs(Fraction(T, 1 << 55) - want) <= Fraction(64 * 6, 1 << 64) + Fraction(1, 1 << 55)
+
+
+def test_fast_conversion_where_it_is_used():
+    """The sums of exponents that oz8_ordinary lets pass: the fast conversion is
+    the general one, and both are the nearest FP64 number (ties away from zero);
+    with the weight 2^-56 of a Gram's last row block too.  Far below, where two
+    scales are usable and their product is not, it would not be."""
+    rng = random.Random(9)
+    Ts = [1 << 32, (1 << 32) + 1, (1 << 62) + 5, (1 << 63) - 1, (1 << 54) + (1 << 1), (1 << 53) - 1]
+    Ts += [rng.getrandbits(b) | 1 << (b - 1) for b in range(33, 64) for _ in range(6)]
+    for e2 in (1120, 1121, 1500, 2046, 2900, 3019, 3020):
+        for shift in (0, 56):
+            for T in Ts + [-t for t in Ts]:
+                base = e2 - BASE - shift
+                y = scaled(T, base)
+                assert scaled_fast(T, base) == y and math.isfinite(y)
+                err = abs(Fraction(y) - Fraction(T) * Fraction(2) ** base)
+                assert err <= Fraction(2) ** (base + max(T.bit_length() - 54, -1))
+                assert err == 0 or T.bit_length() > 53
+    assert scaled_fast(1 << 56, 2 * 359 - BASE) != scaled(1 << 56, 2 * 359 - BASE)  # 1e-200 x 1e-200
