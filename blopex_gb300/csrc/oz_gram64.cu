@@ -375,6 +375,7 @@ __global__ void __launch_bounds__(OZH_THREADS, 1) oz_gram64_kernel(const __grid_
       // share its instruction cache)
 #pragma unroll 1
       for (int i = c0; i < c1 && i < h; i += 4) {
+        __syncwarp();  // (the branch below is taken by single lanes; tcgen05.ld needs the whole warp)
         uint32_t x[8][4];
 #pragma unroll
         for (int c = 0; c < (F == 8 ? 7 : 8); c++)

@@ -401,6 +401,7 @@ __global__ void __launch_bounds__(OZY_THREADS, 1) oz_xc64_kernel(const __grid_co
         for (int g = 0; g < 4; g++) {
           const int j0 = jbase + 4 * g;
           if (j0 >= w) break;
+          __syncwarp();  // (the branches below are taken by single lanes; tcgen05.ld needs the whole warp)
           uint32_t x[8][4];  // the eight levels of four columns
           ozy_tmem_ld(tl + (uint32_t)(4 * g), x);
           // the previous four columns go out only now: their conversions and
@@ -460,6 +461,7 @@ __global__ void __launch_bounds__(OZY_THREADS, 1) oz_xc64_kernel(const __grid_co
           for (int jj = 0; jj < 4; jj++) yp[jj] = y[jj];
           jp = j0;
         }
+        __syncwarp();
         tc_fence_before();
         mbar_arrive(&acc_empty[set]);
         if (jp >= 0) put(yp, jp);

@@ -121,3 +121,21 @@ def test_gram_products_out_of_range(ctx):
     b = ((32 + L(n) / 32 / 304 + 310 + 20) * EPS * mag + n * TINY)[fits]
     assert np.all(err <= b), float((err / b).max())
     assert np.all(np.isinf(G[np.abs(ref) > 1.8e308]))
+
+
+# single rows and columns that leave the common path among ordinary ones: lanes of a
+# warp part ways in every tile and group, and meet again before the next load of
+# accumulators
+def test_gram_mixed_lanes(ctx):
+    rng = np.random.default_rng(24)
+    n, h, w = 150001, 26, 30
+    X, Y = rng.standard_normal((n, h)), rng.standard_normal((n, w))
+    X[:, 2::5] *= 1e-300
+    Y[:, 1::4] *= 1e-305
+    X[256:512, ::3] = 0.0
+    xs, ys = np.abs(X).max(0), np.abs(Y).max(0)
+    G = _gram(ctx, X, Y)
+    with np.errstate(under="ignore"):
+        norm = np.outer(xs.astype(L), ys.astype(L))
+        mag, ref = _products(np.abs(X) / xs, np.abs(Y) / ys) * norm, _products(X / xs, Y / ys) * norm
+    assert np.all(np.abs(G - ref) <= (32 + L(n) / 32 / 304 + 310 + 20) * EPS * mag + n * TINY)
