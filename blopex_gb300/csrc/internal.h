@@ -195,7 +195,7 @@ int gb_oz_xc(gpu_Context* ctx, long n, const blk_cols* X, int h, const double* C
              const blk_cols* Y, int w, const blk_cols* Z, int z_dtype, const blk_cols* Y32);
 /* the same product with the accuracy of FP64 arithmetic (oz_xc64.cu) */
 int gb_oz_xc64(gpu_Context* ctx, long n, const blk_cols* X, int h, const double* C, int ldc,
-               const blk_cols* Y, int w, const blk_cols* Z, int z_dtype, const blk_cols* Y32);
+               const blk_cols* Y, int w, const blk_cols* Z, int z_dtype);
 /* and for FP64 blocks of any widths and alignments; Z FP64, may be Y.  X must
    not overlap Y when h or w > 64 */
 int gb_oz_bymat64(gpu_Context* ctx, long n, const blk_cols* X, int h, const double* C, int ldc,

@@ -1,8 +1,7 @@
 // oz_xc64.cu -- block update Y = X C (+ Z) with the accuracy of FP64 arithmetic on
 // the tensor cores, by error-free splitting (oz8_common.cuh): X an FP64 block of
 // n rows and h <= 64 columns, C the FP64 h x w coordinate block (w <= 64) on the
-// device, Z an optional FP32 or FP64 block, Y FP64 (and optionally its FP32
-// shadow Y32).  It is serial_Multi_VectorByMatrix (blopex_serial_double/
+// device, Z an optional FP32 or FP64 block, Y FP64.  It is serial_Multi_VectorByMatrix (blopex_serial_double/
 // multivector/multi_vector.c:474-524), for callers' large FP64 blocks
 // (gb_bymat_large) and gpu_BlockUpdate's mode 2.
 //
@@ -40,7 +39,7 @@
 //               column 32 (t + u);
 //   warps 0-7   read a unit's eight level accumulators (lane = row; warps w and
 //               w + 4 share TMEM lanes and take 16 of the unit's 32 columns
-//               each), recombine and store Y (and Y32).
+//               each), recombine and store Y.
 // Every wait is bounded; a timeout sets an error word and all roles finish.
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -62,10 +61,9 @@
 
 struct ozy_params {
   const void *x[64], *z[64];
-  void *y[64], *y32[64];
+  void* y[64];
   const double* C;
   int ldc, h, w, z_kind;  // z_kind: 0 none, 1 FP32, 2 FP64
-  int has_y32;
   long n;
   long polls;  // limit of one pipeline wait
   int* err;
@@ -88,10 +86,6 @@ static __device__ __forceinline__ uint32_t ozy_ld32(const void* p, long i)
 static __device__ __forceinline__ void ozy_st(void* p, long i, double v)
 {
   asm volatile("st.global.f64 [%0], %1;" ::"l"(__cvta_generic_to_global((double*)p + i)), "d"(v) : "memory");
-}
-static __device__ __forceinline__ void ozy_st32(void* p, long i, float v)
-{
-  asm volatile("st.global.f32 [%0], %1;" ::"l"(__cvta_generic_to_global((float*)p + i)), "f"(v) : "memory");
 }
 
 // the Z values of one row in columns j0 .. j0 + 3 (bit patterns; 0 outside)
@@ -157,7 +151,6 @@ __global__ void __launch_bounds__(OZY_THREADS, 1) oz_xc64_kernel(const __grid_co
   __shared__ const void* s_x[64];
   __shared__ void* s_y[64];
   __shared__ const void* s_z[64];
-  __shared__ void* s_y32[64];
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int h = prm.h, w = prm.w;
@@ -182,7 +175,6 @@ __global__ void __launch_bounds__(OZY_THREADS, 1) oz_xc64_kernel(const __grid_co
     s_x[tid] = tid < h ? prm.x[tid] : nullptr;
     s_y[tid] = tid < w ? prm.y[tid] : nullptr;
     s_z[tid] = (tid < w && prm.z_kind) ? prm.z[tid] : nullptr;
-    s_y32[tid] = (tid < w && prm.has_y32) ? prm.y32[tid] : nullptr;
   }
   // C: one scale per column, digits as the B operand (row j = output column,
   // K = input column); rows j >= w and columns i >= h are zero
@@ -389,11 +381,6 @@ __global__ void __launch_bounds__(OZY_THREADS, 1) oz_xc64_kernel(const __grid_co
 #pragma unroll
           for (int jj = 0; jj < 4; jj++)
             if (row < prm.n && j0 + jj < w) ozy_st(s_y[j0 + jj], row, y[jj]);
-          if (prm.has_y32) {
-#pragma unroll
-            for (int jj = 0; jj < 4; jj++)
-              if (row < prm.n && j0 + jj < w) ozy_st32(s_y32[j0 + jj], row, oz_to_float(y[jj]));
-          }
         };
         // (not unrolled: the roles of a scheduler's warps share its instruction
         // cache)
@@ -489,8 +476,7 @@ __global__ void ozy_check_kernel(const int* err, int* status)
 
 // columns [0, h) x [0, w) of the tables, h, w <= 64; polls <= 0: the default limit
 static int ozy_launch(gpu_Context* ctx, long n, const void* const* X, int h, const double* C, int ldc,
-                      const void* const* Y, int w, const void* const* Z, int z_kind, const void* const* Y32,
-                      int polls, int* err)
+                      const void* const* Y, int w, const void* const* Z, int z_kind, int polls, int* err)
 {
   ozy_params prm;
   memset(&prm, 0, sizeof(prm));
@@ -498,14 +484,12 @@ static int ozy_launch(gpu_Context* ctx, long n, const void* const* X, int h, con
   for (int j = 0; j < w; j++) {
     prm.y[j] = (void*)Y[j];
     if (z_kind) prm.z[j] = Z[j];
-    if (Y32) prm.y32[j] = (void*)Y32[j];
   }
   prm.C = C;
   prm.ldc = ldc;
   prm.h = h;
   prm.w = w;
   prm.z_kind = z_kind;
-  prm.has_y32 = Y32 != NULL;
   prm.n = n;
   prm.polls = polls > 0 ? (long)polls : TC_WAIT_LIMIT;
   prm.err = err;
@@ -520,7 +504,7 @@ static int ozy_launch(gpu_Context* ctx, long n, const void* const* X, int h, con
 }
 
 extern "C" int gb_oz_xc64(gpu_Context* ctx, long n, const blk_cols* X, int h, const double* C, int ldc,
-                        const blk_cols* Y, int w, const blk_cols* Z, int z_dtype, const blk_cols* Y32)
+                        const blk_cols* Y, int w, const blk_cols* Z, int z_dtype)
 {
   if (n <= 0 || w <= 0) return 0;
   if (h < 1 || h > 64 || w > 64)
@@ -534,10 +518,9 @@ extern "C" int gb_oz_xc64(gpu_Context* ctx, long n, const blk_cols* X, int h, co
   const int zk = Z ? (z_dtype == GPU_MV_FLOAT64 ? 2 : 1) : 0;
   gb_prof_rec pr;
   gb_prof_begin(ctx, &pr, GB_K_OZ_XC);
-  const int rc = ozy_launch(ctx, n, X->col, h, C, ldc, Y->col, w, Z ? Z->col : NULL, zk, Y32 ? Y32->col : NULL,
-                            ctx->opt.wait_polls, err);
+  const int rc = ozy_launch(ctx, n, X->col, h, C, ldc, Y->col, w, Z ? Z->col : NULL, zk, ctx->opt.wait_polls, err);
   const double zb = zk == 2 ? 8.0 * w : (zk == 1 ? 4.0 * w : 0.0);
-  gb_prof_end(ctx, &pr, (double)n * (8.0 * h + 8.0 * w + zb + (Y32 ? 4.0 * w : 0.0)),
+  gb_prof_end(ctx, &pr, (double)n * (8.0 * h + 8.0 * w + zb),
               2.0 * n * h * w);
   if (rc) return rc;
   ozy_check_kernel<<<1, 1, 0, (cudaStream_t)ctx->stream>>>(err, ctx->dcount + 5);
@@ -557,8 +540,8 @@ extern "C" int gb_oz_bymat64(gpu_Context* ctx, long n, const blk_cols* X, int h,
     for (int i0 = 0; i0 < h; i0 += 64) {
       const int hi = h - i0 < 64 ? h - i0 : 64;
       const void* const* z = i0 ? Y->col + j0 : (Z ? Z->col + j0 : NULL);
-      if (ozy_launch(ctx, n, X->col + i0, hi, C + i0 + (size_t)j0 * ldc, ldc, Y->col + j0, wj, z, z ? 2 : 0,
-                     NULL, 0, ctx->dcount + 5))
+      if (ozy_launch(ctx, n, X->col + i0, hi, C + i0 + (size_t)j0 * ldc, ldc, Y->col + j0, wj, z, z ? 2 : 0, 0,
+                     ctx->dcount + 5))
         return -1;
     }
   }

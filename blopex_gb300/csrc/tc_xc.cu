@@ -363,7 +363,7 @@ extern "C" int gpu_BlockUpdate(gpu_MultiVector* X, const double* C_host, int ldc
     else if (mode == 1)
       rc = gb_tc_xc(ctx, X->size, &cx, h, C, ldc, &cy, w, Z ? &cz : NULL);
     else
-      rc = gb_oz_xc64(ctx, X->size, &cx, h, C, ldc, &cy, w, Z ? &cz : NULL, Z ? Z->dtype : 0, NULL);
+      rc = gb_oz_xc64(ctx, X->size, &cx, h, C, ldc, &cy, w, Z ? &cz : NULL, Z ? Z->dtype : 0);
   }
   int err = 0;
   if (!rc) rc = gb_device_error(ctx, &err);
