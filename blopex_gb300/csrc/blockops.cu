@@ -562,11 +562,25 @@ extern "C" int gb_bymat(gpu_Context* ctx, int dtype, long n, const blk_cols* X, 
 // the reason given at gb_gram_large.
 #define XC_TENSOR_MIN 1.6e7
 
+// whether a column of X shares memory with a column of Y (`bytes` long each)
+extern "C" int gb_cols_overlap(const blk_cols* X, int h, const blk_cols* Y, int w, size_t bytes)
+{
+  for (int i = 0; i < h; i++)
+    for (int j = 0; j < w; j++) {
+      const uintptr_t x = (uintptr_t)X->col[i], y = (uintptr_t)Y->col[j];
+      if (x < y + bytes && y < x + bytes) return 1;
+    }
+  return 0;
+}
+
 extern "C" int gb_bymat_large(gpu_Context* ctx, int dtype, long n, const blk_cols* X, int h,
                               const double* C, int ldc, const blk_cols* Y, int w, const blk_cols* Z)
 {
   if (w <= 0 || n <= 0) return 0;
-  if (dtype != GPU_MV_FLOAT64 || h <= 0 || (double)n * h * w < XC_TENSOR_MIN)
+  // (in place: gb_bymat, whose CTAs read all of their rows of X before they write;
+  // the tensor-core kernel comes back to X for the entries that it sums directly)
+  if (dtype != GPU_MV_FLOAT64 || h <= 0 || (double)n * h * w < XC_TENSOR_MIN ||
+      gb_cols_overlap(X, h, Y, w, sizeof(double) * (size_t)n))
     return gb_bymat(ctx, dtype, n, X, h, C, ldc, Y, w, Z);
   gb_prof_rec pr;
   gb_prof_begin(ctx, &pr, GB_K_XC);

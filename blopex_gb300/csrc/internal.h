@@ -127,6 +127,8 @@ int gb_bymat(gpu_Context* ctx, int dtype, long n, const blk_cols* X, int h, cons
 /* the same for callers outside the solver: large FP64 products on the tensor cores */
 int gb_bymat_large(gpu_Context* ctx, int dtype, long n, const blk_cols* X, int h, const double* C,
                    int ldc, const blk_cols* Y, int w, const blk_cols* Z);
+/* whether a column of X shares memory with a column of Y (bytes long each) */
+int gb_cols_overlap(const blk_cols* X, int h, const blk_cols* Y, int w, size_t bytes);
 /* the same with C upper triangular (explicit zeros below the diagonal) */
 int gb_bymat_tri(gpu_Context* ctx, int dtype, long n, const blk_cols* X, int h, const double* C,
                  int ldc, const blk_cols* Y, int w);
@@ -193,11 +195,12 @@ int gb_tc_xc(gpu_Context* ctx, long n, const blk_cols* X, int h, const double* C
    or FP64 (z_dtype); Y32 optional FP32 copy of Y */
 int gb_oz_xc(gpu_Context* ctx, long n, const blk_cols* X, int h, const double* C, int ldc,
              const blk_cols* Y, int w, const blk_cols* Z, int z_dtype, const blk_cols* Y32);
-/* the same product with the accuracy of FP64 arithmetic (oz_xc64.cu) */
+/* the same product with the accuracy of FP64 arithmetic (oz_xc64.cu); X must not
+   overlap Y */
 int gb_oz_xc64(gpu_Context* ctx, long n, const blk_cols* X, int h, const double* C, int ldc,
                const blk_cols* Y, int w, const blk_cols* Z, int z_dtype);
 /* and for FP64 blocks of any widths and alignments; Z FP64, may be Y.  X must
-   not overlap Y when h or w > 64 */
+   not overlap Y */
 int gb_oz_bymat64(gpu_Context* ctx, long n, const blk_cols* X, int h, const double* C, int ldc,
                   const blk_cols* Y, int w, const blk_cols* Z);
 /* the CTAs' sums of X' Y for FP64 blocks of any widths and alignments

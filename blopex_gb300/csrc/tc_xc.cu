@@ -362,6 +362,8 @@ extern "C" int gpu_BlockUpdate(gpu_MultiVector* X, const double* C_host, int ldc
       rc = gb_bymat(ctx, X->dtype, X->size, &cx, h, C, ldc, &cy, w, Z ? &cz : NULL);
     else if (mode == 1)
       rc = gb_tc_xc(ctx, X->size, &cx, h, C, ldc, &cy, w, Z ? &cz : NULL);
+    else if (gb_cols_overlap(&cx, h, &cy, w, sizeof(double) * (size_t)X->size))
+      rc = gb_oz_xc(ctx, X->size, &cx, h, C, ldc, &cy, w, Z ? &cz : NULL, Z ? Z->dtype : 0, NULL);  // reads X once
     else
       rc = gb_oz_xc64(ctx, X->size, &cx, h, C, ldc, &cy, w, Z ? &cz : NULL, Z ? Z->dtype : 0);
   }

@@ -139,3 +139,43 @@ def test_gram_mixed_lanes(ctx):
         norm = np.outer(xs.astype(L), ys.astype(L))
         mag, ref = _products(np.abs(X) / xs, np.abs(Y) / ys) * norm, _products(X / xs, Y / ys) * norm
     assert np.all(np.abs(G - ref) <= (32 + L(n) / 32 / 304 + 310 + 20) * EPS * mag + n * TINY)
+
+
+def _in_place(ctx, X, C, add):
+    """Y = X C (+ Y) with Y on the first columns of X."""
+    n, (h, w) = X.shape[0], C.shape
+    t = torch.from_numpy(np.ascontiguousarray(X.T)).cuda()
+    torch.cuda.synchronize()
+    mx = S.MultiVector.wrap_device(ctx, t.data_ptr(), n, n, h)
+    my = S.MultiVector.wrap_device(ctx, t.data_ptr(), n, n, w)
+    Cf = np.asfortranarray(C)
+    (i, xx), (j, yy) = _wrap(ctx, mx), _wrap(ctx, my)
+    f = ctx.lib.mv_MultiVectorXapy if add else ctx.lib.mv_MultiVectorByMatrix
+    f(xx, h, h, w, Cf.ctypes.data, yy)
+    assert ctx.last_error() == ""
+    return t.cpu().numpy()[:w].T
+
+
+# as always right in place: up to 32 output columns, any number of input columns
+@pytest.mark.parametrize("n,h,w,add", [(20001, 32, 32, False), (30001, 33, 32, True), (9001, 96, 32, False),
+                                       (5003, 130, 25, True)])
+def test_update_in_place(ctx, n, h, w, add):
+    rng = np.random.default_rng(n)
+    X, C = rng.standard_normal((n, h)), rng.standard_normal((h, w)) / 8
+    X[::9] *= 1e-300
+    ref = X.astype(L) @ C + (X[:, :w] if add else 0)
+    mag = np.abs(X).astype(L) @ np.abs(C) + (np.abs(X[:, :w]) if add else 0)
+    Y = _in_place(ctx, X, C, add)
+    assert np.all(np.abs(Y - ref) <= (h + 3) * EPS * mag + (h + 1) * TINY)
+
+
+def test_split_update_in_place(ctx):
+    """gpu_BlockUpdate mode 2 with Y = X, to the bound of its splitting."""
+    rng = np.random.default_rng(41)
+    n, h = 30000, 64
+    X, C = rng.standard_normal((n, h)), np.asfortranarray(rng.standard_normal((h, h)))
+    X[::9] *= 1e-300
+    mx = S.MultiVector.from_host(ctx, X)
+    assert ctx.lib.gpu_BlockUpdate(mx.handle, C.ctypes.data, h, mx.handle, None, 2) == 0, ctx.last_error()
+    b = h * 2.0 ** -38 * np.outer(np.abs(X).max(1), np.abs(C).max(0))
+    assert np.all(np.abs(mx.to_host() - X @ C) <= b + 2.0 ** -45 * (np.abs(X) @ np.abs(C)))
