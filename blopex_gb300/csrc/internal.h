@@ -195,12 +195,12 @@ int gb_tc_xc(gpu_Context* ctx, long n, const blk_cols* X, int h, const double* C
    or FP64 (z_dtype); Y32 optional FP32 copy of Y */
 int gb_oz_xc(gpu_Context* ctx, long n, const blk_cols* X, int h, const double* C, int ldc,
              const blk_cols* Y, int w, const blk_cols* Z, int z_dtype, const blk_cols* Y32);
-/* the same product with the accuracy of FP64 arithmetic (oz_xc64.cu); X must not
-   overlap Y */
+/* the same product from 55 bits of each factor (oz_xc64.cu): |error| up to
+   2^-53 (h + 1) max |row of X| max |column of C|; X must not overlap Y */
 int gb_oz_xc64(gpu_Context* ctx, long n, const blk_cols* X, int h, const double* C, int ldc,
                const blk_cols* Y, int w, const blk_cols* Z, int z_dtype);
-/* and for FP64 blocks of any widths and alignments; Z FP64, may be Y.  X must
-   not overlap Y */
+/* and for FP64 blocks of any widths and alignments, every entry within the bound
+   of FP64 multiply-adds; Z FP64, may be Y.  X must not overlap Y */
 int gb_oz_bymat64(gpu_Context* ctx, long n, const blk_cols* X, int h, const double* C, int ldc,
                   const blk_cols* Y, int w, const blk_cols* Z);
 /* the CTAs' sums of X' Y for FP64 blocks of any widths and alignments

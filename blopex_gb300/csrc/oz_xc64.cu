@@ -1,47 +1,65 @@
 // oz_xc64.cu -- block update Y = X C (+ Z) with the accuracy of FP64 arithmetic on
 // the tensor cores, by error-free splitting (oz8_common.cuh): X an FP64 block of
 // n rows and h <= 64 columns, C the FP64 h x w coordinate block (w <= 64) on the
-// device, Z an optional FP32 or FP64 block, Y FP64.  It is serial_Multi_VectorByMatrix (blopex_serial_double/
-// multivector/multi_vector.c:474-524), for callers' large FP64 blocks
-// (gb_bymat_large) and gpu_BlockUpdate's mode 2.
+// device, Z an optional FP32 or FP64 block, Y FP64.  It is
+// serial_Multi_VectorByMatrix (blopex_serial_double/multivector/multi_vector.c:
+// 474-524), for callers' large FP64 blocks (gb_bymat_large) and gpu_BlockUpdate's
+// mode 2.
 //
 // Scales: each row of X (its h values) and each column of C share one power of
 // two; both are cut into 7 8-bit digits (55 fraction bits).  Level L = t + u of
 // the digit products is accumulated exactly in FP32 in TMEM (at most 7 products
 // of 2^14 over 64 columns: below 2^23); the epilogue recombines the eight levels
 // into one 64-bit integer, rounds it to FP64 with integer operations and adds Z.
-// |Y - (X C + Z)| is below that of a sum of h fused multiply-adds (6e-17
-// against 2.0e-16 relative on random blocks, h = 32).
 //
-// Rows or columns whose scale the digits cannot carry (infinities, NaN, values
-// below 2^-960), and products whose scale is below 2^-924, are summed directly
-// with FP64 FMAs by the epilogue, entry by entry.
+// Accuracy.  The digits alone (gpu_BlockUpdate's mode 2) are off by up to
+// 2^-55 S S' (|x/S| + |c/S'| + 1.3) (1-norms; S, S' the scales: every value cut
+// below 2^-55 of its scale, products of levels 8 and up left out, T rounded): less
+// than the roundings of fused multiply-adds on random blocks (6e-17 against 2.0e-16
+// relative, h = 32), and more, or everything, where a row's large values meet
+// zeros or small values of C.  Callers' products (BOUND) are held to the bound of
+// the multiply-adds, m 2^-53 sum |x_i c_ij| with the m nonzeros of column j of C
+// (+ the rounding of Z), in every entry: the magnitudes of the top digits are
+// multiplied as well (an eighth slice, a ninth accumulator).  D = sum |d_0(x)|
+// |d_0(c)| bounds sum |x_i c_ij| / (S S') from below by (D - 0.502 (N + N')) 2^-14,
+// N and N' being the sums of the top digits, which bound the 1-norms from above
+// by (N + h / 2) / 128.  The digits serve where
+//   2^-55 ((N + N' + h) / 128 + 1.3) <= (m - 1) 2^-53 (D - 0.502 (N + N')) 2^-14,
+// the last of the m roundings being that of the sum.  Other entries are summed
+// directly with FP64 FMAs by the epilogue, in the order of bymat_kernel: 1 in 10^5
+// of random blocks of 32 columns; all of a column of C with one nonzero (a copy of
+// X's column comes back as it is), most where X's large columns meet C's zeros.  So
+// are rows or columns whose scale the digits cannot carry (infinities, NaN,
+// values below 2^-960), and products whose scale is below 2^-924.
 //
 // What bounds it: instruction issue, the half-rate integer pipe above all (~17
 // integer instructions per X value in the producers, ~30 per Y value in the
 // epilogue); FP64 FMAs instead would need h w / 2 cycles per row and SM (2 per
-// cycle), 2,048 at h = w = 64 against ~115 here.  Measured, 2,097,152 rows:
-// 32 x 32 0.43 ms (FMAs 3.5), 64 x 64 0.83 (11.7), 64 x 64 with an FP32 Z 1.11
-// (1.56 for oz_xc.cu, whose six 7-bit digits stop at 42 bits).  Hence no
+// cycle), 2,048 at h = w = 64.  With D the narrower units cost more MMAs, each of
+// which reads its 4 KB of A.  Measured, 2,097,152 rows, with D (without; FMAs):
+// 16 x 16 0.31 ms (-; 0.91), 32 x 32 0.55 (0.46; 3.5), 64 x 64 1.33 (0.88; 13.8);
+// 32 x 32 with X's columns graded over 18 decades 3.9 ms.  Hence no
 // shared-memory staging of X: its columns are read by coalesced 8-byte loads
 // straight into registers (any alignment and spacing of the columns), all 32 of
 // a thread in flight at once, while the MMAs of the previous tile run.
 //
 // Per CTA (one per SM, persistent over 128-row tiles; a tile's output columns
-// are taken 32 at a time, "units", into two alternating TMEM accumulator sets
-// so the MMAs of one unit overlap the epilogue of the previous one):
+// are taken 32 at a time, "units", into two alternating TMEM accumulator sets --
+// with D 16 at a time, three sets -- so that the MMAs of one unit overlap the
+// epilogue of the ones before):
 //   warps 8-15  producers: warp p holds rows 32 (p mod 4) .. + 31 (lane = row)
 //               of 32 columns in registers, finds the rows' scales and writes
 //               the digit slices in the 128-byte-swizzled K-major layout;
 //   warp 16     allocates TMEM; one thread issues tcgen05.mma.kind::f16
 //               (M = 128, K = 16): for X slice t one MMA per K step against the
 //               C slices stacked along N, so that level t + u lands at TMEM
-//               column 32 (t + u);
-//   warps 0-7   read a unit's eight level accumulators (lane = row; warps w and
-//               w + 4 share TMEM lanes and take 16 of the unit's 32 columns
-//               each), recombine and store Y.
+//               column 32 (16) (t + u), and D behind them;
+//   warps 0-7   read a unit's accumulators (lane = row; warps w and w + 4 share
+//               TMEM lanes and take half of the unit's columns each), recombine
+//               and store Y.
 // Every wait is bounded; a timeout sets an error word and all roles finish.
 #include <cuda_runtime.h>
+#include <math.h>
 #include <stdint.h>
 #include <string.h>
 
@@ -52,12 +70,21 @@
 #define OZY_THREADS 544
 #define OZY_NPROD 256
 #define OZY_ASLICE 16384          // 128 rows x 128 bytes
-#define OZY_BSLICE 4096           // 32 rows x 128 bytes (one unit's columns of one slice)
-#define OZY_UNIT 32               // output columns per unit
-#define OZY_SET (8 * OZY_UNIT)    // TMEM columns of one accumulator set
-#define OZY_C_BYTES (2 * OZY_S * OZY_BSLICE)  // [unit half][slice][32 rows][128 B]
-#define OZY_A_BYTES (OZY_S * OZY_ASLICE)
-#define OZY_SMEM (OZY_C_BYTES + OZY_A_BYTES + 1024)
+#define OZY_TILES 8               // tiles whose rows' scales and sums are kept
+
+// BOUND: every entry held to the bound of FP64 FMAs
+template <bool BOUND>
+struct ozy_cfg {
+  static constexpr int SLICES = BOUND ? OZY_S + 1 : OZY_S;  // the digits' and, last, the magnitudes of the top digits
+  static constexpr int UNIT = BOUND ? 16 : 32;              // output columns per unit
+  static constexpr int SETS = BOUND ? 3 : 2;
+  static constexpr int LEVELS = BOUND ? 9 : 8;              // accumulators of a column: levels 0-7 (and D)
+  static constexpr int SET = LEVELS * UNIT;                 // TMEM columns of one accumulator set
+  static constexpr int BSLICE = UNIT * 128;                 // one unit's columns of one slice
+  static constexpr int C_BYTES = 64 * 128 * SLICES;         // [unit][slice][UNIT rows][128 B]
+  static constexpr int SMEM = C_BYTES + SLICES * OZY_ASLICE + 1024;
+  static_assert(SETS * SET <= 512, "accumulators exceed TMEM");
+};
 
 struct ozy_params {
   const void *x[64], *z[64];
@@ -105,14 +132,15 @@ static __device__ __forceinline__ void ozy_load_z(int z_kind, const void* const*
   }
 }
 
-// the eight levels of four output columns of this warp's rows (not waited for)
-static __device__ __forceinline__ void ozy_tmem_ld(uint32_t taddr, uint32_t (&v)[8][4])
+// the accumulators of four output columns of this warp's rows (not waited for)
+template <int UNIT, int LEVELS>
+static __device__ __forceinline__ void ozy_tmem_ld(uint32_t taddr, uint32_t (&v)[LEVELS][4])
 {
 #pragma unroll
-  for (int L = 0; L < 8; L++)
+  for (int L = 0; L < LEVELS; L++)
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
                  : "=r"(v[L][0]), "=r"(v[L][1]), "=r"(v[L][2]), "=r"(v[L][3])
-                 : "r"(taddr + (uint32_t)(L * OZY_UNIT)));
+                 : "r"(taddr + (uint32_t)(L * UNIT)));
 }
 
 // one entry of X C by FP64 FMAs, in column order
@@ -120,8 +148,31 @@ static __device__ __noinline__ double ozy_direct(const void* const* s_x, const d
                                                  long row)
 {
   double acc = 0.0;
-  for (int i = 0; i < h; i++) acc = fma(((const double*)s_x[i])[row], C[i + (size_t)j * ldc], acc);
+#pragma unroll 8
+  for (int i = 0; i < h; i++) acc = fma(ozy_ld(s_x[i], row), C[i + (size_t)j * ldc], acc);
   return acc;
+}
+
+// the two FP16 sums of the magnitudes of eight digits (four words)
+static __device__ __forceinline__ uint32_t oz8_hadd2(uint32_t a, uint32_t b)
+{
+  uint32_t d;
+  asm("add.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  return d;
+}
+static __device__ __forceinline__ uint32_t ozy_magnitudes(const uint32_t (&d)[4], uint32_t (&m)[4])
+{
+#pragma unroll
+  for (int k = 0; k < 4; k++) m[k] = d[k] & 0x7FFF7FFFu;
+  return oz8_hadd2(oz8_hadd2(m[0], m[1]), oz8_hadd2(m[2], m[3]));
+}
+static __device__ __forceinline__ float ozy_both(uint32_t h2)
+{
+  float lo, hi;
+  asm("{\n .reg .b16 l, h;\n mov.b32 {l, h}, %2;\n cvt.f32.f16 %0, l;\n cvt.f32.f16 %1, h;\n}\n"
+      : "=f"(lo), "=f"(hi)
+      : "r"(h2));
+  return lo + hi;
 }
 
 // a group's largest exponent, raised to 1 (unsafe) when it holds nothing but
@@ -132,19 +183,28 @@ static __device__ __forceinline__ int ozy_group_exp(uint32_t mag, bool nonzero)
   return e == 0 && nonzero ? 1 : e;
 }
 
+template <bool BOUND>
 __global__ void __launch_bounds__(OZY_THREADS, 1) oz_xc64_kernel(const __grid_constant__ ozy_params prm)
 {
+  using K = ozy_cfg<BOUND>;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = smem_align1024(smem_raw);
-  unsigned char* cdig = smem;                // [half][S][32 rows][128 B]
-  unsigned char* adig = smem + OZY_C_BYTES;  // [S][128 rows][128 B]
-  __shared__ uint64_t a_full[4], a_empty[4], acc_full[2], acc_empty[2], done_bar;
+  unsigned char* cdig = smem;               // [unit][slice][UNIT rows][128 B]
+  unsigned char* adig = smem + K::C_BYTES;  // [slice][128 rows][128 B]
+  __shared__ uint64_t a_full[4], a_empty[4], acc_full[K::SETS], acc_empty[K::SETS], done_bar;
   __shared__ uint32_t tmem_base;
   __shared__ int abort_flag;
-  __shared__ int colexp[64];
+  __shared__ __align__(16) int colexp[64];
+  // the digits serve where D >= kappa (N + N') + const: by column, kappa and the rest
+  __shared__ __align__(16) float colkappa[BOUND ? 64 : 4], colneed[BOUND ? 64 : 4];
+  __shared__ int coltop[64], colnnz[64];  // N' and m
   __shared__ uint32_t colpart[8][64];      // per (8-row group of C, column) largest magnitude word
   __shared__ unsigned char colnz[8][64];   // and whether any value is not zero
-  __shared__ int rowexp[4][128];           // by tile modulo 4 (read by the epilogue)
+  // by tile modulo OZY_TILES (read by the epilogue): scales, and N by column half
+  // (two FP16 sums).  Written for tile i once the MMAs of tile i - 2 are done, hence
+  // the epilogue with every unit two or three before that tile's last: tile i - 5
+  __shared__ int rowexp[OZY_TILES][128];
+  __shared__ uint32_t rowtop[BOUND ? OZY_TILES : 1][2][128];
   __shared__ int rowpart[2][2][128];       // by tile modulo 2: per (column half, row) exponent
   // column pointers: shared memory serves a runtime index in a few cycles,
   // where the kernel-parameter table behind it does not
@@ -155,7 +215,7 @@ __global__ void __launch_bounds__(OZY_THREADS, 1) oz_xc64_kernel(const __grid_co
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int h = prm.h, w = prm.w;
   const int ksteps = (h + 15) >> 4;
-  const int nh = (w + OZY_UNIT - 1) / OZY_UNIT;  // units per tile
+  const int nh = (w + K::UNIT - 1) / K::UNIT;  // units per tile
   const long ntiles = (prm.n + 127) / 128;
   const long my_tiles = (long)blockIdx.x < ntiles ? (ntiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
 
@@ -165,13 +225,14 @@ __global__ void __launch_bounds__(OZY_THREADS, 1) oz_xc64_kernel(const __grid_co
       mbar_init(&a_full[k], OZY_NPROD);
       mbar_init(&a_empty[k], 1);
     }
-    for (int b = 0; b < 2; b++) {
+    for (int b = 0; b < K::SETS; b++) {
       mbar_init(&acc_full[b], 1);
       mbar_init(&acc_empty[b], 256);
     }
     mbar_init(&done_bar, 1);
   }
   if (tid < 64) {
+    coltop[tid] = colnnz[tid] = 0;
     s_x[tid] = tid < h ? prm.x[tid] : nullptr;
     s_y[tid] = tid < w ? prm.y[tid] : nullptr;
     s_z[tid] = (tid < w && prm.z_kind) ? prm.z[tid] : nullptr;
@@ -212,21 +273,30 @@ __global__ void __launch_bounds__(OZY_THREADS, 1) oz_xc64_kernel(const __grid_co
     const int E = ozy_group_exp(mag, nz);
     if (cg == 0) colexp[j] = oz8_code(E);
     uint32_t lo[8], hi[8], pk[OZY_S][4];
+    int nnz = 0;
 #pragma unroll
     for (int c = 0; c < 8; c++) {
       const int i = cg * 8 + c;
       const double v = (j < w && i < h) ? prm.C[i + (size_t)j * prm.ldc] : 0.0;
+      nnz += v != 0.0;
       lo[c] = (uint32_t)__double2loint(v);
       hi[c] = (uint32_t)__double2hiint(v);
     }
     oz8_digits8(lo, hi, oz8_scale(E), pk);
-    // rows of one unit half hold its 32 output columns; within a half the
-    // slices are stacked, so one MMA takes several slices as a single operand
-    const int jr = j & 31, hf = j >> 5;
-    const uint32_t off = (uint32_t)jr * 128u + ((uint32_t)(cg ^ (jr & 7)) << 4);
+    // a unit's slices of 16 output columns are stacked, so one MMA takes several
+    // of them as a single operand
+    const int jr = j & (K::UNIT - 1);
+    unsigned char* dst = cdig + (j / K::UNIT) * K::SLICES * K::BSLICE + jr * 128 + ((cg ^ (jr & 7)) << 4);
 #pragma unroll
     for (int t = 0; t < OZY_S; t++)
-      *(uint4*)(cdig + (hf * OZY_S + t) * OZY_BSLICE + off) = make_uint4(pk[t][0], pk[t][1], pk[t][2], pk[t][3]);
+      *(uint4*)(dst + t * K::BSLICE) = make_uint4(pk[t][0], pk[t][1], pk[t][2], pk[t][3]);
+    if (BOUND) {
+      uint32_t m[4];
+      const uint32_t top = ozy_magnitudes(pk[0], m);
+      *(uint4*)(dst + OZY_S * K::BSLICE) = make_uint4(m[0], m[1], m[2], m[3]);
+      atomicAdd(&coltop[j], (int)ozy_both(top));
+      atomicAdd(&colnnz[j], nnz);
+    }
   }
   fence_proxy_async();
   tc_fence_before();
@@ -281,7 +351,8 @@ __global__ void __launch_bounds__(OZY_THREADS, 1) oz_xc64_kernel(const __grid_co
       named_bar(1 + (pw & 3), 64);
       const int E = max(rowpart[i & 1][0][r], rowpart[i & 1][1][r]);
       const uint32_t es = oz8_scale(E);
-      if (half == 0) rowexp[i & 3][r] = oz8_code(E);
+      if (half == 0) rowexp[i % OZY_TILES][r] = oz8_code(E);
+      uint32_t top = 0;  // the sums of the magnitudes of the top digits: integers up to 2048
 #pragma unroll
       for (int k = 0; k < 4; k++) {
         if (k >= ksteps) break;
@@ -301,6 +372,12 @@ __global__ void __launch_bounds__(OZY_THREADS, 1) oz_xc64_kernel(const __grid_co
 #pragma unroll
           for (int t = 0; t < OZY_S; t++)
             *(uint4*)(adig + t * OZY_ASLICE + off) = make_uint4(pk[t][0], pk[t][1], pk[t][2], pk[t][3]);
+          if (BOUND) {
+            uint32_t m[4];
+            top = oz8_hadd2(top, ozy_magnitudes(pk[0], m));
+            *(uint4*)(adig + OZY_S * OZY_ASLICE + off) = make_uint4(m[0], m[1], m[2], m[3]);
+            if (k + 1 == ksteps) rowtop[i % OZY_TILES][half][r] = top;
+          }
           fence_proxy_async();
           mbar_arrive(&a_full[k]);
         }
@@ -313,13 +390,14 @@ __global__ void __launch_bounds__(OZY_THREADS, 1) oz_xc64_kernel(const __grid_co
       long u = 0;  // units issued
       for (long i = 0; i < my_tiles && !abort_flag; i++) {
         for (int hf = 0; hf < nh; hf++, u++) {
-          const int set = (int)(u & 1);
-          if (u >= 2 && !mbar_wait_n(&acc_empty[set], (uint32_t)(((u >> 1) - 1) & 1), &abort_flag, prm.polls)) {
+          const int set = (int)(u % K::SETS);
+          if (u >= K::SETS &&
+              !mbar_wait_n(&acc_empty[set], (uint32_t)((u / K::SETS - 1) & 1), &abort_flag, prm.polls)) {
             abort_flag = 1;
             atomicExch(prm.err, 15);
             break;
           }
-          const uint32_t d = tmem + (uint32_t)(set * OZY_SET);
+          const uint32_t d = tmem + (uint32_t)(set * K::SET);
           for (int ks = 0; ks < ksteps; ks++) {
             if (hf == 0 && !mbar_wait_n(&a_full[ks], (uint32_t)(i & 1), &abort_flag, prm.polls)) {
               abort_flag = 1;
@@ -327,15 +405,17 @@ __global__ void __launch_bounds__(OZY_THREADS, 1) oz_xc64_kernel(const __grid_co
               break;
             }
             tc_fence_after();
-            const uint32_t ab = abase + ks * 32, cb = cbase + hf * OZY_S * OZY_BSLICE + ks * 32;
+            const uint32_t ab = abase + ks * 32, cb = cbase + hf * K::SLICES * K::BSLICE + ks * 32;
             // slice t against C slices u0 .. u0 + nu - 1 (levels t + u0 ..).
             // t = 1 first: in the first K step its seven levels 1-7 start from
             // zero, level 0 from t = 0, u = 0, and everything else accumulates
-            auto mma = [&](int t, int u0, int nu, bool fresh) {
-              mma_bf16(d + (uint32_t)((t + u0) * OZY_UNIT), sw128_desc(ab + t * OZY_ASLICE),
-                       sw128_desc(cb + u0 * OZY_BSLICE), f16_idesc(128, OZY_UNIT * nu),
+            auto mma_at = [&](int level, int t, int u0, int nu, bool fresh) {
+              mma_bf16(d + (uint32_t)(level * K::UNIT), sw128_desc(ab + t * OZY_ASLICE),
+                       sw128_desc(cb + u0 * K::BSLICE), f16_idesc(128, K::UNIT * nu),
                        (!fresh || ks > 0) ? 1u : 0u);
             };
+            auto mma = [&](int t, int u0, int nu, bool fresh) { mma_at(t + u0, t, u0, nu, fresh); };
+            if (BOUND) mma_at(8, OZY_S, OZY_S, 1, true);  // D
             mma(1, 0, 7, true);
             if (ks == 0) {
               mma(0, 0, 1, true);
@@ -356,16 +436,23 @@ __global__ void __launch_bounds__(OZY_THREADS, 1) oz_xc64_kernel(const __grid_co
     // ------------------------------------------------------- epilogue
     const int quarter = warp & 3, chalf = warp >> 2;
     const int r = 32 * quarter + lane;
+    if (BOUND && tid < 64) {
+      const float inv = 1.0f / (float)(colnnz[tid] - 1);
+      const bool sums = colnnz[tid] > 1;  // (at most one product: none but the direct ones)
+      colkappa[tid] = sums ? 0.503f + 32.01f * inv : 0.f;
+      colneed[tid] = sums ? colkappa[tid] * (float)coltop[tid] + (32.01f * (float)h + 5330.f) * inv : HUGE_VALF;
+    }
+    if (BOUND) named_bar(5, 256);
     long u = 0;
     bool stop = false;
     for (long i = 0; i < my_tiles && !stop; i++) {
       const long row = (blockIdx.x + i * gridDim.x) * 128 + r;
       for (int hf = 0; hf < nh; hf++, u++) {
-        const int set = (int)(u & 1);
-        const int jbase = hf * OZY_UNIT + 16 * chalf;  // this warp's 16 columns
+        const int set = (int)(u % K::SETS);
+        const int jbase = hf * K::UNIT + K::UNIT / 2 * chalf;  // this warp's columns
         unsigned long long zn[4];  // Z, four columns ahead
         ozy_load_z(prm.z_kind, s_z, jbase, w, row, prm.n, zn);
-        const bool got = mbar_wait_n(&acc_full[set], (uint32_t)((u >> 1) & 1), &abort_flag, prm.polls);
+        const bool got = mbar_wait_n(&acc_full[set], (uint32_t)((u / K::SETS) & 1), &abort_flag, prm.polls);
         if (!__all_sync(0xffffffffu, got)) {  // tcgen05.ld needs the whole warp
           abort_flag = 1;
           atomicExch(prm.err, 16);
@@ -373,8 +460,10 @@ __global__ void __launch_bounds__(OZY_THREADS, 1) oz_xc64_kernel(const __grid_co
           break;
         }
         tc_fence_after();
-        const int er = rowexp[i & 3][r];
-        const uint32_t tl = tmem + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(set * OZY_SET + 16 * chalf);
+        const int er = rowexp[i % OZY_TILES][r];
+        float top = 0.f;
+        if (BOUND) top = ozy_both(rowtop[i % OZY_TILES][0][r]) + ozy_both(rowtop[i % OZY_TILES][1][r]);
+        const uint32_t tl = tmem + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(set * K::SET + K::UNIT / 2 * chalf);
         double yp[4];
         int jp = -1;
         auto put = [&](const double(&y)[4], int j0) {
@@ -385,43 +474,49 @@ __global__ void __launch_bounds__(OZY_THREADS, 1) oz_xc64_kernel(const __grid_co
         // (not unrolled: the roles of a scheduler's warps share its instruction
         // cache)
 #pragma unroll 1
-        for (int g = 0; g < 4; g++) {
+        for (int g = 0; g < K::UNIT / 8; g++) {
           const int j0 = jbase + 4 * g;
           if (j0 >= w) break;
           __syncwarp();  // (the branches below are taken by single lanes; tcgen05.ld needs the whole warp)
-          uint32_t x[8][4];  // the eight levels of four columns
-          ozy_tmem_ld(tl + (uint32_t)(4 * g), x);
+          uint32_t x[K::LEVELS][4];  // the eight levels (and D) of four columns
+          ozy_tmem_ld<K::UNIT, K::LEVELS>(tl + (uint32_t)(4 * g), x);
           // the previous four columns go out only now: their conversions and
           // additions have had this group's start to finish in
           if (g > 0) put(yp, jp);
           unsigned long long zb[4];
 #pragma unroll
           for (int jj = 0; jj < 4; jj++) zb[jj] = zn[jj];
-          if (g < 3) ozy_load_z(prm.z_kind, s_z, j0 + 4, w, row, prm.n, zn);
+          if (g + 1 < K::UNIT / 8) ozy_load_z(prm.z_kind, s_z, j0 + 4, w, row, prm.n, zn);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
           // (no branch among the entries: their integer chains overlap)
           double y[4];
           long long T[4];
           // out of the ordinary: the general conversion, or the direct sum
-          int e2[4];
-          bool odd = false;
+          const int4 ec4 = *(const int4*)&colexp[j0];
+          const float4 kp = *(const float4*)&colkappa[BOUND ? j0 : 0], nd4 = *(const float4*)&colneed[BOUND ? j0 : 0];
+          const int ec[4] = {ec4.x, ec4.y, ec4.z, ec4.w};
+          const float nd[4] = {fmaf(kp.x, top, nd4.x), fmaf(kp.y, top, nd4.y), fmaf(kp.z, top, nd4.z),
+                               fmaf(kp.w, top, nd4.w)};
+          bool odd = false, weak[4];
 #pragma unroll
           for (int jj = 0; jj < 4; jj++) {
             T[jj] = oz8_combine<false>(x[0][jj], x[1][jj], x[2][jj], x[3][jj], x[4][jj], x[5][jj], x[6][jj], x[7][jj]);
-            e2[jj] = er + colexp[j0 + jj];
+            weak[jj] = BOUND && !(__uint_as_float(x[K::LEVELS - 1][jj]) >= nd[jj]);
             // (|T| < 2^32: cancellation, a zero)
-            odd |= !oz8_ordinary(e2[jj]) || (uint32_t)((T[jj] >> 32) + 1) <= 1u;
+            odd |= !oz8_ordinary(er + ec[jj]) || (uint32_t)((T[jj] >> 32) + 1) <= 1u || weak[jj];
           }
           if (odd) {
 #pragma unroll
             for (int jj = 0; jj < 4; jj++) {
-              y[jj] = oz8_scaled(T[jj], e2[jj] - OZ8_BASE);
-              if (row < prm.n && j0 + jj < w && oz8_direct(er, colexp[j0 + jj]))
+              y[jj] = oz8_scaled(T[jj], er + ec[jj] - OZ8_BASE);
+              // (of a row or column of zeros T is 0)
+              if (row < prm.n && j0 + jj < w &&
+                  (oz8_direct(er, ec[jj]) || (er && ec[jj] && weak[jj])))
                 y[jj] = ozy_direct(s_x, prm.C, prm.ldc, h, j0 + jj, row);
             }
           } else {
 #pragma unroll
-            for (int jj = 0; jj < 4; jj++) y[jj] = oz8_scaled_fast(T[jj], e2[jj] - OZ8_BASE);
+            for (int jj = 0; jj < 4; jj++) y[jj] = oz8_scaled_fast(T[jj], er + ec[jj] - OZ8_BASE);
           }
           if (prm.z_kind == 1) {
             bool cvt = false;
@@ -475,6 +570,7 @@ __global__ void ozy_check_kernel(const int* err, int* status)
 }
 
 // columns [0, h) x [0, w) of the tables, h, w <= 64; polls <= 0: the default limit
+template <bool BOUND>
 static int ozy_launch(gpu_Context* ctx, long n, const void* const* X, int h, const double* C, int ldc,
                       const void* const* Y, int w, const void* const* Z, int z_kind, int polls, int* err)
 {
@@ -493,12 +589,12 @@ static int ozy_launch(gpu_Context* ctx, long n, const void* const* X, int h, con
   prm.n = n;
   prm.polls = polls > 0 ? (long)polls : TC_WAIT_LIMIT;
   prm.err = err;
-  if (cudaFuncSetAttribute(oz_xc64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, OZY_SMEM) !=
-      cudaSuccess)
-    return gb_fail(ctx, "oz_xc64: cannot reserve %d bytes of shared memory", OZY_SMEM);
+  const int smem = ozy_cfg<BOUND>::SMEM;
+  if (cudaFuncSetAttribute(oz_xc64_kernel<BOUND>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+    return gb_fail(ctx, "oz_xc64: cannot reserve %d bytes of shared memory", smem);
   const long ntiles = (n + 127) / 128;
   const unsigned nctas = (unsigned)(ntiles < ctx->num_sms ? ntiles : ctx->num_sms);
-  oz_xc64_kernel<<<nctas, OZY_THREADS, OZY_SMEM, (cudaStream_t)ctx->stream>>>(prm);
+  oz_xc64_kernel<BOUND><<<nctas, OZY_THREADS, smem, (cudaStream_t)ctx->stream>>>(prm);
   gb_count_launch(1);
   return gb_cuda_check(ctx, (int)cudaGetLastError(), "oz_xc64");
 }
@@ -518,7 +614,7 @@ extern "C" int gb_oz_xc64(gpu_Context* ctx, long n, const blk_cols* X, int h, co
   const int zk = Z ? (z_dtype == GPU_MV_FLOAT64 ? 2 : 1) : 0;
   gb_prof_rec pr;
   gb_prof_begin(ctx, &pr, GB_K_OZ_XC);
-  const int rc = ozy_launch(ctx, n, X->col, h, C, ldc, Y->col, w, Z ? Z->col : NULL, zk, ctx->opt.wait_polls, err);
+  const int rc = ozy_launch<false>(ctx, n, X->col, h, C, ldc, Y->col, w, Z ? Z->col : NULL, zk, ctx->opt.wait_polls, err);
   const double zb = zk == 2 ? 8.0 * w : (zk == 1 ? 4.0 * w : 0.0);
   gb_prof_end(ctx, &pr, (double)n * (8.0 * h + 8.0 * w + zb),
               2.0 * n * h * w);
@@ -529,19 +625,22 @@ extern "C" int gb_oz_xc64(gpu_Context* ctx, long n, const blk_cols* X, int h, co
 }
 
 // The FP64 block update of gb_bymat for any widths: 64 output columns at a
-// time, and within them 64 input columns at a time, the later ones added to
-// the sum so far.  A wait that gives up (with the default limit, whatever the
+// time, and within them up to 64 input columns at a time, the later ones added to
+// the sum so far.  (The parts' nonzeros add up to the column's, so that the
+// roundings of the parts and of the additions stay within its bound.)  A wait that gives up (with the default limit, whatever the
 // context's option) is reported in the device error word.
 extern "C" int gb_oz_bymat64(gpu_Context* ctx, long n, const blk_cols* X, int h, const double* C, int ldc,
                              const blk_cols* Y, int w, const blk_cols* Z)
 {
+  // (input columns in equal parts: a part of one or two columns would be summed directly)
+  const int hc = (h + (h + 63) / 64 - 1) / ((h + 63) / 64);
   for (int j0 = 0; j0 < w; j0 += 64) {
     const int wj = w - j0 < 64 ? w - j0 : 64;
-    for (int i0 = 0; i0 < h; i0 += 64) {
-      const int hi = h - i0 < 64 ? h - i0 : 64;
+    for (int i0 = 0; i0 < h; i0 += hc) {
+      const int hi = h - i0 < hc ? h - i0 : hc;
       const void* const* z = i0 ? Y->col + j0 : (Z ? Z->col + j0 : NULL);
-      if (ozy_launch(ctx, n, X->col + i0, hi, C + i0 + (size_t)j0 * ldc, ldc, Y->col + j0, wj, z, z ? 2 : 0, 0,
-                     ctx->dcount + 5))
+      if (ozy_launch<true>(ctx, n, X->col + i0, hi, C + i0 + (size_t)j0 * ldc, ldc, Y->col + j0, wj, z, z ? 2 : 0, 0,
+                           ctx->dcount + 5))
         return -1;
     }
   }

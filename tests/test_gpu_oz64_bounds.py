@@ -4,6 +4,8 @@ update, (32 + n / 32 / 304 + 310) 2^-53 sum |x_ri y_rj| for a Gram product (32
 roundings in a chunk, the chunks of a split, at most 304 splits).  The blocks
 are graded, localised and extreme ones, which a scale shared by a group of
 values does not absorb."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -139,6 +141,139 @@ def test_gram_mixed_lanes(ctx):
         norm = np.outer(xs.astype(L), ys.astype(L))
         mag, ref = _products(np.abs(X) / xs, np.abs(Y) / ys) * norm, _products(X / xs, Y / ys) * norm
     assert np.all(np.abs(G - ref) <= (32 + L(n) / 32 / 304 + 310 + 20) * EPS * mag + n * TINY)
+
+
+def test_update_mixed_lanes(ctx):
+    rng = np.random.default_rng(23)
+    n, h, w = 30001, 40, 41
+    X, C = rng.standard_normal((n, h)), rng.standard_normal((h, w))
+    X[::7] *= 1e-305
+    X[3::11] = 0.0
+    X[5::13, 1:] = 0.0
+    C[:, 3::5] *= 1e-170
+    Y0 = rng.standard_normal((n, w)) * 1e-150
+    Y = _update(ctx, X, C, Y0)
+    ref = X.astype(L) @ C + Y0
+    mag = np.abs(X).astype(L) @ np.abs(C)
+    assert np.all(np.abs(Y - ref) <= (h + 2) * EPS * mag + EPS * (mag + np.abs(Y0)) + (h + 1) * TINY)
+
+
+class _Cols(ctypes.Structure):
+    """blk_cols of internal.h."""
+    _fields_ = [("col", ctypes.c_void_p * 384)]
+
+
+def _columns(t):
+    c = _Cols()
+    for i in range(t.shape[0]):
+        c.col[i] = t[i].data_ptr()
+    return c
+
+
+def _dev(a):
+    return torch.from_numpy(np.ascontiguousarray(a.T)).cuda()
+
+
+def _tensor_update(ctx, X, C, Z=None):
+    """The tensor-core kernel of the callers' products, whatever the size."""
+    n, (h, w) = X.shape[0], C.shape
+    x, c, y = _dev(X), _dev(C), torch.full((w, n), 7.0, dtype=torch.float64, device="cuda")
+    if Z is not None:
+        y.copy_(_dev(Z))
+    torch.cuda.synchronize()
+    cy = _columns(y)
+    rc = ctx.lib.gb_oz_bymat64(ctypes.c_void_p(ctx.handle), ctypes.c_long(n), ctypes.byref(_columns(x)), h,
+                               ctypes.c_void_p(c.data_ptr()), h, ctypes.byref(cy), w,
+                               ctypes.byref(cy) if Z is not None else None)
+    assert rc == 0, ctx.last_error()
+    assert ctx.device_error() == 0
+    return y.cpu().numpy().T
+
+
+def _check_update(X, C, Z, Y):
+    h = X.shape[1]
+    ref, mag = X.astype(L) @ C, np.abs(X).astype(L) @ np.abs(C)
+    b = (h + 2) * EPS * mag + (h + 1) * TINY
+    if Z is not None:
+        ref = ref + Z
+        b = b + EPS * (np.abs(ref) + b)
+    err = np.abs(Y - ref)
+    assert np.all(err <= b), (float((err / b).max()), np.argwhere(err > b)[:3])
+
+
+def _grade(kind, n, h, rng):
+    """Factors for the columns (or entries) of X, of very different size."""
+    if kind == "even":
+        return np.ones(h)
+    if kind == "columns":  # columns that have converged to different degrees
+        return 10.0 ** -rng.uniform(0, 20, size=h)
+    if kind == "steps":
+        return np.array([1.0, 1e-3, 1e-9, 1e-13, 1e-17, 1e-30])[np.arange(h) % 6]
+    return 10.0 ** -rng.uniform(0, 25, size=(n, h))  # every entry its own
+
+
+def _coordinates(kind, h, w, rng):
+    C = rng.standard_normal((h, w))
+    if kind == "identity":
+        return np.eye(h, w)
+    if kind == "permutation":
+        return np.eye(h)[rng.permutation(h)][:, :w] * 3.0
+    if kind == "diagonal":
+        return np.eye(h, w) * 10.0 ** rng.uniform(-12, 12, size=(h, 1))
+    if kind == "triangular":
+        return np.triu(C)
+    if kind == "rows":  # graded the other way
+        return C * 10.0 ** rng.uniform(0, 20, size=(h, 1))
+    return C
+
+
+# shapes: one column, units of 16 columns partly empty, one to four units, K steps
+# partly empty, one to several tiles
+@pytest.mark.parametrize("n,h,w", [(700, 1, 1), (300, 5, 16), (4001, 16, 17), (2500, 33, 40), (1999, 64, 64)])
+@pytest.mark.parametrize("grade", ["even", "columns", "steps", "entries"])
+@pytest.mark.parametrize("coords", ["full", "identity", "permutation", "diagonal", "triangular", "rows"])
+def test_update_of_graded_blocks(ctx, n, h, w, grade, coords):
+    rng = np.random.default_rng(n + len(grade) + 7 * len(coords))
+    X = rng.standard_normal((n, h)) * _grade(grade, n, h, rng)
+    C = _coordinates(coords, h, w, rng)
+    Z = rng.standard_normal((n, C.shape[1])) * 1e-9 if coords == "full" else None
+    _check_update(X, C, Z, _tensor_update(ctx, X, C, Z))
+
+
+# the interpreter's entry, more than 64 input columns (the parts keep the bound of the whole)
+@pytest.mark.parametrize("n,h,w,grade,coords,add", [
+    (120001, 12, 12, "columns", "identity", False), (50001, 20, 17, "steps", "full", True),
+    (20003, 32, 32, "entries", "triangular", False), (5003, 70, 64, "columns", "full", True),
+    (2101, 130, 70, "steps", "rows", False), (2503, 129, 65, "entries", "identity", True)])
+def test_update_of_large_graded_blocks(ctx, n, h, w, grade, coords, add):
+    rng = np.random.default_rng(n + h)
+    X = rng.standard_normal((n, h)) * _grade(grade, n, h, rng)
+    C = _coordinates(coords, h, w, rng)
+    Y0 = rng.standard_normal((n, w)) * 1e-12 if add else None
+    _check_update(X, C, Y0, _update(ctx, X, C, Y0))
+
+
+def test_update_copies_columns_exactly(ctx):
+    """C = I: every output column is an input column, to the last bit."""
+    rng = np.random.default_rng(31)
+    n, h = 60000, 24
+    X = rng.standard_normal((n, h)) * 10.0 ** -rng.uniform(0, 40, size=h)
+    assert np.array_equal(_update(ctx, X, np.eye(h)), X)
+
+
+def test_update_of_random_blocks_is_no_further_off_than_multiply_adds(ctx):
+    rng = np.random.default_rng(32)
+    for n, h, w in ((20000, 8, 16), (20000, 16, 16), (20000, 32, 32), (10000, 64, 64)):
+        X, C = rng.standard_normal((n, h)), rng.standard_normal((h, w))
+        ref = X.astype(L) @ C
+        mx, my = S.MultiVector.from_host(ctx, X), S.MultiVector(ctx, n, w)
+        Cf = np.asfortranarray(C)
+        assert ctx.lib.gpu_BlockUpdate(mx.handle, Cf.ctypes.data, h, my.handle, None, 0) == 0
+        err = []
+        for Y in (my.to_host(), _tensor_update(ctx, X, C)):
+            d = (Y - ref).astype(np.float64)
+            err.append((np.abs(d).max(), np.sqrt(np.mean(d * d))))
+        assert err[1][0] <= err[0][0] and err[1][1] <= err[0][1], (h, w, err)
 
 
 def _in_place(ctx, X, C, add):

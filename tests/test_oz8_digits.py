@@ -205,3 +205,49 @@ def test_fast_conversion_where_it_is_used():
                 assert err <= Fraction(2) ** (base + max(T.bit_length() - 54, -1))
                 assert err == 0 or T.bit_length() > 53
     assert scaled_fast(1 << 56, 2 * 359 - BASE) != scaled(1 << 56, 2 * 359 - BASE)  # 1e-200 x 1e-200
+
+
+def _update_entry(x, c):
+    """One entry of the update from digits: the result, and whether the sums of the
+    top digits let it stand (oz_xc64.cu)."""
+    Ex, Ec = max(map(bexp, x)), max(map(bexp, c))
+    dx, dc = [signed(v, Ex) for v in x], [signed(v, Ec) for v in c]
+    lev = [sum(a[t] * b[L_ - t] for a, b in zip(dx, dc) for t in range(S) if 0 <= L_ - t < S) for L_ in range(8)]
+    reg, T = combine(lev, False)
+    assert reg == T
+    N, N2 = sum(abs(d[0]) for d in dx), sum(abs(d[0]) for d in dc)
+    D = sum(abs(a[0] * b[0]) for a, b in zip(dx, dc))
+    m = sum(v != 0 for v in c)
+    if m < 2:
+        return scaled(T, Ex + Ec - BASE), False
+    kappa = f32(0.503) + f32(32.01) / f32(m - 1)
+    need = f32(kappa * f32(N)) + f32(f32(kappa * f32(N2)) + (f32(32.01) * f32(len(x)) + f32(5330)) / f32(m - 1))
+    return scaled(T, Ex + Ec - BASE), D >= need
+
+
+def test_update_entries_that_stand_keep_the_bound_of_multiply_adds():
+    """m 2^-53 sum |x_i c_i|, m the nonzeros of c, whatever the values' sizes; and
+    random ones do stand."""
+    rng = random.Random(17)
+    stood = dict.fromkeys(("even", "graded", "sparse", "top"), 0)
+    for trial in range(1600):
+        kind = list(stood)[trial % 4]
+        h = rng.choice([2, 3, 8, 16, 32, 64])
+        x, c = [rng.gauss(0, 1) for _ in range(h)], [rng.gauss(0, 1) for _ in range(h)]
+        if kind == "graded":
+            x = [v * 10.0 ** -rng.uniform(0, 18) for v in x]
+            c = [v * 10.0 ** -rng.uniform(0, rng.choice([1, 18])) for v in c]
+        elif kind == "sparse":
+            c = [v if rng.random() < 0.3 else 0.0 for v in c]
+            c[0] = c[0] or 1.0
+        elif kind == "top":  # values just below the places where a top digit rounds
+            x = [rng.choice([1 - 2.0 ** -53, 0.0039, 0.00390624, 0.0117, 2.0 ** -30]) for _ in x]
+        y, ok = _update_entry(x, c)
+        if not ok:
+            continue
+        stood[kind] += h >= 32
+        exact = sum(Fraction(a) * Fraction(b) for a, b in zip(x, c))
+        mag = sum(abs(Fraction(a) * Fraction(b)) for a, b in zip(x, c))
+        m = sum(v != 0 for v in c)
+        assert abs(Fraction(y) - exact) <= m * Fraction(1, 1 << 53) * mag, (kind, h, trial)
+    assert stood["even"] > 100 and stood["graded"] > 0 and stood["sparse"] > 20
