@@ -139,7 +139,8 @@ static __device__ __forceinline__ long long oz8_combine(uint32_t s0, uint32_t s1
   const int a4 = (int)(__float_as_uint(y4) - b24), a5 = (int)(__float_as_uint(y5) - b24);
   const int a6 = (int)(i6 * 256u + i7 - b24 * 257u + 8192u) >> 14;
   const long long t = (long long)a1 * 131072 + ((long long)a4 * 1024 + (long long)(a5 * 4 + a6));
-  return HALF ? ((t + 1) >> 1) + ((long long)a0 << 32) : t + ((long long)a0 << 33);
+  // (an odd t to the even half: always up, the sums over many groups drifted)
+  return HALF ? ((t + ((t >> 1) & 1)) >> 1) + ((long long)a0 << 32) : t + ((long long)a0 << 33);
 }
 
 // FP64 nearest to T 2^base, |T| < 2^63, from integer operations only (ties
