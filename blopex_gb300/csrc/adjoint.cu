@@ -150,10 +150,10 @@ int project(adj_state* a, gpu_MultiVector* L, gpu_MultiVector* R, gpu_MultiVecto
   cols_of(R, &cr);
   cols_of(y, &cy);
   const int k = a->k;
-  if (gb_gram_large(a->ctx, GPU_MV_FLOAT64, a->n, &cr, k, &cy, k, a->M, k)) return -1;
+  if (gb_gram(a->ctx, GPU_MV_FLOAT64, a->n, &cr, k, &cy, k, a->M, k)) return -1;
   adj_neg_kernel<<<(k * k + 255) / 256, 256, 0, S(a->ctx)>>>(k * k, a->M);
   gb_count_launch(1);
-  return gb_bymat_large(a->ctx, GPU_MV_FLOAT64, a->n, &cl, k, a->M, k, &cy, k, &cy);
+  return gb_bymat(a->ctx, GPU_MV_FLOAT64, a->n, &cl, k, a->M, k, &cy, k, &cy);
 }
 
 int dots(adj_state* a, gpu_MultiVector* x, gpu_MultiVector* y, double* out)
@@ -277,7 +277,7 @@ extern "C" int gpu_EigenvectorAdjoint(gpu_MultiVector* X, const double* lambda, 
     adj_inspace_kernel<<<(unsigned)((kk + 255) / 256), 256, 0, S(ctx)>>>(k, a.M, a.lam, a.glam, HUGE_VAL,
                                                                          a.M);
     gb_count_launch(1);
-    rc = gb_bymat_large(ctx, GPU_MV_FLOAT64, a.n, &cx, k, a.M, k, &cw, k, NULL);
+    rc = gb_bymat(ctx, GPU_MV_FLOAT64, a.n, &cx, k, a.M, k, &cw, k, NULL);
     if (xg)
       for (int i = 0; i < k; i++) xg[i] = 0.0;
   } else if (!rc) {
@@ -285,12 +285,12 @@ extern "C" int gpu_EigenvectorAdjoint(gpu_MultiVector* X, const double* lambda, 
     for (int i = 0; i < k; i++) lmax = fmax(lmax, fabs(lambda[i]));
     const double tol_deg = 1e-12 * (lmax > 0.0 ? lmax : 1.0);
     // S = X'G; x_i'g_i for the mass term; W = X M (in-space part + glam)
-    rc = gb_gram_large(ctx, GPU_MV_FLOAT64, a.n, &cx, k, &cg, k, a.Sg, k);
+    rc = gb_gram(ctx, GPU_MV_FLOAT64, a.n, &cx, k, &cg, k, a.Sg, k);
     if (!rc) {
       adj_inspace_kernel<<<(unsigned)((kk + 255) / 256), 256, 0, S(ctx)>>>(k, a.Sg, a.lam, a.glam,
                                                                            tol_deg, a.M);
       gb_count_launch(1);
-      rc = gb_bymat_large(ctx, GPU_MV_FLOAT64, a.n, &cx, k, a.M, k, &cw, k, NULL);
+      rc = gb_bymat(ctx, GPU_MV_FLOAT64, a.n, &cx, k, a.M, k, &cw, k, NULL);
     }
     if (!rc && xg) {
       double* hs = (double*)malloc(sizeof(double) * kk);
@@ -300,7 +300,7 @@ extern "C" int gpu_EigenvectorAdjoint(gpu_MultiVector* X, const double* lambda, 
       free(hs);
     }
     // r = -(I - B X X') G = BX S - G ; mu = 0
-    if (!rc) rc = gb_bymat_large(ctx, GPU_MV_FLOAT64, a.n, &cbx, k, a.Sg, k, &cr, k, NULL);
+    if (!rc) rc = gb_bymat(ctx, GPU_MV_FLOAT64, a.n, &cbx, k, a.Sg, k, &cr, k, NULL);
     if (!rc) rc = gb_axpby(ctx, GPU_MV_FLOAT64, a.n, -1.0, &cg, 1.0, &cr, k);
     if (!rc) rc = gb_axpby(ctx, GPU_MV_FLOAT64, a.n, 0.0, &cr, 0.0, &cmu, k);
     if (!rc) rc = dots(&a, a.r, a.r, a.bn2);
