@@ -431,17 +431,17 @@ extern "C" int gb_gram(gpu_Context* ctx, int dtype, long n, const blk_cols* X, i
   return gram_launch<float, 4, 4>(ctx, n, X, h, Y, w, G, ldg);
 }
 
-// Callers' products (the interpreter's entry, the adjoint): FP64 ones of at
-// least GRAM_TENSOR_MIN multiply-adds on the tensor cores (oz_gram64.cu), with
-// an error no larger.  The FP64 pipe takes 0.17 ms for them at its 0.58 T
-// multiply-adds/s, the tensor-core kernel 0.05 to 0.07 (65,536 x 32 x 32: 45 us
+// A caller's products (the interpreter's entry): FP64 ones of at least
+// GRAM_TENSOR_MIN multiply-adds on the tensor cores (oz_gram64.cu), checked there
+// against the bound of multiply-adds.  The FP64 pipe takes 0.17 ms for them at its
+// 0.58 T multiply-adds/s, the tensor-core kernel 0.05 to 0.07 (65,536 x 32 x 32: 45 us
 // against 125; 16,384 x 32 x 32: 51 against 30).  The solver keeps gb_gram: the
 // signs of its Ritz vectors follow the last bits of these sums, and a solve
 // returns the same iterates, bit for bit, as it always did.
 #define GRAM_TENSOR_MIN 1e8
 
 extern "C" int gb_gram_large(gpu_Context* ctx, int dtype, long n, const blk_cols* X, int h,
-                             const blk_cols* Y, int w, double* G, int ldg)
+                             const blk_cols* Y, int w, double* G, int ldg, int* verdict)
 {
   if (h <= 0 || w <= 0) return 0;
   if (dtype != GPU_MV_FLOAT64 || (double)n * h * w < GRAM_TENSOR_MIN)
@@ -451,12 +451,12 @@ extern "C" int gb_gram_large(gpu_Context* ctx, int dtype, long n, const blk_cols
   long splits;
   gb_prof_rec pr;
   gb_prof_begin(ctx, &pr, GB_K_GRAM);
-  if (gb_oz_gram64(ctx, n, X, h, Y, w, sym, &partial, &splits)) return -1;
+  if (gb_oz_gram64(ctx, n, X, h, Y, w, sym, &partial, &splits, verdict)) return -1;
   gb_pdl(gram_reduce_kernel, (h * w + 31) / 32, 256, 0, S(ctx), partial, (int)splits, 1, splits, h * w, h, sym ? 2 : 0, G,
                                                             ldg);
   gb_prof_end(ctx, &pr, 8.0 * n * (sym ? h : h + w), sym ? (double)n * h * (h + 1) : 2.0 * n * h * w);
   gb_count_launch(1);
-  return CUDA_LAUNCH_CHECK(ctx, "gram64");
+  return CUDA_LAUNCH_CHECK(ctx, "gram64") ? -1 : 1;
 }
 
 // ------------------------------------------------------------------------

@@ -118,9 +118,11 @@ int gb_mv_fill_cols(const gpu_MultiVector* x, blk_cols* t, int offset);
    X(:,0:h)' * Y(:,0:w); X and Y share dtype. */
 int gb_gram(gpu_Context* ctx, int dtype, long n, const blk_cols* X, int h, const blk_cols* Y,
             int w, double* G, int ldg);
-/* the same for callers outside the solver: large FP64 products on the tensor cores */
+/* the same for callers that read the result on the host: large FP64 products on the
+   tensor cores.  Returns 1 when those took the product: the caller then reads
+   *verdict (device), and takes the product again with gb_gram when it is not 0 */
 int gb_gram_large(gpu_Context* ctx, int dtype, long n, const blk_cols* X, int h, const blk_cols* Y,
-                  int w, double* G, int ldg);
+                  int w, double* G, int ldg, int* verdict);
 /* Y(:,j) = sum_i X(:,i) C(i,j) [+ Z(:,j)], C FP64 device column-major (ldc) */
 int gb_bymat(gpu_Context* ctx, int dtype, long n, const blk_cols* X, int h, const double* C,
              int ldc, const blk_cols* Y, int w, const blk_cols* Z);
@@ -205,9 +207,10 @@ int gb_oz_bymat64(gpu_Context* ctx, long n, const blk_cols* X, int h, const doub
                   const blk_cols* Y, int w, const blk_cols* Z);
 /* the CTAs' sums of X' Y for FP64 blocks of any widths and alignments
    (oz_gram64.cu), in the workspace: [split][w][h], *splits of them; sym: X and
-   Y are the same columns */
+   Y are the same columns; *verdict (device): 1 when an entry may be further off than
+   FP64 multiply-adds, else 0 */
 int gb_oz_gram64(gpu_Context* ctx, long n, const blk_cols* X, int h, const blk_cols* Y, int w, int sym,
-                 const double** partial, long* splits);
+                 const double** partial, long* splits, int* verdict);
 /* FP64-accurate Gram G = L' [L Q_0 Q_1 ...] on the tensor cores (oz_gram.cu):
    L a block of h <= 64 columns, FP32 or FP64 (ldt); nq <= 4 blocks Q_b of up
    to 64 columns each, FP32 or FP64 (qdt[b]); every column 16-byte aligned and

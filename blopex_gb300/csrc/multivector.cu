@@ -300,14 +300,22 @@ static void gi_InnerProd(void* x_, void* y_, BlopexInt gh, BlopexInt h, BlopexIn
     gb_fail(ctx, "MultiInnerProd: shape mismatch");
     return;
   }
-  double* g = (double*)gb_device_alloc(ctx, sizeof(double) * (size_t)(h > 0 ? h : 1) * (w > 0 ? w : 1));
+  // the product and, behind it, the verdict on a product of the tensor cores
+  const size_t hw = (size_t)(h > 0 ? h : 0) * (w > 0 ? w : 0);
+  double* g = (double*)gb_device_alloc(ctx, sizeof(double) * (hw + 1));
   if (!g) return;
   blk_cols a, b;
   gb_mv_fill_cols(x, &a, 0);
   gb_mv_fill_cols(y, &b, 0);
-  if (gb_gram_large(ctx, x->dtype, x->size, &a, h, &b, w, g, h) == 0) {
-    double* tmp = (double*)malloc(sizeof(double) * (size_t)h * w);
-    if (gb_memcpy_d2h(ctx, tmp, g, sizeof(double) * (size_t)h * w) == 0)
+  const int tensor = gb_gram_large(ctx, x->dtype, x->size, &a, h, &b, w, g, h, (int*)(g + hw));
+  if (tensor >= 0) {
+    double* tmp = (double*)malloc(sizeof(double) * (hw + 1));
+    int rc = gb_memcpy_d2h(ctx, tmp, g, sizeof(double) * (hw + tensor));
+    if (!rc && tensor && *(int*)(tmp + hw) != 0) {
+      rc = gb_gram(ctx, x->dtype, x->size, &a, h, &b, w, g, h);
+      if (!rc) rc = gb_memcpy_d2h(ctx, tmp, g, sizeof(double) * hw);
+    }
+    if (!rc)
       for (int j = 0; j < w; j++)
         for (int i = 0; i < h; i++) ((double*)v)[i + (size_t)j * gh] = tmp[i + (size_t)j * h];
     free(tmp);

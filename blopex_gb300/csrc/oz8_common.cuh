@@ -101,6 +101,29 @@ static __device__ __forceinline__ void oz8_digits8(const uint32_t* lo, const uin
   }
 }
 
+// the magnitudes of the top digits of eight values (their four words), and these
+// added up into two FP16 numbers: integers, exact up to 2048
+static __device__ __forceinline__ uint32_t oz8_hadd2(uint32_t a, uint32_t b)
+{
+  uint32_t d;
+  asm("add.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  return d;
+}
+static __device__ __forceinline__ uint32_t oz8_magnitudes(const uint32_t (&d)[4], uint32_t (&m)[4])
+{
+#pragma unroll
+  for (int k = 0; k < 4; k++) m[k] = d[k] & 0x7FFF7FFFu;
+  return oz8_hadd2(oz8_hadd2(m[0], m[1]), oz8_hadd2(m[2], m[3]));
+}
+static __device__ __forceinline__ float oz8_both(uint32_t h2)
+{
+  float lo, hi;
+  asm("{\n .reg .b16 l, h;\n mov.b32 {l, h}, %2;\n cvt.f32.f16 %0, l;\n cvt.f32.f16 %1, h;\n}\n"
+      : "=f"(lo), "=f"(hi)
+      : "r"(h2));
+  return lo + hi;
+}
+
 // The exact integer T = sum_L S_L 256^(7 - L) of the eight level sums, in
 // units of 2^15 (rounded once, at 2^-55 of the scales' product): |S_0..3| <=
 // 2^22, the others up to 2^23.  FP32 to integer by adding 1.5 2^23 (exact to

@@ -31,6 +31,21 @@
 // rows: 32 x 32 0.63 ms (FP64 FMAs 3.9; HBM 0.16), 64 x 64 1.61 (14.5), X'X of 64
 // 1.25 (7.9).  Relative error 2.1e-16 on random blocks (FMAs 6 to 9e-16).
 //
+// Accuracy.  Within a group of R rows, scales S and S', the digits are off by up to
+// 2^-55 S S' (|x/S| + |y/S'| + 4) (1-norms: every value cut below 2^-55 of its
+// scale, products of levels 8 and up left out, T rounded), which is small beside the
+// roundings of multiply-adds only where sum |x_r y_r| is not far below S S' -- not,
+// say, for columns that are large in different rows.  So the result is checked.
+// The producers sum the groups' Q = sum S^2 and P = sum (S |x/S|)^2 of every column
+// (1-norms from the top digits), which bound the error of an entry by
+// 2^-55 (sqrt(P Q') + sqrt(Q P') + 4 sqrt(Q Q')); gram64_cover_kernel adds up
+// |x_r y_r| over an eighth of the rows in FP32, rounded down, a lower bound of
+// sum |x_r y_r|; and gram64_verdict_kernel asks for an error of at most
+// OZH_ROUNDINGS 2^-53 of it.  Together with the additions over groups and CTAs that
+// is within (32 + n / 9728 + 310) 2^-53 sum |x_r y_r|, the bound of the kernels of
+// blockops.cu.  Random blocks pass with a factor of 20 to spare; when an entry does
+// not, the caller takes the product again with FP64 multiply-adds.
+//
 // Columns whose scale the digits cannot carry in some group (infinities, NaN,
 // values below 2^-960) and pairs of columns whose product's scale is below 2^-924
 // are summed directly there with FP64 FMAs.
@@ -46,17 +61,21 @@
 // Every wait is bounded; a timeout sets the device error word and the outputs
 // become NaN.
 #include <cuda_runtime.h>
+#include <math.h>
 #include <stdint.h>
 #include <string.h>
 
 #include "internal.h"
 #include "oz8_common.cuh"
+#include "pdl.cuh"
 
 #define OZH_THREADS 544
 #define OZH_PROD 8               // producer warps
 #define OZH_STAGE 32             // rows per stage
 #define OZH_MAXST 4              // stages of the ring
 #define OZH_SMEM_MAX 225280
+#define OZH_ROUNDINGS 128        // units of 2^-53 sum |x y| that the digits may be off
+#define OZH_SAMPLE 256           // one chunk of 32 rows in so many is covered
 
 struct ozh_params {
   const void *x[BLK_MAXCOLS], *y[BLK_MAXCOLS];
@@ -64,6 +83,7 @@ struct ozh_params {
   int nst, acc_off, smem;  // ring stages, offset of the FP64 sums, bytes
   long n;
   double* partial;         // [CTA][w][h]
+  double* norms;           // [CTA][Q, P][h + w]
   int* err;
 };
 
@@ -112,6 +132,7 @@ __global__ void __launch_bounds__(OZH_THREADS, 1) oz_gram64_kernel(const __grid_
   __shared__ int abort_flag;
   __shared__ int cexp[4][128];         // scales, by group modulo 4: X's columns, then from 64 Y's
   __shared__ const void* s_col[128];
+  __shared__ double s_norm[2][128];    // Q and P of the columns
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int ti = blockIdx.y % prm.tx, tj = blockIdx.y / prm.tx;
@@ -128,6 +149,7 @@ __global__ void __launch_bounds__(OZH_THREADS, 1) oz_gram64_kernel(const __grid_
   const int nsets = hpad <= 32 ? 2 : 1;
 
   if (tid < 128) {
+    s_norm[0][tid] = s_norm[1][tid] = 0.0;
     const int c = tid & 63;
     s_col[tid] = tid < 64 ? (c < h ? prm.x[i0 + c] : nullptr) : (c < w ? prm.y[j0 + c] : nullptr);
   }
@@ -176,6 +198,8 @@ __global__ void __launch_bounds__(OZH_THREADS, 1) oz_gram64_kernel(const __grid_
     uint32_t emax[2] = {0, 0};      // the largest magnitude word so far of the group being scouted
     uint32_t anyb[2] = {0, 0};      // any bit set (subnormals)
     uint32_t es[2] = {0, 0};
+    uint32_t top2[2] = {0, 0};      // the top digits' magnitudes of up to four stages,
+    float topf[2] = {0.f, 0.f};     // and of the group so far
 #pragma unroll
     for (int m = 0; m < 2; m++) {
       const int u = pw + OZH_PROD * m;
@@ -220,6 +244,21 @@ __global__ void __launch_bounds__(OZH_THREADS, 1) oz_gram64_kernel(const __grid_
       }
       emax[m] = anyb[m] = 0;
     };
+    // the group's part of Q and P (|x/S| <= (top digits + R / 2) / 128)
+    auto measure = [&](int m) {
+      float t = topf[m];
+      t += __shfl_xor_sync(0xffffffffu, t, 1);
+      t += __shfl_xor_sync(0xffffffffu, t, 2);
+      topf[m] = 0.f;
+      const int E = (int)(es[m] >> 20);  // 0xFFF: zeros
+      if (q == 0 && col[m] && E < 2047 && E >= 64) {
+        // (S^2 has to fit: other columns fail the check)
+        const double S = E >= 542 && E <= 1502 ? __hiloint2double((E + 1) << 20, 0) : HUGE_VAL;
+        const double P = S * (double)(t * 0.0078125f + (float)R * 0.00390625f);
+        s_norm[0][slot[m]] += S * S;
+        s_norm[1][slot[m]] += P * P;
+      }
+    };
     auto row_of = [&](long g) { return (blockIdx.x + g * gridDim.x) * R; };
     uint2 v[8];
     if (my_groups > 0) {
@@ -262,6 +301,12 @@ __global__ void __launch_bounds__(OZH_THREADS, 1) oz_gram64_kernel(const __grid_
                 hi[e] = v[e].y;
               }
               oz8_digits8(lo, hi, es[m], pk);
+              uint32_t mag[4];
+              top2[m] = oz8_hadd2(top2[m], oz8_magnitudes(pk[0], mag));
+              if ((s & 3) == 3) {
+                topf[m] += oz8_both(top2[m]);
+                top2[m] = 0;
+              }
             }
             // the next unit's values
             if (m + 1 < mine)
@@ -284,10 +329,22 @@ __global__ void __launch_bounds__(OZH_THREADS, 1) oz_gram64_kernel(const __grid_
           phase ^= 1;
         }
       }
-      if (more) {
 #pragma unroll
-        for (int m = 0; m < 2; m++)
-          if (m < mine) settle(m, g + 1);
+      for (int m = 0; m < 2; m++) {
+        if (m < mine) {
+          measure(m);
+          if (more) settle(m, g + 1);
+        }
+      }
+    }
+    // X's columns from the tiles of the first column, Y's from those of the first row
+#pragma unroll
+    for (int m = 0; m < 2; m++) {
+      if (q == 0 && col[m] && (slot[m] < 64 ? tj : ti) == 0) {
+        double* out = prm.norms + (size_t)blockIdx.x * 2 * (prm.h + prm.w) +
+                      (slot[m] < 64 ? i0 + slot[m] : prm.h + j0 + slot[m] - 64);
+        out[0] = s_norm[0][slot[m]];
+        out[prm.h + prm.w] = s_norm[1][slot[m]];
       }
     }
   } else if (warp == 16) {
@@ -443,8 +500,131 @@ __global__ void __launch_bounds__(OZH_THREADS, 1) oz_gram64_kernel(const __grid_
   }
 }
 
+// Lower bounds of sum |x_r y_r|: the CTAs' sums over every gridDim.z-th of the sampled
+// chunks (32 rows of each OZH_SAMPLE, moving through them), 32 x 32 entries, in FP32 on
+// values cut to 20 bits and scaled by a power of two near the column's rms scale
+// (from Q; values 2^40 above it count as that much, far smaller ones as 0).
+// FP32 arithmetic takes 20 us at 2,097,152 x 32 x 32.
+__global__ void __launch_bounds__(256) gram64_cover_kernel(blk_cols X, int h, blk_cols Y, int w, int sym, long n,
+                                                           const double* __restrict__ norms, int parts, long groups,
+                                                           double* __restrict__ cover, int* verdict)
+{
+  gb_pdl_entry();
+  __shared__ float xs[32][33], ys[32][33];
+  __shared__ double sq[64][5];
+  __shared__ int eref[64];  // the columns' reference exponents (biased): X's, Y's
+  const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
+  const int i0 = blockIdx.x * 32, j0 = blockIdx.y * 32;
+  if (t == 0 && blockIdx.x + blockIdx.y + blockIdx.z == 0) *verdict = 0;
+  {
+    const int c = t >> 2;
+    const int k = c < 32 ? i0 + c : j0 + c - 32;
+    double s = 0.0;
+    if (k < (c < 32 ? h : w))
+      for (int p = t & 3; p < parts; p += 4) s += norms[(size_t)p * 2 * (h + w) + (c < 32 || sym ? k : h + k)];
+    sq[c][t & 3] = s;
+  }
+  __syncthreads();
+  if (t < 64) {
+    const double s = (sq[t][0] + sq[t][1] + sq[t][2] + sq[t][3]) / (double)groups;
+    const int e = (int)((uint32_t)__double2hiint(s) >> 20) - 1023;  // of the mean of S^2
+    eref[t] = s > 0.0 && e < 1000 ? 1022 + (e >> 1) : 1022;
+  }
+  __syncthreads();
+  // a value's place in the tile: row t % 32 of the chunk, columns t / 32 + 8 k
+  const uint32_t* col[8];
+  int ref[8];
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    const int c = (t >> 5) + 8 * k;
+    col[k] = (const uint32_t*)(c < 32 ? (i0 + c < h ? X.col[i0 + c] : NULL) : (j0 + c - 32 < w ? Y.col[j0 + c - 32] : NULL));
+    ref[k] = eref[c] - 127;
+  }
+  const long blocks = (n + OZH_SAMPLE - 1) / OZH_SAMPLE;
+  float acc[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+  uint32_t v[8];
+  auto load = [&](long b) {
+    long r = b * OZH_SAMPLE + 32 * ((5 * b + (b >> 3)) & (OZH_SAMPLE / 32 - 1));
+    if (r >= n) r = b * OZH_SAMPLE;
+    r += t & 31;
+#pragma unroll
+    for (int k = 0; k < 8; k++) v[k] = b < blocks && col[k] && r < n ? col[k][2 * r + 1] : 0u;  // the high word
+  };
+  load(blockIdx.z);
+  for (long b = blockIdx.z; b < blocks; b += gridDim.z) {
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      // biased FP32 exponent e - ref, the leading 20 bits of the fraction
+      const int d = (int)(v[k] & 0x7FFFFFFFu) - (ref[k] << 20);
+      const int e = d < 0x100000 ? 0 : min(d, 167 << 20);
+      const float f = __int_as_float(e << 3);
+      const int c = (t >> 5) + 8 * k;
+      if (c < 32)
+        xs[c][t & 31] = f;
+      else
+        ys[c - 32][t & 31] = f;
+    }
+    __syncthreads();
+    load(b + gridDim.z);
+#pragma unroll 8
+    for (int r = 0; r < 32; r++) {
+      const float x0 = xs[tx][r], x1 = xs[tx + 16][r], y0 = ys[ty][r], y1 = ys[ty + 16][r];
+      acc[0][0] = fmaf(x0, y0, acc[0][0]);
+      acc[0][1] = fmaf(x0, y1, acc[0][1]);
+      acc[1][0] = fmaf(x1, y0, acc[1][0]);
+      acc[1][1] = fmaf(x1, y1, acc[1][1]);
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int a = 0; a < 2; a++)
+#pragma unroll
+    for (int b = 0; b < 2; b++) {
+      const int ii = tx + 16 * a, jj = ty + 16 * b;
+      if (i0 + ii < h && j0 + jj < w)
+        cover[((size_t)blockIdx.z * w + j0 + jj) * h + i0 + ii] =
+            (double)acc[a][b] * __hiloint2double(eref[ii] << 20, 0) * __hiloint2double(eref[32 + jj] << 20, 0);
+    }
+}
+
+// *verdict |= 1 where the digits' error may exceed its share
+__global__ void __launch_bounds__(256) gram64_verdict_kernel(const double* __restrict__ norms, int parts,
+                                                             const double* __restrict__ cover, int covers, int h,
+                                                             int w, int sym, int* verdict)
+{
+  gb_pdl_entry();
+  __shared__ double sm[5][8][33];
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+  const long E = (long)h * w, e = min(blockIdx.x * 32L + x, E - 1);
+  const int i = (int)(e % h), j = (int)(e / h), yj = sym ? j : h + j, hw = h + w;
+  double s[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+#pragma unroll 4
+  for (int p = y; p < covers; p += 8) s[0] += cover[(size_t)p * E + e];
+#pragma unroll 4
+  for (int p = y; p < parts; p += 8) {
+    const double* np = norms + (size_t)p * 2 * hw;
+    s[1] += np[i];
+    s[2] += np[hw + i];
+    s[3] += np[yj];
+    s[4] += np[hw + yj];
+  }
+#pragma unroll
+  for (int k = 0; k < 5; k++) sm[k][y][x] = s[k];
+  __syncthreads();
+  if (y) return;
+#pragma unroll
+  for (int k = 0; k < 5; k++) {
+    s[k] = 0.0;
+    for (int q = 0; q < 8; q++) s[k] += sm[k][q][x];
+  }
+  const double qx = sqrt(s[1]), px = sqrt(s[2]), qy = sqrt(s[3]), py = sqrt(s[4]);
+  // (0.9: the roundings of the FP32 sums)
+  const bool ok = qx == 0.0 || qy == 0.0 || px * qy + qx * py + 4.0 * qx * qy <= 0.9 * 4.0 * OZH_ROUNDINGS * s[0];
+  if (!ok) *verdict = 1;
+}
+
 template <int F>
-static int ozh_launch(gpu_Context* ctx, ozh_params& prm, long* splits)
+static int ozh_launch(gpu_Context* ctx, ozh_params& prm, long* splits, int* verdict)
 {
   const int WPAD = 128 / F;
   const long R = (F == 2 ? 4 : 8) * OZH_STAGE;
@@ -465,22 +645,40 @@ static int ozh_launch(gpu_Context* ctx, ozh_params& prm, long* splits)
   if (gx < 1) gx = 1;
   if (gx > ngroups) gx = ngroups;
   *splits = gx;
-  double* partial = (double*)gb_workspace(ctx, sizeof(double) * (size_t)gx * prm.h * prm.w);
+  // CTAs of the check: two an SM, as many chunks as there are at most
+  const int cx = (prm.h + 31) / 32, cy = (prm.w + 31) / 32;
+  const long blocks = (prm.n + OZH_SAMPLE - 1) / OZH_SAMPLE;
+  long cz = 2L * ctx->num_sms / (cx * cy);
+  if (cz < 1) cz = 1;
+  if (cz > blocks) cz = blocks;
+  const size_t np = (size_t)gx * prm.h * prm.w, nn = (size_t)gx * 2 * (prm.h + prm.w);
+  double* partial = (double*)gb_workspace(ctx, sizeof(double) * (np + nn + (size_t)cz * prm.h * prm.w));
   if (!partial) return -1;
   prm.partial = partial;
+  prm.norms = partial + np;
+  double* cover = prm.norms + nn;
   if (cudaFuncSetAttribute(oz_gram64_kernel<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, prm.smem) !=
       cudaSuccess)
     return gb_fail(ctx, "oz_gram64: cannot reserve %d bytes of shared memory", prm.smem);
   oz_gram64_kernel<F><<<dim3((unsigned)gx, (unsigned)(prm.tx * ty)), OZH_THREADS, prm.smem,
                         (cudaStream_t)ctx->stream>>>(prm);
-  gb_count_launch(1);
+  blk_cols X, Y;
+  for (int c = 0; c < prm.h; c++) X.col[c] = prm.x[c];
+  for (int c = 0; c < prm.w; c++) Y.col[c] = prm.y[c];
+  cudaStream_t st = (cudaStream_t)ctx->stream;
+  gb_pdl(gram64_cover_kernel, dim3(cx, cy, (unsigned)cz), 256, 0, st, X, prm.h, Y, prm.w, prm.sym, prm.n, prm.norms,
+         (int)gx, ngroups, cover, verdict);
+  gb_pdl(gram64_verdict_kernel, (prm.h * prm.w + 31) / 32, 256, 0, st, prm.norms, (int)gx, cover, (int)cz, prm.h, prm.w,
+         prm.sym, verdict);
+  gb_count_launch(3);
   return gb_cuda_check(ctx, (int)cudaGetLastError(), "oz_gram64");
 }
 
 // The CTAs' sums of X' Y in the context's workspace, [split][w][h]; *splits of
-// them.  sym: X and Y are the same columns.
+// them.  sym: X and Y are the same columns.  *verdict (device): 1 when an entry may
+// be further off than FP64 multiply-adds.
 extern "C" int gb_oz_gram64(gpu_Context* ctx, long n, const blk_cols* X, int h, const blk_cols* Y, int w, int sym,
-                            const double** partial, long* splits)
+                            const double** partial, long* splits, int* verdict)
 {
   ozh_params prm;
   memset(&prm, 0, sizeof(prm));
@@ -493,11 +691,11 @@ extern "C" int gb_oz_gram64(gpu_Context* ctx, long n, const blk_cols* X, int h, 
   prm.err = ctx->dcount + 5;
   int rc;
   if (w > 32)
-    rc = ozh_launch<2>(ctx, prm, splits);
+    rc = ozh_launch<2>(ctx, prm, splits, verdict);
   else if (w > 16)
-    rc = ozh_launch<4>(ctx, prm, splits);
+    rc = ozh_launch<4>(ctx, prm, splits, verdict);
   else
-    rc = ozh_launch<8>(ctx, prm, splits);
+    rc = ozh_launch<8>(ctx, prm, splits, verdict);
   *partial = prm.partial;
   return rc;
 }

@@ -153,28 +153,6 @@ static __device__ __noinline__ double ozy_direct(const void* const* s_x, const d
   return acc;
 }
 
-// the two FP16 sums of the magnitudes of eight digits (four words)
-static __device__ __forceinline__ uint32_t oz8_hadd2(uint32_t a, uint32_t b)
-{
-  uint32_t d;
-  asm("add.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-  return d;
-}
-static __device__ __forceinline__ uint32_t ozy_magnitudes(const uint32_t (&d)[4], uint32_t (&m)[4])
-{
-#pragma unroll
-  for (int k = 0; k < 4; k++) m[k] = d[k] & 0x7FFF7FFFu;
-  return oz8_hadd2(oz8_hadd2(m[0], m[1]), oz8_hadd2(m[2], m[3]));
-}
-static __device__ __forceinline__ float ozy_both(uint32_t h2)
-{
-  float lo, hi;
-  asm("{\n .reg .b16 l, h;\n mov.b32 {l, h}, %2;\n cvt.f32.f16 %0, l;\n cvt.f32.f16 %1, h;\n}\n"
-      : "=f"(lo), "=f"(hi)
-      : "r"(h2));
-  return lo + hi;
-}
-
 // a group's largest exponent, raised to 1 (unsafe) when it holds nothing but
 // subnormals
 static __device__ __forceinline__ int ozy_group_exp(uint32_t mag, bool nonzero)
@@ -292,9 +270,9 @@ __global__ void __launch_bounds__(OZY_THREADS, 1) oz_xc64_kernel(const __grid_co
       *(uint4*)(dst + t * K::BSLICE) = make_uint4(pk[t][0], pk[t][1], pk[t][2], pk[t][3]);
     if (BOUND) {
       uint32_t m[4];
-      const uint32_t top = ozy_magnitudes(pk[0], m);
+      const uint32_t top = oz8_magnitudes(pk[0], m);
       *(uint4*)(dst + OZY_S * K::BSLICE) = make_uint4(m[0], m[1], m[2], m[3]);
-      atomicAdd(&coltop[j], (int)ozy_both(top));
+      atomicAdd(&coltop[j], (int)oz8_both(top));
       atomicAdd(&colnnz[j], nnz);
     }
   }
@@ -374,7 +352,7 @@ __global__ void __launch_bounds__(OZY_THREADS, 1) oz_xc64_kernel(const __grid_co
             *(uint4*)(adig + t * OZY_ASLICE + off) = make_uint4(pk[t][0], pk[t][1], pk[t][2], pk[t][3]);
           if (BOUND) {
             uint32_t m[4];
-            top = oz8_hadd2(top, ozy_magnitudes(pk[0], m));
+            top = oz8_hadd2(top, oz8_magnitudes(pk[0], m));
             *(uint4*)(adig + OZY_S * OZY_ASLICE + off) = make_uint4(m[0], m[1], m[2], m[3]);
             if (k + 1 == ksteps) rowtop[i % OZY_TILES][half][r] = top;
           }
@@ -462,7 +440,7 @@ __global__ void __launch_bounds__(OZY_THREADS, 1) oz_xc64_kernel(const __grid_co
         tc_fence_after();
         const int er = rowexp[i % OZY_TILES][r];
         float top = 0.f;
-        if (BOUND) top = ozy_both(rowtop[i % OZY_TILES][0][r]) + ozy_both(rowtop[i % OZY_TILES][1][r]);
+        if (BOUND) top = oz8_both(rowtop[i % OZY_TILES][0][r]) + oz8_both(rowtop[i % OZY_TILES][1][r]);
         const uint32_t tl = tmem + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(set * K::SET + K::UNIT / 2 * chalf);
         double yp[4];
         int jp = -1;

@@ -314,3 +314,89 @@ def test_split_update_in_place(ctx):
     assert ctx.lib.gpu_BlockUpdate(mx.handle, C.ctypes.data, h, mx.handle, None, 2) == 0, ctx.last_error()
     b = h * 2.0 ** -38 * np.outer(np.abs(X).max(1), np.abs(C).max(0))
     assert np.all(np.abs(mx.to_host() - X @ C) <= b + 2.0 ** -45 * (np.abs(X) @ np.abs(C)))
+
+
+def _gram_blocks(kind, n, h, w, rng):
+    X, Y = rng.standard_normal((n, h)), rng.standard_normal((n, w))
+    r = np.arange(n)[:, None]
+    if kind == "localised":  # columns that are large in different rows of every group
+        X *= 10.0 ** -(3.0 * ((r + np.arange(h)) % 7))
+        Y *= 10.0 ** -(3.0 * ((r + 3 + np.arange(w)) % 7))
+    elif kind == "disjoint":  # large where the other is zero
+        X[::2] *= 1e-18
+        Y[1::2] = 0.0
+    elif kind == "dominant":  # one entry a column, where the other block vanishes
+        X[rng.integers(0, n, h), np.arange(h)] = 1e12
+        big = np.abs(X).max(1) >= 1e12
+        Y[big] = 0.0
+    elif kind == "entries":
+        X *= 10.0 ** -rng.uniform(0, 25, size=X.shape)
+        Y *= 10.0 ** -rng.uniform(0, 25, size=Y.shape)
+    elif kind == "rows":  # an amplitude that falls over the domain, in both
+        X *= np.exp(-40.0 * r / n)
+        Y *= np.exp(-40.0 * r / n)
+    elif kind == "opposite":
+        X *= np.exp(-40.0 * r / n)
+        Y *= np.exp(-40.0 * (n - r) / n)
+    elif kind == "sparse":
+        X *= rng.random(X.shape) < 0.02
+        Y *= rng.random(Y.shape) < 0.02
+    elif kind == "heavy":
+        X = np.exp(3 * X)
+        Y = np.exp(3 * Y)
+    return X, Y
+
+
+# each variant of the kernel (w <= 16, <= 32, more), more than a tile, X'X
+@pytest.mark.parametrize("n,h,w", [(500001, 17, 12), (200003, 20, 30), (60001, 40, 45), (30001, 70, 65), (150001, 27, 0)])
+@pytest.mark.parametrize("kind", ["even", "localised", "disjoint", "dominant", "entries", "rows", "opposite", "sparse",
+                                  "heavy"])
+def test_gram_of_graded_blocks(ctx, n, h, w, kind):
+    rng = np.random.default_rng(n + len(kind))
+    X, Y = _gram_blocks(kind, n, h, w if w else h, rng)
+    if w == 0:
+        Y = X
+    _check_gram(X, Y, _gram(ctx, X, Y))
+
+
+def _modes(n_grid, k):
+    """Orthonormal eigenvectors of the Laplacian on a square."""
+    s = np.sin(np.pi * np.outer(np.arange(1, n_grid + 1), np.arange(1, 9)) / (n_grid + 1))
+    return np.stack([np.outer(s[:, a % 8], s[:, (a * 3 + 1) % 8]).ravel() for a in range(k)], axis=1)
+
+
+# what users' blocks look like passes the check: the tensor cores' four launches and
+# no second product
+@pytest.mark.parametrize("kind", ["normal", "scaled", "uniform", "laplace", "modes"])
+def test_gram_of_ordinary_blocks_needs_no_second_product(ctx, kind):
+    rng = np.random.default_rng(51)
+    n, h, w = 512 * 512, 20, 24
+    X, Y = rng.standard_normal((n, h)), rng.standard_normal((n, w))
+    if kind == "scaled":
+        X, Y = X * 10.0 ** rng.uniform(-30, 30, size=h), Y * n ** -0.5
+    elif kind == "uniform":
+        X, Y = rng.random((n, h)), rng.random((n, w)) - 0.5
+    elif kind == "laplace":
+        X, Y = rng.laplace(size=(n, h)), rng.laplace(size=(n, w))
+    elif kind == "modes":
+        X, Y = _modes(512, h), _modes(512, w)
+    mx, my = S.MultiVector.from_host(ctx, X), S.MultiVector.from_host(ctx, Y)
+    (i, xx), (j, yy) = _wrap(ctx, mx), _wrap(ctx, my)
+    G = np.empty((h, w), order="F")
+    ctx.lib.mv_MultiVectorByMultiVector(xx, yy, h, h, w, G.ctypes.data)
+    before = ctx.lib.gpu_KernelLaunchCount()
+    ctx.lib.mv_MultiVectorByMultiVector(xx, yy, h, h, w, G.ctypes.data)
+    assert ctx.lib.gpu_KernelLaunchCount() - before == 4
+    _check_gram(X, Y, G)
+
+
+def test_gram_of_random_blocks_is_no_further_off_than_multiply_adds(ctx):
+    rng = np.random.default_rng(52)
+    for n, h, w in ((400000, 20, 15), (300000, 16, 32), (40000, 64, 64)):
+        X, Y = rng.standard_normal((n, h)), rng.standard_normal((n, w))
+        ref = _products(X, Y)
+        # (parts below the tensor cores' size, by multiply-adds)
+        fma = np.hstack([np.vstack([_gram(ctx, X[:, a:a + 8], Y[:, b:b + 8]) for a in range(0, h, 8)])
+                         for b in range(0, w, 8)])
+        err = [float(np.sqrt(np.mean((g - ref).astype(np.float64) ** 2))) for g in (fma, _gram(ctx, X, Y))]
+        assert err[1] <= err[0], (h, w, err)
