@@ -586,7 +586,7 @@ extern "C" int gb_bymat_large(gpu_Context* ctx, int dtype, long n, const blk_col
   gb_prof_begin(ctx, &pr, GB_K_XC);
   const int rc = gb_oz_bymat64(ctx, n, X, h, C, ldc, Y, w, Z);
   gb_prof_end(ctx, &pr, 8.0 * n * (h + w + (Z ? w : 0)), 2.0 * n * h * w);
-  return rc;
+  return rc ? -1 : 1;
 }
 
 extern "C" int gb_bymat_tri(gpu_Context* ctx, int dtype, long n, const blk_cols* X, int h,

@@ -120,13 +120,16 @@ int gb_gram(gpu_Context* ctx, int dtype, long n, const blk_cols* X, int h, const
             int w, double* G, int ldg);
 /* the same for callers that read the result on the host: large FP64 products on the
    tensor cores.  Returns 1 when those took the product: the caller then reads
-   *verdict (device), and takes the product again with gb_gram when it is not 0 */
+   verdict[0 .. 1] (device): [1] the error word of a wait that gave up (reported and
+   cleared with gb_device_error); [0] not 0: to be taken again with gb_gram */
 int gb_gram_large(gpu_Context* ctx, int dtype, long n, const blk_cols* X, int h, const blk_cols* Y,
                   int w, double* G, int ldg, int* verdict);
 /* Y(:,j) = sum_i X(:,i) C(i,j) [+ Z(:,j)], C FP64 device column-major (ldc) */
 int gb_bymat(gpu_Context* ctx, int dtype, long n, const blk_cols* X, int h, const double* C,
              int ldc, const blk_cols* Y, int w, const blk_cols* Z);
-/* the same for callers outside the solver: large FP64 products on the tensor cores */
+/* the same for callers outside the solver: large FP64 products on the tensor cores.
+   Returns 1 when those took the product: the caller then asks gb_device_error
+   whether a wait gave up (Y holds NaN where it is incomplete) */
 int gb_bymat_large(gpu_Context* ctx, int dtype, long n, const blk_cols* X, int h, const double* C,
                    int ldc, const blk_cols* Y, int w, const blk_cols* Z);
 /* whether a column of X shares memory with a column of Y (bytes long each) */
@@ -207,8 +210,8 @@ int gb_oz_bymat64(gpu_Context* ctx, long n, const blk_cols* X, int h, const doub
                   const blk_cols* Y, int w, const blk_cols* Z);
 /* the CTAs' sums of X' Y for FP64 blocks of any widths and alignments
    (oz_gram64.cu), in the workspace: [split][w][h], *splits of them; sym: X and
-   Y are the same columns; *verdict (device): 1 when an entry may be further off than
-   FP64 multiply-adds, else 0 */
+   Y are the same columns; verdict[0] (device): 1 when an entry may be further off than
+   FP64 multiply-adds, else 0; [1]: the device error word */
 int gb_oz_gram64(gpu_Context* ctx, long n, const blk_cols* X, int h, const blk_cols* Y, int w, int sym,
                  const double** partial, long* splits, int* verdict);
 /* FP64-accurate Gram G = L' [L Q_0 Q_1 ...] on the tensor cores (oz_gram.cu):

@@ -311,7 +311,12 @@ static void gi_InnerProd(void* x_, void* y_, BlopexInt gh, BlopexInt h, BlopexIn
   if (tensor >= 0) {
     double* tmp = (double*)malloc(sizeof(double) * (hw + 1));
     int rc = gb_memcpy_d2h(ctx, tmp, g, sizeof(double) * (hw + tensor));
-    if (!rc && tensor && *(int*)(tmp + hw) != 0) {
+    const int* verdict = (const int*)(tmp + hw);
+    if (!rc && tensor && verdict[1] != 0) {
+      int err = 0;
+      gb_device_error(ctx, &err);
+      gb_fail(ctx, "MultiInnerProd: tensor-core kernel timed out (code %d)", verdict[1]);  // tmp holds NaN
+    } else if (!rc && tensor && verdict[0] != 0) {
       rc = gb_gram(ctx, x->dtype, x->size, &a, h, &b, w, g, h);
       if (!rc) rc = gb_memcpy_d2h(ctx, tmp, g, sizeof(double) * hw);
     }
@@ -368,7 +373,10 @@ static void vecmat(void* x_, BlopexInt gh, BlopexInt h, BlopexInt w, void* v, vo
   blk_cols a, b;
   gb_mv_fill_cols(x, &a, 0);
   gb_mv_fill_cols(y, &b, 0);
-  gb_bymat_large(ctx, x->dtype, x->size, &a, h, c, h, &b, w, add ? &b : NULL);
+  int err = 0;
+  if (gb_bymat_large(ctx, x->dtype, x->size, &a, h, c, h, &b, w, add ? &b : NULL) == 1 &&
+      gb_device_error(ctx, &err) == 0 && err)
+    gb_fail(ctx, "MultiVecMat: tensor-core kernel timed out (code %d)", err);
   gb_sync(ctx);
   gb_device_free(c);
 }

@@ -82,6 +82,7 @@ struct ozh_params {
   int h, w, tx, sym;       // tx: tiles along x; sym: X and Y are the same columns
   int nst, acc_off, smem;  // ring stages, offset of the FP64 sums, bytes
   long n;
+  long polls;              // limit of one pipeline wait
   double* partial;         // [CTA][w][h]
   double* norms;           // [CTA][Q, P][h + w]
   int* err;
@@ -281,7 +282,7 @@ __global__ void __launch_bounds__(OZH_THREADS, 1) oz_gram64_kernel(const __grid_
       const bool more = g + 1 < my_groups;
 #pragma unroll 1
       for (int s = 0; s < SPG; s++) {
-        if (!abort_flag && !mbar_wait_n(&a_empty[buf], phase, &abort_flag, TC_WAIT_LIMIT)) {
+        if (!abort_flag && !mbar_wait_n(&a_empty[buf], phase, &abort_flag, prm.polls)) {
           abort_flag = 1;
           atomicExch(prm.err, 31);
         }
@@ -355,14 +356,14 @@ __global__ void __launch_bounds__(OZH_THREADS, 1) oz_gram64_kernel(const __grid_
       uint32_t phase = 0;
       for (long g = 0; g < my_groups && !abort_flag; g++) {
         const int set = (int)(g % nsets);
-        if (g >= nsets && !mbar_wait_n(&acc_empty[set], (uint32_t)((g / nsets - 1) & 1), &abort_flag, TC_WAIT_LIMIT)) {
+        if (g >= nsets && !mbar_wait_n(&acc_empty[set], (uint32_t)((g / nsets - 1) & 1), &abort_flag, prm.polls)) {
           abort_flag = 1;
           atomicExch(prm.err, 32);
           break;
         }
         const uint32_t d = tmem + (uint32_t)(set * 256);
         for (int s = 0; s < SPG; s++) {
-          if (!mbar_wait_n(&a_full[buf], phase, &abort_flag, TC_WAIT_LIMIT)) {
+          if (!mbar_wait_n(&a_full[buf], phase, &abort_flag, prm.polls)) {
             abort_flag = 1;
             atomicExch(prm.err, 33);
             break;
@@ -418,7 +419,7 @@ __global__ void __launch_bounds__(OZH_THREADS, 1) oz_gram64_kernel(const __grid_
     bool ok = true;
     for (long g = 0; g < my_groups; g++) {
       const int set = (int)(g % nsets);
-      const bool got = mbar_wait_n(&acc_full[set], (uint32_t)((g / nsets) & 1), &abort_flag, TC_WAIT_LIMIT);
+      const bool got = mbar_wait_n(&acc_full[set], (uint32_t)((g / nsets) & 1), &abort_flag, prm.polls);
       if (!__all_sync(0xffffffffu, got)) {  // tcgen05.ld needs the whole warp
         abort_flag = 1;
         atomicExch(prm.err, 34);
@@ -515,7 +516,7 @@ __global__ void __launch_bounds__(256) gram64_cover_kernel(blk_cols X, int h, bl
   __shared__ int eref[64];  // the columns' reference exponents (biased): X's, Y's
   const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
   const int i0 = blockIdx.x * 32, j0 = blockIdx.y * 32;
-  if (t == 0 && blockIdx.x + blockIdx.y + blockIdx.z == 0) *verdict = 0;
+  if (t == 0 && blockIdx.x + blockIdx.y + blockIdx.z == 0) verdict[0] = 0;
   {
     const int c = t >> 2;
     const int k = c < 32 ? i0 + c : j0 + c - 32;
@@ -587,14 +588,15 @@ __global__ void __launch_bounds__(256) gram64_cover_kernel(blk_cols X, int h, bl
     }
 }
 
-// *verdict |= 1 where the digits' error may exceed its share
+// verdict[0] = 1 where the digits' error may exceed its share; [1]: the error word
 __global__ void __launch_bounds__(256) gram64_verdict_kernel(const double* __restrict__ norms, int parts,
                                                              const double* __restrict__ cover, int covers, int h,
-                                                             int w, int sym, int* verdict)
+                                                             int w, int sym, const int* err, int* verdict)
 {
   gb_pdl_entry();
   __shared__ double sm[5][8][33];
   const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+  if (blockIdx.x == 0 && threadIdx.x == 0) verdict[1] = *err;
   const long E = (long)h * w, e = min(blockIdx.x * 32L + x, E - 1);
   const int i = (int)(e % h), j = (int)(e / h), yj = sym ? j : h + j, hw = h + w;
   double s[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
@@ -620,7 +622,7 @@ __global__ void __launch_bounds__(256) gram64_verdict_kernel(const double* __res
   const double qx = sqrt(s[1]), px = sqrt(s[2]), qy = sqrt(s[3]), py = sqrt(s[4]);
   // (0.9: the roundings of the FP32 sums)
   const bool ok = qx == 0.0 || qy == 0.0 || px * qy + qx * py + 4.0 * qx * qy <= 0.9 * 4.0 * OZH_ROUNDINGS * s[0];
-  if (!ok) *verdict = 1;
+  if (!ok) verdict[0] = 1;
 }
 
 template <int F>
@@ -669,14 +671,15 @@ static int ozh_launch(gpu_Context* ctx, ozh_params& prm, long* splits, int* verd
   gb_pdl(gram64_cover_kernel, dim3(cx, cy, (unsigned)cz), 256, 0, st, X, prm.h, Y, prm.w, prm.sym, prm.n, prm.norms,
          (int)gx, ngroups, cover, verdict);
   gb_pdl(gram64_verdict_kernel, (prm.h * prm.w + 31) / 32, 256, 0, st, prm.norms, (int)gx, cover, (int)cz, prm.h, prm.w,
-         prm.sym, verdict);
+         prm.sym, prm.err, verdict);
   gb_count_launch(3);
   return gb_cuda_check(ctx, (int)cudaGetLastError(), "oz_gram64");
 }
 
 // The CTAs' sums of X' Y in the context's workspace, [split][w][h]; *splits of
-// them.  sym: X and Y are the same columns.  *verdict (device): 1 when an entry may
-// be further off than FP64 multiply-adds.
+// them.  sym: X and Y are the same columns.  verdict[0] (device): 1 when an entry may
+// be further off than FP64 multiply-adds; [1]: the device error word (a wait that
+// gave up; the CTA's sums are NaN).
 extern "C" int gb_oz_gram64(gpu_Context* ctx, long n, const blk_cols* X, int h, const blk_cols* Y, int w, int sym,
                             const double** partial, long* splits, int* verdict)
 {
@@ -688,6 +691,7 @@ extern "C" int gb_oz_gram64(gpu_Context* ctx, long n, const blk_cols* X, int h, 
   prm.w = w;
   prm.sym = sym;
   prm.n = n;
+  prm.polls = ctx->opt.wait_polls > 0 ? (long)ctx->opt.wait_polls : TC_WAIT_LIMIT;
   prm.err = ctx->dcount + 5;
   int rc;
   if (w > 32)

@@ -57,7 +57,8 @@
 //   warps 0-7   read a unit's accumulators (lane = row; warps w and w + 4 share
 //               TMEM lanes and take half of the unit's columns each), recombine
 //               and store Y.
-// Every wait is bounded; a timeout sets an error word and all roles finish.
+// Every wait is bounded; a timeout sets an error word, the outputs become NaN and
+// all roles finish.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -435,6 +436,15 @@ __global__ void __launch_bounds__(OZY_THREADS, 1) oz_xc64_kernel(const __grid_co
           abort_flag = 1;
           atomicExch(prm.err, 16);
           stop = true;
+          // nothing is left as it was: NaN in this warp's part of the units to come
+          for (long i1 = i; i1 < my_tiles; i1++) {
+            const long row1 = (blockIdx.x + i1 * gridDim.x) * 128 + r;
+            for (int h1 = i1 == i ? hf : 0; h1 < nh; h1++)
+              for (int c = 0; c < K::UNIT / 2; c++) {
+                const int j = h1 * K::UNIT + K::UNIT / 2 * chalf + c;
+                if (row1 < prm.n && j < w) ozy_st(s_y[j], row1, __longlong_as_double(0x7ff8000000000000LL));
+              }
+          }
           break;
         }
         tc_fence_after();
@@ -605,8 +615,8 @@ extern "C" int gb_oz_xc64(gpu_Context* ctx, long n, const blk_cols* X, int h, co
 // The FP64 block update of gb_bymat for any widths: 64 output columns at a
 // time, and within them up to 64 input columns at a time, the later ones added to
 // the sum so far.  (The parts' nonzeros add up to the column's, so that the
-// roundings of the parts and of the additions stay within its bound.)  A wait that gives up (with the default limit, whatever the
-// context's option) is reported in the device error word.
+// roundings of the parts and of the additions stay within its bound.)  A wait that
+// gives up is reported in the device error word.
 extern "C" int gb_oz_bymat64(gpu_Context* ctx, long n, const blk_cols* X, int h, const double* C, int ldc,
                              const blk_cols* Y, int w, const blk_cols* Z)
 {
@@ -617,8 +627,8 @@ extern "C" int gb_oz_bymat64(gpu_Context* ctx, long n, const blk_cols* X, int h,
     for (int i0 = 0; i0 < h; i0 += hc) {
       const int hi = h - i0 < hc ? h - i0 : hc;
       const void* const* z = i0 ? Y->col + j0 : (Z ? Z->col + j0 : NULL);
-      if (ozy_launch<true>(ctx, n, X->col + i0, hi, C + i0 + (size_t)j0 * ldc, ldc, Y->col + j0, wj, z, z ? 2 : 0, 0,
-                           ctx->dcount + 5))
+      if (ozy_launch<true>(ctx, n, X->col + i0, hi, C + i0 + (size_t)j0 * ldc, ldc, Y->col + j0, wj, z, z ? 2 : 0,
+                           ctx->opt.wait_polls, ctx->dcount + 5))
         return -1;
     }
   }

@@ -400,3 +400,51 @@ def test_gram_of_random_blocks_is_no_further_off_than_multiply_adds(ctx):
                          for b in range(0, w, 8)])
         err = [float(np.sqrt(np.mean((g - ref).astype(np.float64) ** 2))) for g in (fma, _gram(ctx, X, Y))]
         assert err[1] <= err[0], (h, w, err)
+
+
+# (a poll a wait: the kernels give up on the first copy or product that is not there yet)
+def test_update_gives_up_cleanly():
+    c = S.Context(0)
+    rng = np.random.default_rng(61)
+    n, h, w = 300000, 32, 24
+    X, C = rng.standard_normal((n, h)), rng.standard_normal((h, w))
+    ref, mag = X @ C, np.abs(X) @ np.abs(C)
+    mx, my = S.MultiVector.from_host(c, X), S.MultiVector(c, n, w)
+    Cf = np.asfortranarray(C)
+    (i, xx), (j, yy) = _wrap(c, mx), _wrap(c, my)
+
+    def call():
+        my.upload(np.full((n, w), 3e33))
+        c.lib.mv_MultiVectorByMatrix(xx, h, h, w, Cf.ctypes.data, yy)
+        return my.to_host()
+
+    c.set_options(wait_polls=1)
+    Y = call()
+    c.set_options(wait_polls=0)
+    assert "timed out" in c.last_error()
+    assert c.device_error() == 0  # read and cleared by the call that failed
+    done = ~np.isnan(Y)
+    assert not done.all()
+    assert np.all(np.abs(Y - ref)[done] <= 80 * 2.0 ** -53 * mag[done])
+    assert np.all(np.abs(call() - ref) <= 80 * 2.0 ** -53 * mag)
+    assert c.device_error() == 0
+    c.close()
+
+
+def test_gram_gives_up_cleanly():
+    c = S.Context(0)
+    rng = np.random.default_rng(62)
+    n, h, w = 300000, 24, 30
+    X, Y = rng.standard_normal((n, h)), rng.standard_normal((n, w))
+    mx, my = S.MultiVector.from_host(c, X), S.MultiVector.from_host(c, Y)
+    (i, xx), (j, yy) = _wrap(c, mx), _wrap(c, my)
+    G = np.zeros((h, w), order="F")
+    c.set_options(wait_polls=1)
+    c.lib.mv_MultiVectorByMultiVector(xx, yy, h, h, w, G.ctypes.data)
+    c.set_options(wait_polls=0)
+    assert "timed out" in c.last_error()
+    assert np.isnan(G).all()
+    assert c.device_error() == 0
+    c.lib.mv_MultiVectorByMultiVector(xx, yy, h, h, w, G.ctypes.data)
+    _check_gram(X, Y, G)
+    c.close()
