@@ -180,6 +180,8 @@ __global__ void __launch_bounds__(256) gram_reduce_kernel(const double* __restri
 //   8,000 x 10 x 10: 16 us with the reduction against 96 (padded tile, 28 CTAs);
 //   262,144 x 8 x 8: 60 us against 504.
 #define GRAMP_T 512
+#define GRAMP_ROWS_SMEM (64 * 1024)                   // most of the staged rows (one group of 128 columns: 33 KB)
+#define GRAMP_SMEM (GRAMP_ROWS_SMEM + 8 * GRAMP_T)  // and the groups' sums
 template <bool SYM>
 __global__ void __launch_bounds__(GRAMP_T) gram_packed_kernel(blk_cols X, int h, blk_cols Y, int w, long n,
                                                               long rows_per_split, int sub, int groups,
@@ -385,7 +387,7 @@ static int gram_packed(gpu_Context* ctx, long n, const blk_cols* X, int h, const
   const int E = SYM ? h * (h + 1) / 2 : h * w, E32 = (E + 31) & ~31, nc = SYM ? h : h + w;
   int groups = GRAMP_T / E32;
   if (groups > chunks) groups = (int)chunks;
-  while (groups > 1 && 32 * groups * (nc | 1) * 8 > 64 * 1024) groups /= 2;
+  while (groups > 1 && 32 * groups * (nc | 1) * 8 > GRAMP_ROWS_SMEM) groups /= 2;
   // few splits: several CTAs a split, each leaving its chunks' sums
   int sub = 1;
   if (splits <= ctx->num_sms) {
@@ -396,7 +398,9 @@ static int gram_packed(gpu_Context* ctx, long n, const blk_cols* X, int h, const
   double* partial = (double*)gb_workspace(ctx, sizeof(double) * (size_t)nparts * E);
   if (!partial) return -1;
   const int smem = 8 * (32 * groups * (nc | 1) + groups * E32);
-  if (cudaFuncSetAttribute(gram_packed_kernel<SYM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+  if (smem > 40 * 1024 &&  // (always the most: the limit is the function's, for all threads)
+      cudaFuncSetAttribute(gram_packed_kernel<SYM>, cudaFuncAttributeMaxDynamicSharedMemorySize, GRAMP_SMEM) !=
+          cudaSuccess)
     return gb_fail(ctx, "gram: cannot reserve %d bytes of shared memory", smem);
   gb_prof_rec pr;
   gb_prof_begin(ctx, &pr, GB_K_GRAM);

@@ -249,8 +249,9 @@ extern "C" int gb_cholqr_factor(gpu_Context* ctx, double* A, int ld, int m, int*
   gb_prof_rec pr;
   gb_prof_begin(ctx, &pr, GB_K_CHOLQR);
   const int smem = m <= CHOLQR_SMEM_M ? (int)(2 * sizeof(double) * (size_t)m * m) : 0;
-  if (smem > 48 * 1024 &&
-      cudaFuncSetAttribute(cholqr_factor_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+  if (smem > 40 * 1024 &&  // (always the most: the limit is the function's, for all threads)
+      cudaFuncSetAttribute(cholqr_factor_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           2 * (int)sizeof(double) * CHOLQR_SMEM_M * CHOLQR_SMEM_M) != cudaSuccess)
     return gb_fail(ctx, "cholqr_factor: cannot reserve %d bytes of shared memory", smem);
   gb_pdl(cholqr_factor_kernel, 1, DENSE_THREADS, smem, S(ctx), A, ld, m, info, W, force, smem > 0);
   gb_prof_end(ctx, &pr, 16.0 * m * m, (double)m * m * m / 1.5);

@@ -659,7 +659,9 @@ static int ozh_launch(gpu_Context* ctx, ozh_params& prm, long* splits, int* verd
   prm.partial = partial;
   prm.norms = partial + np;
   double* cover = prm.norms + nn;
-  if (cudaFuncSetAttribute(oz_gram64_kernel<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, prm.smem) !=
+  // (prm.smem <= OZH_SMEM_MAX but for the rounding of acc_off; the limit is the
+  // function's, for all threads)
+  if (cudaFuncSetAttribute(oz_gram64_kernel<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, OZH_SMEM_MAX + 1024) !=
       cudaSuccess)
     return gb_fail(ctx, "oz_gram64: cannot reserve %d bytes of shared memory", prm.smem);
   oz_gram64_kernel<F><<<dim3((unsigned)gx, (unsigned)(prm.tx * ty)), OZH_THREADS, prm.smem,

@@ -1411,7 +1411,10 @@ static void rr_reduce(gpu_Context* ctx, double* A, double* B, int ld, int m, int
   const size_t mm = (size_t)m * m;
   if (m <= RR_CHOL_SMEM_M) {
     const int sm = (int)(sizeof(double) * (size_t)m * m);
-    cudaFuncSetAttribute(rr_chol64_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+    // (here and below the most a kernel takes at any order: the limit is the
+    // function's, and another thread's smaller one would refuse this launch)
+    cudaFuncSetAttribute(rr_chol64_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)sizeof(double) * RR_CHOL_SMEM_M * RR_CHOL_SMEM_M);
     RR_STAGE(GB_K_RR_CHOL, m3 / 3,
              (gb_pdl(rr_chol64_kernel<true>, 1, RR_THREADS, sm, st, B, ld, m, s, info, report_below)));
   } else {
@@ -1433,7 +1436,8 @@ static void rr_tridiag_path(gpu_Context* ctx, double* A, int ld, int m, int nev,
   const double m3 = (double)m * m * m;
   if (m <= RR_TRD_SMEM_M) {
     const int sm = (int)(sizeof(double) * (size_t)m * (m + 1) / 2);
-    cudaFuncSetAttribute(rr_tridiag_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+    cudaFuncSetAttribute(rr_tridiag_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)sizeof(double) * RR_TRD_SMEM_M * (RR_TRD_SMEM_M + 1) / 2);
     RR_STAGE(GB_K_RR_TRID, 4.0 * m3 / 3.0,
              (gb_pdl(rr_tridiag_smem_kernel, 1, RR_TRD_THREADS, sm, st, m, s)));
   } else {
@@ -1441,14 +1445,15 @@ static void rr_tridiag_path(gpu_Context* ctx, double* A, int ld, int m, int nev,
   }
   const int sb = (int)rr_bisect_smem(m);
   if (sb > 32 * 1024)
-    cudaFuncSetAttribute(rr_bisect_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sb);
+    cudaFuncSetAttribute(rr_bisect_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rr_bisect_smem(RR_MAX_M));
   RR_STAGE(GB_K_RR_EIG, 0.0, (gb_pdl(rr_bisect_kernel, nev, 32 * RR_BIS_WARPS, sb, st, m, s)));
   RR_STAGE(GB_K_RR_EIG, 0.0, (gb_pdl(rr_invit_kernel, nev, 32, 0, st, m, s)));
   // Cholesky-QR twice: Z <- Z inv(U), U'U = Z'Z
   const dim3 gs = rr_gemm_grid(nev, nev, 1), gz = rr_gemm_grid(m, nev, 1);
   const int sc = nev <= RR_CHOLINV_SMEM_M ? (int)(2 * sizeof(double) * (size_t)nev * nev) : 0;
   if (sc > 40 * 1024)
-    cudaFuncSetAttribute(rr_cholinv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sc);
+    cudaFuncSetAttribute(rr_cholinv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         2 * (int)sizeof(double) * RR_CHOLINV_SMEM_M * RR_CHOLINV_SMEM_M);
   for (int round = 0; round < 2; round++) {
     rr_gemm_t zz = {s.X, m, 1, s.X, m, s.S, nev, nev, nev, m};
     RR_STAGE(GB_K_RR_GEMM, 2.0 * m * nev * nev, (gb_pdl(rr_gemm_kernel, gs, RR_GEMM_TM * RR_GEMM_TN, 0, st, zz, zz, s.status)));
@@ -1475,8 +1480,10 @@ static void rr_jacobi32_path(gpu_Context* ctx, double* A, int ld, int m, int nev
   // Jacobi: every CTA holds C (m*m) and `rows` rows of V
   const int nsplit = m <= 96 ? 1 : 4;
   const int rows = (m + nsplit - 1) / nsplit;
-  const size_t sm_jac = ((size_t)m * rr_pad(m) + (size_t)rows * rr_pad(m)) * sizeof(float);
-  cudaFuncSetAttribute(rr_jacobi32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_jac);
+  auto jac_smem = [](int m, int rows) { return ((size_t)m * rr_pad(m) + (size_t)rows * rr_pad(m)) * sizeof(float); };
+  const size_t sm_jac = jac_smem(m, rows);
+  cudaFuncSetAttribute(rr_jacobi32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)jac_smem(RR_MAX_SMEM_M, (RR_MAX_SMEM_M + 3) / 4));
   RR_STAGE(GB_K_RR_JAC32, 0.0, (gb_pdl(rr_jacobi32_kernel, nsplit, RR_THREADS, sm_jac, st, m, rows, s)));
   gb_pdl(rr_vsort_kernel, 1, RR_THREADS, 0, st, m, s);
   int launches = 2;
