@@ -12,6 +12,7 @@
 // deterministic run to run.
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <math.h>
 #include <string.h>
 
 #include "internal.h"
@@ -435,22 +436,34 @@ extern "C" int gb_gram(gpu_Context* ctx, int dtype, long n, const blk_cols* X, i
   return gram_launch<float, 4, 4>(ctx, n, X, h, Y, w, G, ldg);
 }
 
-// A caller's products (the interpreter's entry): FP64 ones of at least
-// GRAM_TENSOR_MIN multiply-adds on the tensor cores (oz_gram64.cu), checked there
-// against the bound of multiply-adds.  The FP64 pipe takes 0.17 ms for them at its
-// 0.58 T multiply-adds/s, the tensor-core kernel 0.05 to 0.07 (65,536 x 32 x 32: 45 us
-// against 125; 16,384 x 32 x 32: 51 against 30).  The solver keeps gb_gram: the
-// signs of its Ritz vectors follow the last bits of these sums, and a solve
-// returns the same iterates, bit for bit, as it always did.
+// A caller's products (the interpreter's entry): large FP64 ones on the tensor cores
+// (oz_gram64.cu), checked there against the bound of multiply-adds.  Those cost a
+// row as much for all blocks whose 8-column units its eight producer warps hold at
+// once (0.27 ns a row, 0.6 with two units a warp), the multiply-adds what their
+// entries take (2.0 ps each; X'X half).  Measured, 2,097,152 rows, multiply-adds and
+// tensor cores: 8 x 8 287 and 545 us, 16 x 8 552 and 561, 12 x 12 690 and 560, 16 x 16
+// 1058 and 568 (X'X 676 and 556), 32 x 4 555 and 642, 32 x 32 5.5 ms and 696, 64 x 4 1102
+// and 1221, 64 x 8 2138 and 1243, 64 x 64 14.6 ms and 1755.  The four launches take 30 us:
+// 262,144 x 16 x 16 147 and 91, 20,000 x 32 x 32 89 and 40, x 64 x 4 31 and 49.  The solver
+// keeps gb_gram: the signs of its Ritz vectors follow the last bits of these sums,
+// and a solve returns the same iterates, bit for bit, as it always did.
 #define GRAM_TENSOR_MIN 1e8
+#define GRAM_TENSOR_ENTRIES 132
+
+static int gram_on_tensor_cores(long n, int h, int w, int sym)
+{
+  const int units = (h + 7) / 8 + (sym ? 0 : (w + 7) / 8);
+  return (double)n * h * w >= GRAM_TENSOR_MIN &&
+         (sym ? h * (h + 1) / 2 : h * w) >= GRAM_TENSOR_ENTRIES * ((units + 7) / 8);
+}
 
 extern "C" int gb_gram_large(gpu_Context* ctx, int dtype, long n, const blk_cols* X, int h,
                              const blk_cols* Y, int w, double* G, int ldg, int* verdict)
 {
   if (h <= 0 || w <= 0) return 0;
-  if (dtype != GPU_MV_FLOAT64 || (double)n * h * w < GRAM_TENSOR_MIN)
-    return gb_gram(ctx, dtype, n, X, h, Y, w, G, ldg);
   const int sym = h == w && memcmp(X->col, Y->col, sizeof(void*) * (size_t)h) == 0;
+  if (dtype != GPU_MV_FLOAT64 || !gram_on_tensor_cores(n, h, w, sym))
+    return gb_gram(ctx, dtype, n, X, h, Y, w, G, ldg);
   const double* partial;
   long splits;
   gb_prof_rec pr;
@@ -559,12 +572,35 @@ extern "C" int gb_bymat(gpu_Context* ctx, int dtype, long n, const blk_cols* X, 
   return bymat_launch(ctx, dtype, n, X, h, C, ldc, Y, w, Z, 0);
 }
 
-// Callers' updates (the interpreter's entries, the adjoint): FP64 ones of at
-// least XC_TENSOR_MIN multiply-adds on the tensor cores (oz_xc64.cu), with a
-// smaller error: 2,097,152 x 32 x 32 0.43 ms against 3.5; 262,144 x 8 x 8 42 us
-// against 53; a launch costs it 20 us at least.  The solver keeps gb_bymat, for
-// the reason given at gb_gram_large.
+// Callers' updates (the interpreter's entries): large FP64 ones on the tensor cores
+// (oz_xc64.cu), within the bound of multiply-adds.  Measured, 2,097,152 rows,
+// multiply-adds and tensor cores: 4 x 16 336 and 899 us, 8 x 8 355 and 343, 10 x 10 614 and 333,
+// 12 x 12 718 and 294, 16 x 4 534 and 243, 16 x 16 881 and 295, 32 x 32 3454 and 509, 64 x 4
+// 2148 and 500, 64 x 64 13.8 ms and 1302; 65,536 x 12 x 12 35 and 20, 20,000 x 16 x 16 17 and 14, x 32 x 32
+// 54 and 19.  From 12 input columns on, few of random entries are summed directly
+// (8 columns: 3%, 12: 1%, 16: 0.3%); summed directly an entry costs up to three times its
+// multiply-adds (32 x 32, C triangular, 3.1 ms; identity 5.8; 16 x 16 triangular
+// 1.4; X's columns graded over 18 decades 3.9).  Hence the look at C: at most one column
+// in eight may be of few values (its 1-norm below h / 8 of its largest).  The solver
+// keeps gb_bymat, for the reason given at gb_gram_large.
 #define XC_TENSOR_MIN 1.6e7
+#define XC_TENSOR_H 12
+
+static int update_on_tensor_cores(long n, int h, int w, const double* C, int ldc)
+{
+  if (h < XC_TENSOR_H || (double)n * h * w < XC_TENSOR_MIN) return 0;
+  int sparse = 0;
+  for (int j = 0; j < w; j++) {
+    double sum = 0.0, big = 0.0;
+    for (int i = 0; i < h; i++) {
+      const double a = fabs(C[i + (size_t)j * ldc]);
+      sum += a;
+      big = a > big ? a : big;
+    }
+    sparse += !(sum * 8 >= big * h && big > 0.0);  // (zeros and NaN count as sparse)
+  }
+  return sparse * 8 <= w;
+}
 
 // whether a column of X shares memory with a column of Y (`bytes` long each)
 extern "C" int gb_cols_overlap(const blk_cols* X, int h, const blk_cols* Y, int w, size_t bytes)
@@ -578,12 +614,13 @@ extern "C" int gb_cols_overlap(const blk_cols* X, int h, const blk_cols* Y, int 
 }
 
 extern "C" int gb_bymat_large(gpu_Context* ctx, int dtype, long n, const blk_cols* X, int h,
-                              const double* C, int ldc, const blk_cols* Y, int w, const blk_cols* Z)
+                              const double* C, int ldc, const double* C_host, int ldch,
+                              const blk_cols* Y, int w, const blk_cols* Z)
 {
   if (w <= 0 || n <= 0) return 0;
   // (in place: gb_bymat, whose CTAs read all of their rows of X before they write;
   // the tensor-core kernel comes back to X for the entries that it sums directly)
-  if (dtype != GPU_MV_FLOAT64 || h <= 0 || (double)n * h * w < XC_TENSOR_MIN ||
+  if (dtype != GPU_MV_FLOAT64 || h <= 0 || !update_on_tensor_cores(n, h, w, C_host, ldch) ||
       gb_cols_overlap(X, h, Y, w, sizeof(double) * (size_t)n))
     return gb_bymat(ctx, dtype, n, X, h, C, ldc, Y, w, Z);
   gb_prof_rec pr;

@@ -127,11 +127,11 @@ int gb_gram_large(gpu_Context* ctx, int dtype, long n, const blk_cols* X, int h,
 /* Y(:,j) = sum_i X(:,i) C(i,j) [+ Z(:,j)], C FP64 device column-major (ldc) */
 int gb_bymat(gpu_Context* ctx, int dtype, long n, const blk_cols* X, int h, const double* C,
              int ldc, const blk_cols* Y, int w, const blk_cols* Z);
-/* the same for callers outside the solver: large FP64 products on the tensor cores.
-   Returns 1 when those took the product: the caller then asks gb_device_error
+/* the same for callers outside the solver: large FP64 products on the tensor cores,
+   chosen by the sizes and by C's values (C_host, ldch: C on the host).  Returns 1 when those took the product: the caller then asks gb_device_error
    whether a wait gave up (Y holds NaN where it is incomplete) */
 int gb_bymat_large(gpu_Context* ctx, int dtype, long n, const blk_cols* X, int h, const double* C,
-                   int ldc, const blk_cols* Y, int w, const blk_cols* Z);
+                   int ldc, const double* C_host, int ldch, const blk_cols* Y, int w, const blk_cols* Z);
 /* whether a column of X shares memory with a column of Y (bytes long each) */
 int gb_cols_overlap(const blk_cols* X, int h, const blk_cols* Y, int w, size_t bytes);
 /* the same with C upper triangular (explicit zeros below the diagonal) */

@@ -374,7 +374,7 @@ static void vecmat(void* x_, BlopexInt gh, BlopexInt h, BlopexInt w, void* v, vo
   gb_mv_fill_cols(x, &a, 0);
   gb_mv_fill_cols(y, &b, 0);
   int err = 0;
-  if (gb_bymat_large(ctx, x->dtype, x->size, &a, h, c, h, &b, w, add ? &b : NULL) == 1 &&
+  if (gb_bymat_large(ctx, x->dtype, x->size, &a, h, c, h, (const double*)v, gh, &b, w, add ? &b : NULL) == 1 &&
       gb_device_error(ctx, &err) == 0 && err)
     gb_fail(ctx, "MultiVecMat: tensor-core kernel timed out (code %d)", err);
   gb_sync(ctx);

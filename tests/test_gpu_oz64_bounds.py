@@ -448,3 +448,43 @@ def test_gram_gives_up_cleanly():
     c.lib.mv_MultiVectorByMultiVector(xx, yy, h, h, w, G.ctypes.data)
     _check_gram(X, Y, G)
     c.close()
+
+
+# with a poll a wait the tensor cores give up, multiply-adds do not: which took the
+# product.  (narrow blocks of many rows, for which these are faster, and C of few values)
+@pytest.mark.parametrize("n,h,w,coords,tensor", [
+    (4000000, 2, 2, "full", False), (262144, 8, 8, "full", False), (1 << 21, 11, 2, "full", False),
+    (1 << 20, 12, 12, "full", True), (200000, 32, 32, "full", True), (30000, 96, 40, "full", True),
+    (200000, 32, 32, "identity", False), (200000, 32, 32, "triangular", False), (200000, 32, 32, "diagonal", False),
+    (200000, 32, 32, "rows", False)])
+def test_updates_that_the_tensor_cores_take(n, h, w, coords, tensor):
+    c = S.Context(0)
+    rng = np.random.default_rng(71)
+    mx, my = S.MultiVector(c, n, h), S.MultiVector(c, n, w)
+    mx.set_random(1)
+    Cf = np.asfortranarray(_coordinates(coords, h, w, rng))
+    (i, xx), (j, yy) = _wrap(c, mx), _wrap(c, my)
+    c.set_options(wait_polls=1)
+    c.lib.mv_MultiVectorByMatrix(xx, h, h, w, Cf.ctypes.data, yy)
+    c.set_options(wait_polls=0)
+    assert ("timed out" in c.last_error()) == tensor
+    c.close()
+
+
+@pytest.mark.parametrize("n,h,w,tensor", [
+    (1 << 21, 8, 8, False), (1 << 21, 16, 8, False), (1 << 21, 32, 4, False), (1 << 19, 64, 4, False),
+    (1 << 21, 15, 0, False), (1 << 20, 16, 0, True), (1 << 20, 12, 12, True), (1 << 19, 64, 8, True),
+    (30000, 64, 64, True), (40000, 70, 65, True)])
+def test_gram_products_that_the_tensor_cores_take(ctx, n, h, w, tensor):
+    mx = S.MultiVector(ctx, n, h)
+    mx.set_random(1)
+    my = mx
+    if w:
+        my = S.MultiVector(ctx, n, w)
+        my.set_random(2)
+    w = w or h
+    (i, xx), (j, yy) = _wrap(ctx, mx), _wrap(ctx, my)
+    G = np.empty((h, w), order="F")
+    before = ctx.lib.gpu_KernelLaunchCount()
+    ctx.lib.mv_MultiVectorByMultiVector(xx, yy, h, h, w, G.ctypes.data)
+    assert ctx.lib.gpu_KernelLaunchCount() - before == (4 if tensor else 2)
