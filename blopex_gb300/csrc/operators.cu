@@ -33,6 +33,7 @@
 #include "tc_common.cuh"
 #include "blas32.cuh"
 #include "pdl.cuh"
+#include "st_tiles.h"
 
 enum { OPK_CSR = 1, OPK_ST7 = 2, OPK_ST5 = 3, OPK_ST27 = 4, OPK_DIAG = 5, OPK_PCG = 6 };
 
@@ -400,7 +401,7 @@ __global__ void __launch_bounds__(256) st7_ring_kernel(int nx, int ny, int nz,
 //     staged a cell instead of 3.3; one leaves more CTAs (st7t_planes).
 //   A thread has four cells in x of one row (16-byte shared loads and stores,
 //     x neighbours by shuffles): a third fewer instructions than four rows of one.
-//   Strips of about ST7T_STRIP tiles, z before the next strip, so that the CTAs
+//   Strips of about ST_STRIP tiles, z before the next strip, so that the CTAs
 //     that share halo planes run within a few columns of each other; whole planes
 //     first let the z halo fall out of L2 (256^3, 64 columns: 1729 us, strips of
 //     8, 16, 32 tiles: 1474, 1459, 1513; 512 x 256 x 128: 1972, 1471, 1471, 1497).
@@ -408,7 +409,6 @@ __global__ void __launch_bounds__(256) st7_ring_kernel(int nx, int ny, int nz,
 //     halos read twice), before 1797; 128^3, 17 columns: 64 us against 71;
 //     32^3, 64 columns: 9 us against 39.
 #define ST7T_DEPTH 3
-#define ST7T_STRIP 16
 template <int NP>  // planes a CTA
 struct st7t_cfg {
   static constexpr int PLANE = 34 * 40;                                   // floats of a centre plane
@@ -480,12 +480,9 @@ __global__ void __launch_bounds__(256, NP == 1 ? 4 : 3) st7_tma_kernel(
   const int t = threadIdx.x, tx = t & 7, ty = t >> 3, warp = t >> 5, lane = t & 31;
   const int tiles_x = (nx + 31) / 32, tiles_y = (ny + 31) / 32;
   const unsigned b = blockIdx.x;
-  // tiles in strips of `strip` tile rows, z before the next strip
-  const unsigned per = (unsigned)(tiles_x * strip) * ((nz + NP - 1) / NP);
-  const int s0 = (int)(b / per) * strip;
-  const unsigned rest = b % per, in_strip = (unsigned)(tiles_x * min(strip, tiles_y - s0));
-  const int k0 = NP * (int)(rest / in_strip), tile = (int)(rest % in_strip);
-  const int i0 = (tile % tiles_x) * 32, j0 = (s0 + tile / tiles_x) * 32;
+  int bx, by, layer;
+  st_tile(b, tiles_x, tiles_y, (nz + NP - 1) / NP, strip, &bx, &by, &layer);
+  const int i0 = 32 * bx, j0 = 32 * by, k0 = NP * layer;
   const long plane = (long)nx * ny;
   // columns c0 .. c0 + w - 1
   const int c0 = blockIdx.y * cpg, w = min(cpg, wall - c0);
@@ -766,11 +763,9 @@ __global__ void __launch_bounds__(32 * ST27T_ROWS, ST27T_MINB)
   const int t = threadIdx.x, tx = t & 31, ty = t >> 5;
   const int tiles_x = (nx + 31) / 32, tiles_y = (ny + ST27T_ROWS - 1) / ST27T_ROWS;
   const unsigned b = blockIdx.x;
-  const unsigned per = (unsigned)(tiles_x * strip) * ((nz + NZ - 1) / NZ);
-  const int s0 = (int)(b / per) * strip;
-  const unsigned rest = b % per, in_strip = (unsigned)(tiles_x * min(strip, tiles_y - s0));
-  const int k0 = NZ * (int)(rest / in_strip), tile = (int)(rest % in_strip);
-  const int i0 = (tile % tiles_x) * 32, j0 = (s0 + tile / tiles_x) * ST27T_ROWS;
+  int bx, by, layer;
+  st_tile(b, tiles_x, tiles_y, (nz + NZ - 1) / NZ, strip, &bx, &by, &layer);
+  const int i0 = 32 * bx, j0 = ST27T_ROWS * by, k0 = NZ * layer;
   const int c0 = blockIdx.y * cpg, w = min(cpg, wall - c0);
   if (t == 0) {
     abort_flag = 0;
@@ -1176,7 +1171,7 @@ static int st27t_pays(const gpu_Operator* op, int w)
 static void st27t_launch(gpu_Operator* op, const CUtensorMap& tm, const st7t_cols& pc, const blk_cols& yc, int w)
 {
   gpu_Context* ctx = op->ctx;
-  const int tiles_x = (op->nx + 31) / 32, strip = tiles_x < ST7T_STRIP ? ST7T_STRIP / tiles_x : 1;
+  const int strip = st_strip((op->nx + 31) / 32, (op->ny + ST27T_ROWS - 1) / ST27T_ROWS);
   const long ctas = st27t_ctas(op);
   long groups = (long)ST27T_MINB * ctx->num_sms / ctas;  // as st7t_launch
   if (groups > (w + 3) / 4) groups = (w + 3) / 4;
@@ -1218,7 +1213,7 @@ static int st7t_launch(gpu_Operator* op, const CUtensorMap& tmc, const CUtensorM
   if (groups > (w + 3) / 4) groups = (w + 3) / 4;
   if (groups < 1) groups = 1;
   const int cpg = (int)((w + groups - 1) / groups);
-  const int tiles_x = (op->nx + 31) / 32, strip = tiles_x < ST7T_STRIP ? ST7T_STRIP / tiles_x : 1;
+  const int strip = st_strip((op->nx + 31) / 32, (op->ny + 31) / 32);
   const dim3 grid((unsigned)ctas, (unsigned)((w + cpg - 1) / cpg));
   gb_pdl(st7_tma_kernel<NP, DOT>, grid, 256, smem, S(ctx), op->nx, op->ny, op->nz, op->c32[0], op->c32[1], op->c32[2],
                                                        (float)op->shift, tmc, tmz, pc, yc, w, cpg, strip, yvec,
