@@ -41,6 +41,26 @@ static __device__ __forceinline__ void acc_pair32(float& s, float& c, float s2, 
   c = __fadd_rn(__fadd_rn(c, c2), e);
 }
 
+static __device__ __forceinline__ void two_sum32(float& s, float& e, float a, float b)
+{
+  s = __fadd_rn(a, b);
+  const float bp = __fsub_rn(s, a);
+  e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bp)), __fsub_rn(b, bp));
+}
+
+// (s, c, d) += (s2, c2, d2): the roundings of the second word kept in a third, for
+// long merges of compensated sums
+static __device__ __forceinline__ void acc_triple32(float& s, float& c, float& d, float s2, float c2, float d2)
+{
+  float t, e, u, g, v, h;
+  two_sum32(t, e, s, s2);
+  two_sum32(u, g, c, c2);
+  two_sum32(v, h, u, e);
+  s = t;
+  c = v;
+  d = __fadd_rn(__fadd_rn(d, d2), __fadd_rn(g, h));
+}
+
 static __device__ __forceinline__ void warp_pair_sum32(float& s, float& c)
 {
 #pragma unroll

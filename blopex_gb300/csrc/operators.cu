@@ -450,17 +450,25 @@ static __device__ __forceinline__ void st7t_issue(uint32_t slot, const CUtensorM
 }
 
 // a column's sum over the CTA of the threads' compensated sums, by one warp (all
-// eight warps' values in a fixed order), into the CTA's partial
+// eight warps' values in a fixed order), into the CTA's partial.  With three words,
+// and a thread's cells of each plane summed apart, its error is that of FP64 sums of
+// the warps' pairs (restated on the CPU, 2 M products: of equal signs 5.8e-16 of their
+// sum, with two words and 8 cells 1.1e-15; of mixed signs 2.2e-18 and 9.5e-18)
 static __device__ __forceinline__ void st7t_dot_store(const float2* red, double* out, int lane)
 {
-  float s = 0.f, c = 0.f;
+  float s = 0.f, c = 0.f, d = 0.f;
 #pragma unroll
   for (int q = 0; q < 8; q++) {
     const float2 v = red[32 * q + lane];
-    acc_pair32(s, c, v.x, v.y);
+    acc_triple32(s, c, d, v.x, v.y, 0.f);
   }
-  warp_pair_sum32(s, c);
-  if (lane == 0) *out = (double)s + (double)c;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const float s2 = __shfl_xor_sync(0xffffffffu, s, o), c2 = __shfl_xor_sync(0xffffffffu, c, o),
+                d2 = __shfl_xor_sync(0xffffffffu, d, o);
+    acc_triple32(s, c, d, s2, c2, d2);
+  }
+  if (lane == 0) *out = (double)s + ((double)c + (double)d);
 }
 
 template <int NP, bool DOT>
@@ -600,7 +608,14 @@ __global__ void __launch_bounds__(256, NP == 1 ? 4 : 3) st7_tma_kernel(
           } else {
             __stcs(yp, o.x), __stcs(yp + 1, o.y), __stcs(yp + 2, o.z), __stcs(yp + 3, o.w);
           }
-          if (DOT) acc_prod32x4(xs, xc, c, o);
+          if (DOT) {
+            float ps = 0.f, pc = 0.f;
+            acc_prod32x4(ps, pc, c, o);
+            if (p == 0)
+              xs = ps, xc = pc;
+            else
+              acc_pair32(xs, xc, ps, pc);
+          }
         }
       }
     } else {
