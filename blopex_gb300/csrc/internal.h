@@ -128,8 +128,9 @@ int gb_gram_large(gpu_Context* ctx, int dtype, long n, const blk_cols* X, int h,
 int gb_bymat(gpu_Context* ctx, int dtype, long n, const blk_cols* X, int h, const double* C,
              int ldc, const blk_cols* Y, int w, const blk_cols* Z);
 /* the same for callers outside the solver: large FP64 products on the tensor cores,
-   chosen by the sizes and by C's values (C_host, ldch: C on the host).  Returns 1 when those took the product: the caller then asks gb_device_error
-   whether a wait gave up (Y holds NaN where it is incomplete) */
+   chosen by the sizes and by C's values (C_host, ldch: C on the host).  Returns 1
+   when those took the product: the caller then asks gb_device_error whether a wait
+   gave up (Y holds NaN where it is incomplete) */
 int gb_bymat_large(gpu_Context* ctx, int dtype, long n, const blk_cols* X, int h, const double* C,
                    int ldc, const double* C_host, int ldch, const blk_cols* Y, int w, const blk_cols* Z);
 /* whether a column of X shares memory with a column of Y (bytes long each) */

@@ -1153,7 +1153,7 @@ static int st7t_maps(const gpu_Operator* op, const gpu_MultiVector* X, int np, C
   return 0;
 }
 
-// the map of st27_tma_kernel: boxes 40 x 10 x np (the conditions of st7t_maps)
+// the map of st27_tma_kernel: boxes 40 x 6 x np (the conditions of st7t_maps)
 static int st27t_map(const gpu_Operator* op, const gpu_MultiVector* X, int np, CUtensorMap* m)
 {
   PFN_cuTensorMapEncodeTiled_v12000 enc = st7t_encoder();
@@ -1193,8 +1193,8 @@ static void st27t_launch(gpu_Operator* op, const CUtensorMap& tm, const st7t_col
   if (groups < 1) groups = 1;
   const int cpg = (int)((w + groups - 1) / groups);
   const dim3 grid((unsigned)ctas, (unsigned)((w + cpg - 1) / cpg));
-  gb_pdl(st27_tma_kernel<ST27T_NZ>, grid, 32 * ST27T_ROWS, st27t_cfg<ST27T_NZ>::SMEM, S(ctx), 
-      op->nx, op->ny, op->nz, op->w32, (float)op->shift, tm, pc, yc, w, cpg, strip, ctx->dcount + 5);
+  gb_pdl(st27_tma_kernel<ST27T_NZ>, grid, 32 * ST27T_ROWS, st27t_cfg<ST27T_NZ>::SMEM, S(ctx),
+         op->nx, op->ny, op->nz, op->w32, (float)op->shift, tm, pc, yc, w, cpg, strip, ctx->dcount + 5);
 }
 
 static int pcg_apply(gpu_Operator* op, gpu_MultiVector* X, gpu_MultiVector* Y);
@@ -1376,8 +1376,8 @@ static int operator_apply(gpu_Operator* op, gpu_MultiVector* X, gpu_MultiVector*
           gb_count_launch(1);
         }
       } else if (f32 && st7_ring_ok(op, &xc, w))
-        gb_pdl(st7_ring_kernel, (unsigned)(((op->nx + 31) / 32) * ((op->ny + 31) / 32) * (long)op->nz), 256, 0, S(ctx), op->nx, op->ny, op->nz, op->c32[0], op->c32[1],
-                                                op->c32[2], (float)op->shift, xc, yc, w);
+        gb_pdl(st7_ring_kernel, (unsigned)st7t_ctas(op, 1), 256, 0, S(ctx), op->nx, op->ny, op->nz, op->c32[0],
+               op->c32[1], op->c32[2], (float)op->shift, xc, yc, w);
       else if (f32)
         gb_pdl(st7_kernel<float>, tb, ST_TX * ST_TY, 0, S(ctx), op->nx, op->ny, op->nz, op->c32[0],
                                                             op->c32[1], op->c32[2], (float)op->shift,

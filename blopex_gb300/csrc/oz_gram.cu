@@ -97,7 +97,9 @@ struct ozg_params {
 // digit slices behind them 1024-byte aligned (the MMA descriptors' swizzle
 // atom); dynamic plus static shared memory within the 227 KB of a CTA
 static_assert(sizeof(ozg_params) <= 32764, "oz_gram parameters exceed the kernel parameter space");
-static_assert(OZG_RAW % 1024 == 0 && 2 * OZG_RAW <= OZG_RAWS && OZG_MAXSLOTS + 3 < OZG_CSLOTS + 1, "raw buffers must keep the digit slices 1024-byte aligned");
+static_assert(OZG_RAW % 1024 == 0 && 2 * OZG_RAW <= OZG_RAWS,
+              "raw buffers must keep the digit slices 1024-byte aligned");
+static_assert(OZG_MAXSLOTS + 3 <= OZG_CSLOTS, "a chunk's scales are overwritten before it is folded");
 static_assert(OZG_SMEM + 12288 <= 232448, "oz_gram shared memory exceeds a CTA's 227 KB");
 
 // rows x columns tile of a column run: x = first row, the run's columns all
@@ -139,7 +141,8 @@ __global__ void __launch_bounds__(OZG_THREADS, 1) oz_gram_kernel(const __grid_co
   unsigned char* raws = smem;                  // [nslots][raw]: columns at s_off
   unsigned char* adig = smem + prm.nslots * prm.raw;    // [S][128 rows][128 B]
   // a_full, a_empty: the digits of rows 0-31 and 32-63
-  __shared__ uint64_t raw_full[OZG_MAXSLOTS], raw_empty[OZG_MAXSLOTS], scale_full[OZG_MAXSLOTS], a_full[2], a_empty[2], acc_full[2], acc_empty[2], done_bar;
+  __shared__ uint64_t raw_full[OZG_MAXSLOTS], raw_empty[OZG_MAXSLOTS], scale_full[OZG_MAXSLOTS];
+  __shared__ uint64_t a_full[2], a_empty[2], acc_full[2], acc_empty[2], done_bar;
   __shared__ uint32_t tmem_base;
   __shared__ int abort_flag;
   // this tile's column pointers and kinds (0 absent, 1 FP32, 2 FP64) in shared

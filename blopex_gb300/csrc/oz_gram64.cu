@@ -504,11 +504,12 @@ __global__ void __launch_bounds__(OZH_THREADS, 1) oz_gram64_kernel(const __grid_
 // Lower bounds of sum |x_r y_r|: the CTAs' sums over every gridDim.z-th of the sampled
 // chunks (32 rows of each OZH_SAMPLE, moving through them), 32 x 32 entries, in FP32 on
 // values cut to 20 bits and scaled by a power of two near the column's rms scale
-// (from Q; values 2^40 above it count as that much, far smaller ones as 0).
-// FP32 arithmetic takes 20 us at 2,097,152 x 32 x 32.
+// (from Q; values 2^40 above it count as that much, far smaller ones as 0).  The
+// CTAs of the first layer also leave the columns' Q and P over all groups in tot.
 __global__ void __launch_bounds__(256) gram64_cover_kernel(blk_cols X, int h, blk_cols Y, int w, int sym, long n,
                                                            const double* __restrict__ norms, int parts, long groups,
-                                                           double* __restrict__ cover, int* verdict)
+                                                           double* __restrict__ tot, double* __restrict__ cover,
+                                                           int* verdict)
 {
   gb_pdl_entry();
   __shared__ float xs[32][33], ys[32][33];
@@ -519,11 +520,27 @@ __global__ void __launch_bounds__(256) gram64_cover_kernel(blk_cols X, int h, bl
   if (t == 0 && blockIdx.x + blockIdx.y + blockIdx.z == 0) verdict[0] = 0;
   {
     const int c = t >> 2;
-    const int k = c < 32 ? i0 + c : j0 + c - 32;
+    const int k = c < 32 ? i0 + c : j0 + c - 32, hw = h + w;
+    const bool on = k < (c < 32 ? h : w);
+    const double* np = norms + (c < 32 || sym ? k : h + k);
     double s = 0.0;
-    if (k < (c < 32 ? h : w))
-      for (int p = t & 3; p < parts; p += 4) s += norms[(size_t)p * 2 * (h + w) + (c < 32 || sym ? k : h + k)];
+    if (on)
+#pragma unroll 4
+      for (int p = t & 3; p < parts; p += 4) s += np[(size_t)p * 2 * hw];
     sq[c][t & 3] = s;
+    if (blockIdx.z == 0 && (c < 32 ? blockIdx.y : blockIdx.x) == 0) {  // (whole warps)
+      double q = 0.0;
+      if (on)
+        for (int p = t & 3; p < parts; p += 4) q += np[(size_t)p * 2 * hw + hw];
+      for (int o = 1; o < 4; o <<= 1) {
+        s += __shfl_xor_sync(0xffffffffu, s, o);
+        q += __shfl_xor_sync(0xffffffffu, q, o);
+      }
+      if (on && (t & 3) == 0) {
+        tot[c < 32 ? k : h + k] = s;
+        tot[hw + (c < 32 ? k : h + k)] = q;
+      }
+    }
   }
   __syncthreads();
   if (t < 64) {
@@ -538,7 +555,8 @@ __global__ void __launch_bounds__(256) gram64_cover_kernel(blk_cols X, int h, bl
 #pragma unroll
   for (int k = 0; k < 8; k++) {
     const int c = (t >> 5) + 8 * k;
-    col[k] = (const uint32_t*)(c < 32 ? (i0 + c < h ? X.col[i0 + c] : NULL) : (j0 + c - 32 < w ? Y.col[j0 + c - 32] : NULL));
+    const int i = i0 + c, j = j0 + c - 32;
+    col[k] = (const uint32_t*)(c < 32 ? (i < h ? X.col[i] : NULL) : (j < w ? Y.col[j] : NULL));
     ref[k] = eref[c] - 127;
   }
   const long blocks = (n + OZH_SAMPLE - 1) / OZH_SAMPLE;
@@ -589,39 +607,29 @@ __global__ void __launch_bounds__(256) gram64_cover_kernel(blk_cols X, int h, bl
 }
 
 // verdict[0] = 1 where the digits' error may exceed its share; [1]: the error word
-__global__ void __launch_bounds__(256) gram64_verdict_kernel(const double* __restrict__ norms, int parts,
+__global__ void __launch_bounds__(256) gram64_verdict_kernel(const double* __restrict__ tot,
                                                              const double* __restrict__ cover, int covers, int h,
-                                                             int w, int sym, const int* err, int* verdict)
+                                                             int w, const int* err, int* verdict)
 {
   gb_pdl_entry();
-  __shared__ double sm[5][8][33];
-  const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+  __shared__ double sm[32][9];
+  const int x = threadIdx.x & 7, y = threadIdx.x >> 3;  // 8 entries a CTA, 32 threads each
   if (blockIdx.x == 0 && threadIdx.x == 0) verdict[1] = *err;
-  const long E = (long)h * w, e = min(blockIdx.x * 32L + x, E - 1);
-  const int i = (int)(e % h), j = (int)(e / h), yj = sym ? j : h + j, hw = h + w;
-  double s[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+  const long E = (long)h * w, e = min(blockIdx.x * 8L + x, E - 1);
+  double s = 0.0;
 #pragma unroll 4
-  for (int p = y; p < covers; p += 8) s[0] += cover[(size_t)p * E + e];
-#pragma unroll 4
-  for (int p = y; p < parts; p += 8) {
-    const double* np = norms + (size_t)p * 2 * hw;
-    s[1] += np[i];
-    s[2] += np[hw + i];
-    s[3] += np[yj];
-    s[4] += np[hw + yj];
-  }
-#pragma unroll
-  for (int k = 0; k < 5; k++) sm[k][y][x] = s[k];
+  for (int p = y; p < covers; p += 32) s += cover[(size_t)p * E + e];
+  sm[y][x] = s;
   __syncthreads();
+  if (y >= 4) return;
+  for (int q = y + 4; q < 32; q += 4) s += sm[q][x];
+  s += __shfl_xor_sync(0xffffffffu, s, 8);
+  s += __shfl_xor_sync(0xffffffffu, s, 16);
   if (y) return;
-#pragma unroll
-  for (int k = 0; k < 5; k++) {
-    s[k] = 0.0;
-    for (int q = 0; q < 8; q++) s[k] += sm[k][q][x];
-  }
-  const double qx = sqrt(s[1]), px = sqrt(s[2]), qy = sqrt(s[3]), py = sqrt(s[4]);
+  const int i = (int)(e % h), j = h + (int)(e / h), hw = h + w;
+  const double qx = sqrt(tot[i]), px = sqrt(tot[hw + i]), qy = sqrt(tot[j]), py = sqrt(tot[hw + j]);
   // (0.9: the roundings of the FP32 sums)
-  const bool ok = qx == 0.0 || qy == 0.0 || px * qy + qx * py + 4.0 * qx * qy <= 0.9 * 4.0 * OZH_ROUNDINGS * s[0];
+  const bool ok = qx == 0.0 || qy == 0.0 || px * qy + qx * py + 4.0 * qx * qy <= 0.9 * 4.0 * OZH_ROUNDINGS * s;
   if (!ok) verdict[0] = 1;
 }
 
@@ -647,18 +655,18 @@ static int ozh_launch(gpu_Context* ctx, ozh_params& prm, long* splits, int* verd
   if (gx < 1) gx = 1;
   if (gx > ngroups) gx = ngroups;
   *splits = gx;
-  // CTAs of the check: two an SM, as many chunks as there are at most
+  // CTAs of the check: four an SM, as many chunks as there are at most
   const int cx = (prm.h + 31) / 32, cy = (prm.w + 31) / 32;
   const long blocks = (prm.n + OZH_SAMPLE - 1) / OZH_SAMPLE;
-  long cz = 2L * ctx->num_sms / (cx * cy);
+  long cz = 4L * ctx->num_sms / (cx * cy);
   if (cz < 1) cz = 1;
   if (cz > blocks) cz = blocks;
-  const size_t np = (size_t)gx * prm.h * prm.w, nn = (size_t)gx * 2 * (prm.h + prm.w);
-  double* partial = (double*)gb_workspace(ctx, sizeof(double) * (np + nn + (size_t)cz * prm.h * prm.w));
+  const size_t np = (size_t)gx * prm.h * prm.w, nt = (size_t)2 * (prm.h + prm.w), nn = (size_t)gx * nt;
+  double* partial = (double*)gb_workspace(ctx, sizeof(double) * (np + nn + nt + (size_t)cz * prm.h * prm.w));
   if (!partial) return -1;
   prm.partial = partial;
   prm.norms = partial + np;
-  double* cover = prm.norms + nn;
+  double *tot = prm.norms + nn, *cover = tot + nt;
   // (prm.smem <= OZH_SMEM_MAX but for the rounding of acc_off; the limit is the
   // function's, for all threads)
   if (cudaFuncSetAttribute(oz_gram64_kernel<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, OZH_SMEM_MAX + 1024) !=
@@ -671,9 +679,8 @@ static int ozh_launch(gpu_Context* ctx, ozh_params& prm, long* splits, int* verd
   for (int c = 0; c < prm.w; c++) Y.col[c] = prm.y[c];
   cudaStream_t st = (cudaStream_t)ctx->stream;
   gb_pdl(gram64_cover_kernel, dim3(cx, cy, (unsigned)cz), 256, 0, st, X, prm.h, Y, prm.w, prm.sym, prm.n, prm.norms,
-         (int)gx, ngroups, cover, verdict);
-  gb_pdl(gram64_verdict_kernel, (prm.h * prm.w + 31) / 32, 256, 0, st, prm.norms, (int)gx, cover, (int)cz, prm.h, prm.w,
-         prm.sym, prm.err, verdict);
+         (int)gx, ngroups, tot, cover, verdict);
+  gb_pdl(gram64_verdict_kernel, (prm.h * prm.w + 7) / 8, 256, 0, st, tot, cover, (int)cz, prm.h, prm.w, prm.err, verdict);
   gb_count_launch(3);
   return gb_cuda_check(ctx, (int)cudaGetLastError(), "oz_gram64");
 }

@@ -1456,10 +1456,12 @@ static void rr_tridiag_path(gpu_Context* ctx, double* A, int ld, int m, int nev,
                          2 * (int)sizeof(double) * RR_CHOLINV_SMEM_M * RR_CHOLINV_SMEM_M);
   for (int round = 0; round < 2; round++) {
     rr_gemm_t zz = {s.X, m, 1, s.X, m, s.S, nev, nev, nev, m};
-    RR_STAGE(GB_K_RR_GEMM, 2.0 * m * nev * nev, (gb_pdl(rr_gemm_kernel, gs, RR_GEMM_TM * RR_GEMM_TN, 0, st, zz, zz, s.status)));
+    RR_STAGE(GB_K_RR_GEMM, 2.0 * m * nev * nev,
+             (gb_pdl(rr_gemm_kernel, gs, RR_GEMM_TM * RR_GEMM_TN, 0, st, zz, zz, s.status)));
     RR_STAGE(GB_K_RR_EIG, 0.0, (gb_pdl(rr_cholinv_kernel, 1, 256, sc, st, nev, s, sc > 0)));
     rr_gemm_t zu = {s.X, m, 0, s.P, nev, s.Xn, m, m, nev, nev};
-    RR_STAGE(GB_K_RR_GEMM, 2.0 * m * nev * nev, (gb_pdl(rr_gemm_kernel, gz, RR_GEMM_TM * RR_GEMM_TN, 0, st, zu, zu, s.status)));
+    RR_STAGE(GB_K_RR_GEMM, 2.0 * m * nev * nev,
+             (gb_pdl(rr_gemm_kernel, gz, RR_GEMM_TM * RR_GEMM_TN, 0, st, zu, zu, s.status)));
     double* t = s.X;
     s.X = s.Xn;
     s.Xn = t;
