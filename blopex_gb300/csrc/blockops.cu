@@ -581,14 +581,18 @@ extern "C" int gb_bymat(gpu_Context* ctx, int dtype, long n, const blk_cols* X, 
 // (8 columns: 3%, 12: 1%, 16: 0.3%); summed directly an entry costs up to three times its
 // multiply-adds (32 x 32, C triangular, 3.1 ms; identity 5.8; 16 x 16 triangular
 // 1.4; X's columns graded over 18 decades 3.9).  Hence the look at C: at most one column
-// in eight may be of few values (its 1-norm below h / 8 of its largest).  The solver
-// keeps gb_bymat, for the reason given at gb_gram_large.
+// in eight may be of few values (its 1-norm below h / 8 of its largest).  And a launch
+// of 64 x 64 columns takes 20 us at least, C's digits above all, 36 of them for 384 x
+// 384: 3000 x 200 x 200 263 and 322, 6000 rows 576 and 330; 3000 x 384 x 384 1038 and 879,
+// 1500 rows 411 and 878.  The solver keeps gb_bymat, for the reason given at
+// gb_gram_large.
 #define XC_TENSOR_MIN 1.6e7
 #define XC_TENSOR_H 12
+#define XC_TENSOR_ROWS 5000
 
 static int update_on_tensor_cores(long n, int h, int w, const double* C, int ldc)
 {
-  if (h < XC_TENSOR_H || (double)n * h * w < XC_TENSOR_MIN) return 0;
+  if (h < XC_TENSOR_H || n < XC_TENSOR_ROWS || (double)n * h * w < XC_TENSOR_MIN) return 0;
   int sparse = 0;
   for (int j = 0; j < w; j++) {
     double sum = 0.0, big = 0.0;
@@ -605,11 +609,20 @@ static int update_on_tensor_cores(long n, int h, int w, const double* C, int ldc
 // whether a column of X shares memory with a column of Y (`bytes` long each)
 extern "C" int gb_cols_overlap(const blk_cols* X, int h, const blk_cols* Y, int w, size_t bytes)
 {
-  for (int i = 0; i < h; i++)
+  uintptr_t lo = UINTPTR_MAX, hi = 0;  // Y's columns
+  for (int j = 0; j < w; j++) {
+    const uintptr_t y = (uintptr_t)Y->col[j];
+    lo = y < lo ? y : lo;
+    hi = y > hi ? y : hi;
+  }
+  for (int i = 0; i < h; i++) {
+    const uintptr_t x = (uintptr_t)X->col[i];
+    if (x >= hi + bytes || lo >= x + bytes) continue;
     for (int j = 0; j < w; j++) {
-      const uintptr_t x = (uintptr_t)X->col[i], y = (uintptr_t)Y->col[j];
+      const uintptr_t y = (uintptr_t)Y->col[j];
       if (x < y + bytes && y < x + bytes) return 1;
     }
+  }
   return 0;
 }
 

@@ -454,6 +454,7 @@ def test_gram_gives_up_cleanly():
 # product.  (narrow blocks of many rows, for which these are faster, and C of few values)
 @pytest.mark.parametrize("n,h,w,coords,tensor", [
     (4000000, 2, 2, "full", False), (262144, 8, 8, "full", False), (1 << 21, 11, 2, "full", False),
+    (700, 200, 200, "full", False), (1500, 384, 384, "full", False), (4000, 96, 70, "full", False),
     (1 << 20, 12, 12, "full", True), (200000, 32, 32, "full", True), (30000, 96, 40, "full", True),
     (200000, 32, 32, "identity", False), (200000, 32, 32, "triangular", False), (200000, 32, 32, "diagonal", False),
     (200000, 32, 32, "rows", False)])
@@ -488,3 +489,15 @@ def test_gram_products_that_the_tensor_cores_take(ctx, n, h, w, tensor):
     before = ctx.lib.gpu_KernelLaunchCount()
     ctx.lib.mv_MultiVectorByMultiVector(xx, yy, h, h, w, G.ctypes.data)
     assert ctx.lib.gpu_KernelLaunchCount() - before == (4 if tensor else 2)
+
+
+# more than 64 columns on either side, by the tensor-core kernel itself: parts of equal width
+@pytest.mark.parametrize("n,h,w", [(2101, 130, 70), (1503, 129, 65), (999, 65, 64), (700, 64, 129)])
+@pytest.mark.parametrize("grade,coords,add", [("even", "full", True), ("columns", "rows", False),
+                                              ("entries", "triangular", True)])
+def test_update_in_parts(ctx, n, h, w, grade, coords, add):
+    rng = np.random.default_rng(n + w)
+    X = rng.standard_normal((n, h)) * _grade(grade, n, h, rng)
+    C = _coordinates(coords, h, w, rng)
+    Z = rng.standard_normal((n, w)) * 1e-10 if add else None
+    _check_update(X, C, Z, _tensor_update(ctx, X, C, Z))
