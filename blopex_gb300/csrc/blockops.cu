@@ -443,7 +443,7 @@ extern "C" int gb_gram(gpu_Context* ctx, int dtype, long n, const blk_cols* X, i
 // entries take (2.0 ps each; X'X half).  Measured, 2,097,152 rows, multiply-adds and
 // tensor cores: 8 x 8 287 and 545 us, 16 x 8 552 and 561, 12 x 12 690 and 560, 16 x 16
 // 1058 and 568 (X'X 676 and 556), 32 x 4 555 and 642, 32 x 32 5.5 ms and 696, 64 x 4 1102
-// and 1221, 64 x 8 2138 and 1243, 64 x 64 14.6 ms and 1755.  The four launches take 30 us:
+// and 1221, 64 x 8 2138 and 1243, 64 x 64 14.6 ms and 1755.  The three launches take 30 us:
 // 262,144 x 16 x 16 147 and 91, 20,000 x 32 x 32 89 and 40, x 64 x 4 31 and 49.  The solver
 // keeps gb_gram: the signs of its Ritz vectors follow the last bits of these sums,
 // and a solve returns the same iterates, bit for bit, as it always did.
@@ -464,16 +464,11 @@ extern "C" int gb_gram_large(gpu_Context* ctx, int dtype, long n, const blk_cols
   const int sym = h == w && memcmp(X->col, Y->col, sizeof(void*) * (size_t)h) == 0;
   if (dtype != GPU_MV_FLOAT64 || !gram_on_tensor_cores(n, h, w, sym))
     return gb_gram(ctx, dtype, n, X, h, Y, w, G, ldg);
-  const double* partial;
-  long splits;
   gb_prof_rec pr;
   gb_prof_begin(ctx, &pr, GB_K_GRAM);
-  if (gb_oz_gram64(ctx, n, X, h, Y, w, sym, &partial, &splits, verdict)) return -1;
-  gb_pdl(gram_reduce_kernel, (h * w + 31) / 32, 256, 0, S(ctx), partial, (int)splits, 1, splits, h * w, h, sym ? 2 : 0, G,
-                                                            ldg);
+  const int rc = gb_oz_gram64(ctx, n, X, h, Y, w, sym, G, ldg, verdict);
   gb_prof_end(ctx, &pr, 8.0 * n * (sym ? h : h + w), sym ? (double)n * h * (h + 1) : 2.0 * n * h * w);
-  gb_count_launch(1);
-  return CUDA_LAUNCH_CHECK(ctx, "gram64") ? -1 : 1;
+  return rc ? -1 : 1;
 }
 
 // ------------------------------------------------------------------------

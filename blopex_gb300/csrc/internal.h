@@ -209,12 +209,11 @@ int gb_oz_xc64(gpu_Context* ctx, long n, const blk_cols* X, int h, const double*
    of FP64 multiply-adds; Z FP64, may be Y.  X must not overlap Y */
 int gb_oz_bymat64(gpu_Context* ctx, long n, const blk_cols* X, int h, const double* C, int ldc,
                   const blk_cols* Y, int w, const blk_cols* Z);
-/* the CTAs' sums of X' Y for FP64 blocks of any widths and alignments
-   (oz_gram64.cu), in the workspace: [split][w][h], *splits of them; sym: X and
-   Y are the same columns; verdict[0] (device): 1 when an entry may be further off than
-   FP64 multiply-adds, else 0; [1]: the device error word */
+/* G = X' Y (device, ldg) for FP64 blocks of any widths and alignments (oz_gram64.cu);
+   sym: X and Y are the same columns; verdict[0] (device): 1 when an entry may be
+   further off than FP64 multiply-adds, else 0; [1]: the device error word */
 int gb_oz_gram64(gpu_Context* ctx, long n, const blk_cols* X, int h, const blk_cols* Y, int w, int sym,
-                 const double** partial, long* splits, int* verdict);
+                 double* G, int ldg, int* verdict);
 /* FP64-accurate Gram G = L' [L Q_0 Q_1 ...] on the tensor cores (oz_gram.cu):
    L a block of h <= 64 columns, FP32 or FP64 (ldt); nq <= 4 blocks Q_b of up
    to 64 columns each, FP32 or FP64 (qdt[b]); every column 16-byte aligned and

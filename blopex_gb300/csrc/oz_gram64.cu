@@ -11,8 +11,8 @@
 // into the entry's FP64 sum: one FP64 addition per group where fused
 // multiply-adds spend one per row, on a pipe that takes 16 cycles for a warp.
 // Each CTA (one per SM) covers every gridDim.x-th group of a tile of up to 64 x
-// 64 entries; gram_reduce_kernel adds the CTAs' sums in a fixed order (X'X from
-// its lower triangle, so that it comes out symmetric).
+// 64 entries; gram64_finish_kernel adds the CTAs' sums, 32 chains and a tree (X'X
+// from its lower triangle, so that it comes out symmetric).
 //
 // Operands.  B: the digit slices of the tile's X columns, stacked along N.  A:
 // the slices of its Y columns, wpad = 16, 32 or 64 rows each, stacked along M so
@@ -40,7 +40,7 @@
 // (1-norms from the top digits), which bound the error of an entry by
 // 2^-55 (sqrt(P Q') + sqrt(Q P') + 4 sqrt(Q Q')); gram64_cover_kernel adds up
 // |x_r y_r| over an eighth of the rows in FP32, rounded down, a lower bound of
-// sum |x_r y_r|; and gram64_verdict_kernel asks for an error of at most
+// sum |x_r y_r|; and gram64_finish_kernel asks for an error of at most
 // OZH_ROUNDINGS 2^-53 of it.  Together with the additions over groups and CTAs that
 // is within (32 + n / 9728 + 310) 2^-53 sum |x_r y_r|, the bound of the kernels of
 // blockops.cu.  Random blocks pass with a factor of 20 to spare; when an entry does
@@ -606,35 +606,48 @@ __global__ void __launch_bounds__(256) gram64_cover_kernel(blk_cols X, int h, bl
     }
 }
 
-// verdict[0] = 1 where the digits' error may exceed its share; [1]: the error word
-__global__ void __launch_bounds__(256) gram64_verdict_kernel(const double* __restrict__ tot,
-                                                             const double* __restrict__ cover, int covers, int h,
-                                                             int w, const int* err, int* verdict)
+// G from the CTAs' sums, 32 threads an entry: strides of 32 in order, then a tree of
+// the 32 (in one chain, 152 sums of growing size were the largest part of the error:
+// 30,000 x 64 x 64 5.6e-16, multiply-adds 4.7e-16).  verdict[0] = 1 where the digits'
+// error may exceed its share; [1]: the error word
+__global__ void __launch_bounds__(256) gram64_finish_kernel(const double* __restrict__ partial, int parts,
+                                                            const double* __restrict__ tot,
+                                                            const double* __restrict__ cover, int covers, int h, int w,
+                                                            int sym, const int* err, double* __restrict__ G, int ldg,
+                                                            int* verdict)
 {
   gb_pdl_entry();
-  __shared__ double sm[32][9];
-  const int x = threadIdx.x & 7, y = threadIdx.x >> 3;  // 8 entries a CTA, 32 threads each
+  __shared__ double sm[2][32][9];
+  const int x = threadIdx.x & 7, y = threadIdx.x >> 3;  // 8 entries a CTA
   if (blockIdx.x == 0 && threadIdx.x == 0) verdict[1] = *err;
-  const long E = (long)h * w, e = min(blockIdx.x * 8L + x, E - 1);
-  double s = 0.0;
+  const long E = (long)h * w, e0 = blockIdx.x * 8L + x, e = min(e0, E - 1);
+  const int i = (int)(e % h), j = (int)(e / h), hw = h + w;
+  const long src = sym && i < j ? (long)i * h + j : e;
+  double g = 0.0, s = 0.0;
+#pragma unroll 4
+  for (int p = y; p < parts; p += 32) g += partial[(size_t)p * E + src];
 #pragma unroll 4
   for (int p = y; p < covers; p += 32) s += cover[(size_t)p * E + e];
-  sm[y][x] = s;
-  __syncthreads();
-  if (y >= 4) return;
-  for (int q = y + 4; q < 32; q += 4) s += sm[q][x];
-  s += __shfl_xor_sync(0xffffffffu, s, 8);
-  s += __shfl_xor_sync(0xffffffffu, s, 16);
-  if (y) return;
-  const int i = (int)(e % h), j = h + (int)(e / h), hw = h + w;
-  const double qx = sqrt(tot[i]), px = sqrt(tot[hw + i]), qy = sqrt(tot[j]), py = sqrt(tot[hw + j]);
+  sm[0][y][x] = g;
+  sm[1][y][x] = s;
+  for (int o = 16; o > 0; o >>= 1) {
+    __syncthreads();
+    if (y < o) {
+      sm[0][y][x] += sm[0][y + o][x];
+      sm[1][y][x] += sm[1][y + o][x];
+    }
+  }
+  if (y || e0 >= E) return;
+  G[(size_t)j * ldg + i] = sm[0][0][x];
+  const double qx = sqrt(tot[i]), px = sqrt(tot[hw + i]), qy = sqrt(tot[h + j]), py = sqrt(tot[hw + h + j]);
   // (0.9: the roundings of the FP32 sums)
-  const bool ok = qx == 0.0 || qy == 0.0 || px * qy + qx * py + 4.0 * qx * qy <= 0.9 * 4.0 * OZH_ROUNDINGS * s;
+  const bool ok =
+      qx == 0.0 || qy == 0.0 || px * qy + qx * py + 4.0 * qx * qy <= 0.9 * 4.0 * OZH_ROUNDINGS * sm[1][0][x];
   if (!ok) verdict[0] = 1;
 }
 
 template <int F>
-static int ozh_launch(gpu_Context* ctx, ozh_params& prm, long* splits, int* verdict)
+static int ozh_launch(gpu_Context* ctx, ozh_params& prm, double* G, int ldg, int* verdict)
 {
   const int WPAD = 128 / F;
   const long R = (F == 2 ? 4 : 8) * OZH_STAGE;
@@ -654,7 +667,6 @@ static int ozh_launch(gpu_Context* ctx, ozh_params& prm, long* splits, int* verd
   long gx = ctx->num_sms / (prm.tx * ty);
   if (gx < 1) gx = 1;
   if (gx > ngroups) gx = ngroups;
-  *splits = gx;
   // CTAs of the check: four an SM, as many chunks as there are at most
   const int cx = (prm.h + 31) / 32, cy = (prm.w + 31) / 32;
   const long blocks = (prm.n + OZH_SAMPLE - 1) / OZH_SAMPLE;
@@ -680,17 +692,17 @@ static int ozh_launch(gpu_Context* ctx, ozh_params& prm, long* splits, int* verd
   cudaStream_t st = (cudaStream_t)ctx->stream;
   gb_pdl(gram64_cover_kernel, dim3(cx, cy, (unsigned)cz), 256, 0, st, X, prm.h, Y, prm.w, prm.sym, prm.n, prm.norms,
          (int)gx, ngroups, tot, cover, verdict);
-  gb_pdl(gram64_verdict_kernel, (prm.h * prm.w + 7) / 8, 256, 0, st, tot, cover, (int)cz, prm.h, prm.w, prm.err, verdict);
+  gb_pdl(gram64_finish_kernel, (prm.h * prm.w + 7) / 8, 256, 0, st, partial, (int)gx, tot, cover, (int)cz, prm.h, prm.w,
+         prm.sym, prm.err, G, ldg, verdict);
   gb_count_launch(3);
   return gb_cuda_check(ctx, (int)cudaGetLastError(), "oz_gram64");
 }
 
-// The CTAs' sums of X' Y in the context's workspace, [split][w][h]; *splits of
-// them.  sym: X and Y are the same columns.  verdict[0] (device): 1 when an entry may
-// be further off than FP64 multiply-adds; [1]: the device error word (a wait that
-// gave up; the CTA's sums are NaN).
+// G = X' Y (ldg, device).  sym: X and Y are the same columns.  verdict[0] (device): 1
+// when an entry may be further off than FP64 multiply-adds; [1]: the device error
+// word (a wait that gave up; the CTA's sums are NaN).
 extern "C" int gb_oz_gram64(gpu_Context* ctx, long n, const blk_cols* X, int h, const blk_cols* Y, int w, int sym,
-                            const double** partial, long* splits, int* verdict)
+                            double* G, int ldg, int* verdict)
 {
   ozh_params prm;
   memset(&prm, 0, sizeof(prm));
@@ -702,13 +714,7 @@ extern "C" int gb_oz_gram64(gpu_Context* ctx, long n, const blk_cols* X, int h, 
   prm.n = n;
   prm.polls = ctx->opt.wait_polls > 0 ? (long)ctx->opt.wait_polls : TC_WAIT_LIMIT;
   prm.err = ctx->dcount + 5;
-  int rc;
-  if (w > 32)
-    rc = ozh_launch<2>(ctx, prm, splits, verdict);
-  else if (w > 16)
-    rc = ozh_launch<4>(ctx, prm, splits, verdict);
-  else
-    rc = ozh_launch<8>(ctx, prm, splits, verdict);
-  *partial = prm.partial;
-  return rc;
+  if (w > 32) return ozh_launch<2>(ctx, prm, G, ldg, verdict);
+  if (w > 16) return ozh_launch<4>(ctx, prm, G, ldg, verdict);
+  return ozh_launch<8>(ctx, prm, G, ldg, verdict);
 }
