@@ -5,8 +5,8 @@
 // On this GPU the FP64 pipe runs at 1/64 of the FP32 rate, so an FP32 dot
 // product that accumulates in FP64 is bound by its DFMAs, not by HBM.  Here
 // each product a b is made exact as p + e (e = fma(a, b, -p)) and added to a
-// compensated FP32 sum (Knuth's two-sum); every 64 terms the pair (s, c) is
-// flushed into an FP64 accumulator.  The intrinsics keep the compiler from
+// compensated FP32 sum (Knuth's two-sum); after at most 64 terms the pair (s, c)
+// goes into an FP64 accumulator or, first, is merged with other threads' pairs.  The intrinsics keep the compiler from
 // contracting the two-sum into FMAs, which would break its error term.
 #pragma once
 #include <cuda_runtime.h>

@@ -405,8 +405,8 @@ __global__ void __launch_bounds__(256) st7_ring_kernel(int nx, int ny, int nz,
 //     that share halo planes run within a few columns of each other; whole planes
 //     first let the z halo fall out of L2 (256^3, 64 columns: 1729 us, strips of
 //     8, 16, 32 tiles: 1474, 1459, 1513; 512 x 256 x 128: 1972, 1471, 1471, 1497).
-//   256^3, 64 columns: 1455 us, 5.9 TB/s of blocks and coefficients (6.1 with the
-//     halos read twice), before 1797; 128^3, 17 columns: 64 us against 71;
+//   256^3, 64 columns: 1455 us, 5.9 TB/s of blocks (6.04 with the coefficients),
+//     before 1797; 128^3, 17 columns: 64 us against 71;
 //     32^3, 64 columns: 9 us against 39.
 #define ST7T_DEPTH 3
 template <int NP>  // planes a CTA
@@ -725,7 +725,7 @@ __global__ void __launch_bounds__(256) st27_kernel(int nx, int ny, int nz, const
 // weights in registers over the columns.  Same terms in the same order as
 // st27_kernel, which gathers 27 values a cell through L1 by 64-bit addresses.
 //
-// Bound by shared-memory reads (18 a cell: 74% of the pipe).  The four layers are
+// Bound by shared-memory reads (18 a cell: 71% of the pipe, 69% of the issue slots).  The four layers are
 // read once for both cells; three cells (15 a cell) spill, and four columns a step
 // share a wait and a barrier and interleave their dependent sums (100^3, 128
 // columns: 640 us with one column a step and 3 x 256 threads at 80 registers, 456
@@ -1771,7 +1771,7 @@ __global__ void pcg_ratio_kernel(int k, const double* num, const double* den, do
 //   512^2 5-point, 8 columns, FP64, 20 steps: 1700 us against 2390, 1530 with the
 //   launches overlapped (FP64 pipe: 14 instructions an entry and step, 1010 us; the
 //   ordered sums 11 us a step);
-//   128^3 7-point, 17 columns, FP32, 20 steps: 5980 us against 7120, 5140 with the
+//   128^3 7-point, 17 columns, FP32, 20 steps: 5980 us against 7120, 5170 with the
 //   two-plane stencil and the launches overlapped (HBM 4000).
 // FP32 (16-byte aligned columns): float4 access, inner products as gb_dot_cols'
 // FP32 path (exact products, compensated FP32 sums flushed to FP64).  FP64: the

@@ -37,7 +37,7 @@
 //                   column of [L Q_b]; warps w and w + 4 share TMEM lanes and
 //                   take 32 of the 64 L columns each).
 // Bound by the instructions that cut the digits (integer and FP32 pipes; 20 warps
-// of 96 registers cover each other's latencies to half the issue rate).  Measured,
+// of 96 registers cover each other's latencies to 58% of the issue slots).  Measured,
 // 2 M rows, 64 FP64 + 33 + 33 FP32 columns (HBM 240 us): 2240 us with 64-bit
 // shifts and one value at a time, six warps for scales and digits, a barrier
 // between them, and one MMA a digit pair (40 of N = 64, bound by the shared-memory

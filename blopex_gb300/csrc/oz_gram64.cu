@@ -22,14 +22,15 @@
 // 19 (f = 2), 11 (f = 4) or 7 (f = 8) MMA columns per X column instead of 34.
 // Row block q's sums carry the weight 2^(-8 q); they are added up at the end.
 //
-// What bounds it: the producers' latency, then the integer pipe (half rate), ~17
-// instructions per value cut and ~30 per entry and group recombined, and with h
-// > 32 the epilogue, whose 512 TMEM columns leave no second set.  So the values
-// are read straight into registers by coalesced loads (four lanes a column, any
-// alignment), not staged; a group's scales are found one group ahead from the
-// same columns (the second read of a value comes from L2).  Measured, 2,097,152
-// rows: 32 x 32 0.63 ms (FP64 FMAs 3.9; HBM 0.16), 64 x 64 1.61 (14.5), X'X of 64
-// 1.25 (7.9).  Relative error 2.1e-16 on random blocks (FMAs 6 to 9e-16).
+// What bounds it: the producers' instructions and latency, ~17 instructions per value
+// cut and ~30 per entry and group recombined (32 x 32: 50% of the issue slots, 54% of
+// the ALU pipe), and with h > 32 the epilogue, whose 512 TMEM columns leave no second
+// set.  So the values are read straight into registers by coalesced loads (four
+// lanes a column, any alignment), not staged; a group's scales are found one group
+// ahead from the same columns (the second read of a value comes from L2).  Measured,
+// 2,097,152 rows, all three kernels: 32 x 32 0.70 ms (FP64 FMAs 3.9 to 5.5; HBM 0.16),
+// 64 x 64 1.75 (14.6), X'X of 64 1.42 (7.9).  Error against 64 bits on random blocks 3.0
+// to 8.3e-16 of the norm (FMAs 3.8e-16 to 1.2e-15).
 //
 // Accuracy.  Within a group of R rows, scales S and S', the digits are off by up to
 // 2^-55 S S' (|x/S| + |y/S'| + 4) (1-norms: every value cut below 2^-55 of its

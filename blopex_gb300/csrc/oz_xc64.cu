@@ -32,13 +32,13 @@
 // are rows or columns whose scale the digits cannot carry (infinities, NaN,
 // values below 2^-960), and products whose scale is below 2^-924.
 //
-// What bounds it: instruction issue, the half-rate integer pipe above all (~17
-// integer instructions per X value in the producers, ~30 per Y value in the
-// epilogue); FP64 FMAs instead would need h w / 2 cycles per row and SM (2 per
-// cycle), 2,048 at h = w = 64.  With D the narrower units cost more MMAs, each of
-// which reads its 4 KB of A.  Measured, 2,097,152 rows, with D (without; FMAs):
-// 16 x 16 0.31 ms (-; 0.91), 32 x 32 0.55 (0.46; 3.5), 64 x 64 1.33 (0.88; 13.8);
-// 32 x 32 with X's columns graded over 18 decades 3.9 ms.  Hence no
+// What bounds it: instructions, ~17 integer ones per X value in the producers and
+// ~30 per Y value in the epilogue (32 x 32: 63% of the issue slots, 52% of the ALU
+// pipe, 17 warps to cover their latencies); FP64 FMAs instead would need h w / 2
+// cycles per row and SM (2 per cycle), 2,048 at h = w = 64.  With D the narrower
+// units cost more MMAs, each of which reads its 4 KB of A.  Measured, 2,097,152 rows,
+// with D (without; FMAs): 16 x 16 0.29 ms (-; 0.88), 32 x 32 0.51 (0.46; 3.45), 64 x 64
+// 1.30 (0.88; 13.8); 32 x 32 with X's columns graded over 18 decades 3.9 ms.  Hence no
 // shared-memory staging of X: its columns are read by coalesced 8-byte loads
 // straight into registers (any alignment and spacing of the columns), all 32 of
 // a thread in flight at once, while the MMAs of the previous tile run.

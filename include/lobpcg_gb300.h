@@ -228,9 +228,13 @@ int gpu_ExplicitGram(gpu_MultiVector* X, gpu_MultiVector* R, gpu_MultiVector* P,
    (blopex_serial_double/multivector/multi_vector.c:474-524) with the fused
    accumulate of the solver's X update.  mode 0: CUDA-core kernel (FP64 or FP32
    blocks); mode 1: tensor cores, compensated 3xTF32 (FP32 blocks, h <= 128,
-   w <= 64, 16-byte aligned columns); mode 2: tensor cores, products with the
-   accuracy of FP64 arithmetic by error-free splitting into seven 8-bit digits
-   (FP64 X and Y, h <= 64, w <= 64; Z FP32 or FP64).  Z may be NULL. */
+   w <= 64, 16-byte aligned columns); mode 2: tensor cores, error-free splitting into
+   seven 8-bit digits (FP64 X and Y, h <= 64, w <= 64; Z FP32 or FP64): an entry is
+   off by at most (h + 1) 2^-53 max |row of X| max |column of C| and the roundings of
+   the sum, so block columns of very different size want mode 0 or
+   mv_MultiVectorByMatrix, which keep the bound of multiply-adds in every entry.  Y
+   may overlap X (up to 32 columns in mode 0); mode 2 then takes six 7-bit digits.
+   Z may be NULL. */
 int gpu_BlockUpdate(gpu_MultiVector* X, const double* C_host, int ldc, gpu_MultiVector* Y,
                     gpu_MultiVector* Z, int mode);
 
