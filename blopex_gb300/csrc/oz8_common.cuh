@@ -14,9 +14,9 @@
 // product of their groups' scales, one rounding of FP64.
 //
 // The integer (ALU) pipe issues at half the rate of the FMA pipe and is the
-// busiest of these kernels (52 to 54%): hence the truncation, the sign applied by the packed FMA that
-// also takes the bias out of the digits, and the constant byte in the fixed
-// point word that one byte permutation turns into fp16 numbers.
+// busiest of these kernels (52 to 54%): hence the truncation, the sign applied by
+// the packed FMA that also takes the bias out of the digits, and the constant byte in
+// the fixed point word that one byte permutation turns into fp16 numbers.
 #define OZ8_S 7
 #define OZ8_F 55
 
