@@ -767,7 +767,7 @@ template <int NZ>
 __global__ void __launch_bounds__(32 * ST27T_ROWS, ST27T_MINB)
     st27_tma_kernel(int nx, int ny, int nz, const float* __restrict__ wt, float shift,
                     const __grid_constant__ CUtensorMap tm, const __grid_constant__ st7t_cols XC,
-                    const __grid_constant__ blk_cols Y, int wall, int cpg, int strip, int* err)
+                    const __grid_constant__ blk_cols Y, int wall, int cpg, int strip, long polls, int* err)
 {
   gb_pdl_entry();
   using C = st27t_cfg<NZ>;
@@ -823,7 +823,7 @@ __global__ void __launch_bounds__(32 * ST27T_ROWS, ST27T_MINB)
 #pragma unroll 1
   for (int st = 0; st < steps; st++) {
     const uint32_t parity = (uint32_t)((st / ST27T_DEPTH) & 1);
-    const bool ok = !abort_flag && mbar_wait(&bar[slot], parity, &abort_flag);
+    const bool ok = !abort_flag && mbar_wait_n(&bar[slot], parity, &abort_flag, polls);
     if (!ok) abort_flag = 1;
     else if (t == 0) waited = st + 1;
     __syncthreads();  // step st landed; every thread is done with the slot of st - 1
@@ -1194,7 +1194,8 @@ static void st27t_launch(gpu_Operator* op, const CUtensorMap& tm, const st7t_col
   const int cpg = (int)((w + groups - 1) / groups);
   const dim3 grid((unsigned)ctas, (unsigned)((w + cpg - 1) / cpg));
   gb_pdl(st27_tma_kernel<ST27T_NZ>, grid, 32 * ST27T_ROWS, st27t_cfg<ST27T_NZ>::SMEM, S(ctx),
-         op->nx, op->ny, op->nz, op->w32, (float)op->shift, tm, pc, yc, w, cpg, strip, ctx->dcount + 5);
+         op->nx, op->ny, op->nz, op->w32, (float)op->shift, tm, pc, yc, w, cpg, strip,
+         ctx->opt.wait_polls > 0 ? (long)ctx->opt.wait_polls : TC_WAIT_LIMIT, ctx->dcount + 5);
 }
 
 static int pcg_apply(gpu_Operator* op, gpu_MultiVector* X, gpu_MultiVector* Y);
@@ -1399,8 +1400,6 @@ static int operator_apply(gpu_Operator* op, gpu_MultiVector* X, gpu_MultiVector*
       if (f32 && st27t_pays(op, w) && st27t_map(op, X, ST27T_NZ + 2, &tmc) == 0) {
         st7t_cols pc;
         for (int c = 0; c < w; c++) pc.c[c] = X->active[c];
-        if (tc_apply_wait_polls(ctx->opt.wait_polls, S(ctx)) != cudaSuccess)
-          return gb_fail(ctx, "stencil27: cannot set the wait limit");
         st27t_launch(op, tmc, pc, yc, w);
       } else if (f32)
         gb_pdl(st27_kernel<float>, blocks, 256, 0, S(ctx), op->nx, op->ny, op->nz, op->w32,

@@ -71,3 +71,26 @@ def test_solves_of_several_threads():
         assert flag == 0 and err == "", (k, flag, err)
     first = {k: min(lam[0] for kk, _, _, lam in out if kk == k) for k in (3, 12, 25, 40)}
     assert np.ptp(list(first.values())) <= 1e-6 * max(first.values())
+
+
+def test_wait_limit_of_another_threads_context():
+    """A context's wait_polls (a poll a wait, so that its kernels give up) is its own:
+    the 27-point stencil of another thread's context runs with the default limit."""
+    nx = ny = nz = 40
+    w = P.stencil27_weights(nx, ny, nz, 1)
+    codes, bad = [], []
+
+    def apply(polls, times, out):
+        ctx = S.Context(0)
+        A = S.Stencil27(ctx, nx, ny, nz, w, 0.5)
+        X = S.MultiVector.from_host(ctx, np.random.default_rng(1).standard_normal((nx * ny * nz, 16)), S.FLOAT32)
+        Y = S.MultiVector(ctx, nx * ny * nz, 16, S.FLOAT32)
+        ctx.set_options(wait_polls=polls)
+        for _ in range(times):
+            A.apply(X, Y)
+            out.append(ctx.device_error())
+        ctx.set_options(wait_polls=0)
+        ctx.close()
+
+    _run([(apply, (1, 1500, codes)), (apply, (0, 1500, bad))])
+    assert any(codes) and not any(bad), (sum(map(bool, codes)), sum(map(bool, bad)))
